@@ -100,6 +100,7 @@ struct bmxg_ctx {
     int traj_T = -1, traj_k = 0;
     double traj_dt = 0.0;
 
+    bool rod_walk = false;    // no room for the rod pair lists: FP64 rod steps walk the stencil
     bool vel32 = false;       // the last step's velocities are in the FP32F buffers
     bool vel64_zero = false;  // the FP64 velocity planes (vx .. wz) hold zeros: a load zeroed them
                               // and no kernel that writes them ran since
@@ -222,6 +223,7 @@ void free_state(bmxg_ctx *ctx)
     for (void *p : ctx->allocs) cudaFree(p);
     ctx->allocs.clear();
     ctx->S = DevState{};
+    ctx->rod_walk = false;
     ctx->d_geoms = nullptr;
     ctx->d_cbase = nullptr;
     ctx->scan_scratch = nullptr;
@@ -1144,15 +1146,15 @@ int enqueue_step(bmxg_ctx *ctx, double dt, int precision, int a, int resync)
         if (k1) cudaEventRecord(k1, st);
     } else {
         const int rg = grid_for(ctx, ctx->sh_rod, n);
-        // FP32F: the flat pipeline over the pairs the bookkeeping records
-        const bool pipe = precision == BMXG_FP32F && S.rnb;
+        // the flat pipeline over the pairs the bookkeeping records
+        const bool pipe = S.rnb != nullptr;
         if (pipe) cudaMemsetAsync(S.rctl, 0, sizeof(RodCtl), st);
-        LAUNCH(launch_rod_book(S, P, a, pipe, rg, ctx->sh_rod.block, st));
+        LAUNCH(launch_rod_book(S, P, a, precision, pipe, rg, ctx->sh_rod.block, st));
         if (k0) cudaEventRecord(k0, st);
         if (pipe)
-            LAUNCH(launch_rod_pairs(S, P, a, ctx->nsm, (int)n, st));
+            LAUNCH(launch_rod_pairs(S, P, a, precision, ctx->nsm, (int)n, st));
         else
-            LAUNCH(launch_rod_force(S, P, a, precision, rg, ctx->sh_rod.block, st));
+            LAUNCH(launch_rod_force(S, P, a, rg, ctx->sh_rod.block, st));
         if (k1) cudaEventRecord(k1, st);
         LAUNCH(launch_rod_update(S, dt, a, mgrd, mblk, st));
     }
@@ -1221,18 +1223,31 @@ int step_setup(bmxg_ctx *ctx, int32_t nsteps, int32_t precision)
         if (rc) return rc;
         drop_graphs(ctx);
     }
-    if (ctx->S.has_rods && precision == BMXG_FP32F && !ctx->S.rnb) {  // the FP32F rod pipeline's buffers
+    // the rod pipelines' buffers (the queue's length is an int)
+    if (ctx->S.has_rods && !ctx->S.rnb &&
+        !(precision == BMXG_FP64 && (ctx->rod_walk || ctx->n > (1LL << 26)))) {
         const size_t n = (size_t)ctx->n;
         int2 *nb = nullptr, *work = nullptr;
         int *cnt = nullptr;
         double *res = nullptr;
         RodCtl *ctl = nullptr;
+        const size_t held = ctx->allocs.size();
         int rc = dalloc(ctx, &nb, n * kRodCap);
         if (!rc) rc = dalloc(ctx, &cnt, n);
         if (!rc) rc = dalloc(ctx, &res, n * kRodCap * 6);
         if (!rc) rc = dalloc(ctx, &work, n * kRodCap);
         if (!rc) rc = dalloc(ctx, &ctl, 1);
-        if (rc) return rc;
+        if (rc) {
+            // no room for the lists (2 KB per segment): the FP64 form walks
+            while (ctx->allocs.size() > held) {
+                cudaFree(ctx->allocs.back());
+                ctx->allocs.pop_back();
+            }
+            (void)cudaGetLastError();
+            if (precision != BMXG_FP64 || rc != BMXG_ERR_OOM) return rc;
+            ctx->rod_walk = true;
+            return BMXG_OK;
+        }
         ctx->S.rnb = nb;
         ctx->S.rcnt = cnt;
         ctx->S.rres = res;

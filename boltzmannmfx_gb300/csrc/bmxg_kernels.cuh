@@ -51,7 +51,7 @@ constexpr int kListBins = 0;         // list mode keeps its frozen bins in buffe
 constexpr int kListStepBlock = 128;  // k_list_step's default block (at most 256; autotuned)
 constexpr int kListBuildBlock = 128; // k_list_build's default block (one slot per thread; at most 256)
 constexpr int kSphereBlock = 64;     // per-step sphere kernels' block (one slot per thread)
-constexpr int kRodCap = 32;          // gated pairs per segment the FP32F rod pipeline holds (more: the
+constexpr int kRodCap = 32;          // gated pairs per segment the rod pipelines hold (more: the
                                      // segment walks its stencil in the segment kernel)
 
 // Per-step counters of the FP32F rod pipeline (k_rod.cu).
@@ -253,11 +253,11 @@ int launch_tile_step(const TileBufs &B, const TileGeom &T, const DevParams &P, d
 // ---- rods and mixed states (k_rod.cu) ------------------------------------
 int launch_rod_mobility(const DevState &S, const DevParams &P, int grid, int block, cudaStream_t st);
 // list: also record each segment's gated pairs (the FP32F pipeline)
-int launch_rod_book(const DevState &S, const DevParams &P, int a, bool list, int grid, int block, cudaStream_t st);
+int launch_rod_book(const DevState &S, const DevParams &P, int a, int precision, bool list, int grid, int block,
+                    cudaStream_t st);
 // the FP32F pipeline after the bookkeeping: FP32 pairs, FP64 pairs, per-segment sums
-int launch_rod_pairs(const DevState &S, const DevParams &P, int a, int nsm, int n, cudaStream_t st);
-int launch_rod_force(const DevState &S, const DevParams &P, int a, int precision, int grid, int block,
-                      cudaStream_t st);
+int launch_rod_pairs(const DevState &S, const DevParams &P, int a, int precision, int nsm, int n, cudaStream_t st);
+int launch_rod_force(const DevState &S, const DevParams &P, int a, int grid, int block, cudaStream_t st);
 int launch_rod_update(const DevState &S, double dt, int a, int grid, int block, cudaStream_t st);
 // one ParticleExchange substep: conc / out 3 planes (A, B, C), slot order; xpar host
 int launch_exchange(const DevState &S, const DevParams &P, int a, const double *vol, const double *conc, double *out,

@@ -241,15 +241,23 @@ __device__ __forceinline__ bool rod_gate(const DevState &S, const DevGeom &G, co
 }
 
 // ---- bookkeeping ----------------------------------------------------------
-// LIST: also record the segment's gated pairs, in the order of its walk, for
-// the FP32F pipeline (rnb, rcnt; the step's largest count into rctl->kmax).
-template <bool LIST>
+// kRodList: also record the segment's gated pairs, in the order of its walk,
+// for the flat pipelines (rnb, rcnt; the step's largest count into
+// rctl->kmax).  kRodQueue (the FP64 pipeline): and queue every recorded pair
+// for k_rod_pair64, a warp's pairs together, one atomic per warp.
+enum { kRodPlain = 0, kRodList = 1, kRodQueue = 2 };
+
+template <int MODE>
 __global__ void k_rod_book(const DevState S, const DevParams P, int a)
 {
+    constexpr bool LIST = MODE != kRodPlain;
     const int b = a ^ 1;
     const int n = S.n;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    // (same trip count for every lane of a warp)
+    for (int base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
+        const int i = base + threadIdx.x;
         int cnt = 0;
+        if (i < n) {
         S.fflag[i] = 0;  // flag resets of bmx_pc_interaction.cpp:178-180
         S.sflag[i] = 0;
         S.nflag[i] = 0;
@@ -327,9 +335,24 @@ __global__ void k_rod_book(const DevState S, const DevParams P, int a)
                 e.y |= ((site == 1 || site == 2) ? site : 0) << 9;
             }
             S.rcnt[i] = cnt;
-            const unsigned m = __activemask();
-            const int w = __reduce_max_sync(m, min(cnt, kRodCap));
-            if ((threadIdx.x & 31) == __ffs(m) - 1 && w > 0) atomicMax(&S.rctl->kmax, w);
+        }
+        }
+        if (MODE == kRodList) {
+            const int w = __reduce_max_sync(0xffffffffu, min(cnt, kRodCap));
+            if ((threadIdx.x & 31) == 0 && w > 0) atomicMax(&S.rctl->kmax, w);
+        }
+        if (MODE == kRodQueue) {
+            const int lane = threadIdx.x & 31;
+            const int x = (cnt <= kRodCap) ? cnt : 0;  // (a longer list is walked)
+            int o = x;
+            for (int q = 1; q < 32; q <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, o, q);
+                if (lane >= q) o += v;
+            }
+            int at = 0;
+            if (lane == 31 && o > 0) at = atomicAdd(&S.rctl->nwork, o);
+            at = __shfl_sync(0xffffffffu, at, 31) + o - x;
+            for (int k = 0; k < x; ++k) S.rwork[at + k] = make_int2(i, k);
         }
     }
 }
@@ -406,6 +429,59 @@ __device__ __forceinline__ void rod_velocity32(const float *ni, float L, const f
     acc[3] += 0.5f * ((ax[1] * w1[2] - ax[2] * w1[1]) - (ax[1] * w2[2] - ax[2] * w2[1]));
     acc[4] += 0.5f * ((ax[2] * w1[0] - ax[0] * w1[2]) - (ax[2] * w2[0] - ax[0] * w2[2]));
     acc[5] += 0.5f * ((ax[0] * w1[1] - ax[1] * w1[0]) - (ax[0] * w2[1] - ax[1] * w2[0]));
+}
+
+// The same in FP64 (the plain form), from the two site positions as the
+// reference computes them.
+__device__ __forceinline__ void rod_velocity64(const double *ni, double Li, const double *Sv, const double *Dv,
+                                               const double4_32a &mb, double xi, double yi, double zi, double ri,
+                                               const DevParams &P, double *acc)
+{
+    const double ns = ni[0] * Sv[0] + ni[1] * Sv[1] + ni[2] * Sv[2];
+    double rv[3];
+    for (int k = 0; k < 3; ++k) {
+        acc[k] = 0.5 * (mb.x * Sv[k] + mb.y * ns * ni[k]);
+        rv[k] = (-0.5 * ni[k] * Li) - (0.5 * ni[k] * Li);  // site 1 minus site 2
+    }
+    const double c = mb.z;
+    acc[3] = c * (rv[1] * Dv[2] - rv[2] * Dv[1]);
+    acc[4] = c * (rv[2] * Dv[0] - rv[0] * Dv[2]);
+    acc[5] = c * (rv[0] * Dv[1] - rv[1] * Dv[0]);
+    // growth-surface force on both sites (bmx_cell_interaction_K.H:1067-1281;
+    // its mobility block :1176-1265 is overwritten there and has no effect)
+    double u1[3], u2[3], ax[3];
+    const double pc[3] = {xi, yi, zi};
+    for (int k = 0; k < 3; ++k) {
+        u1[k] = pc[k] - 0.5 * ni[k] * Li;
+        u2[k] = pc[k] + 0.5 * ni[k] * Li;
+        ax[k] = u1[k] - u2[k];
+    }
+    double w1[3] = {0.0, 0.0, wall_law(u1[2], ri, P)};
+    double w2[3] = {0.0, 0.0, wall_law(u2[2], ri, P)};
+    const double ra = sqrt(ax[0] * ax[0] + ax[1] * ax[1] + ax[2] * ax[2]);
+    const double un[3] = {ax[0] / ra, ax[1] / ra, ax[2] / ra};
+    const double fn = (w1[0] - w2[0]) * un[0] + (w1[1] - w2[1]) * un[1] + (w1[2] - w2[2]) * un[2];
+    double vw[3];
+    for (int k = 0; k < 3; ++k) {
+        w1[k] -= 0.5 * fn * un[k];
+        w2[k] += 0.5 * fn * un[k];
+    }
+    for (int k = 0; k < 3; ++k) vw[k] = 0.5 * (w1[k] + w2[k]);
+    for (int k = 0; k < 3; ++k) {
+        w1[k] -= 0.5 * vw[k];
+        w2[k] -= 0.5 * vw[k];
+    }
+    double rw[3];
+    rw[0] = 0.5 * (ax[1] * w1[2] - ax[2] * w1[1]);
+    rw[1] = 0.5 * (ax[2] * w1[0] - ax[0] * w1[2]);
+    rw[2] = 0.5 * (ax[0] * w1[1] - ax[1] * w1[0]);
+    rw[0] += -0.5 * (ax[1] * w2[2] - ax[2] * w2[1]);
+    rw[1] += -0.5 * (ax[2] * w2[0] - ax[0] * w2[2]);
+    rw[2] += -0.5 * (ax[0] * w2[1] - ax[1] * w2[0]);
+    for (int k = 0; k < 3; ++k) {
+        acc[k] += vw[k];
+        acc[3 + k] += rw[k];
+    }
 }
 
 // ---- force gather ----------------------------------------------------------
@@ -532,68 +608,31 @@ __device__ __forceinline__ void rod_force_slot(const DevState &S, const DevParam
                 for (int c = 0; c < 6; ++c) S.fc[(size_t)c * n + i] = acc[c];
                 return;
             }
-            const double ns = ni[0] * Sv[0] + ni[1] * Sv[1] + ni[2] * Sv[2];
-            double rv[3];
-            for (int k = 0; k < 3; ++k) {
-                acc[k] = 0.5 * (mb.x * Sv[k] + mb.y * ns * ni[k]);
-                rv[k] = (-0.5 * ni[k] * Li) - (0.5 * ni[k] * Li);  // site 1 minus site 2
-            }
-            const double c = mb.z;
-            acc[3] = c * (rv[1] * Dv[2] - rv[2] * Dv[1]);
-            acc[4] = c * (rv[2] * Dv[0] - rv[0] * Dv[2]);
-            acc[5] = c * (rv[0] * Dv[1] - rv[1] * Dv[0]);
-            // growth-surface force on both sites (bmx_cell_interaction_K.H:1067-1281;
-            // its mobility block :1176-1265 is overwritten there and has no effect)
-            double u1[3], u2[3], ax[3];
-            const double pc[3] = {xi, yi, zi};
-            for (int k = 0; k < 3; ++k) {
-                u1[k] = pc[k] - 0.5 * ni[k] * Li;
-                u2[k] = pc[k] + 0.5 * ni[k] * Li;
-                ax[k] = u1[k] - u2[k];
-            }
-            double w1[3] = {0.0, 0.0, wall_law(u1[2], ri, P)};
-            double w2[3] = {0.0, 0.0, wall_law(u2[2], ri, P)};
-            const double ra = sqrt(ax[0] * ax[0] + ax[1] * ax[1] + ax[2] * ax[2]);
-            const double un[3] = {ax[0] / ra, ax[1] / ra, ax[2] / ra};
-            const double fn = (w1[0] - w2[0]) * un[0] + (w1[1] - w2[1]) * un[1] + (w1[2] - w2[2]) * un[2];
-            double vw[3];
-            for (int k = 0; k < 3; ++k) {
-                w1[k] -= 0.5 * fn * un[k];
-                w2[k] += 0.5 * fn * un[k];
-            }
-            for (int k = 0; k < 3; ++k) vw[k] = 0.5 * (w1[k] + w2[k]);
-            for (int k = 0; k < 3; ++k) {
-                w1[k] -= 0.5 * vw[k];
-                w2[k] -= 0.5 * vw[k];
-            }
-            double rw[3];
-            rw[0] = 0.5 * (ax[1] * w1[2] - ax[2] * w1[1]);
-            rw[1] = 0.5 * (ax[2] * w1[0] - ax[0] * w1[2]);
-            rw[2] = 0.5 * (ax[0] * w1[1] - ax[1] * w1[0]);
-            rw[0] += -0.5 * (ax[1] * w2[2] - ax[2] * w2[1]);
-            rw[1] += -0.5 * (ax[2] * w2[0] - ax[0] * w2[2]);
-            rw[2] += -0.5 * (ax[0] * w2[1] - ax[1] * w2[0]);
-            for (int k = 0; k < 3; ++k) {
-                acc[k] += vw[k];
-                acc[3 + k] += rw[k];
-            }
+            rod_velocity64(ni, Li, Sv, Dv, mb, xi, yi, zi, ri, P, acc);
             S.fix_site[i] = 0;  // evaluateSurfaceForce (:1060)
         }
         for (int c = 0; c < 6; ++c) S.fc[(size_t)c * n + i] = acc[c];
     }
 }
 
-template <int PREC>
+// The plain FP64 form without pair lists (no room for them).
 __global__ void __launch_bounds__(128) k_rod_force(const DevState S, const DevParams P, int a)
 {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < S.n; i += gridDim.x * blockDim.x)
-        rod_force_slot<PREC>(S, P, a, i);
+        rod_force_slot<BMXG_FP64_FORM>(S, P, a, i);
 }
 
-// ---- FP32F pipeline ---------------------------------------------------------
-// With every segment's gated pairs recorded by k_rod_book, the FP32F force
-// gather runs flat instead of one stencil walk per thread (whose lanes
-// diverge over pair counts and over the FP32 and FP64 paths):
+// ---- flat pipelines -----------------------------------------------------------
+// With every segment's gated pairs recorded by k_rod_book, the force gather
+// runs flat instead of one stencil walk per thread (whose lanes diverge over
+// pair counts and, in the FP32F form, over the FP32 and FP64 paths).
+// Plain FP64 form: k_rod_book queues every pair, k_rod_pair64<true> evaluates
+// one per thread in full warps, k_rod_seg64 adds a segment's pairs in list
+// order (the walk's FP64 values in the walk's order: bit-identical to it).
+// GB300 issues FP64 at 2 lanes per clock per SM whatever the mask, and the walk
+// kept 6 of 32 lanes busy: 50 000 segments in 500 trees, 10 steps and the
+// load 8.29 -> 3.35 ms.
+// FP32F form:
 //   k_rod_pair32  one pair per thread (pair k of segment i); evaluates it in
 //                 FP32 where the FP32F form allows, else queues it;
 //   k_rod_pair64  the queued pairs, one per thread, in FP64 (full warps on
@@ -690,15 +729,32 @@ __global__ void __launch_bounds__(256) k_rod_pair32(const DevState S, const DevP
     }
 }
 
+// ALL: the queue holds every recorded pair (k_rod_book<kRodQueue>, the plain
+// FP64 form) and the pair's bonded sites are looked up here; else they come
+// with the queue entry (k_rod_pair32).
+template <bool ALL>
 __global__ void __launch_bounds__(128) k_rod_pair64(const DevState S, const DevParams P, int a)
 {
+    const int b = a ^ 1;
     const int n = S.n;
     const int nw = S.rctl->nwork;
     for (int w = blockIdx.x * blockDim.x + threadIdx.x; w < nw; w += gridDim.x * blockDim.x) {
         const int2 it = S.rwork[w];
-        const int i = it.x, k = it.y & 255, si = (it.y >> 8) & 15, sj = (it.y >> 12) & 15;
+        const int i = it.x, k = it.y & 255;
+        int si = (it.y >> 8) & 15, sj = (it.y >> 12) & 15;
         const int2 e = S.rnb[(size_t)k * n + i];
         const int j = e.x;
+        if (ALL) {
+            const int isite = (e.y >> 9) & 3;
+            if (isite) {
+                const int jb = find_in_plane_table(S.tab[b], n, j, S.id[i], S.cpu[i]);
+                if (jb >= 0) {
+                    const int s2 = __ldg(&S.tab[b][(size_t)(9 + jb) * n + j]);
+                    si = isite;
+                    sj = (s2 == 1 || s2 == 2) ? s2 : 0;
+                }
+            }
+        }
         int dxs, dys, dzs, sx, sy;
         decode_pair(e.y, dxs, dys, dzs, sx, sy);
         const DevGeom &G = geom_of(S, i);
@@ -750,6 +806,32 @@ __global__ void __launch_bounds__(128) k_rod_seg32(const DevState S, const DevPa
         const float nif[3] = {axi.x, axi.y, axi.z};
         rod_velocity32(nif, axi.w, sv, dv, S.mob[i], d2f_rn(S.z[a][i] - P.z_wall), S.rel[a][i].w, P, af);
         for (int c = 0; c < 6; ++c) S.fc[(size_t)c * n + i] = f2d_int(af[c]);
+        S.fix_site[i] = 0;  // evaluateSurfaceForce (bmx_cell_interaction_K.H:1060)
+    }
+}
+
+// The plain FP64 form's segments: the pairs' sums in list order, as the walk
+// adds them, then mobility and surface force in FP64.
+__global__ void __launch_bounds__(64) k_rod_seg64(const DevState S, const DevParams P, int a)
+{
+    const int n = S.n;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const int cnt = S.rcnt[i];
+        if (S.ctype[i] != kFungi || cnt > kRodCap) {
+            rod_force_slot<BMXG_FP64_FORM>(S, P, a, i);
+            continue;
+        }
+        double Sv[3] = {0.0, 0.0, 0.0}, Dv[3] = {0.0, 0.0, 0.0};
+        for (int k = 0; k < cnt; ++k)
+            for (int c = 0; c < 3; ++c) {
+                Sv[c] += S.rres[((size_t)c * kRodCap + k) * n + i];
+                Dv[c] += S.rres[((size_t)(3 + c) * kRodCap + k) * n + i];
+            }
+        const double4_32a tri = S.trig[a][i];
+        const double ni[3] = {tri.y * tri.z, tri.y * tri.w, tri.x};
+        double acc[6];
+        rod_velocity64(ni, S.clen[i], Sv, Dv, S.mob[i], S.x[a][i], S.y[a][i], S.z[a][i], S.rad[i], P, acc);
+        for (int c = 0; c < 6; ++c) S.fc[(size_t)c * n + i] = acc[c];
         S.fix_site[i] = 0;  // evaluateSurfaceForce (bmx_cell_interaction_K.H:1060)
     }
 }
@@ -973,30 +1055,31 @@ int launch_rod_mobility(const DevState &S, const DevParams &P, int grid, int blo
     return 1;
 }
 
-int launch_rod_book(const DevState &S, const DevParams &P, int a, bool list, int grid, int block, cudaStream_t st)
+int launch_rod_book(const DevState &S, const DevParams &P, int a, int precision, bool list, int grid, int block,
+                    cudaStream_t st)
 {
-    if (list)
-        k_rod_book<true><<<grid, block, 0, st>>>(S, P, a);
-    else
-        k_rod_book<false><<<grid, block, 0, st>>>(S, P, a);
+    if (!list) k_rod_book<kRodPlain><<<grid, block, 0, st>>>(S, P, a);
+    else if (precision == BMXG_FP64_FORM) k_rod_book<kRodQueue><<<grid, block, 0, st>>>(S, P, a);
+    else k_rod_book<kRodList><<<grid, block, 0, st>>>(S, P, a);
     return 1;
 }
 
-int launch_rod_pairs(const DevState &S, const DevParams &P, int a, int nsm, int n, cudaStream_t st)
+int launch_rod_pairs(const DevState &S, const DevParams &P, int a, int precision, int nsm, int n, cudaStream_t st)
 {
+    if (precision == BMXG_FP64_FORM) {
+        k_rod_pair64<true><<<nsm * 8, 64, 0, st>>>(S, P, a);
+        k_rod_seg64<<<(n + 63) / 64, 64, 0, st>>>(S, P, a);
+        return 2;
+    }
     k_rod_pair32<<<nsm * 8, 256, 0, st>>>(S, P, a);
-    k_rod_pair64<<<nsm * 4, 128, 0, st>>>(S, P, a);
+    k_rod_pair64<false><<<nsm * 4, 128, 0, st>>>(S, P, a);
     k_rod_seg32<<<(n + 127) / 128, 128, 0, st>>>(S, P, a);
     return 3;
 }
 
-int launch_rod_force(const DevState &S, const DevParams &P, int a, int precision, int grid, int block,
-                      cudaStream_t st)
+int launch_rod_force(const DevState &S, const DevParams &P, int a, int grid, int block, cudaStream_t st)
 {
-    if (precision == BMXG_FP64_FORM)
-        k_rod_force<BMXG_FP64_FORM><<<grid, block, 0, st>>>(S, P, a);
-    else
-        k_rod_force<BMXG_FP32F_FORM><<<grid, block, 0, st>>>(S, P, a);
+    k_rod_force<<<grid, block, 0, st>>>(S, P, a);
     return 1;
 }
 
