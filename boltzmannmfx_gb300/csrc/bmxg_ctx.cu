@@ -264,17 +264,7 @@ void stencil_shape(bmxg_ctx *ctx, const Shape &s, int64_t n, int *grid, int *blo
     }
 }
 
-DevParams dev_params(const bmxg_params &p)
-{
-    DevParams d{p.bndry_width, p.stiffness,     p.z_wall,      p.z_bndry_width, p.z_stiffness,
-                p.z_gravity,   p.bond_strength, p.bond_cutoff, p.viscosity,     p.neighborhood};
-    d.bw32 = (float)d.bw;
-    d.k32 = (float)d.k;
-    d.z_k32 = (float)d.z_k;
-    d.z_bw32 = (float)d.z_bw;
-    d.z_g32 = (float)d.z_g;
-    return d;
-}
+DevParams dev_params(const bmxg_params &p) { return make_dev_params(p); }
 
 int check_params(const bmxg_params *p)
 {

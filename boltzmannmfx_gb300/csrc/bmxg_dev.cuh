@@ -20,6 +20,8 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "bmxg_fp64.cuh"
+
 namespace bmxg {
 
 constexpr double kPi = 3.14159265358979323846;  // M_PI as the reference uses it
@@ -101,7 +103,23 @@ struct DevParams {
     // bw, k, z_k, z_bw, z_g rounded to FP32 on the host for the FP32F list
     // kernels (a conversion per thread is an FP64-pipe instruction)
     float bw32, k32, z_k32, z_bw32, z_g32;
+    double z_gk;  // z_g z_k, the wall law's gravity factor (one rounding, as the law multiplies them first)
 };
+
+// DevParams of the caller's parameters (P: bmxg_params).
+template <class P>
+inline DevParams make_dev_params(const P &p)
+{
+    DevParams d{p.bndry_width, p.stiffness,     p.z_wall,      p.z_bndry_width, p.z_stiffness,
+                p.z_gravity,   p.bond_strength, p.bond_cutoff, p.viscosity,     p.neighborhood};
+    d.bw32 = (float)d.bw;
+    d.k32 = (float)d.k;
+    d.z_k32 = (float)d.z_k;
+    d.z_bw32 = (float)d.z_bw;
+    d.z_g32 = (float)d.z_g;
+    d.z_gk = d.z_g * d.z_k;
+    return d;
+}
 
 // Bin index along one axis in the coordinates of the box grown by one cell:
 // (int)((x - plo)*dxi - lo) with lo = -1, as AMReX's NeighborList bins.
@@ -171,10 +189,10 @@ __device__ __forceinline__ bool finite_bits(double x)
 // loop after |x|/len + 1 iterations; a non-finite x is caught by the caller).
 __device__ __forceinline__ double wrap1(double x, double lo, double hi, double len)
 {
-    if (x > hi) {
+    if (lt_bits(hi, x)) {
         for (int it = 0; x > hi && it < 64; ++it) x = __dsub_rn(x, len);
         if (x < lo) x = lo;
-    } else if (x < lo) {
+    } else if (lt_bits(x, lo)) {
         for (int it = 0; x < lo && it < 64; ++it) x = __dadd_rn(x, len);
         if (x > hi) x = hi;
     }

@@ -215,16 +215,21 @@ __device__ __forceinline__ void rebin_slot(const DevState &S, const DevGeom &G, 
 }
 
 // Growth-surface cubic law of one site at height z
-// (bmx_cell_interaction_K.H:1019-1030, :1099-1121).
+// (bmx_cell_interaction_K.H:1019-1030, :1099-1121).  The branches above and
+// below the surface are one product c t t w with selected factors (the same
+// roundings; a warp whose lanes differ would issue both branches), and the
+// comparisons read the bits: FP64 instructions are what the callers run out of.
 __device__ __forceinline__ double wall_law(double z, double rS, const DevParams &P)
 {
     const double dz = z - P.z_wall;
     const double rA = rS + P.z_bw;
-    double v;
-    if (dz > 0.0 && dz < rA) v = -P.z_k * (dz - rA) * (dz - rA) * (dz - rS);
-    else if (dz <= 0.0) v = P.z_k * rA * rA * rS;
-    else v = 0.0;
-    v -= P.z_g * P.z_k * rA * rA * rS;
+    const bool below = le_bits(dz, 0.0);
+    const bool near = !below && lt_bits(dz, rA) && !is_nan_bits(dz);
+    const double t = near ? dz - rA : rA;
+    const double w = near ? dz - rS : rS;
+    double v = (near ? -P.z_k : P.z_k) * t * t * w;
+    if (!below && !near) v = 0.0;
+    v -= P.z_gk * rA * rA * rS;
     return v;
 }
 

@@ -43,7 +43,7 @@ __device__ __forceinline__ PairLaw pair_law(double r, double rS, double rA, doub
 
 __device__ __forceinline__ double mobility_of(double r, double mu)
 {
-    return mu > 0.0 ? 1.0 / (6.0 * kPi * mu * r) : 1.0;
+    return mu > 0.0 ? div_rn(1.0, 6.0 * kPi * mu * r) : 1.0;
 }
 
 __device__ __forceinline__ double wall_slope(double z, double rS, const DevParams &P)
@@ -179,13 +179,14 @@ __device__ __forceinline__ bool dfwd_term(const DevState &S, const DevGeom &G, c
     if (!G.nbh_trivial && !(r2 <= P.nbh)) return false;
     const double rj = S.rad[j];
     const double rlm = ri + rj + P.bw;
-    if (!(r2 <= (rlm - kSmall) * (rlm - kSmall))) return false;
+    if (!le_nonneg(r2, (rlm - kSmall) * (rlm - kSmall))) return false;
     const double rS = ri + rj, rA = rS + P.bw;
-    const double rn = sqrt(r2);
-    const double ux = dx / rn, uy = dy / rn, uz = dz / rn;
+    Divisor by;
+    const double rn = sqrt_rn(r2, &by);
+    const double ux = div_by(dx, by), uy = div_by(dy, by), uz = div_by(dz, by);
     const double abar = 0.5 * (ai + (D.adh ? D.adh[j] : 0.0));
     const PairLaw q = pair_law(rn, rS, rA, P.k, P.bw, abar);
-    const double s = 1.0 / (1.0 + D.gamma * (mi + mobility_of(rj, D.mu)));
+    const double s = div_rn(1.0, 1.0 + D.gamma * (mi + mobility_of(rj, D.mu)));
     const double F = mi * (q.f * s);
     t[0] = F * ux;
     t[1] = F * uy;
@@ -210,24 +211,25 @@ __device__ __forceinline__ bool dadj_term(const DevState &S, const DevGeom &G, c
     if (!G.nbh_trivial && !(r2 <= P.nbh)) return false;
     const double rj = S.rad[j];
     const double rlm = rk + rj + P.bw;
-    if (!(r2 <= (rlm - kSmall) * (rlm - kSmall))) return false;
+    if (!le_nonneg(r2, (rlm - kSmall) * (rlm - kSmall))) return false;
     const double rS = rk + rj, rA = rS + P.bw;
-    const double rn = sqrt(r2);
-    if (!(rn < rA)) return false;  // f, f' and all parameter slopes vanish
-    const double u[3] = {d[0] / rn, d[1] / rn, d[2] / rn};
+    Divisor by;
+    const double rn = sqrt_rn(r2, &by);
+    if (!lt_bits(rn, rA)) return false;  // f, f' and all parameter slopes vanish
+    const double u[3] = {div_by(d[0], by), div_by(d[1], by), div_by(d[2], by)};
     const double mj = mobility_of(rj, D.mu);
-    const double dmj = D.mu > 0.0 ? -mj / D.mu : 0.0;
+    const double dmj = D.mu > 0.0 ? div_rn(-mj, D.mu) : 0.0;
     const double abar = 0.5 * (ak + (D.adh ? D.adh[j] : 0.0));
     const PairLaw q = pair_law(rn, rS, rA, P.k, P.bw, abar);
     const double M = mk + mj;
-    const double s = 1.0 / (1.0 + D.gamma * M);
+    const double s = div_rn(1.0, 1.0 + D.gamma * M);
     const double Ft = q.f * s, dFt = q.df * s;
     const double lj[3] = {lin[j], lin[(size_t)n + j], lin[(size_t)2 * n + j]};
     // w = m_k lam'_k - m_j lam'_j ; J w = dFt u (u.w) + (Ft/r)(w - u (u.w))
     double w[3];
     for (int c = 0; c < 3; ++c) w[c] = mk * lk[c] - mj * lj[c];
     const double uw = u[0] * w[0] + u[1] * w[1] + u[2] * w[2];
-    const double fr = Ft / rn;
+    const double fr = div_by(Ft, by);
     for (int c = 0; c < 3; ++c) t[c] = dFt * u[c] * uw + fr * (w[c] - u[c] * uw);
     // parameter slopes of v_k (this pair's term m_k Ft u), against lam'_k
     const double lu = lk[0] * u[0] + lk[1] * u[1] + lk[2] * u[2];
@@ -313,7 +315,7 @@ __global__ void __launch_bounds__(256) k_dfwd(const DevState S, const DevParams 
             });
         if (act) {
             const DevGeom &G = S.geoms[col];
-            const double vx = fx + 0.0, vy = fy + 0.0, vz = fz + wall_law(zi, ri, P);
+            const double vx = plus_zero(fx), vy = plus_zero(fy), vz = fz + wall_law(zi, ri, P);
             double nx = xi + dt * vx, ny = yi + dt * vy;
             const double nz = zi + dt * vz;
             if (G.per[0]) nx = wrap1(nx, G.plo[0], G.phi[0], G.len[0]);
@@ -369,7 +371,7 @@ __global__ void __launch_bounds__(256) k_dadj(const DevState S, const DevParams 
             o[2] = S.z[a][k];
             o[3] = rk;
             o[4] = mk;
-            o[5] = D.mu > 0.0 ? -mk / D.mu : 0.0;
+            o[5] = D.mu > 0.0 ? div_rn(-mk, D.mu) : 0.0;
             o[6] = D.adh ? D.adh[k] : 0.0;
             o[7] = lin[k];
             o[8] = lin[(size_t)n + k];

@@ -43,7 +43,7 @@ constexpr size_t kOffOrig = align256(kOffTmp + sizeof(int) * kMaxN);
 constexpr size_t kOffStart = align256(kOffOrig + sizeof(int) * kMaxN);
 constexpr size_t kOffCount = align256(kOffStart + sizeof(int) * (kMaxCols + 1));
 constexpr size_t kOffScan = align256(kOffCount + sizeof(int) * kMaxCols);
-constexpr size_t kScratchBytes = align256(kOffScan + sizeof(int) * (kMaxCols / 4096 + 4));
+constexpr size_t kScratchBytes = align256(kOffScan + sizeof(int) * (kMaxCols / 1024 + 2));
 
 static __device__ __align__(256) unsigned char g_scratch[kScratchBytes];
 
@@ -159,9 +159,7 @@ extern "C" int bmxg_sphere_step_noalloc(const bmxg_params *params, const bmxg_ge
     const int block = 256;
     const int grid = (int)std::min<int64_t>((n + block - 1) / block, 4096);
     k_iota<<<grid, block, 0, st>>>(S.orig, (int)n);
-    const DevParams P{params->bndry_width, params->stiffness,     params->z_wall,      params->z_bndry_width,
-                      params->z_stiffness,  params->z_gravity,     params->bond_strength, params->bond_cutoff,
-                      params->viscosity,    params->neighborhood};
+    const DevParams P = make_dev_params(*params);
     launch_bin(S, 0, grid, block, st);
     launch_rebuild(S, 0, scan, grid, block, st);
     launch_sphere_step(S, P, dt / 1.0, 0, BMXG_FP64_FORM, grid, block, st);

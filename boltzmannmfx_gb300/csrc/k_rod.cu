@@ -66,22 +66,22 @@ __device__ void min_distance(const T *a1, const T *a2, const T *b1, const T *b2,
     T ti = T(0), tj = T(0);
     bool search = false;
     if (Aij == T(0)) {
-        ti = Bi / Aii;
-        tj = Bj / Ajj;
+        ti = qdiv(Bi, Aii);
+        tj = qdiv(Bj, Ajj);
     } else if (det == T(0)) {
-        const T t0 = Bj / Ajj;
+        const T t0 = qdiv(Bj, Ajj);
         if (in01(t0)) { ti = T(0); tj = t0; }
         else {
-            const T t1 = (Bj + rirj) / Ajj;
+            const T t1 = qdiv(Bj + rirj, Ajj);
             if (in01(t1)) { ti = T(1); tj = t1; }
             else search = true;
         }
     } else {
-        ti = (Ajj * Bi - Aij * Bj) / det;
-        tj = (Aii * Bj - Aij * Bi) / det;
+        ti = qdiv(Ajj * Bi - Aij * Bj, det);
+        tj = qdiv(Aii * Bj - Aij * Bi, det);
         if (in01(ti)) {
             if (tj < T(0) || tj > T(1)) {
-                const T t0 = Bi / Aii, t1 = (Bi + rirj) / Aii;
+                const T t0 = qdiv(Bi, Aii), t1 = qdiv(Bi + rirj, Aii);
                 if (in01(t0) && in01(t1)) {
                     const T s0 = sq3(a1[0] + t0 * ri[0] - b1[0], a1[1] + t0 * ri[1] - b1[1],
                                      a1[2] + t0 * ri[2] - b1[2]);
@@ -93,7 +93,7 @@ __device__ void min_distance(const T *a1, const T *a2, const T *b1, const T *b2,
                 else search = true;
             }
         } else if (in01(tj)) {
-            const T t0 = Bj / Ajj, t1 = (Bj + rirj) / Ajj;
+            const T t0 = qdiv(Bj, Ajj), t1 = qdiv(Bj + rirj, Ajj);
             if (in01(t0) && in01(t1)) {
                 const T s0 = sq3(b1[0] + t0 * rj[0] - a1[0], b1[1] + t0 * rj[1] - a1[1],
                                  b1[2] + t0 * rj[2] - a1[2]);
@@ -151,14 +151,14 @@ __device__ void rod_site_forces(const T *r12, const T *ni, T Li, const T *nj, T 
     min_distance(e1, e2, g1, g2, ti, tj);
     T dv[3];
     for (int d = 0; d < 3; ++d) dv[d] = (e1[d] + ti * (e2[d] - e1[d])) - (g1[d] + tj * (g2[d] - g1[d]));
-    const T r = sqrt(dv[0] * dv[0] + dv[1] * dv[1] + dv[2] * dv[2]);
+    const T r = qsqrt(dv[0] * dv[0] + dv[1] * dv[1] + dv[2] * dv[2]);
     if (r_out) *r_out = r;
     // r <= 1e-8: the reference keeps the unnormalised separation (its
     // fallback direction goes to shadowing locals, :744-746); so do we.
     if (r > T(1.0e-8)) {
-        dv[0] /= r;
-        dv[1] /= r;
-        dv[2] /= r;
+        dv[0] = qdiv(dv[0], r);
+        dv[1] = qdiv(dv[1], r);
+        dv[2] = qdiv(dv[2], r);
     }
     const T F = (r < rA) ? -k * (r - rA) * (r - rA) * (r - rS) : T(0);
     if (F != T(0)) {
@@ -458,8 +458,9 @@ __device__ __forceinline__ void rod_velocity64(const double *ni, double Li, cons
     }
     double w1[3] = {0.0, 0.0, wall_law(u1[2], ri, P)};
     double w2[3] = {0.0, 0.0, wall_law(u2[2], ri, P)};
-    const double ra = sqrt(ax[0] * ax[0] + ax[1] * ax[1] + ax[2] * ax[2]);
-    const double un[3] = {ax[0] / ra, ax[1] / ra, ax[2] / ra};
+    Divisor by;
+    (void)sqrt_rn(ax[0] * ax[0] + ax[1] * ax[1] + ax[2] * ax[2], &by);
+    const double un[3] = {div_by(ax[0], by), div_by(ax[1], by), div_by(ax[2], by)};
     const double fn = (w1[0] - w2[0]) * un[0] + (w1[1] - w2[1]) * un[1] + (w1[2] - w2[2]) * un[2];
     double vw[3];
     for (int k = 0; k < 3; ++k) {
@@ -510,9 +511,10 @@ __device__ __forceinline__ void rod_force_slot(const DevState &S, const DevParam
                 const double rlm = ri + rj + P.bw;
                 if (!(r2 <= (rlm - kSmall) * (rlm - kSmall))) return;
                 const double rS = ri + rj, rA = rS + P.bw;
-                const double rn = sqrt(r2);
-                const double ux = d[0] / rn, uy = d[1] / rn, uz = d[2] / rn;
-                const double F = (rn < rA) ? -P.k * (rn - rA) * (rn - rA) * (rn - rS) : 0.0;
+                Divisor by;
+                const double rn = sqrt_rn(r2, &by);
+                const double ux = div_by(d[0], by), uy = div_by(d[1], by), uz = div_by(d[2], by);
+                const double F = lt_bits(rn, rA) ? -P.k * (rn - rA) * (rn - rA) * (rn - rS) : 0.0;
                 acc[0] += F * ux;
                 acc[1] += F * uy;
                 acc[2] += F * uz;
@@ -867,12 +869,14 @@ __global__ void k_rod_update(const DevState S, double dt, int a)
             }
             const double L = S.clen[i];
             om[0] = 0.0;
-            om[1] *= 2.0 / (L * L);
-            om[2] *= 2.0 / (L * L);
-            double on = sqrt(om[1] * om[1] + om[2] * om[2]);
+            const double oL = div_rn(2.0, L * L);
+            om[1] *= oL;
+            om[2] *= oL;
+            Divisor by;
+            const double on = sqrt_rn(om[1] * om[1] + om[2] * om[2], &by);
             if (on > 0.0) {
-                om[1] /= on;
-                om[2] /= on;
+                om[1] = div_by(om[1], by);
+                om[2] = div_by(om[2], by);
             }
             const double c = om[2], s = om[1];
             const double Q[3][3] = {{1.0, 0.0, 0.0}, {0.0, c, -s}, {0.0, s, c}};
@@ -890,8 +894,8 @@ __global__ void k_rod_update(const DevState S, double dt, int a)
                 for (int cc = 0; cc < 3; ++cc) nd[r] += R[r][cc] * q[cc];
             }
             th = acos(nd[2]);
-            const double rho = sqrt(nd[0] * nd[0] + nd[1] * nd[1]);
-            if (rho > 0.0) nd[0] /= rho;
+            const double rho = sqrt_rn(nd[0] * nd[0] + nd[1] * nd[1], &by);
+            if (rho > 0.0) nd[0] = div_by(nd[0], by);
             ph = acos(nd[0]);
             if (nd[1] < 0.0) ph = 2.0 * kPi - ph;
             double st2, ct2, sp2, cp2;

@@ -46,12 +46,13 @@ __device__ __forceinline__ bool sphere_term64(const DevState &S, const DevGeom &
     if (!G.nbh_trivial && !(r2 <= P.nbh)) return false;  // not in the neighbour list
     const double rj = S.rad[j];
     const double rlm = ri + rj + P.bw;                     // maxInteractionDistance
-    if (!(r2 <= (rlm - kSmall) * (rlm - kSmall))) return false;
+    if (!le_nonneg(r2, (rlm - kSmall) * (rlm - kSmall))) return false;
     const double rS = ri + rj;
     const double rA = rS + P.bw;
-    const double rn = sqrt(r2);
-    const double ux = dx / rn, uy = dy / rn, uz = dz / rn;
-    const double F = (rn < rA) ? -P.k * (rn - rA) * (rn - rA) * (rn - rS) : 0.0;
+    Divisor by;
+    const double rn = sqrt_rn(r2, &by);
+    const double ux = div_by(dx, by), uy = div_by(dy, by), uz = div_by(dz, by);
+    const double F = lt_bits(rn, rA) ? -P.k * (rn - rA) * (rn - rA) * (rn - rS) : 0.0;
     t[0] = F * ux;
     t[1] = F * uy;
     t[2] = F * uz;
@@ -97,7 +98,7 @@ __global__ void __launch_bounds__(256) k_sphere64(const DevState S, const DevPar
     int *opass = olen + B;  // the round's gate result per thread
     int *wsum = opass + B;  // per warp: staged pairs, then their exclusive scan
     const int b = a ^ 1;
-    const float bwf = (float)P.bw;  // once per thread: a conversion is an FP64-pipe instruction
+    const float bwf = P.bw32;
     for (int base = blockIdx.x * B; base < S.n; base += gridDim.x * B) {
         const int i = base + tid;
         const bool act = i < S.n;
@@ -208,8 +209,8 @@ __global__ void __launch_bounds__(256) k_sphere64(const DevState S, const DevPar
         if (act) {
             const DevGeom &G = S.geoms[col];
             // evaluateSurfaceForce, sphere branch: vcom = (0, 0, wall), vrot = 0
-            const double vx = fx + 0.0;
-            const double vy = fy + 0.0;
+            const double vx = plus_zero(fx);
+            const double vy = plus_zero(fy);
             const double vz = fz + wall_law(zi, ri, P);
             double nx = xi + dt * vx;
             double ny = yi + dt * vy;

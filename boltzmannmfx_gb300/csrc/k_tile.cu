@@ -123,9 +123,10 @@ __global__ void __launch_bounds__(128) k_tile_step(const double *__restrict__ x,
                         if (!(r2 <= (rlm - kSmall) * (rlm - kSmall))) continue;
                         const double rS = ri + rj;
                         const double rA = rS + P.bw;
-                        const double rn = sqrt(r2);
-                        const double ux = dx / rn, uy = dy / rn, uz = dz / rn;
-                        const double F = (rn < rA) ? -P.k * (rn - rA) * (rn - rA) * (rn - rS) : 0.0;
+                        Divisor by;
+                        const double rn = sqrt_rn(r2, &by);
+                        const double ux = div_by(dx, by), uy = div_by(dy, by), uz = div_by(dz, by);
+                        const double F = lt_bits(rn, rA) ? -P.k * (rn - rA) * (rn - rA) * (rn - rS) : 0.0;
                         fx += F * ux;
                         fy += F * uy;
                         fz += F * uz;
