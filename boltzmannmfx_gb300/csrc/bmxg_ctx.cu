@@ -718,11 +718,9 @@ int bmxg_set_state(bmxg_ctx *ctx, const bmxg_particles *p, const int64_t *colony
     if (join.s) CK(cudaStreamWaitEvent(st, ctx->io_ev[1], 0));  // staged positions
     // canonical order of the caller's particles
     LAUNCH(launch_user_bin(S, src_x, src_y, src_z, S.col[1], S.iz[1], grd, blk, st));
-    LAUNCH(launch_scan(S.colcnt, S.colstart[1], (int)ncols, ctx->scan_scratch, st));
-    LAUNCH(launch_user_scatter_canon(S, S.col[1], S.iz[1], S.colstart[1], ctx->uperm, grd, blk, st));
+    LAUNCH(launch_user_sort(S, S.col[1], S.iz[1], S.colstart[0], ctx->scan_scratch, ctx->uperm, grd, blk, st));
     // positions, radii, cell types, bins and offsets into slot order in one
     // pass (slot s is sorted position s, so the sort's bins are the slots')
-    CK(cudaMemcpyAsync(S.colstart[0], S.colstart[1], sizeof(int) * (ncols + 1), cudaMemcpyDeviceToDevice, st));
     LAUNCH(launch_load_slots(S, src_x, src_y, src_z, src_r, src_ct, S.col[1], S.iz[1], ctx->uperm, grd, blk, st));
     // the other fields
     auto up_d = [&](const double *src, double *dst, double fill) -> int {
@@ -1120,9 +1118,6 @@ int enqueue_step(bmxg_ctx *ctx, double dt, int precision, int a, int resync)
     cudaStream_t st = ctx->stream;
     const DevParams P = dev_params(ctx->prm);
     const int b = a ^ 1;
-    // per-step counters (out-of-domain, images, pairs, repairs); `nonfinite` is sticky
-    cudaMemsetAsync(ctx->d_cnt, 0, offsetof(DevCounters, nonfinite), st);
-    cudaMemsetAsync(&ctx->d_cnt->pairs, 0, sizeof(DevCounters) - offsetof(DevCounters, pairs), st);
     const int64_t n = ctx->n;
     const int mblk = ctx->sh_misc.block, mgrd = grid_for(ctx, ctx->sh_misc, n);
     cudaEvent_t k0, k1;
@@ -1138,7 +1133,6 @@ int enqueue_step(bmxg_ctx *ctx, double dt, int precision, int a, int resync)
         const int rg = grid_for(ctx, ctx->sh_rod, n);
         // the flat pipeline over the pairs the bookkeeping records
         const bool pipe = S.rnb != nullptr;
-        if (pipe) cudaMemsetAsync(S.rctl, 0, sizeof(RodCtl), st);
         LAUNCH(launch_rod_book(S, P, a, precision, pipe, rg, ctx->sh_rod.block, st));
         if (k0) cudaEventRecord(k0, st);
         if (pipe)
@@ -1148,7 +1142,7 @@ int enqueue_step(bmxg_ctx *ctx, double dt, int precision, int a, int resync)
         if (k1) cudaEventRecord(k1, st);
         LAUNCH(launch_rod_update(S, dt, a, mgrd, mblk, st));
     }
-    LAUNCH(launch_rebuild(S, b, ctx->scan_scratch, mgrd, mblk, st));
+    LAUNCH(launch_rebuild(S, b, ctx->scan_scratch, mgrd, mblk, st, true));
     return BMXG_OK;
 }
 
@@ -1243,6 +1237,7 @@ int step_setup(bmxg_ctx *ctx, int32_t nsteps, int32_t precision)
         ctx->S.rres = res;
         ctx->S.rwork = work;
         ctx->S.rctl = ctl;
+        CK(cudaMemsetAsync(ctl, 0, sizeof(RodCtl), ctx->stream));  // (then emptied at the end of each step)
         drop_graphs(ctx);
     }
     return BMXG_OK;
@@ -1292,6 +1287,8 @@ int bmxg_step(bmxg_ctx *ctx, double dt, int32_t nsteps, int32_t precision)
     // after a load, if shorter than kListMinSteps, takes the per-step path (a
     // load-step-store caller never reuses a list); later calls build one
     if (int rc = step_setup(ctx, nsteps, precision)) return rc;
+    // the per-step counters (the end of each step clears them for the next)
+    CK(cudaMemsetAsync(ctx->d_cnt, 0, kStepCounters * sizeof(unsigned long long), ctx->stream));
     CK(cudaEventRecord(ctx->ev0, ctx->stream));
     int32_t left = nsteps;
     ctx->kev_used = 0;
@@ -1370,9 +1367,10 @@ int bmxg_step(bmxg_ctx *ctx, double dt, int32_t nsteps, int32_t precision)
     }
     ctx->kev_used = 0;
     ctx->stats.n_kernel_launches = ctx->launches;
-    ctx->stats.n_out_of_domain = (int64_t)ctx->h_cnt->out_of_domain;
-    ctx->stats.n_edge_ghost = (int64_t)ctx->h_cnt->edge_ghost;
-    ctx->stats.n_bond_repairs = (int64_t)ctx->h_cnt->bond_repairs;
+    const DevCounters &hc = *ctx->h_cnt;
+    ctx->stats.n_out_of_domain = (int64_t)(ctx->list_on ? hc.out_of_domain : hc.last_out_of_domain);
+    ctx->stats.n_edge_ghost = (int64_t)(ctx->list_on ? hc.edge_ghost : hc.last_edge_ghost);
+    ctx->stats.n_bond_repairs = (int64_t)(ctx->list_on ? hc.bond_repairs : hc.last_bond_repairs);
     if (ctx->h_cnt->bad_index) return fail(ctx, BMXG_ERR_STATE, "internal: inconsistent bin counts");
     if (ctx->h_cnt->nonfinite) return fail(ctx, BMXG_ERR_NONFINITE, "a step produced a non-finite position");
     if (ctx->h_cnt->range)

@@ -85,17 +85,23 @@ struct alignas(16) FxGeom {
     int pad2;
 };
 
-// Counters a step accumulates on the device.
+// Counters a step accumulates on the device.  The per-step ones come first
+// (kStepCounters of them, cleared together); the re-binning at the end of a
+// step publishes them into last_* and clears them for the next step, so that
+// a step has no clearing node of its own (the list path clears them itself and
+// its last step's are read in place).
 struct DevCounters {
     unsigned long long out_of_domain;
     unsigned long long edge_ghost;
-    unsigned long long nonfinite;
-    unsigned long long bad_index;  // counting-sort slots outside 0..n-1 (skipped; an internal error, sticky)
     unsigned long long pairs;
     unsigned long long bond_repairs;
     unsigned long long moved;
+    unsigned long long nonfinite;  // sticky
+    unsigned long long bad_index;  // counting-sort slots outside 0..n-1 (skipped; an internal error, sticky)
     unsigned long long range;      // list path: a z left the fixed-point range (sticky)
+    unsigned long long last_out_of_domain, last_edge_ghost, last_bond_repairs;
 };
+constexpr int kStepCounters = 5;
 
 // Force parameters, fpar[0..8] (src/chemistry/bmx_cell_interaction.cpp:84-93).
 struct DevParams {

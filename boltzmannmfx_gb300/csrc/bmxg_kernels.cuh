@@ -156,11 +156,10 @@ int launch_bin(const DevState &S, int b, int grid, int block, cudaStream_t st);
 // gate (may be null): the kernels return at once when *gate == 0
 int launch_scan(const int *in, int *out, int n, int *scratch, cudaStream_t st, const int *gate = nullptr);
 size_t scan_scratch_ints(int n);
-// ra: buffer whose FP32 offsets the sorted copies take (default b)
-int launch_scatter_canon(const DevState &S, int b, int grid, int block, cudaStream_t st, int ra = -1,
-                         const int *gate = nullptr);
+// publish: the end of a step (the counters into last_*, cleared, and the rod
+// pipeline's queue emptied)
 int launch_rebuild(const DevState &S, int b, int *scan_scratch, int grid, int block, cudaStream_t st,
-                   int ra = -1, const int *gate = nullptr);
+                   bool publish = false);
 
 // positions, radii, cell types, bins, offsets and identity column order of a
 // freshly sorted state (buffer 0), gathered from the caller-order arrays
@@ -178,9 +177,10 @@ int launch_check_state(const int *ct, const double *r, int n, unsigned long long
 // caller-order staging -> slot order (set_state) and back (get_state)
 int launch_user_bin(const DevState &S, const double *ux, const double *uy, const double *uz,
                      int *ucol, int *uiz, int grid, int block, cudaStream_t st);
-// the caller's particles into column order: uperm[slot] = caller index (keys in lkey)
-int launch_user_scatter_canon(const DevState &S, const int *ucol, const int *uiz, const int *colstart,
-                               int *uperm, int grid, int block, cudaStream_t st);
+// the caller's particles into column order: the column offsets and uperm[slot] =
+// caller index (keys in lkey)
+int launch_user_sort(const DevState &S, const int *ucol, const int *uiz, int *colstart, int *scan_scratch,
+                     int *uperm, int grid, int block, cudaStream_t st);
 int launch_gather_d(double *dst, const double *src, const int *perm, int n, int grid, int block, cudaStream_t st);
 int launch_gather_i(int *dst, const int *src, const int *perm, int n, int planes, int grid, int block, cudaStream_t st);
 int launch_scatter_d(double *dst, const double *src, const int *orig, int n, int grid, int block, cudaStream_t st);
