@@ -1127,7 +1127,7 @@ int enqueue_step(bmxg_ctx *ctx, double dt, int precision, int a, int resync)
         if (k0) cudaEventRecord(k0, st);
         int sg, sb;
         stencil_shape(ctx, sh, n, &sg, &sb);
-        LAUNCH(launch_sphere_step(S, P, dt, a, precision, sg, sb, st, resync));
+        LAUNCH(launch_sphere_step(S, P, dt, a, precision, sg, sb, st, resync, sh.grid > 0));
         if (k1) cudaEventRecord(k1, st);
     } else {
         const int rg = grid_for(ctx, ctx->sh_rod, n);
@@ -1799,6 +1799,16 @@ int bmxg_autotune(bmxg_ctx *ctx, const char *cache_path)
         // which are cleared afterwards
         float best = 1e30f;
         Shape bs = ctx->sh_sphere[prec];
+        {   // the launch rule's own choice (grid 0)
+            Shape sh = ctx->sh_sphere[prec];
+            sh.grid = 0;
+            int sg, sb;
+            stencil_shape(ctx, sh, n, &sg, &sb);
+            if (int rc = timeit(2, 5, [&]() { return launch_sphere_step(S, P, 0.0, ctx->parity, prec, sg, sb,
+                                                                        ctx->stream, 0); }, &best))
+                return rc;
+            bs = sh;
+        }
         const int blocks[] = {64, 128, 256};  // k_sphere is compiled with __launch_bounds__(256)
         for (int blk : blocks) {
             for (int mult = 1; mult <= 64; mult *= 2) {  // up to one slot per thread
@@ -1808,7 +1818,7 @@ int bmxg_autotune(bmxg_ctx *ctx, const char *cache_path)
                 const int grd = grid_for(ctx, sh, n);
                 float ms = 0.0f;
                 if (int rc = timeit(2, 5, [&]() { return launch_sphere_step(S, P, 0.0, ctx->parity, prec, grd, blk,
-                                                                            ctx->stream, 0); }, &ms))
+                                                                            ctx->stream, 0, true); }, &ms))
                     return rc;
                 if (ms < best) {
                     best = ms;
@@ -2023,8 +2033,7 @@ int dfwd_step(bmxg_ctx *ctx, double dt)
     const Shape &sh = ctx->sh_sphere[0];
     int sg, sb;
     stencil_shape(ctx, sh, ctx->n, &sg, &sb);
-    LAUNCH(launch_dfwd(S, dev_params(ctx->prm), diff_params(ctx), dt, a, sg, sb,
-                       ctx->stream));
+    LAUNCH(launch_dfwd(S, dev_params(ctx->prm), diff_params(ctx), dt, a, sg, sb, ctx->stream, sh.grid > 0));
     LAUNCH(launch_rebuild(S, a ^ 1, ctx->scan_scratch, mgrd, mblk, ctx->stream));
     ctx->parity = a ^ 1;
     return BMXG_OK;
@@ -2134,7 +2143,7 @@ int bmxg_backward(bmxg_ctx *ctx, const double *dL_dx, double *dL_dx0, double *dL
         for (int t = c1 - 1; t >= c0; --t) {
             if ((rc = load_pos(ctx, ctx->segbuf + (size_t)(t - c0) * 3 * n))) return rc;
             LAUNCH(launch_dadj(S, P, D, ctx->traj_dt, 0, ctx->lam[cur], ctx->lam[cur ^ 1], ctx->gacc, ctx->gadh,
-                               ag, ab, st));
+                               ag, ab, st, sh.grid > 0));
             cur ^= 1;
         }
     }

@@ -51,6 +51,8 @@ constexpr int kListBins = 0;         // list mode keeps its frozen bins in buffe
 constexpr int kListStepBlock = 128;  // k_list_step's default block (at most 256; autotuned)
 constexpr int kListBuildBlock = 128; // k_list_build's default block (one slot per thread; at most 256)
 constexpr int kSphereBlock = 64;     // per-step sphere kernels' block (one slot per thread)
+constexpr int kWalkNarrow = 65536;   // FP64 steps: 32 slots per block, a warp per neighbour column, up to here
+constexpr int kWalkWide = 400000;    // ... 128 slots per block up to here
 constexpr int kRodCap = 32;          // gated pairs per segment the rod pipelines hold (more: the
                                      // segment walks its stencil in the segment kernel)
 
@@ -199,7 +201,7 @@ int launch_pairs(const DevState &S, const DevParams &P, int a, int64_t *cnt_or_o
 // resync (FP32F only): re-derive every slot's FP32 offsets and bin from its
 // FP64 position this step
 int launch_sphere_step(const DevState &S, const DevParams &P, double dt, int a, int precision,
-                        int grid, int block, cudaStream_t st, int resync = 1);
+                        int grid, int block, cudaStream_t st, int resync = 1, bool pinned = false);
 
 // ---- FP32F neighbour list with a skin (k_list.cu) --------------------------
 // decide: fold the last step's displacement into the bound and decide
@@ -268,9 +270,9 @@ int launch_init_bonds(const DevState &S, const DevParams &P, int a, double rlim,
 
 // ---- differentiation form (k_adjoint.cu) ---------------------------------
 int launch_dfwd(const DevState &S, const DevParams &P, const DiffParams &D, double dt, int a, int grid, int block,
-                cudaStream_t st);
+                cudaStream_t st, bool pinned = false);
 int launch_dadj(const DevState &S, const DevParams &P, const DiffParams &D, double dt, int a, const double *lin,
-                double *lout, double *gacc, double *gadh, int grid, int block, cudaStream_t st);
+                double *lout, double *gacc, double *gadh, int grid, int block, cudaStream_t st, bool pinned = false);
 int launch_dreduce(const double *gacc, int n, int planes, double *out, cudaStream_t st);
 
 }  // namespace bmxg

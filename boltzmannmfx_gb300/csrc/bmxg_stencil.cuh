@@ -155,6 +155,223 @@ __device__ __forceinline__ void col_to_bxy(const DevGeom &G, int col, int &bx, i
     by = q - (bx - 1) * G.n[1] + 1;
 }
 
+// ---- a stencil walk with one warp per neighbour column ----------------------
+// A block holds NS slots (a multiple of 32) and nine warps; warp w walks neighbour column w
+// (x offset w / 3 - 1, y offset w % 3 - 1, the order of the reference's list)
+// for all of them, one slot per lane, 32 at a time, and stages the candidates that pass the
+// caller's FP32 screen.  Nine short independent walks instead of one long
+// chain of dependent loads per slot, and a warp's lanes read the same or
+// adjacent columns.
+constexpr int kWalkCols = 9;
+constexpr int kWalkBlock = 32 * kWalkCols;
+
+// One column of one slot: up to four entries are loaded before any is used.
+// f(t, dzs) for every entry of z bins izi - 1 .. izi + 1 but the slot itself.
+template <class F>
+__device__ __forceinline__ void walk_column(const DevState &S, int a, int lo, int hi, int self_t, int izi, F &&f)
+{
+    const int *__restrict__ siz = S.siz[a];
+    const float4 *__restrict__ srel = S.srel[a];
+    if (hi - lo > 8) {  // (a column can be many bins tall)
+        int l = lo, h = hi;
+        while (l < h) {
+            const int mid = (l + h) >> 1;
+            if (__ldg(&siz[mid]) < izi - 1) l = mid + 1;
+            else h = mid;
+        }
+        lo = l;
+    }
+    for (int t = lo; t < hi; t += 4) {
+        int z[4];
+        float4 q[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int u = min(t + k, hi - 1);
+            z[k] = __ldg(&siz[u]) - izi;
+            q[k] = __ldg(&srel[u]);
+        }
+        if (z[0] > 1) break;  // sorted by z bin: the rest is out of reach
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (t + k < hi && z[k] >= -1 && z[k] <= 1 && t + k != self_t) f(t + k, q[k], z[k]);
+    }
+}
+
+// Shared memory of a block's walk over NS slots (32 per pass of the warps): per
+// column and slot the staged candidates (slot of the neighbour, image code)
+// and, after walk_scan, the end of the column's run among the slot's pairs;
+// the slots' first pairs.
+template <int NS, int STAGE>
+struct WalkMem {
+    int2 stage[kWalkCols * NS][STAGE];
+    int end[kWalkCols][NS];
+    int first[NS + 1];
+    int over[NS];  // the slot staged too many in some column: no pairs here
+    int wsum[NS / 32];
+};
+
+// After every warp wrote its counts into end[w][slot] (more than STAGE:
+// overflow): the counts into runs, over the whole block (it synchronises).
+template <int NS, int STAGE>
+__device__ __forceinline__ void walk_scan(WalkMem<NS, STAGE> &M)
+{
+    const int tid = threadIdx.x, lane = tid & 31;
+    __syncthreads();
+    int x = 0, mine = 0;
+    if (tid < NS) {
+        int run = 0;
+        bool over = false;
+#pragma unroll
+        for (int w = 0; w < kWalkCols; ++w) {
+            const int c = M.end[w][tid];
+            over |= c > STAGE;
+            run += c;
+            M.end[w][tid] = run;
+        }
+        M.over[tid] = over ? 1 : 0;
+        mine = over ? 0 : run;
+        x = mine;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, x, d);
+            if (lane >= d) x += y;
+        }
+        if (NS == 32) M.first[tid + 1] = x;
+        else if (lane == 31) M.wsum[tid >> 5] = x;
+        if (tid == 0) M.first[0] = 0;
+    }
+    __syncthreads();
+    if (NS > 32) {
+        if (tid < NS) {
+            for (int v = 0; v < (tid >> 5); ++v) x += M.wsum[v];
+            M.first[tid + 1] = x;
+        }
+        __syncthreads();
+    }
+}
+
+// Pair t of the block: its slot o and its staged candidate.
+template <int NS, int STAGE>
+__device__ __forceinline__ int2 walk_pair(const WalkMem<NS, STAGE> &M, int t, int &o)
+{
+    o = 0;
+#pragma unroll
+    for (int d = NS / 2; d >= 1; d >>= 1)
+        if (M.first[o + d] <= t) o += d;
+    const int k = t - M.first[o];
+    int w = 0, at = 0;
+#pragma unroll
+    for (int v = 0; v < kWalkCols - 1; ++v) {
+        const int e = M.end[v][o];
+        if (e <= k) {
+            w = v + 1;
+            at = e;
+        }
+    }
+    return M.stage[w * NS + o][k - at];
+}
+
+// The column of warp w around slot i's bin (false: outside a closed face).
+__device__ __forceinline__ bool walk_target(const DevState &S, const DevGeom &G, int a, int bx, int by, int w, int &ii,
+                                            int &jj, int &lo, int &hi, int &sx, int &sy)
+{
+    ii = bx + w / 3 - 1;
+    jj = by + w % 3 - 1;
+    int cc;
+    if (!stencil_row(G, ii, jj, cc, sx, sy)) return false;
+    lo = __ldg(&S.colstart[a][cc]);
+    hi = __ldg(&S.colstart[a][cc + 1]);
+    return true;
+}
+
+// The FP32 screen of the FP64 pair walks: false only when the candidate is
+// certainly beyond the cutoff r_i + r_j + bw, from the FP32 offsets to the bin
+// corners (o: the neighbour bin's minus the slot's) with an absolute slack of 8
+// ulp of the largest bin width that bounds their error; the FP64 gate decides
+// the rest.
+__device__ __forceinline__ bool near_pair32(const float4 me, const float4 q, float ox, float oy, float oz, float bwf,
+                                            float slack)
+{
+    const float ex = (me.x - q.x) - ox;
+    const float ey = (me.y - q.y) - oy;
+    const float ez = (me.z - q.z) - oz;
+    const float r2f = __fmaf_rn(ex, ex, __fmaf_rn(ey, ey, __fmul_rn(ez, ez)));
+    const float lim = __fadd_rn(__fadd_rn(__fadd_rn(me.w, q.w), bwf), slack);
+    return !(r2f > __fmul_rn(lim, lim));
+}
+
+__device__ __forceinline__ float screen_slack(const DevGeom &G)
+{
+    return 8.0f * 1.1920929e-7f * fmaxf(G.dxf[0], fmaxf(G.dxf[1], G.dxf[2]));
+}
+
+// The block's walk of buffer a: every slot's candidates staged, the runs of
+// pairs set up (walk_scan).  own(s, i, colony): the first warp, for each slot.
+template <int NS, int STAGE, class Own>
+__device__ __forceinline__ void walk_block(const DevState &S, int a, float bwf, WalkMem<NS, STAGE> &M, Own &&own)
+{
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (int g = 0; g < NS; g += 32) {
+        const int s = g + lane;
+        const int i = blockIdx.x * NS + s;
+        int cnt = 0;
+        if (i < S.n) {
+            const int col = colony_of(S.cbase, S.ncol, i);
+            const DevGeom &G = S.geoms[col];
+            int bx, by;
+            col_to_bxy(G, S.col[a][i], bx, by);
+            const int izi = S.iz[a][i];
+            const float4 me = S.rel[a][i];
+            const int self_t = S.rank[a][i];
+            if (w == 0) own(s, i, col);
+            const float slack = screen_slack(G), dzb = G.dxf[2];
+            const float ox = (float)(w / 3 - 1) * G.dxf[0], oy = (float)(w % 3 - 1) * G.dxf[1];
+            int ii, jj, lo, hi, sx, sy;
+            if (walk_target(S, G, a, bx, by, w, ii, jj, lo, hi, sx, sy)) {
+                walk_column(S, a, lo, hi, self_t, izi, [&](int t, const float4 q, int dzs) {
+                    if (!near_pair32(me, q, ox, oy, (float)dzs * dzb, bwf, slack)) return;
+                    const int j = __ldg(&S.perm[a][t]);
+                    if ((sx | sy) && !image_in_row(S, G, a, j, ii, jj, sx, sy)) return;
+                    if (cnt < STAGE) M.stage[w * NS + s][cnt] = make_int2(j, (sx + 1) * 3 + (sy + 1));
+                    ++cnt;
+                });
+            }
+        }
+        M.end[w][s] = cnt;
+    }
+    walk_scan(M);
+}
+
+// The block's staged pairs, one per thread: eval(o, e, t) computes pair e of
+// slot o into t[NT] (false: no term); add(t, stride) adds one pair's terms to
+// the sums of slot threadIdx.x, in staging order (the slots' threads are the
+// block's first NS).  term: NT x kWalkBlock values.
+template <int NT, int NS, int STAGE, class Eval, class Add>
+__device__ __forceinline__ void walk_pairs(const WalkMem<NS, STAGE> &M, double *term, unsigned char *opass, Eval &&eval,
+                                           Add &&add)
+{
+    const int tid = threadIdx.x;
+    const int total = M.first[NS];
+    for (int t0 = 0; t0 < total; t0 += kWalkBlock) {
+        const int t = t0 + tid;
+        if (t < total) {
+            int o;
+            const int2 e = walk_pair(M, t, o);
+            double tt[NT];
+            for (int c = 0; c < NT; ++c) tt[c] = 0.0;
+            opass[tid] = eval(o, e, tt) ? 1 : 0;
+            for (int c = 0; c < NT; ++c) term[c * kWalkBlock + tid] = tt[c];
+        }
+        __syncthreads();
+        if (tid < NS) {
+            const int k1 = min(M.first[tid + 1], t0 + kWalkBlock);
+            for (int k = max(M.first[tid], t0); k < k1; ++k)
+                if (opass[k - t0]) add(term + (k - t0));
+        }
+        if (t0 + kWalkBlock < total) __syncthreads();
+    }
+}
+
 // Bin a slot at position (x, y, z): column and z bin into buffer bb, FP32
 // offsets from the bin corner into buffer rb, column count; flag
 // out-of-domain z, images that leave their halo cell, and non-finite positions.

@@ -54,24 +54,11 @@ __device__ __forceinline__ double wall_slope(double z, double rS, const DevParam
     return 0.0;
 }
 
-// The FP32 screen of the FP64 pair walks (as in the FP64 sphere step): false
-// only when the candidate is certainly beyond the cutoff r_i + r_j + bw, from
-// the FP32 offsets to the bin corners with an absolute slack of 8 ulp of the
-// largest bin width that bounds their error; the FP64 gate decides the rest.
+// near_pair32 by bin offsets
 __device__ __forceinline__ bool near32(const float4 me, const float4 q, int dxs, int dys, int dzs, const DevGeom &G,
                                        float bwf, float slack)
 {
-    const float ex = (me.x - q.x) - (float)dxs * G.dxf[0];
-    const float ey = (me.y - q.y) - (float)dys * G.dxf[1];
-    const float ez = (me.z - q.z) - (float)dzs * G.dxf[2];
-    const float r2f = __fmaf_rn(ex, ex, __fmaf_rn(ey, ey, __fmul_rn(ez, ez)));
-    const float lim = __fadd_rn(__fadd_rn(__fadd_rn(me.w, q.w), bwf), slack);
-    return !(r2f > __fmul_rn(lim, lim));
-}
-
-__device__ __forceinline__ float screen_slack(const DevGeom &G)
-{
-    return 8.0f * 1.1920929e-7f * fmaxf(G.dxf[0], fmaxf(G.dxf[1], G.dxf[2]));
+    return near_pair32(me, q, (float)dxs * G.dxf[0], (float)dys * G.dxf[1], (float)dzs * G.dxf[2], bwf, slack);
 }
 
 // ---- staged pair evaluation ----------------------------------------------
@@ -420,6 +407,145 @@ __global__ void __launch_bounds__(256) k_dadj(const DevState S, const DevParams 
     }
 }
 
+// The same two kernels with one warp per neighbour column (bmxg_stencil.cuh),
+// for sizes whose walks are bound by their dependent loads: same pairs, same
+// FP64 operations, same order of the sums.
+template <int NS, int STAGE>
+__global__ void __launch_bounds__(kWalkBlock, 3) k_dfwdw(const DevState S, const DevParams P, DiffParams D, double dt,
+                                                         int a)
+{
+    extern __shared__ __align__(16) unsigned char smw[];
+    auto &M = *reinterpret_cast<WalkMem<NS, STAGE> *>(smw);
+    __shared__ double own[6][NS];
+    __shared__ int ocol[NS];
+    __shared__ double term[3 * kWalkBlock];
+    __shared__ unsigned char opass[kWalkBlock];
+    const int tid = threadIdx.x;
+    const int b = a ^ 1;
+    walk_block(S, a, P.bw32, M, [&](int s, int i, int col) {
+        const double ri = S.rad[i];
+        own[0][s] = S.x[a][i];
+        own[1][s] = S.y[a][i];
+        own[2][s] = S.z[a][i];
+        own[3][s] = ri;
+        own[4][s] = mobility_of(ri, D.mu);
+        own[5][s] = D.adh ? D.adh[i] : 0.0;
+        ocol[s] = col;
+    });
+    double fx = 0.0, fy = 0.0, fz = 0.0;
+    walk_pairs<3>(
+        M, term, opass,
+        [&](int o, int2 e, double *t) {
+            return dfwd_term(S, S.geoms[ocol[o]], P, D, a, own[0][o], own[1][o], own[2][o], own[3][o], own[4][o],
+                             own[5][o], e.x, e.y / 3 - 1, e.y % 3 - 1, t);
+        },
+        [&](const double *t) {
+            fx += t[0];
+            fy += t[kWalkBlock];
+            fz += t[2 * kWalkBlock];
+        });
+    const int i = blockIdx.x * NS + tid;
+    if (tid >= NS || i >= S.n) return;
+    const DevGeom &G = S.geoms[ocol[tid]];
+    const double xi = own[0][tid], yi = own[1][tid], zi = own[2][tid], ri = own[3][tid];
+    if (M.over[tid]) {  // a crowded column: the whole walk, each pair evaluated as it is met
+        int bx, by;
+        col_to_bxy(G, S.col[a][i], bx, by);
+        const float4 me = S.rel[a][i];
+        const float slack = screen_slack(G);
+        walk<true>(S, G, a, i, bx, by, S.iz[a][i], [&](const float4 q, auto slot, int dxs, int dys, int dzs, int sx,
+                                                       int sy) {
+            if (!near32(me, q, dxs, dys, dzs, G, P.bw32, slack)) return;
+            double t[3];
+            if (dfwd_term(S, G, P, D, a, xi, yi, zi, ri, own[4][tid], own[5][tid], slot(), sx, sy, t)) {
+                fx += t[0];
+                fy += t[1];
+                fz += t[2];
+            }
+        });
+    }
+    const double vx = plus_zero(fx), vy = plus_zero(fy), vz = fz + wall_law(zi, ri, P);
+    double nx = xi + dt * vx, ny = yi + dt * vy;
+    const double nz = zi + dt * vz;
+    if (G.per[0]) nx = wrap1(nx, G.plo[0], G.phi[0], G.len[0]);
+    if (G.per[1]) ny = wrap1(ny, G.plo[1], G.phi[1], G.len[1]);
+    S.x[b][i] = nx;
+    S.y[b][i] = ny;
+    S.z[b][i] = nz;
+    S.vx[i] = vx;
+    S.vy[i] = vy;
+    S.vz[i] = vz;
+    rebin_slot(S, G, i, nx, ny, nz, ri, b);
+}
+
+template <int NS, int STAGE>
+__global__ void __launch_bounds__(kWalkBlock, 2) k_dadjw(const DevState S, const DevParams P, DiffParams D, double dt,
+                                                         int a, const double *__restrict__ lin,
+                                                         double *__restrict__ lout, double *__restrict__ gacc,
+                                                         double *__restrict__ gadh)
+{
+    constexpr int NO = 10, NT = 7;
+    extern __shared__ __align__(16) unsigned char smw[];
+    auto &M = *reinterpret_cast<WalkMem<NS, STAGE> *>(smw);
+    __shared__ double own[NS][NO + 1];  // (odd pitch: no bank conflicts between the slots' rows)
+    __shared__ int ocol[NS];
+    __shared__ double term[NT * kWalkBlock];
+    __shared__ unsigned char opass[kWalkBlock];
+    const int tid = threadIdx.x;
+    const int n = S.n;
+    walk_block(S, a, P.bw32, M, [&](int s, int k, int col) {
+        double *o = own[s];
+        const double rk = S.rad[k];
+        const double mk = mobility_of(rk, D.mu);
+        o[0] = S.x[a][k];
+        o[1] = S.y[a][k];
+        o[2] = S.z[a][k];
+        o[3] = rk;
+        o[4] = mk;
+        o[5] = D.mu > 0.0 ? div_rn(-mk, D.mu) : 0.0;
+        o[6] = D.adh ? D.adh[k] : 0.0;
+        o[7] = lin[k];
+        o[8] = lin[(size_t)n + k];
+        o[9] = lin[(size_t)2 * n + k];
+        ocol[s] = col;
+    });
+    double acc[NT];
+    for (int c = 0; c < NT; ++c) acc[c] = 0.0;
+    walk_pairs<NT>(
+        M, term, opass,
+        [&](int ow, int2 e, double *t) {
+            return dadj_term(S, S.geoms[ocol[ow]], P, D, a, lin, n, own[ow], e.x, e.y / 3 - 1, e.y % 3 - 1, t);
+        },
+        [&](const double *t) {
+            for (int c = 0; c < NT; ++c) acc[c] += t[c * kWalkBlock];
+        });
+    const int k = blockIdx.x * NS + tid;
+    if (tid >= NS || k >= n) return;
+    const double *o = own[tid];
+    if (M.over[tid]) {
+        const DevGeom &G = S.geoms[ocol[tid]];
+        int bx, by;
+        col_to_bxy(G, S.col[a][k], bx, by);
+        const float4 me = S.rel[a][k];
+        const float slack = screen_slack(G);
+        walk<true>(S, G, a, k, bx, by, S.iz[a][k], [&](const float4 q, auto slot, int dxs, int dys, int dzs, int sx,
+                                                       int sy) {
+            if (!near32(me, q, dxs, dys, dzs, G, P.bw32, slack)) return;
+            double t[NT];
+            if (dadj_term(S, G, P, D, a, lin, n, o, slot(), sx, sy, t))
+                for (int c = 0; c < NT; ++c) acc[c] += t[c];
+        });
+    }
+    const double wz = wall_slope(o[2], o[3], P);
+    lout[k] = o[7] + dt * acc[0];
+    lout[(size_t)n + k] = o[8] + dt * acc[1];
+    lout[(size_t)2 * n + k] = o[9] + dt * (acc[2] + wz * o[9]);
+    gacc[k] += dt * acc[3];
+    gacc[(size_t)n + k] += dt * acc[4];
+    gacc[(size_t)2 * n + k] += dt * acc[5];
+    gadh[k] += dt * acc[6];
+}
+
 // deterministic sum of per-slot gradient planes (one block, fixed order)
 __global__ void k_dreduce(const double *gacc, int n, int planes, double *out)
 {
@@ -449,10 +575,15 @@ void allow_smem(K kernel, size_t need)
 }
 
 int launch_dfwd(const DevState &S, const DevParams &P, const DiffParams &D, double dt, int a, int grid, int block,
-                cudaStream_t st)
+                cudaStream_t st, bool pinned)
 {
     const size_t smem = staged_smem(block, 6, 3);
-    if (S.srel[a]) {
+    // (the FP64 step's rule, launch_sphere_step.  Measured, us per step of the forward / the backward sweep
+    // with recomputation, one thread per slot -> a warp per column: 1000 spheres 57 -> 23 / 144 -> 77, 20 000
+    // 79 -> 40 / 195 -> 129, 40 000 82 -> 61 / 207 -> 192)
+    if (S.srel[a] && !pinned && S.n <= kWalkNarrow) {
+        k_dfwdw<32, 6><<<(S.n + 31) / 32, kWalkBlock, sizeof(WalkMem<32, 6>), st>>>(S, P, D, dt, a);
+    } else if (S.srel[a]) {
         allow_smem(k_dfwd<true>, smem);
         k_dfwd<true><<<grid, block, smem, st>>>(S, P, D, dt, a);
     } else {
@@ -463,10 +594,13 @@ int launch_dfwd(const DevState &S, const DevParams &P, const DiffParams &D, doub
 }
 
 int launch_dadj(const DevState &S, const DevParams &P, const DiffParams &D, double dt, int a, const double *lin,
-                double *lout, double *gacc, double *gadh, int grid, int block, cudaStream_t st)
+                double *lout, double *gacc, double *gadh, int grid, int block, cudaStream_t st, bool pinned)
 {
     const size_t smem = staged_smem(block, 10, 7);
-    if (S.srel[a]) {
+    if (S.srel[a] && !pinned && S.n <= kWalkNarrow) {
+        k_dadjw<32, 6><<<(S.n + 31) / 32, kWalkBlock, sizeof(WalkMem<32, 6>), st>>>(S, P, D, dt, a, lin, lout, gacc,
+                                                                                     gadh);
+    } else if (S.srel[a]) {
         allow_smem(k_dadj<true>, smem);
         k_dadj<true><<<grid, block, smem, st>>>(S, P, D, dt, a, lin, lout, gacc, gadh);
     } else {

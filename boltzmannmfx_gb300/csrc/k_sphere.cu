@@ -25,6 +25,8 @@
 //        might change.  Away from the faces the FP64 bin cannot change, so
 //        the neighbour lists stay exactly the reference's.
 // Roofline: HBM / L2 bound gather; no dense contraction, so no tensor cores.
+#include <atomic>
+
 #include "bmxg_stencil.cuh"
 
 namespace bmxg {
@@ -229,6 +231,78 @@ __global__ void __launch_bounds__(256) k_sphere64(const DevState S, const DevPar
     }
 }
 
+// The same step with one warp per neighbour column (bmxg_stencil.cuh): the
+// staged pairs one per thread over the block, the sums and the slots' updates
+// in its first warps.  Same pairs, same FP64 operations, same order of the sums.
+template <int NS, int STAGE>
+__global__ void __launch_bounds__(kWalkBlock, 3) k_sphere64w(const DevState S, const DevParams P, double dt, int a)
+{
+    extern __shared__ __align__(16) unsigned char smw[];
+    auto &M = *reinterpret_cast<WalkMem<NS, STAGE> *>(smw);
+    __shared__ double opos[NS][4];
+    __shared__ int ocol[NS];
+    __shared__ double term[3 * kWalkBlock];
+    __shared__ unsigned char opass[kWalkBlock];
+    const int tid = threadIdx.x;
+    const int b = a ^ 1;
+    walk_block(S, a, P.bw32, M, [&](int s, int i, int col) {
+        opos[s][0] = S.x[a][i];
+        opos[s][1] = S.y[a][i];
+        opos[s][2] = S.z[a][i];
+        opos[s][3] = S.rad[i];
+        ocol[s] = col;
+    });
+    double fx = 0.0, fy = 0.0, fz = 0.0;
+    walk_pairs<3>(
+        M, term, opass,
+        [&](int o, int2 e, double *t) {
+            return sphere_term64(S, S.geoms[ocol[o]], P, a, opos[o][0], opos[o][1], opos[o][2], opos[o][3], e.x,
+                                 e.y / 3 - 1, e.y % 3 - 1, t);
+        },
+        [&](const double *t) {
+            fx += t[0];
+            fy += t[kWalkBlock];
+            fz += t[2 * kWalkBlock];
+        });
+    const int i = blockIdx.x * NS + tid;
+    if (tid >= NS || i >= S.n) return;
+    const DevGeom &G = S.geoms[ocol[tid]];
+    const double xi = opos[tid][0], yi = opos[tid][1], zi = opos[tid][2], ri = opos[tid][3];
+    if (M.over[tid]) {  // a crowded column: the whole walk, each pair evaluated as it is met
+        int bx, by;
+        col_to_bxy(G, S.col[a][i], bx, by);
+        const float4 me = S.rel[a][i];
+        const float slack = screen_slack(G);
+        walk<true>(S, G, a, i, bx, by, S.iz[a][i], [&](const float4 q, auto slot, int dxs, int dys, int dzs, int sx,
+                                                       int sy) {
+            if (!near_pair32(me, q, (float)dxs * G.dxf[0], (float)dys * G.dxf[1], (float)dzs * G.dxf[2], P.bw32, slack))
+                return;
+            double t[3];
+            if (sphere_term64(S, G, P, a, xi, yi, zi, ri, slot(), sx, sy, t)) {
+                fx += t[0];
+                fy += t[1];
+                fz += t[2];
+            }
+        });
+    }
+    // evaluateSurfaceForce, sphere branch: vcom = (0, 0, wall), vrot = 0
+    const double vx = plus_zero(fx);
+    const double vy = plus_zero(fy);
+    const double vz = fz + wall_law(zi, ri, P);
+    double nx = xi + dt * vx;
+    double ny = yi + dt * vy;
+    const double nz = zi + dt * vz;
+    if (G.per[0]) nx = wrap1(nx, G.plo[0], G.phi[0], G.len[0]);
+    if (G.per[1]) ny = wrap1(ny, G.plo[1], G.phi[1], G.len[1]);
+    S.x[b][i] = nx;
+    S.y[b][i] = ny;
+    S.z[b][i] = nz;
+    S.vx[i] = vx;
+    S.vy[i] = vy;
+    S.vz[i] = vz;
+    rebin_slot(S, G, i, nx, ny, nz, ri, b);
+}
+
 template <bool SORTED>
 __global__ void __launch_bounds__(256, 5) k_sphere32(const DevState S, const DevParams P, float dtf, int a,
                                                   int resync)
@@ -316,33 +390,57 @@ __global__ void __launch_bounds__(256, 5) k_sphere32(const DevState S, const Dev
 
 }  // namespace
 
-// k_sphere64's dynamic shared memory above the default 48 KB for 256-thread
-// blocks: the attribute, once per device
-template <bool SORTED>
-void allow_sphere64_smem()
+// A kernel's dynamic shared memory above the default 48 KB: the attribute,
+// once per device (known: a bit per device, set twice at worst).
+template <class K>
+static void allow_smem_once(K kernel, size_t bytes, std::atomic<unsigned long long> &known)
 {
-    static unsigned long long done = 0ull;  // a bit per device (set twice at worst: idempotent)
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return;
-    if (dev < 64 && ((done >> dev) & 1ull)) return;
-    if (cudaFuncSetAttribute(k_sphere64<SORTED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)sphere64_smem(256)) == cudaSuccess &&
+    if (dev < 64 && ((known.load(std::memory_order_relaxed) >> dev) & 1ull)) return;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess &&
         dev < 64)
-        done |= 1ull << dev;
+        known.fetch_or(1ull << dev, std::memory_order_relaxed);
+}
+
+// Which FP64 kernel a sorted state takes: one warp per neighbour column where
+// the slots are too few for a thread each to hide the walk's dependent loads
+// (32 slots per block up to kWalkNarrow slots, 128 up to kWalkWide), one thread
+// per slot above, where the walk's instructions count and not its latency.
+// Measured, us per step with the re-binning, one thread per slot / 32 / 128
+// slots per block: 1000 spheres 39 / 17 / -, 20 000 50 / 30 / 44, 40 000 54 / 41 / 48,
+// 80 000 69 / 65 / 59, 160 000 96 / 109 / 77, 500 000 (host load and store
+// included) 698 / 814 / 698, 688 000 in 64 colonies 445 / 552 / 483.
+static int sphere64_slots(int n)
+{
+    return n <= kWalkNarrow ? 32 : (n <= kWalkWide ? 128 : 0);
 }
 
 int launch_sphere_step(const DevState &S, const DevParams &P, double dt, int a, int precision, int grid,
-                       int block, cudaStream_t st, int resync)
+                       int block, cudaStream_t st, int resync, bool pinned)
 {
     const bool sorted = S.srel[a] != nullptr;  // the context keeps sorted copies; bare callers do not
     if (precision == BMXG_FP64_FORM) {
+        const int ns = (sorted && !pinned) ? sphere64_slots(S.n) : 0;
+        if (ns == 32) {
+            k_sphere64w<32, 6><<<(S.n + 31) / 32, kWalkBlock, sizeof(WalkMem<32, 6>), st>>>(S, P, dt, a);
+            return 1;
+        }
+        if (ns == 128) {
+            static std::atomic<unsigned long long> known{0};
+            allow_smem_once(k_sphere64w<128, 4>, sizeof(WalkMem<128, 4>), known);
+            k_sphere64w<128, 4><<<(S.n + 127) / 128, kWalkBlock, sizeof(WalkMem<128, 4>), st>>>(S, P, dt, a);
+            return 1;
+        }
         // (block a multiple of 32, at most 256: the block stages and evaluates its pairs together)
         const size_t smem = sphere64_smem(block);
         if (sorted) {
-            allow_sphere64_smem<true>();
+            static std::atomic<unsigned long long> known{0};
+            allow_smem_once(k_sphere64<true>, sphere64_smem(256), known);
             k_sphere64<true><<<grid, block, smem, st>>>(S, P, dt, a);
         } else {
-            allow_sphere64_smem<false>();
+            static std::atomic<unsigned long long> known{0};
+            allow_smem_once(k_sphere64<false>, sphere64_smem(256), known);
             k_sphere64<false><<<grid, block, smem, st>>>(S, P, dt, a);
         }
     } else {
