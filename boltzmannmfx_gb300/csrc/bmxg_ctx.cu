@@ -66,7 +66,6 @@ struct bmxg_ctx {
     int *scan_scratch = nullptr;
     // staging in caller order
     double *ud = nullptr;  // n doubles
-    int *ui = nullptr;     // 13 n ints
     int *uperm = nullptr;
 
     int64_t n = 0;
@@ -132,13 +131,26 @@ struct bmxg_ctx {
     cudaEvent_t io_ev[8] = {};
     char *io_buf = nullptr;
     size_t io_cap = 0;
-    unsigned long long *d_chk = nullptr;    // state-check flags (4), device
+    char *aos_buf = nullptr;                // planes (and staged records) of the AoS entry point, grown
+    size_t aos_cap = 0;
+    bool pageable = false;                  // the device reads pageable host memory in place
+    unsigned long long *d_chk = nullptr;    // state-check flags (4) and the comparison of a load (1), device
     unsigned long long *h_chk = nullptr;    // and pinned host
 };
 
 namespace {
 
 int sync_fp64(bmxg_ctx *ctx);
+
+// What a load checks of a state (launch_check_state), when the caller has done so.
+struct StateCheck {
+    bool rods;
+    double rmax;
+};
+int load_state(bmxg_ctx *ctx, const bmxg_particles *p, const int64_t *colony_offsets, int where,
+               const StateCheck *known);
+int check_state(bmxg_ctx *ctx, const int *ct, const double *r, int64_t n, StateCheck *out);
+int read_check(bmxg_ctx *ctx, StateCheck *out);
 
 int fail(bmxg_ctx *c, int code, const std::string &msg)
 {
@@ -229,7 +241,6 @@ void free_state(bmxg_ctx *ctx)
     ctx->scan_scratch = nullptr;
     ctx->cell_scratch = nullptr;
     ctx->ud = nullptr;
-    ctx->ui = nullptr;
     ctx->uperm = nullptr;
     ctx->have_state = false;
     ctx->list_valid = false;
@@ -421,6 +432,9 @@ int bmxg_create(const bmxg_params *params, int32_t ncolonies, const bmxg_geometr
     }
     cudaError_t e = cudaGetDevice(&ctx->device);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&ctx->nsm, cudaDevAttrMultiProcessorCount, ctx->device);
+    int paged = 0;
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&paged, cudaDevAttrPageableMemoryAccess, ctx->device);
+    ctx->pageable = paged != 0;
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->own_stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreate(&ctx->ev0);
     if (e == cudaSuccess) e = cudaEventCreate(&ctx->ev1);
@@ -430,8 +444,8 @@ int bmxg_create(const bmxg_params *params, int32_t ncolonies, const bmxg_geometr
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->io_stream, cudaStreamNonBlocking);
     for (cudaEvent_t &ev : ctx->io_ev)
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
-    if (e == cudaSuccess) e = cudaMalloc(&ctx->d_chk, 4 * sizeof(unsigned long long));
-    if (e == cudaSuccess) e = cudaMallocHost(&ctx->h_chk, 4 * sizeof(unsigned long long));
+    if (e == cudaSuccess) e = cudaMalloc(&ctx->d_chk, 5 * sizeof(unsigned long long));
+    if (e == cudaSuccess) e = cudaMallocHost(&ctx->h_chk, 5 * sizeof(unsigned long long));
     if (e != cudaSuccess) {
         ctx->err = cudaGetErrorString(e);
         bmxg_destroy(ctx);
@@ -461,6 +475,7 @@ void bmxg_destroy(bmxg_ctx *ctx)
     for (cudaEvent_t ev : ctx->io_ev)
         if (ev) cudaEventDestroy(ev);
     if (ctx->io_buf) cudaFree(ctx->io_buf);
+    if (ctx->aos_buf) cudaFree(ctx->aos_buf);
     if (ctx->d_chk) cudaFree(ctx->d_chk);
     if (ctx->h_chk) cudaFreeHost(ctx->h_chk);
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);
@@ -508,6 +523,16 @@ int bmxg_set_stream(bmxg_ctx *ctx, void *stream)
 
 int bmxg_set_state(bmxg_ctx *ctx, const bmxg_particles *p, const int64_t *colony_offsets, int where)
 {
+    return load_state(ctx, p, colony_offsets, where, nullptr);
+}
+
+}  // extern "C"
+
+namespace {
+
+int load_state(bmxg_ctx *ctx, const bmxg_particles *p, const int64_t *colony_offsets, int where,
+               const StateCheck *known)
+{
     if (!ctx) return BMXG_ERR_ARG;
     (void)cudaGetLastError();  // drop a non-sticky error another library left on this thread
     if (!p || p->n < 0 || !p->x || !p->y || !p->z || !p->radius || !p->cell_type)
@@ -539,7 +564,7 @@ int bmxg_set_state(bmxg_ctx *ctx, const bmxg_particles *p, const int64_t *colony
                                !p->id && !p->cpu && !p->n_bnds && !p->seg_id1 && !p->seg_id2 && !p->site &&
                                !p->position && !p->fuse_tip && !p->fix_site && !p->fuse_flag &&
                                !p->split_flag && !p->new_flag && !p->dltd;
-    const bool same_cand = n && only_required && ctx->have_state && ctx->n == n && ctx->offsets == off &&
+    const bool same_cand = n && !known && only_required && ctx->have_state && ctx->n == n && ctx->offsets == off &&
                            !ctx->S.has_rods;
     // the comparison reads the device's FP64 positions
     if (same_cand) {
@@ -553,9 +578,23 @@ int bmxg_set_state(bmxg_ctx *ctx, const bmxg_particles *p, const int64_t *colony
     const int *src_ct = p->cell_type;
     JoinIo join{nullptr};
     cudaStream_t st0 = ctx->stream, st1 = ctx->io_stream;
+    {   // staging of the positions, radii and cell types (36 B) and of the other fields (up to 200 B, 24 of them)
+        auto staged = [&](const void *f, size_t align) {
+            return f && (where == BMXG_HOST || reinterpret_cast<uintptr_t>(f) % align != 0);
+        };
+        size_t bytes = (where == BMXG_HOST) ? (size_t)n * 36 + 512 : 0;
+        for (const double *f : {p->velx, p->vely, p->velz, p->wx, p->wy, p->wz, p->c_length, p->theta, p->phi,
+                                p->area, p->bond_scale})
+            if (staged(f, 8)) bytes += (size_t)n * 8 + 16;
+        for (const int32_t *f : {p->id, p->cpu, p->fuse_tip, p->position, p->fix_site, p->fuse_flag, p->split_flag,
+                                 p->new_flag, p->n_bnds})
+            if (staged(f, 4)) bytes += (size_t)n * 4 + 16;
+        for (const int32_t *f : {p->seg_id1, p->seg_id2, p->site})
+            if (staged(f, 4)) bytes += (size_t)n * 16 + 16;
+        if (staged(p->dltd, 4)) bytes += (size_t)n * 24 + 16;
+        if (int rc0 = ensure_io(ctx, bytes)) return rc0;
+    }
     if (n && where == BMXG_HOST) {
-        int rc0 = ensure_io(ctx, (size_t)n * 36 + 256);
-        if (rc0) return rc0;
         double *bx = (double *)ctx->io_buf, *by = bx + n, *bz = by + n, *br = bz + n;
         int *bct = (int *)(br + n);
         CK(cudaEventRecord(ctx->io_ev[0], st0));  // earlier kernels on st0 are done with the staging
@@ -579,25 +618,29 @@ int bmxg_set_state(bmxg_ctx *ctx, const bmxg_particles *p, const int64_t *colony
         cudaStream_t st = ctx->stream;
         const int grd = grid_for(ctx, ctx->sh_misc, n), blk = ctx->sh_misc.block;
         const DevState &S = ctx->S;
-        CK(cudaMemsetAsync(ctx->d_chk, 0, sizeof(unsigned long long), st));
+        unsigned long long *diff = ctx->d_chk + 4;
+        CK(cudaMemsetAsync(ctx->d_chk, 0, 5 * sizeof(unsigned long long), st));
+        // (the checks of a full load go along: one read-back decides both)
+        Shape sh;
+        LAUNCH(launch_check_state(src_ct, src_r, (int)n, ctx->d_chk, grid_for(ctx, sh, n), sh.block, st));
         if (join.s) {  // each field as its copy lands: only the last comparison follows the copies
-            LAUNCH(launch_same_state(S, ctx->parity, nullptr, nullptr, nullptr, src_r, src_ct, ctx->d_chk, grd, blk,
+            LAUNCH(launch_same_state(S, ctx->parity, nullptr, nullptr, nullptr, src_r, src_ct, diff, grd, blk,
                                      st));
             CK(cudaStreamWaitEvent(st, ctx->io_ev[6], 0));
-            LAUNCH(launch_same_state(S, ctx->parity, src_x, nullptr, nullptr, nullptr, nullptr, ctx->d_chk, grd, blk,
+            LAUNCH(launch_same_state(S, ctx->parity, src_x, nullptr, nullptr, nullptr, nullptr, diff, grd, blk,
                                      st));
             CK(cudaStreamWaitEvent(st, ctx->io_ev[7], 0));
-            LAUNCH(launch_same_state(S, ctx->parity, nullptr, src_y, nullptr, nullptr, nullptr, ctx->d_chk, grd, blk,
+            LAUNCH(launch_same_state(S, ctx->parity, nullptr, src_y, nullptr, nullptr, nullptr, diff, grd, blk,
                                      st));
             CK(cudaStreamWaitEvent(st, ctx->io_ev[1], 0));
-            LAUNCH(launch_same_state(S, ctx->parity, nullptr, nullptr, src_z, nullptr, nullptr, ctx->d_chk, grd, blk,
+            LAUNCH(launch_same_state(S, ctx->parity, nullptr, nullptr, src_z, nullptr, nullptr, diff, grd, blk,
                                      st));
         } else {
-            LAUNCH(launch_same_state(S, ctx->parity, src_x, src_y, src_z, src_r, src_ct, ctx->d_chk, grd, blk, st));
+            LAUNCH(launch_same_state(S, ctx->parity, src_x, src_y, src_z, src_r, src_ct, diff, grd, blk, st));
         }
-        CK(cudaMemcpyAsync(ctx->h_chk, ctx->d_chk, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
+        CK(cudaMemcpyAsync(ctx->h_chk, ctx->d_chk, 5 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
-        if (ctx->h_chk[0] == 0) {
+        if (ctx->h_chk[4] == 0) {
             // velocities to zero (unless no kernel wrote them since the last
             // load zeroed them) and the counters; stream-ordered before
             // whatever the caller enqueues next
@@ -621,33 +664,28 @@ int bmxg_set_state(bmxg_ctx *ctx, const bmxg_particles *p, const int64_t *colony
     // cell types decide which path runs (rods need their fields) and the
     // largest radius whether the FP32F list is exact: checked on the device,
     // one small read-back
-    bool rods = false;
-    double rmax = 0.0;
-    if (n) {
-        CK(cudaMemsetAsync(ctx->d_chk, 0, 4 * sizeof(unsigned long long), st0));
-        Shape sh;
-        launch_check_state(src_ct, src_r, (int)n, ctx->d_chk, grid_for(ctx, sh, n), sh.block, st0);
-        CK(cudaGetLastError());
-        CK(cudaMemcpyAsync(ctx->h_chk, ctx->d_chk, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st0));
-        const cudaError_t e = cudaStreamSynchronize(st0);
-        if (e != cudaSuccess) return fail(ctx, BMXG_ERR_CUDA, std::string("state check: ") + cudaGetErrorString(e));
-        const unsigned long long *h = ctx->h_chk;
-        if (h[0]) return fail(ctx, BMXG_ERR_ARG, "cell_type must be 0 or 1");
-        rods = h[1] != 0;
-        const uint64_t rb = h[2];
-        std::memcpy(&rmax, &rb, sizeof(rmax));
-        if (h[3]) rmax = std::nan("");
+    StateCheck chk{false, 0.0};
+    if (known) {
+        chk = *known;
+    } else if (same_cand) {
+        if (int rc0 = read_check(ctx, &chk)) return rc0;
+    } else if (n) {
+        if (int rc0 = check_state(ctx, src_ct, src_r, n, &chk)) return rc0;
     }
+    const bool rods = chk.rods;
+    const double rmax = chk.rmax;
     if (rods && (!p->c_length || !p->theta || !p->phi || !p->area || !p->id || !p->cpu || !p->n_bnds ||
                  !p->seg_id1 || !p->seg_id2 || !p->site))
         return fail(ctx, BMXG_ERR_ARG, "rod segments need c_length, theta, phi, area, id, cpu and the bond table");
 
-    CK(cudaStreamSynchronize(ctx->stream));
     // Same particle count, colony layout and cell-type mix as the loaded
     // state: keep the device buffers (and the captured step graphs, which
     // only hold their addresses) and overwrite the contents.
     const bool reuse = ctx->have_state && ctx->n == n && ctx->offsets == off && ctx->S.has_rods == (rods ? 1 : 0);
-    if (!reuse) free_state(ctx);
+    if (!reuse) {
+        CK(cudaStreamSynchronize(ctx->stream));
+        free_state(ctx);
+    }
     ctx->n = n;
     ctx->offsets = off;
     build_geoms(ctx);
@@ -681,7 +719,7 @@ int bmxg_set_state(bmxg_ctx *ctx, const bmxg_particles *p, const int64_t *colony
     AL(S.vx, n); AL(S.vy, n); AL(S.vz, n); AL(S.wx, n); AL(S.wy, n); AL(S.wz, n);
     AL(S.vxf, n); AL(S.vyf, n); AL(S.vzf, n);
     AL(ctx->scan_scratch, scan_scratch_ints((int)ncols));
-    AL(ctx->ud, n); AL(ctx->ui, 13 * n + 1); AL(ctx->uperm, n);
+    AL(ctx->ud, n); AL(ctx->uperm, n);
     if (rods) {
         AL(S.clen, n); AL(S.area, n); AL(S.bscale, n);
         for (int k = 0; k < 2; ++k) { AL(S.theta[k], n); AL(S.phi[k], n); AL(S.trig[k], n); AL(S.tab[k], 13 * n); }
@@ -721,59 +759,38 @@ int bmxg_set_state(bmxg_ctx *ctx, const bmxg_particles *p, const int64_t *colony
     LAUNCH(launch_user_sort(S, S.col[1], S.iz[1], S.colstart[0], ctx->scan_scratch, ctx->uperm, grd, blk, st));
     // positions, radii, cell types, bins and offsets into slot order in one
     // pass (slot s is sorted position s, so the sort's bins are the slots')
-    LAUNCH(launch_load_slots(S, src_x, src_y, src_z, src_r, src_ct, S.col[1], S.iz[1], ctx->uperm, grd, blk, st));
-    // the other fields
-    auto up_d = [&](const double *src, double *dst, double fill) -> int {
-        if (src) {
-            CK(cudaMemcpyAsync(ctx->ud, src, sizeof(double) * n, kind, st));
-            LAUNCH(launch_gather_d(dst, ctx->ud, ctx->uperm, (int)n, grd, blk, st));
-        } else if (fill == 0.0) {
-            CK(cudaMemsetAsync(dst, 0, sizeof(double) * n, st));
-        } else {
-            std::vector<double> h((size_t)n, fill);
-            CK(cudaMemcpyAsync(ctx->ud, h.data(), sizeof(double) * n, cudaMemcpyHostToDevice, st));
-            CK(cudaStreamSynchronize(st));
-            CK(cudaMemcpyAsync(dst, ctx->ud, sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
+    // The other fields: read in place from device arrays (aligned ones), else
+    // staged behind the positions; then gathered in one kernel.
+    char *stage = ctx->io_buf + (((size_t)(where == BMXG_HOST ? n : 0) * 36 + 255) / 256) * 256;
+    rc = BMXG_OK;
+    auto field = [&](const void *src, size_t bytes, size_t align) -> const void * {
+        if (!src || rc) return nullptr;
+        if (where == BMXG_DEVICE && (reinterpret_cast<uintptr_t>(src) % align) == 0) return src;
+        const cudaError_t e = cudaMemcpyAsync(stage, src, bytes, kind, st);
+        if (e != cudaSuccess) {
+            rc = fail(ctx, BMXG_ERR_CUDA, std::string("load of a field: ") + cudaGetErrorString(e));
+            return nullptr;
         }
-        return BMXG_OK;
+        const void *q = stage;
+        stage += (bytes + 15) / 16 * 16;
+        return q;
     };
-    auto up_i = [&](const int32_t *src, int *dst, int planes, int fill) -> int {
-        if (src) {
-            CK(cudaMemcpyAsync(ctx->ui, src, sizeof(int) * n * planes, kind, st));
-            LAUNCH(launch_gather_i(dst, ctx->ui, ctx->uperm, (int)n, planes, grd, blk, st));
-        } else {
-            CK(cudaMemsetAsync(dst, fill == 0 ? 0 : 0xff, sizeof(int) * n * planes, st));
-        }
-        return BMXG_OK;
+    auto fd = [&](const double *src) { return static_cast<const double *>(field(src, sizeof(double) * n, 8)); };
+    auto fi = [&](const int32_t *src, int planes) {
+        return static_cast<const int *>(field(src, sizeof(int) * n * planes, 4));
     };
-    if ((rc = up_d(p->velx, S.vx, 0.0))) return rc;
-    if ((rc = up_d(p->vely, S.vy, 0.0))) return rc;
-    if ((rc = up_d(p->velz, S.vz, 0.0))) return rc;
-    if ((rc = up_d(p->wx, S.wx, 0.0))) return rc;
-    if ((rc = up_d(p->wy, S.wy, 0.0))) return rc;
-    if ((rc = up_d(p->wz, S.wz, 0.0))) return rc;
+    const double *const vel[6] = {fd(p->velx), fd(p->vely), fd(p->velz), fd(p->wx), fd(p->wy), fd(p->wz)};
+    if (rc) return rc;
+    LAUNCH(launch_load_slots(S, src_x, src_y, src_z, src_r, src_ct, vel, S.col[1], S.iz[1], ctx->uperm, grd, blk,
+                             st));
     if (rods) {
-        if ((rc = up_d(p->c_length, S.clen, 0.0))) return rc;
-        if ((rc = up_d(p->area, S.area, 0.0))) return rc;
-        if ((rc = up_d(p->bond_scale, S.bscale, 1.0))) return rc;
-        if ((rc = up_d(p->theta, S.theta[0], 0.0))) return rc;
-        if ((rc = up_d(p->phi, S.phi[0], 0.0))) return rc;
-        if ((rc = up_i(p->id, S.id, 1, 0))) return rc;
-        if ((rc = up_i(p->cpu, S.cpu, 1, 0))) return rc;
-        if ((rc = up_i(p->fuse_tip, S.fuse_tip, 1, 0))) return rc;
-        if ((rc = up_i(p->position, S.position, 1, 0))) return rc;
-        if ((rc = up_i(p->fix_site, S.fix_site, 1, 0))) return rc;
-        if ((rc = up_i(p->fuse_flag, S.fflag, 1, 0))) return rc;
-        if ((rc = up_i(p->split_flag, S.sflag, 1, 0))) return rc;
-        if ((rc = up_i(p->new_flag, S.nflag, 1, 0))) return rc;
-        if ((rc = up_i(p->dltd, S.dltd, 6, -1))) return rc;
-        // bond table planes: n_bnds, ids[4], cpus[4], sites[4]
-        if ((rc = up_i(p->n_bnds, S.tab[0], 1, 0))) return rc;
-        if ((rc = up_i(p->seg_id1, S.tab[0] + n, 4, 0))) return rc;
-        if ((rc = up_i(p->seg_id2, S.tab[0] + 5 * n, 4, 0))) return rc;
-        if ((rc = up_i(p->site, S.tab[0] + 9 * n, 4, 0))) return rc;
-        LAUNCH(launch_trig(S, 0, grd, blk, st));
-        LAUNCH(launch_rod_mobility(S, dev_params(ctx->prm), grd, blk, st));
+        const RodFields F{fd(p->c_length), fd(p->area), fd(p->bond_scale), fd(p->theta), fd(p->phi),
+                          fi(p->id, 1), fi(p->cpu, 1), fi(p->fuse_tip, 1), fi(p->position, 1), fi(p->fix_site, 1),
+                          fi(p->fuse_flag, 1), fi(p->split_flag, 1), fi(p->new_flag, 1), fi(p->dltd, 6),
+                          fi(p->n_bnds, 1), fi(p->seg_id1, 4), fi(p->seg_id2, 4), fi(p->site, 4)};
+        if (rc) return rc;
+        const int rblk = 128;
+        LAUNCH(launch_load_rods(S, dev_params(ctx->prm), F, ctx->uperm, (int)((n + rblk - 1) / rblk), rblk, st));
     }
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(ctx->h_cnt, ctx->d_cnt, sizeof(DevCounters), cudaMemcpyDeviceToHost, st));
@@ -797,6 +814,112 @@ int bmxg_set_state(bmxg_ctx *ctx, const bmxg_particles *p, const int64_t *colony
     return BMXG_OK;
 }
 
+// The check's read-back (h_chk) as a StateCheck.
+int read_check(bmxg_ctx *ctx, StateCheck *out)
+{
+    const unsigned long long *h = ctx->h_chk;
+    if (h[0]) return fail(ctx, BMXG_ERR_ARG, "cell_type must be 0 or 1");
+    out->rods = h[1] != 0;
+    const uint64_t rb = h[2];
+    std::memcpy(&out->rmax, &rb, sizeof(out->rmax));
+    if (h[3]) out->rmax = std::nan("");
+    return BMXG_OK;
+}
+
+// Cell types, presence of rods and the largest radius of device arrays in
+// caller order (synchronises the stream).
+int check_state(bmxg_ctx *ctx, const int *ct, const double *r, int64_t n, StateCheck *out)
+{
+    cudaStream_t st = ctx->stream;
+    CK(cudaMemsetAsync(ctx->d_chk, 0, 4 * sizeof(unsigned long long), st));
+    Shape sh;
+    LAUNCH(launch_check_state(ct, r, (int)n, ctx->d_chk, grid_for(ctx, sh, n), sh.block, st));
+    CK(cudaMemcpyAsync(ctx->h_chk, ctx->d_chk, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
+    const cudaError_t e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) return fail(ctx, BMXG_ERR_CUDA, std::string("state check: ") + cudaGetErrorString(e));
+    return read_check(ctx, out);
+}
+
+constexpr int64_t kStoreFused = 65536;
+
+// bmxg_get_state through one kernel: straight into device arrays, or into the
+// staging and from there into host arrays.
+int store_fused(bmxg_ctx *ctx, bmxg_particles *p, bool host, bool fx)
+{
+    const int64_t n = ctx->n;
+    const DevState &S = ctx->S;
+    cudaStream_t st = ctx->stream;
+    struct Out {
+        void *dst;
+        char *from;
+        size_t bytes;
+    };
+    std::vector<Out> outs;
+    size_t used = 0;
+    // spheres have no rod fields (those arrays are left alone)
+    const bool rods = S.has_rods != 0;
+    struct Want {
+        void *dst;
+        size_t bytes;
+    };
+    const size_t d8 = sizeof(double) * (size_t)n, i4 = sizeof(int) * (size_t)n;
+    Want w[] = {{p->x, d8},          {p->y, d8},         {p->z, d8},
+                {p->velx, d8},       {p->vely, d8},      {p->velz, d8},
+                {p->wx, d8},         {p->wy, d8},        {p->wz, d8},
+                {rods ? p->theta : nullptr, d8},         {rods ? p->phi : nullptr, d8},
+                {rods ? p->n_bnds : nullptr, i4},        {rods ? p->seg_id1 : nullptr, 4 * i4},
+                {rods ? p->seg_id2 : nullptr, 4 * i4},   {rods ? p->site : nullptr, 4 * i4},
+                {rods ? p->position : nullptr, i4},      {rods ? p->fix_site : nullptr, i4},
+                {rods ? p->fuse_flag : nullptr, i4},     {rods ? p->split_flag : nullptr, i4},
+                {rods ? p->new_flag : nullptr, i4},      {rods ? p->dltd : nullptr, 6 * i4}};
+    if (host) {
+        for (const Want &q : w)
+            if (q.dst) used += (q.bytes + 15) / 16 * 16;
+        if (int rc = ensure_io(ctx, used)) return rc;
+        used = 0;
+    }
+    void *at[sizeof(w) / sizeof(w[0])];
+    for (size_t k = 0; k < sizeof(w) / sizeof(w[0]); ++k) {
+        at[k] = w[k].dst;
+        if (!host || !w[k].dst) continue;
+        at[k] = ctx->io_buf + used;
+        outs.push_back({w[k].dst, ctx->io_buf + used, w[k].bytes});
+        used += (w[k].bytes + 15) / 16 * 16;
+    }
+    StoreFields F;
+    F.x = (double *)at[0];
+    F.y = (double *)at[1];
+    F.z = (double *)at[2];
+    for (int k = 0; k < 6; ++k) F.v[k] = (double *)at[3 + k];
+    F.theta = (double *)at[9];
+    F.phi = (double *)at[10];
+    F.n_bnds = (int *)at[11];
+    F.seg_id1 = (int *)at[12];
+    F.seg_id2 = (int *)at[13];
+    F.site = (int *)at[14];
+    F.position = (int *)at[15];
+    F.fix_site = (int *)at[16];
+    F.fflag = (int *)at[17];
+    F.sflag = (int *)at[18];
+    F.nflag = (int *)at[19];
+    F.dltd = (int *)at[20];
+    LAUNCH(launch_store(S, ctx->parity, F, fx, ctx->vel32, st));
+    if (fx) ctx->fx_ahead = false;
+    for (const Out &o : outs) CK(cudaMemcpyAsync(o.dst, o.from, o.bytes, cudaMemcpyDeviceToHost, st));
+    if (!rods && ctx->stepped)  // a step of spheres only clears the fusion flags (bmx_pc_interaction.cpp:178-180)
+        for (int32_t *f : {p->fuse_flag, p->split_flag, p->new_flag}) {
+            if (!f) continue;
+            if (host) std::memset(f, 0, i4);
+            else CK(cudaMemsetAsync(f, 0, i4, st));
+        }
+    CK(cudaStreamSynchronize(st));
+    return BMXG_OK;
+}
+
+}  // namespace
+
+extern "C" {
+
 int bmxg_get_state(bmxg_ctx *ctx, bmxg_particles *p, int where)
 {
     if (!ctx) return BMXG_ERR_ARG;
@@ -804,10 +927,9 @@ int bmxg_get_state(bmxg_ctx *ctx, bmxg_particles *p, int where)
     if (!ctx->have_state) return fail(ctx, BMXG_ERR_STATE, "no state loaded");
     if (!p || p->n != ctx->n) return fail(ctx, BMXG_ERR_ARG, "particle count differs from the loaded state");
     if (where != BMXG_HOST && where != BMXG_DEVICE) return fail(ctx, BMXG_ERR_ARG, "bad `where`");
-    // positions still in the list's fixed point: host arrays asking for x, y
-    // and z get each axis converted as it is stored (one pass instead of a
-    // conversion and a scatter); otherwise all three are converted first
-    const bool fx_store = ctx->fx_ahead && where == BMXG_HOST && p->x && p->y && p->z;
+    // positions still in the list's fixed point are converted as they are
+    // stored, where all three axes are asked for; otherwise first
+    const bool fx_store = ctx->fx_ahead && p->x && p->y && p->z;
     if (!fx_store) {
         if (int rc = sync_fp64(ctx)) return rc;
     }
@@ -819,36 +941,36 @@ int bmxg_get_state(bmxg_ctx *ctx, bmxg_particles *p, int where)
     const int blk = ctx->sh_misc.block;
     const int grd = grid_for(ctx, ctx->sh_misc, n);
     const int a = ctx->parity;
-    // Device arrays receive the caller-order scatter directly.  Host arrays:
-    // each field is scattered into one of two staging halves on the compute
-    // stream and copied out on the copy stream, so that the copy of one field
-    // overlaps the scatter of the next.
+    // Device arrays receive the caller-order scatter directly, every field in
+    // one kernel.  Host arrays of rod states and of few particles go through
+    // the same kernel into the staging, then out field by field; of many
+    // spheres: each field is scattered into one of two staging halves on the
+    // compute stream and copied out on the copy stream, so that the copy of one
+    // field overlaps the scatter of the next (500 000 spheres: six scatters of
+    // 6 us behind copies of 21 us; below kStoreFused the launches cost more).
+    if (!host || S.has_rods || n <= kStoreFused) return store_fused(ctx, p, host, fx_store);
     JoinIo join{nullptr};
     int used = 0;
-    const bool pipe = host;  // (copies on `st` instead measured slower at every size)
-    if (host) {
+    {
         int rc0 = ensure_io(ctx, (size_t)n * 48 + 256);
         if (rc0) return rc0;
     }
-    if (pipe) {
-        CK(cudaEventRecord(ctx->io_ev[0], st));
-        CK(cudaStreamWaitEvent(st1, ctx->io_ev[0], 0));
-        join.s = st1;
-    }
+    CK(cudaEventRecord(ctx->io_ev[0], st));
+    CK(cudaStreamWaitEvent(st1, ctx->io_ev[0], 0));
+    join.s = st1;
     char *half[2] = {ctx->io_buf, ctx->io_buf + (size_t)n * 24 + 128};
     // destination of the next field: the caller's array or a staging half
     cudaError_t wait_err = cudaSuccess;
     auto begin = [&](void *dst) -> void * {
-        if (!host) return dst;
+        (void)dst;
         const int h = used & 1;
-        if (pipe && used >= 2) {  // the half's previous copy-out is done
+        if (used >= 2) {  // the half's previous copy-out is done
             const cudaError_t e = cudaStreamWaitEvent(st, ctx->io_ev[4 + h], 0);
             if (e != cudaSuccess) wait_err = e;
         }
         return half[h];
     };
     auto finish = [&](void *dst, size_t bytes) -> int {
-        if (!host) return BMXG_OK;
         CK(wait_err);
         const int h = used & 1;
         CK(cudaEventRecord(ctx->io_ev[2 + h], st));
@@ -863,12 +985,6 @@ int bmxg_get_state(bmxg_ctx *ctx, bmxg_particles *p, int where)
         double *o = (double *)begin(dst);
         LAUNCH(launch_scatter_d(o, src, S.orig, (int)n, grd, blk, st));
         return finish(dst, sizeof(double) * n);
-    };
-    auto out_i = [&](int32_t *dst, const int *src, int planes) -> int {
-        if (!dst || !src) return BMXG_OK;
-        int *o = (int *)begin(dst);
-        LAUNCH(launch_scatter_i(o, src, S.orig, (int)n, planes, grd, blk, st));
-        return finish(dst, sizeof(int) * n * planes);
     };
     auto out_f = [&](double *dst, const float *src) -> int {  // FP32F velocities, widened
         if (!dst || !src) return BMXG_OK;
@@ -902,29 +1018,13 @@ int bmxg_get_state(bmxg_ctx *ctx, bmxg_particles *p, int where)
     if ((rc = out_d(p->wx, S.wx))) return rc;
     if ((rc = out_d(p->wy, S.wy))) return rc;
     if ((rc = out_d(p->wz, S.wz))) return rc;
-    if (S.has_rods) {
-        if ((rc = out_d(p->theta, S.theta[a]))) return rc;
-        if ((rc = out_d(p->phi, S.phi[a]))) return rc;
-        if ((rc = out_i(p->n_bnds, S.tab[a], 1))) return rc;
-        if ((rc = out_i(p->seg_id1, S.tab[a] + n, 4))) return rc;
-        if ((rc = out_i(p->seg_id2, S.tab[a] + 5 * n, 4))) return rc;
-        if ((rc = out_i(p->site, S.tab[a] + 9 * n, 4))) return rc;
-        if ((rc = out_i(p->position, S.position, 1))) return rc;
-        if ((rc = out_i(p->fix_site, S.fix_site, 1))) return rc;
-        if ((rc = out_i(p->fuse_flag, S.fflag, 1))) return rc;
-        if ((rc = out_i(p->split_flag, S.sflag, 1))) return rc;
-        if ((rc = out_i(p->new_flag, S.nflag, 1))) return rc;
-        if ((rc = out_i(p->dltd, S.dltd, 6))) return rc;
-    } else if (ctx->stepped && where == BMXG_HOST) {
+    if (ctx->stepped) {
         // spheres: the step only clears the fusion flags (bmx_pc_interaction.cpp:178-180)
         for (int32_t *f : {p->fuse_flag, p->split_flag, p->new_flag})
             if (f) std::memset(f, 0, sizeof(int32_t) * n);
-    } else if (ctx->stepped) {
-        for (int32_t *f : {p->fuse_flag, p->split_flag, p->new_flag})
-            if (f) CK(cudaMemsetAsync(f, 0, sizeof(int32_t) * n, st));
     }
     CK(cudaStreamSynchronize(st));
-    if (pipe) CK(cudaStreamSynchronize(st1));
+    CK(cudaStreamSynchronize(st1));
     return BMXG_OK;
 }
 
@@ -1386,6 +1486,67 @@ int bmxg_evolve_particles(bmxg_ctx *ctx, double dt, double *cost_per_colony, int
     if (nsubsteps) *nsubsteps = 1;
     if (cost_per_colony)  // "NumParticles" knapsack weight (bmx_pc_interaction.cpp:470-473)
         for (int c = 0; c < ctx->ncol; ++c) cost_per_colony[c] = (double)(ctx->offsets[c + 1] - ctx->offsets[c]);
+    return BMXG_OK;
+}
+
+int bmxg_evolve_particles_aos(bmxg_ctx *ctx, void *particles, int64_t n, int32_t nreal, int32_t nint,
+                              const int64_t *colony_offsets, double dt, double *cost_per_colony, int32_t *nsubsteps)
+{
+    if (!ctx || n < 0 || (n > 0 && !particles)) return BMXG_ERR_ARG;
+    if (nreal <= 24 || nint <= 34) return BMXG_ERR_ARG;  // up to bond_scale and cpu (bmx_chem.H:38-118)
+    AosLayout L;
+    L.rdata = 3 * sizeof(double);
+    L.idata = L.rdata + (size_t)nreal * sizeof(double) + 2 * sizeof(int);
+    L.stride = (L.idata + (size_t)nint * sizeof(int) + 7) / 8 * 8;
+    bmxg_particles s;
+    std::memset(&s, 0, sizeof(s));
+    s.n = n;
+    if (n == 0 || n > (1LL << 30)) return bmxg_set_state(ctx, &s, colony_offsets, BMXG_DEVICE);  // (refused there)
+    (void)cudaGetLastError();
+    cudaStream_t st = ctx->stream;
+    // the records in place where the device reads the host's pages, else staged whole
+    const size_t N = (size_t)n;
+    const bool in_place = ctx->pageable && (reinterpret_cast<uintptr_t>(particles) & 7u) == 0;
+    const size_t planes = N * (15 * sizeof(double) + 28 * sizeof(int));
+    const size_t rec_at = (planes + 255) / 256 * 256;
+    const size_t need = rec_at + (in_place ? 0 : N * L.stride);
+    if (need > ctx->aos_cap) {
+        CK(cudaStreamSynchronize(st));
+        if (ctx->aos_buf) cudaFree(ctx->aos_buf);
+        ctx->aos_buf = nullptr;
+        ctx->aos_cap = 0;
+        CK(cudaMalloc(&ctx->aos_buf, need));
+        ctx->aos_cap = need;
+    }
+    unsigned char *rec = in_place ? static_cast<unsigned char *>(particles)
+                                  : reinterpret_cast<unsigned char *>(ctx->aos_buf + rec_at);
+    if (!in_place) CK(cudaMemcpyAsync(rec, particles, N * L.stride, cudaMemcpyHostToDevice, st));
+    double *d = reinterpret_cast<double *>(ctx->aos_buf);
+    int *q = reinterpret_cast<int *>(d + 15 * N);
+    // the first record's type says which fields to expect (the check decides)
+    int32_t first = 0;
+    std::memcpy(&first, static_cast<const unsigned char *>(particles) + L.idata + 5 * sizeof(int), sizeof(first));
+    const bool guess = first == BMXG_FUNGI;
+    LAUNCH(launch_aos_load(rec, L, (int)n, guess, d, q, st));
+    StateCheck chk;
+    if (int rc = check_state(ctx, q, d + 3 * N, n, &chk)) return rc;
+    if (chk.rods && !guess) LAUNCH(launch_aos_load(rec, L, (int)n, true, d, q, st));
+    s.x = d; s.y = d + N; s.z = d + 2 * N; s.radius = d + 3 * N;
+    s.velx = d + 9 * N; s.vely = d + 10 * N; s.velz = d + 11 * N;
+    s.wx = d + 12 * N; s.wy = d + 13 * N; s.wz = d + 14 * N;
+    s.cell_type = q;
+    if (chk.rods) {
+        s.c_length = d + 4 * N; s.theta = d + 5 * N; s.phi = d + 6 * N; s.area = d + 7 * N; s.bond_scale = d + 8 * N;
+        s.id = q + N; s.cpu = q + 2 * N; s.n_bnds = q + 3 * N;
+        s.seg_id1 = q + 4 * N; s.seg_id2 = q + 8 * N; s.site = q + 12 * N;
+        s.position = q + 16 * N; s.fuse_tip = q + 17 * N; s.fix_site = q + 18 * N;
+        s.fuse_flag = q + 19 * N; s.split_flag = q + 20 * N; s.new_flag = q + 21 * N; s.dltd = q + 22 * N;
+    }
+    if (int rc = load_state(ctx, &s, colony_offsets, BMXG_DEVICE, &chk)) return rc;
+    if (int rc = bmxg_evolve_particles(ctx, dt, cost_per_colony, nsubsteps)) return rc;
+    LAUNCH(launch_aos_store(rec, L, ctx->S, ctx->parity, st));
+    if (!in_place) CK(cudaMemcpyAsync(particles, rec, N * L.stride, cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
     return BMXG_OK;
 }
 

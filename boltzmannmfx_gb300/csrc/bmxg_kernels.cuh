@@ -165,9 +165,39 @@ int launch_rebuild(const DevState &S, int b, int *scan_scratch, int grid, int bl
 
 // positions, radii, cell types, bins, offsets and identity column order of a
 // freshly sorted state (buffer 0), gathered from the caller-order arrays
+// (v: the six velocity fields, caller order; null: zeros)
 int launch_load_slots(const DevState &S, const double *ux, const double *uy, const double *uz, const double *ur,
-                      const int *uct, const int *ucol, const int *uiz, const int *uperm, int grid, int block,
-                      cudaStream_t st);
+                      const int *uct, const double *const v[6], const int *ucol, const int *uiz, const int *uperm,
+                      int grid, int block, cudaStream_t st);
+// The fields of rod segments in caller order (device arrays; null: the field's
+// default), gathered into slot order with the segments' trig and mobility.
+struct RodFields {
+    const double *clen, *area, *bscale, *theta, *phi;
+    const int *id, *cpu, *fuse_tip, *position, *fix_site, *fflag, *sflag, *nflag, *dltd, *n_bnds, *seg_id1, *seg_id2,
+        *site;
+};
+int launch_load_rods(const DevState &S, const DevParams &P, const RodFields &F, const int *uperm, int grid, int block,
+                     cudaStream_t st);
+// The state of buffer a scattered to caller order in one pass, the fields asked
+// for (null: not).  fx: the positions come from the list's fixed point (the FP64
+// ones are written too); vel32: the velocities from the FP32F planes.
+struct StoreFields {
+    double *x, *y, *z, *v[6], *theta, *phi;
+    int *n_bnds, *seg_id1, *seg_id2, *site, *position, *fix_site, *fflag, *sflag, *nflag, *dltd;
+};
+int launch_store(const DevState &S, int a, const StoreFields &F, bool fx, bool vel32, cudaStream_t st);
+// AoS records (k_io.cu): bytes per record, of rdata and idata in a record
+struct AosLayout {
+    size_t stride, rdata, idata;
+};
+// The records' fields into planes in caller order: 15 of doubles (x, y, z,
+// radius, c_length, theta, phi, area, bond_scale, velx .. wz), 28 of ints
+// (cell_type, id, cpu, n_bnds, seg_id1[4], seg_id2[4], site[4], position,
+// fuse_tip, fix_site, fuse_flag, split_flag, new_flag, dltd[6]).  Without rods
+// only the fields of spheres (the first four, the velocities, cell_type).
+int launch_aos_load(const unsigned char *rec, const AosLayout &L, int n, bool rods, double *d, int *i, cudaStream_t st);
+// What a step writes, from buffer a into the records.
+int launch_aos_store(unsigned char *rec, const AosLayout &L, const DevState &S, int a, cudaStream_t st);
 // *diff |= 1 when a given field (null: not compared) differs bit for bit from
 // the device state of buffer a (slot s against caller index orig[s])
 int launch_same_state(const DevState &S, int a, const double *x, const double *y, const double *z, const double *r,
@@ -184,12 +214,9 @@ int launch_user_bin(const DevState &S, const double *ux, const double *uy, const
 int launch_user_sort(const DevState &S, const int *ucol, const int *uiz, int *colstart, int *scan_scratch,
                      int *uperm, int grid, int block, cudaStream_t st);
 int launch_gather_d(double *dst, const double *src, const int *perm, int n, int grid, int block, cudaStream_t st);
-int launch_gather_i(int *dst, const int *src, const int *perm, int n, int planes, int grid, int block, cudaStream_t st);
 int launch_scatter_d(double *dst, const double *src, const int *orig, int n, int grid, int block, cudaStream_t st);
 int launch_scatter_f2d(double *dst, const float *src, const int *orig, int n, int grid, int block,
                        cudaStream_t st);
-int launch_scatter_i(int *dst, const int *src, const int *orig, int n, int planes, int grid, int block, cudaStream_t st);
-int launch_trig(const DevState &S, int b, int grid, int block, cudaStream_t st);
 
 // neighbour-list export (k_bin.cu): mode 0 counts per caller index, mode 1 fills
 int launch_pairs(const DevState &S, const DevParams &P, int a, int64_t *cnt_or_offs, int *idx,

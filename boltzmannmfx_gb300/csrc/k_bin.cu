@@ -368,14 +368,6 @@ __global__ void k_gather_d(double *dst, const double *src, const int *perm, int 
         dst[s] = src[perm[s]];
 }
 
-__global__ void k_gather_i(int *dst, const int *src, const int *perm, int n, int planes)
-{
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) {
-        const int u = perm[s];
-        for (int k = 0; k < planes; ++k) dst[(size_t)k * n + s] = src[(size_t)k * n + u];
-    }
-}
-
 __global__ void k_scatter_d(double *dst, const double *src, const int *orig, int n)
 {
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x)
@@ -386,25 +378,6 @@ __global__ void k_scatter_f2d(double *dst, const float *src, const int *orig, in
 {
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x)
         dst[orig[s]] = (double)src[s];
-}
-
-__global__ void k_scatter_i(int *dst, const int *src, const int *orig, int n, int planes)
-{
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) {
-        const int u = orig[s];
-        for (int k = 0; k < planes; ++k) dst[(size_t)k * n + u] = src[(size_t)k * n + s];
-    }
-}
-
-__global__ void k_trig(const DevState S, int b)
-{
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < S.n; i += gridDim.x * blockDim.x) {
-        const double th = S.theta[b][i], ph = S.phi[b][i];
-        double st, ct, sp, cp;
-        sincos(th, &st, &ct);
-        sincos(ph, &sp, &cp);
-        S.trig[b][i] = make_trig(ct, st, cp, sp);
-    }
 }
 
 // Neighbour list of every slot in the reference's order; indices and counts
@@ -512,9 +485,15 @@ __global__ void k_user_canon(const DevState S, const int *ucol, const int *uiz, 
 // position, radius and cell type are gathered from the caller-order arrays,
 // its bins are the caller-order bins of the sort, its column order is the
 // sort's (perm = identity, colstart = the sort's offsets, copied by the
-// caller), and its offsets and counters are place_slot's.
+// caller), and its offsets and counters are place_slot's.  Velocities the caller
+// gives are gathered, the others zero.
+struct VelSrc {
+    const double *v[6];
+};
+
 __global__ void k_load_slots(const DevState S, const double *ux, const double *uy, const double *uz,
-                             const double *ur, const int *uct, const int *ucol, const int *uiz, const int *uperm)
+                             const double *ur, const int *uct, const VelSrc V, const int *ucol, const int *uiz,
+                             const int *uperm)
 {
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < S.n; s += gridDim.x * blockDim.x) {
         const DevGeom &G = geom_of(S, s);
@@ -526,6 +505,12 @@ __global__ void k_load_slots(const DevState S, const double *ux, const double *u
         S.rad[s] = r;
         S.ctype[s] = (int8_t)uct[u];
         S.orig[s] = u;
+        S.vx[s] = V.v[0] ? V.v[0][u] : 0.0;
+        S.vy[s] = V.v[1] ? V.v[1][u] : 0.0;
+        S.vz[s] = V.v[2] ? V.v[2][u] : 0.0;
+        S.wx[s] = V.v[3] ? V.v[3][u] : 0.0;
+        S.wy[s] = V.v[4] ? V.v[4][u] : 0.0;
+        S.wz[s] = V.v[5] ? V.v[5][u] : 0.0;
         int bx, by;
         col_to_bxy(G, ucol[u], bx, by);
         const int bz = uiz[u];
@@ -542,10 +527,11 @@ __global__ void k_load_slots(const DevState S, const double *ux, const double *u
 }  // namespace
 
 int launch_load_slots(const DevState &S, const double *ux, const double *uy, const double *uz, const double *ur,
-                      const int *uct, const int *ucol, const int *uiz, const int *uperm, int grid, int block,
-                      cudaStream_t st)
+                      const int *uct, const double *const v[6], const int *ucol, const int *uiz, const int *uperm,
+                      int grid, int block, cudaStream_t st)
 {
-    k_load_slots<<<grid, block, 0, st>>>(S, ux, uy, uz, ur, uct, ucol, uiz, uperm);
+    const VelSrc V{{v[0], v[1], v[2], v[3], v[4], v[5]}};
+    k_load_slots<<<grid, block, 0, st>>>(S, ux, uy, uz, ur, uct, V, ucol, uiz, uperm);
     return 1;
 }
 
@@ -679,13 +665,6 @@ int launch_gather_d(double *dst, const double *src, const int *perm, int n, int 
     return 1;
 }
 
-int launch_gather_i(int *dst, const int *src, const int *perm, int n, int planes, int grid, int block,
-                     cudaStream_t st)
-{
-    k_gather_i<<<grid, block, 0, st>>>(dst, src, perm, n, planes);
-    return 1;
-}
-
 int launch_scatter_d(double *dst, const double *src, const int *orig, int n, int grid, int block,
                       cudaStream_t st)
 {
@@ -697,19 +676,6 @@ int launch_scatter_f2d(double *dst, const float *src, const int *orig, int n, in
                        cudaStream_t st)
 {
     k_scatter_f2d<<<grid, block, 0, st>>>(dst, src, orig, n);
-    return 1;
-}
-
-int launch_scatter_i(int *dst, const int *src, const int *orig, int n, int planes, int grid, int block,
-                      cudaStream_t st)
-{
-    k_scatter_i<<<grid, block, 0, st>>>(dst, src, orig, n, planes);
-    return 1;
-}
-
-int launch_trig(const DevState &S, int b, int grid, int block, cudaStream_t st)
-{
-    k_trig<<<grid, block, 0, st>>>(S, b);
     return 1;
 }
 

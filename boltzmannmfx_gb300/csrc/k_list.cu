@@ -41,6 +41,7 @@
 // are L2-resident.  HBM bound, no contraction.
 #include <algorithm>
 
+#include "bmxg_fx.cuh"
 #include "bmxg_stencil.cuh"
 
 namespace bmxg {
@@ -84,11 +85,6 @@ __device__ __forceinline__ long long fx_inc(float f, float c, float cl, bool &bi
     // instruction on GB300) fewer
     if (fabsf(p) < 1.8014398509481984e16f) return __float2ll_rn(p) + (long long)__float2int_rn(r);  // 2^54
     return __float2ll_rn(p) + __float2ll_rn(r);
-}
-
-__device__ __forceinline__ unsigned long long fx_join(unsigned h, unsigned l)
-{
-    return ((unsigned long long)h << 32) | l;
 }
 
 // The bound: for any pair, the separation change since the build is, per
@@ -700,52 +696,6 @@ __device__ __forceinline__ unsigned long long to_fx(double x, const FxGeom &F, i
     if (F.per[ax]) return neg ? 0ull - X : X;  // the unsigned wrap is the periodic wrap
     if (neg) return 0ull;
     return over ? ~0ull : X;
-}
-
-// x of a fixed-point coordinate: o + X span / 2^64, the product X ms 2^(es - 64)
-// rounded to nearest even once (then the FP64 addition of a non-zero origin);
-// a periodic coordinate is kept below phi.
-__device__ __forceinline__ double from_fx(unsigned long long X, const FxGeom &F, int ax)
-{
-    const unsigned long long ms = F.ms[ax];
-    const unsigned long long hi = __umul64hi(X, ms), lo = X * ms;
-    unsigned long long t, rest;
-    int E;  // value = t 2^E with t in [2^63, 2^64), rest the bits below t
-    if (hi) {
-        const int lz = __clzll((long long)hi);
-        t = lz ? ((hi << lz) | (lo >> (64 - lz))) : hi;
-        rest = lo << lz;
-        E = F.es[ax] - lz;
-    } else if (lo) {
-        const int lz = __clzll((long long)lo);
-        t = lo << lz;
-        rest = 0ull;
-        E = F.es[ax] - 64 - lz;
-    } else {
-        t = 0ull;
-        rest = 0ull;
-        E = 0;
-    }
-    double v = 0.0;
-    if (t) {
-        unsigned long long m = t >> 11;
-        const unsigned long long rb = (t >> 10) & 1ull;
-        const bool sticky = (t & 0x3ffull) != 0ull || rest != 0ull;
-        m += rb & ((sticky ? 1ull : 0ull) | (m & 1ull));
-        if (m >> 53) {
-            m >>= 1;
-            ++E;
-        }
-        v = __longlong_as_double((long long)((((unsigned long long)(E + 1086)) << 52) | (m & 0xfffffffffffffull)));
-    }
-    if (F.ozero[ax]) {
-        // (periodic with plo = 0: v < len unless rounding reached it)
-        if (F.per[ax] && !(v < F.phi[ax])) v = nextafter(F.phi[ax], 0.0);
-        return v;
-    }
-    double x = F.o[ax] + v;
-    if (F.per[ax] && !(x < F.phi[ax])) x = nextafter(F.phi[ax], -1.0e300);
-    return x;
 }
 
 // Fixed-point positions of buffer a from its FP64 positions and the radii

@@ -364,26 +364,72 @@ __global__ void k_rod_book(const DevState S, const DevParams P, int a)
 // force gather applies, (d0 + db, da - db, (d0 - db) / 2), each the FP64
 // expression the gather evaluated per step before; none of the inputs changes
 // during a step, so it runs when a state or the parameters load.
+__device__ __forceinline__ double4_32a rod_mobility(int ctype, double Li, double sarea, const DevParams &P)
+{
+    double4_32a m = make_trig(0.0, 0.0, 0.0, 0.0);
+    if (ctype == kFungi) {
+        const double area = sarea / 2.0;
+        const double arad = sqrt(area / (4.0 * kPi));
+        const double d0 = 1.0 / (6.0 * kPi * arad * P.visc);
+        double da, db;
+        if (Li > 2.0 * arad) {
+            da = (Li * Li - 2.0 * arad * arad / 3.0) / (4.0 * kPi * pow(Li, 3.0) * P.visc);
+            db = (Li * Li + 2.0 * arad * arad / 3.0) / (8.0 * kPi * pow(Li, 3.0) * P.visc);
+        } else {
+            da = (1.0 - 3.0 * Li / (16.0 * arad)) / (6.0 * kPi * arad * P.visc);
+            db = (1.0 - 9.0 * Li / (32.0 * arad)) / (6.0 * kPi * arad * P.visc);
+        }
+        m = make_trig(d0 + db, da - db, 0.5 * (d0 - db), 0.0);
+    }
+    return m;
+}
+
 __global__ void k_rod_mobility(const DevState S, const DevParams P)
 {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < S.n; i += gridDim.x * blockDim.x) {
-        double4_32a m = make_trig(0.0, 0.0, 0.0, 0.0);
-        if (S.ctype[i] == kFungi) {
-            const double Li = S.clen[i];
-            const double area = S.area[i] / 2.0;
-            const double arad = sqrt(area / (4.0 * kPi));
-            const double d0 = 1.0 / (6.0 * kPi * arad * P.visc);
-            double da, db;
-            if (Li > 2.0 * arad) {
-                da = (Li * Li - 2.0 * arad * arad / 3.0) / (4.0 * kPi * pow(Li, 3.0) * P.visc);
-                db = (Li * Li + 2.0 * arad * arad / 3.0) / (8.0 * kPi * pow(Li, 3.0) * P.visc);
-            } else {
-                da = (1.0 - 3.0 * Li / (16.0 * arad)) / (6.0 * kPi * arad * P.visc);
-                db = (1.0 - 9.0 * Li / (32.0 * arad)) / (6.0 * kPi * arad * P.visc);
-            }
-            m = make_trig(d0 + db, da - db, 0.5 * (d0 - db), 0.0);
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < S.n; i += gridDim.x * blockDim.x)
+        S.mob[i] = rod_mobility(S.ctype[i], S.clen[i], S.area[i], P);
+}
+
+// The segments' fields of a load, gathered into slot order in one pass (18
+// fields: one launch instead of a copy and a gather each), with the trig of
+// the angles and the mobility.
+__global__ void __launch_bounds__(128) k_load_rods(const DevState S, const DevParams P, const RodFields F,
+                                                   const int *__restrict__ uperm)
+{
+    const size_t n = (size_t)S.n;
+    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < S.n; s += gridDim.x * blockDim.x) {
+        const int u = uperm[s];
+        const double L = F.clen ? F.clen[u] : 0.0, area = F.area ? F.area[u] : 0.0;
+        const double th = F.theta ? F.theta[u] : 0.0, ph = F.phi ? F.phi[u] : 0.0;
+        S.clen[s] = L;
+        S.area[s] = area;
+        S.bscale[s] = F.bscale ? F.bscale[u] : 1.0;
+        S.theta[0][s] = th;
+        S.phi[0][s] = ph;
+        S.id[s] = F.id ? F.id[u] : 0;
+        S.cpu[s] = F.cpu ? F.cpu[u] : 0;
+        S.fuse_tip[s] = F.fuse_tip ? F.fuse_tip[u] : 0;
+        S.position[s] = F.position ? F.position[u] : 0;
+        S.fix_site[s] = F.fix_site ? F.fix_site[u] : 0;
+        S.fflag[s] = F.fflag ? F.fflag[u] : 0;
+        S.sflag[s] = F.sflag ? F.sflag[u] : 0;
+        S.nflag[s] = F.nflag ? F.nflag[u] : 0;
+#pragma unroll
+        for (int k = 0; k < 6; ++k) S.dltd[k * n + s] = F.dltd ? F.dltd[k * n + u] : -1;
+        // bond table planes: n_bnds, ids[4], cpus[4], sites[4]
+        int *tab = S.tab[0];
+        tab[s] = F.n_bnds ? F.n_bnds[u] : 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            tab[(1 + k) * n + s] = F.seg_id1 ? F.seg_id1[k * n + u] : 0;
+            tab[(5 + k) * n + s] = F.seg_id2 ? F.seg_id2[k * n + u] : 0;
+            tab[(9 + k) * n + s] = F.site ? F.site[k * n + u] : 0;
         }
-        S.mob[i] = m;
+        double st, ct, sp, cp;
+        sincos(th, &st, &ct);
+        sincos(ph, &sp, &cp);
+        S.trig[0][s] = make_trig(ct, st, cp, sp);
+        S.mob[s] = rod_mobility(S.ctype[s], L, area, P);
     }
 }
 
@@ -1056,6 +1102,13 @@ int launch_exchange(const DevState &S, const DevParams &P, int a, const double *
 int launch_rod_mobility(const DevState &S, const DevParams &P, int grid, int block, cudaStream_t st)
 {
     k_rod_mobility<<<grid, block, 0, st>>>(S, P);
+    return 1;
+}
+
+int launch_load_rods(const DevState &S, const DevParams &P, const RodFields &F, const int *uperm, int grid, int block,
+                     cudaStream_t st)
+{
+    k_load_rods<<<grid, block, 0, st>>>(S, P, F, uperm);
     return 1;
 }
 
