@@ -131,6 +131,8 @@ struct bmxg_ctx {
     cudaEvent_t io_ev[8] = {};
     char *io_buf = nullptr;
     size_t io_cap = 0;
+    char *tile_buf = nullptr;               // workspace of the tile step, grown
+    size_t tile_cap = 0;
     char *aos_buf = nullptr;                // planes (and staged records) of the AoS entry point, grown
     size_t aos_cap = 0;
     bool pageable = false;                  // the device reads pageable host memory in place
@@ -476,6 +478,7 @@ void bmxg_destroy(bmxg_ctx *ctx)
         if (ev) cudaEventDestroy(ev);
     if (ctx->io_buf) cudaFree(ctx->io_buf);
     if (ctx->aos_buf) cudaFree(ctx->aos_buf);
+    if (ctx->tile_buf) cudaFree(ctx->tile_buf);
     if (ctx->d_chk) cudaFree(ctx->d_chk);
     if (ctx->h_chk) cudaFreeHost(ctx->h_chk);
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);
@@ -1599,6 +1602,8 @@ int bmxg_step_tile(bmxg_ctx *ctx, const bmxg_tile *tile, const bmxg_particles *r
         T.len[d] = g.prob_hi[d] - g.prob_lo[d];
         T.n[d] = g.n_cell[d];
         const double dx = T.len[d] / (double)T.n[d];  // the whole-domain step's bin width and inverse
+        T.dx[d] = dx;
+        T.dxf[d] = (float)dx;
         T.dxi[d] = 1.0 / dx;
         T.per[d] = g.is_periodic[d] ? 1 : 0;
         if (tile->lo[d] < 0 || tile->hi[d] < tile->lo[d] || tile->hi[d] >= T.n[d])
@@ -1611,73 +1616,112 @@ int bmxg_step_tile(bmxg_ctx *ctx, const bmxg_tile *tile, const bmxg_particles *r
     if (ncells >= (1LL << 30)) return fail(ctx, BMXG_ERR_UNSUPPORTED, "a tile of more than 2^30 cells");
     T.nbh_trivial = (ctx->prm.neighborhood >= diag2 * (1.0 + 1e-9)) ? 1 : 0;
     const int64_t nt = nr + ng;
+    const int ncols = (T.nt[0] + 2) * (T.nt[1] + 2);
     cudaStream_t st = ctx->stream;
-    // stream-ordered scratch for the call
-    std::vector<void *> mem;
-    auto alloc = [&](auto **p, size_t count) -> bool {
-        void *q = nullptr;
-        if (cudaMallocAsync(&q, std::max<size_t>(count, 1) * sizeof(**p), st) != cudaSuccess) return false;
-        mem.push_back(q);
-        *p = reinterpret_cast<std::remove_reference_t<decltype(*p)>>(q);
-        return true;
+    // device arrays are read and written in place (aligned ones), others staged
+    auto in_place = [&](const void *f, size_t align) {
+        return where == BMXG_DEVICE && reinterpret_cast<uintptr_t>(f) % align == 0;
     };
-    auto release = [&]() {
-        for (void *q : mem) cudaFreeAsync(q, st);
-        mem.clear();
-    };
-    TileBufs B;
-    int *scratch = nullptr;
-    const bool ok = alloc(&B.x, nt) && alloc(&B.y, nt) && alloc(&B.z, nt) && alloc(&B.r, nt) && alloc(&B.ct, nt) &&
-                    alloc(&B.ox, nr) && alloc(&B.oy, nr) && alloc(&B.oz, nr) && alloc(&B.vx, nr) &&
-                    alloc(&B.vy, nr) && alloc(&B.vz, nr) && alloc(&B.cell, nt) && alloc(&B.cnt, ncells) &&
-                    alloc(&B.start, ncells + 1) && alloc(&B.fill, ncells) && alloc(&B.perm, nt) &&
-                    alloc(&B.bad, 3) && alloc(&scratch, scan_scratch_ints((int)ncells));
-    if (!ok) {
-        release();
-        (void)cudaGetLastError();
-        return fail(ctx, BMXG_ERR_OOM, "tile scratch");
+    bool direct = true;
+    for (const double *f : {reals->x, reals->y, reals->z, reals->radius, reals->velx, reals->vely, reals->velz})
+        direct = direct && in_place(f, 8);
+    direct = direct && in_place(reals->cell_type, 4);
+    if (ng) {
+        for (const double *f : {ghosts->x, ghosts->y, ghosts->z, ghosts->radius}) direct = direct && in_place(f, 8);
+        direct = direct && in_place(ghosts->cell_type, 4);
     }
+    // the workspace, kept by the context and grown: what a call clears first
+    size_t used = 0;
+    auto carve = [&](size_t bytes) {
+        const size_t at = used;
+        used += (bytes + 255) / 256 * 256;
+        return at;
+    };
+    const size_t N = (size_t)nt, NR = (size_t)nr;
+    const size_t o_bad = carve(3 * sizeof(unsigned long long) + sizeof(DevCounters));
+    const size_t o_cnt = carve(sizeof(int) * ncols);
+    const size_t cleared = used;
+    const size_t o_pos = carve(sizeof(double) * 4 * N), o_out = carve(sizeof(double) * 6 * NR);
+    const size_t o_rel = carve(sizeof(float4) * N), o_srel = carve(sizeof(float4) * N);
+    const size_t o_key = carve(sizeof(unsigned long long) * N);
+    const size_t o_int = carve(sizeof(int) * 5 * N);
+    const size_t o_start = carve(sizeof(int) * (ncols + 1)), o_scan = carve(sizeof(int) * scan_scratch_ints(ncols));
+    const size_t o_in = carve(direct ? 0 : 36 * N);
+    if (used > ctx->tile_cap) {
+        CK(cudaStreamSynchronize(st));
+        if (ctx->tile_buf) cudaFree(ctx->tile_buf);
+        ctx->tile_buf = nullptr;
+        ctx->tile_cap = 0;
+        if (cudaMalloc(&ctx->tile_buf, used) != cudaSuccess) {
+            (void)cudaGetLastError();
+            return fail(ctx, BMXG_ERR_OOM, "tile scratch");
+        }
+        ctx->tile_cap = used;
+    }
+    char *base = ctx->tile_buf;
+    TileCall C;
+    std::memset(&C, 0, sizeof(C));
+    C.nreal = (int)nr;
+    C.bad = reinterpret_cast<unsigned long long *>(base + o_bad);
+    C.out = reinterpret_cast<double *>(base + o_out);
+    DevState &S = C.S;
+    S.n = (int)nt;
+    S.ncol = 1;
+    S.ncols_total = ncols;
+    S.cnt = reinterpret_cast<DevCounters *>(base + o_bad + 3 * sizeof(unsigned long long));
+    S.x[0] = reinterpret_cast<double *>(base + o_pos);
+    S.y[0] = S.x[0] + N;
+    S.z[0] = S.y[0] + N;
+    S.rad = S.z[0] + N;
+    S.rel[0] = reinterpret_cast<float4 *>(base + o_rel);
+    S.srel[0] = reinterpret_cast<float4 *>(base + o_srel);
+    S.lkey = reinterpret_cast<unsigned long long *>(base + o_key);
+    S.col[0] = reinterpret_cast<int *>(base + o_int);
+    S.iz[0] = S.col[0] + N;
+    S.perm[0] = S.iz[0] + N;
+    S.siz[0] = S.perm[0] + N;
+    S.rank[0] = S.siz[0] + N;
+    S.colcnt = reinterpret_cast<int *>(base + o_cnt);
+    S.colstart[0] = reinterpret_cast<int *>(base + o_start);
+    cudaError_t e = cudaSuccess;
+    char *stage = base + o_in;
     const cudaMemcpyKind kin = (where == BMXG_HOST) ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice;
     const cudaMemcpyKind kout = (where == BMXG_HOST) ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice;
-    cudaError_t e = cudaSuccess;
-    auto in = [&](void *dst, const void *src, size_t bytes) {
-        if (e == cudaSuccess && bytes) e = cudaMemcpyAsync(dst, src, bytes, kin, st);
+    auto in = [&](const void *src, size_t bytes) -> const void * {
+        if (direct || !bytes) return src;
+        if (e == cudaSuccess) e = cudaMemcpyAsync(stage, src, bytes, kin, st);
+        const void *q = stage;
+        stage += bytes;
+        return q;
     };
-    in(B.x, reals->x, 8 * nr);
-    in(B.y, reals->y, 8 * nr);
-    in(B.z, reals->z, 8 * nr);
-    in(B.r, reals->radius, 8 * nr);
-    in(B.ct, reals->cell_type, 4 * nr);
+    auto in_d = [&](const double *src, size_t n) { return static_cast<const double *>(in(src, 8 * n)); };
+    C.rx = in_d(reals->x, NR);
+    C.ry = in_d(reals->y, NR);
+    C.rz = in_d(reals->z, NR);
+    C.rr = in_d(reals->radius, NR);
     if (ng) {
-        in(B.x + nr, ghosts->x, 8 * ng);
-        in(B.y + nr, ghosts->y, 8 * ng);
-        in(B.z + nr, ghosts->z, 8 * ng);
-        in(B.r + nr, ghosts->radius, 8 * ng);
-        in(B.ct + nr, ghosts->cell_type, 4 * ng);
+        C.gx = in_d(ghosts->x, ng);
+        C.gy = in_d(ghosts->y, ng);
+        C.gz = in_d(ghosts->z, ng);
+        C.gr = in_d(ghosts->radius, ng);
+        C.gct = static_cast<const int *>(in(ghosts->cell_type, 4 * (size_t)ng));
     }
-    if (e == cudaSuccess) e = cudaMemsetAsync(B.cnt, 0, sizeof(int) * ncells, st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(B.fill, 0, sizeof(int) * ncells, st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(B.bad, 0, 3 * sizeof(unsigned long long), st);
+    C.rct = static_cast<const int *>(in(reals->cell_type, 4 * NR));
+    double *const dst[6] = {reals->x, reals->y, reals->z, reals->velx, reals->vely, reals->velz};
+    if (e == cudaSuccess) e = cudaMemsetAsync(base, 0, cleared, st);
     if (e == cudaSuccess) {
-        ctx->launches += launch_tile_step(B, T, dev_params(ctx->prm), dt / 1.0, (int)nr, (int)nt, scratch, ctx->nsm, st);
+        ctx->launches += launch_tile_step(C, T, dev_params(ctx->prm), dt / 1.0,
+                                          reinterpret_cast<int *>(base + o_scan), direct ? dst : nullptr, st);
         e = cudaGetLastError();
     }
-    unsigned long long bad[3] = {0ull, 0ull, 0ull};
-    if (e == cudaSuccess) e = cudaMemcpyAsync(bad, B.bad, sizeof(bad), cudaMemcpyDeviceToHost, st);
+    unsigned long long *bad = ctx->h_chk;  // (pinned)
+    if (e == cudaSuccess) e = cudaMemcpyAsync(bad, C.bad, 3 * sizeof(bad[0]), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (e == cudaSuccess && !bad[0] && !bad[1]) {  // (non-finite positions are written, then reported)
-        auto out = [&](void *dst, const void *src) {
-            if (e == cudaSuccess) e = cudaMemcpyAsync(dst, src, 8 * nr, kout, st);
-        };
-        out(reals->x, B.ox);
-        out(reals->y, B.oy);
-        out(reals->z, B.oz);
-        out(reals->velx, B.vx);
-        out(reals->vely, B.vy);
-        out(reals->velz, B.vz);
+    if (e == cudaSuccess && !direct && !bad[0] && !bad[1]) {  // (non-finite positions are written, then reported)
+        for (int k = 0; k < 6 && e == cudaSuccess; ++k)
+            e = cudaMemcpyAsync(dst[k], C.out + (size_t)k * NR, 8 * NR, kout, st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     }
-    release();
     if (e != cudaSuccess) return fail(ctx, BMXG_ERR_CUDA, std::string("tile step: ") + cudaGetErrorString(e));
     if (bad[1]) return fail(ctx, BMXG_ERR_UNSUPPORTED, "the tile step takes spheres (YEAST) only");
     if (bad[0])

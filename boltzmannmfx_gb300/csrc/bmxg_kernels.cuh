@@ -260,24 +260,28 @@ int launch_list_step(const DevState &S, const DevParams &P, double dt, int a, in
 // the whole-domain step) offset by lo, the tile's first cell minus one, so
 // that the tile's own cells are 1..nt and the one-cell halo 0 and nt + 1.
 struct TileGeom {
-    double plo[3], phi[3], len[3], dxi[3];
+    double plo[3], phi[3], len[3], dx[3], dxi[3];
+    float dxf[3];
     int n[3], per[3];
     int lo[3], nt[3];
     int nbh_trivial;
 };
-// Device buffers of one tile call: positions, radii and cell types of the
-// reals then the ghosts; the reals' outputs; cell scratch and counters.
-struct TileBufs {
-    double *x, *y, *z, *r;
-    int *ct;
-    double *ox, *oy, *oz, *vx, *vy, *vz;
-    int *cell, *cnt, *start, *fill, *perm;
+// One tile call: the caller's arrays (device memory), the workspace as a state
+// of the reals then the ghosts (buffer 0: positions, radii, columns of the
+// grown tile, z bins, offsets, sort), the reals' results (6 planes) and flags.
+struct TileCall {
+    const double *rx, *ry, *rz, *rr, *gx, *gy, *gz, *gr;
+    const int *rct, *gct;
+    int nreal;
+    DevState S;
+    double *out;              // new x, y, z and velocity, nreal each
     unsigned long long *bad;  // [3]: a real outside the tile or a ghost outside the halo; a non-sphere;
                               // a non-finite new position
 };
-// bin, count, scan, scatter, order each cell by index, step the reals
-int launch_tile_step(const TileBufs &B, const TileGeom &T, const DevParams &P, double dt, int nreal, int ntot,
-                     int *scan_scratch, int nsm, cudaStream_t st);
+// bin, sort, step; then, with dst, the results into the caller's arrays unless
+// the input was bad (dst[0..2] positions, [3..5] velocities)
+int launch_tile_step(const TileCall &C, const TileGeom &T, const DevParams &P, double dt, int *scan_scratch,
+                     double *const dst[6], cudaStream_t st);
 
 // ---- rods and mixed states (k_rod.cu) ------------------------------------
 int launch_rod_mobility(const DevState &S, const DevParams &P, int grid, int block, cudaStream_t st);

@@ -450,6 +450,28 @@ __device__ __forceinline__ double wall_law(double z, double rS, const DevParams 
     return v;
 }
 
+// The FP64 term of a sphere pair at separation (dx, dy, dz), in the reference's
+// operation order: false when the pair is not in the neighbour list or beyond
+// the cutoff, else the three products F u_x, F u_y, F u_z that the gather adds.
+__device__ __forceinline__ bool sphere_pair64(const DevParams &P, int nbh_trivial, double dx, double dy, double dz,
+                                              double ri, double rj, double *t)
+{
+    const double r2 = dx * dx + dy * dy + dz * dz;
+    if (!nbh_trivial && !(r2 <= P.nbh)) return false;  // not in the neighbour list
+    const double rlm = ri + rj + P.bw;                  // maxInteractionDistance
+    if (!le_nonneg(r2, (rlm - kSmall) * (rlm - kSmall))) return false;
+    const double rS = ri + rj;
+    const double rA = rS + P.bw;
+    Divisor by;
+    const double rn = sqrt_rn(r2, &by);
+    const double ux = div_by(dx, by), uy = div_by(dy, by), uz = div_by(dz, by);
+    const double F = lt_bits(rn, rA) ? -P.k * (rn - rA) * (rn - rA) * (rn - rS) : 0.0;
+    t[0] = F * ux;
+    t[1] = F * uy;
+    t[2] = F * uz;
+    return true;
+}
+
 // Exact float -> double conversion with integer operations (GB300's FP64
 // pipe is the scarce resource here), on the two 32-bit words: for a normal
 // float the high word is the sign, then exponent and mantissa shifted down by

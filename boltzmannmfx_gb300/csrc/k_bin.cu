@@ -177,7 +177,7 @@ __global__ void k_scatter(const DevState S, int b)
         const int r = atomicSub(&S.colcnt[c], 1) - 1;  // leaves colcnt at zero
         const int t = S.colstart[b][c] + r;
         if (t >= 0 && t < S.n) {
-            if (S.lkey) S.lkey[t] = col_key(S.iz[b][i], S.orig[i]);
+            if (S.lkey) S.lkey[t] = col_key(S.iz[b][i], S.orig ? S.orig[i] : i);
             else S.tmp[t] = i;
         } else {
             atomicAdd(&S.cnt->bad_index, 1ULL);
@@ -192,7 +192,7 @@ __global__ void k_canon(const DevState S, int b, int publish)
         const int c = S.col[b][i];
         const int s0 = max(S.colstart[b][c], 0), s1 = min(S.colstart[b][c + 1], S.n);
         const int izi = S.iz[b][i];
-        const unsigned long long key = col_key(izi, S.orig[i]);
+        const unsigned long long key = col_key(izi, S.orig ? S.orig[i] : i);
         int rank = 0;
         if (S.lkey) {
             for (int t = s0; t < s1; ++t) rank += (__ldg(&S.lkey[t]) < key);

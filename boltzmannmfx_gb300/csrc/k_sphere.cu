@@ -34,31 +34,14 @@ namespace bmxg {
 namespace {
 
 // The FP64 pair term of slot i (at xi, yi, zi, radius ri, colony geometry
-// G) from neighbour j under image shift (sx, sy), in the reference's operation
-// order: false when the pair is not in the neighbour list or beyond the
-// cutoff, else the three products F u_x, F u_y, F u_z that the gather adds.
+// G) from neighbour j under image shift (sx, sy).
 __device__ __forceinline__ bool sphere_term64(const DevState &S, const DevGeom &G, const DevParams &P, int a,
                                               double xi, double yi, double zi, double ri, int j, int sx, int sy,
                                               double *t)
 {
     const double xj = sx ? S.x[a][j] + (double)sx * G.len[0] : S.x[a][j];
     const double yj = sy ? S.y[a][j] + (double)sy * G.len[1] : S.y[a][j];
-    const double dx = xi - xj, dy = yi - yj, dz = zi - S.z[a][j];
-    const double r2 = dx * dx + dy * dy + dz * dz;
-    if (!G.nbh_trivial && !(r2 <= P.nbh)) return false;  // not in the neighbour list
-    const double rj = S.rad[j];
-    const double rlm = ri + rj + P.bw;                     // maxInteractionDistance
-    if (!le_nonneg(r2, (rlm - kSmall) * (rlm - kSmall))) return false;
-    const double rS = ri + rj;
-    const double rA = rS + P.bw;
-    Divisor by;
-    const double rn = sqrt_rn(r2, &by);
-    const double ux = div_by(dx, by), uy = div_by(dy, by), uz = div_by(dz, by);
-    const double F = lt_bits(rn, rA) ? -P.k * (rn - rA) * (rn - rA) * (rn - rS) : 0.0;
-    t[0] = F * ux;
-    t[1] = F * uy;
-    t[2] = F * uz;
-    return true;
+    return sphere_pair64(P, G.nbh_trivial, xi - xj, yi - yj, zi - S.z[a][j], ri, S.rad[j], t);
 }
 
 // FP64 plain step.  Each thread walks its slot's stencil and screens the
