@@ -41,6 +41,23 @@ struct Shape {
     int grid = 0;  // 0: derive from occupancy
 };
 
+// Buffers of the differentiation form, grown on demand.
+struct AdjBuf {
+    void *p = nullptr;
+    size_t bytes = 0;
+};
+enum {
+    kAdjCkpt,   // (nseg + 1) x 3n positions, slot order
+    kAdjEnd,    // 3n: the trajectory's end
+    kAdjLam0,   // adjoint of the positions, 3 planes
+    kAdjLam1,
+    kAdjAcc,    // 3n + n: parameter slopes and adhesion slope per slot
+    kAdjOut,    // kReduceOut
+    kAdjSeg,    // ckpt_every x 3n positions of one segment (no room for kAdjTrail)
+    kAdjTrail,  // ckpt_every states of one segment with their columns sorted
+    kAdjBufs
+};
+
 }  // namespace
 
 struct bmxg_ctx {
@@ -91,11 +108,7 @@ struct bmxg_ctx {
     double ext_gamma = 0.0, ext_mu = 0.0;
     double *d_adh = nullptr;                // per-slot adhesion in use (nullptr: zero)
     double *adh_buf = nullptr;              // its buffer, allocated with the state
-    std::vector<void *> dallocs;            // adjoint buffers (freed with the state)
-    double *ckpt = nullptr;                 // (nseg + 1) x 3n positions, slot order
-    double *segbuf = nullptr;               // ckpt_every x 3n positions of one segment
-    double *lam[2] = {nullptr, nullptr};    // adjoint of the positions, 3 planes
-    double *gacc = nullptr, *gadh = nullptr, *gout = nullptr, *xT = nullptr;
+    AdjBuf adj[kAdjBufs];                   // buffers of the trajectory and its adjoint (adj_buf)
     int traj_T = -1, traj_k = 0;
     double traj_dt = 0.0;
 
@@ -196,13 +209,20 @@ void drop_graphs(bmxg_ctx *ctx)
     ctx->graph_kernels.clear();
 }
 
-void free_adjoint(bmxg_ctx *ctx)
+// The trajectory is gone; its buffers stay for the next one while they are small
+// (kAdjointKeep) and the state's arrays stay, else they are given back.
+constexpr size_t kAdjointKeep = 256u << 20;
+
+void free_adjoint(bmxg_ctx *ctx, bool all = false)
 {
-    for (void *p : ctx->dallocs) cudaFree(p);
-    ctx->dallocs.clear();
-    ctx->ckpt = ctx->segbuf = ctx->gacc = ctx->gadh = ctx->gout = ctx->xT = nullptr;
-    ctx->lam[0] = ctx->lam[1] = nullptr;
     ctx->traj_T = -1;
+    size_t held = 0;
+    for (const AdjBuf &b : ctx->adj) held += b.bytes;
+    if (!all && held <= kAdjointKeep) return;
+    for (AdjBuf &b : ctx->adj) {
+        if (b.p) cudaFree(b.p);
+        b = AdjBuf{};
+    }
 }
 
 // Device staging of at least `bytes` for host loads and stores.
@@ -232,7 +252,7 @@ struct JoinIo {
 void free_state(bmxg_ctx *ctx)
 {
     drop_graphs(ctx);
-    free_adjoint(ctx);
+    free_adjoint(ctx, true);
     ctx->d_adh = ctx->adh_buf = nullptr;  // lives in allocs
     for (void *p : ctx->allocs) cudaFree(p);
     ctx->allocs.clear();
@@ -2189,16 +2209,61 @@ int bmxg_set_ext(bmxg_ctx *ctx, const bmxg_ext *ext)
 
 namespace {
 
+// At least `count` values in buffer k.
 template <class T>
-int dalloc_adj(bmxg_ctx *ctx, T **p, size_t count)
+int adj_buf(bmxg_ctx *ctx, int k, T **p, size_t count)
 {
-    void *q = nullptr;
-    if (count == 0) count = 1;
-    CK(cudaMalloc(&q, count * sizeof(T)));
-    ctx->dallocs.push_back(q);
-    *p = (T *)q;
+    AdjBuf &b = ctx->adj[k];
+    const size_t need = std::max<size_t>(count, 1) * sizeof(T);
+    if (b.bytes < need) {
+        if (b.p) cudaFree(b.p);  // (waits for the work that uses it)
+        b = AdjBuf{};
+        CK(cudaMalloc(&b.p, need));
+        b.bytes = need;
+    }
+    *p = static_cast<T *>(b.p);
     return BMXG_OK;
 }
+
+// One state of a segment's recomputation: what a step reads of buffer a, so
+// that the reverse sweep finds each step's positions binned and sorted as the
+// recomputation left them.
+struct Trail {
+    size_t stride, o_pos, o_rel, o_srel, o_int, o_start;
+    char *base = nullptr;
+    size_t n;
+    Trail(size_t n_, size_t ncols) : n(n_)
+    {
+        size_t at = 0;
+        auto carve = [&](size_t bytes) {
+            const size_t o = at;
+            at += (bytes + 255) / 256 * 256;
+            return o;
+        };
+        o_pos = carve(3 * sizeof(double) * n);
+        o_rel = carve(sizeof(float4) * n);
+        o_srel = carve(sizeof(float4) * n);
+        o_int = carve(5 * sizeof(int) * n);
+        o_start = carve(sizeof(int) * (ncols + 1));
+        stride = at;
+    }
+    // entry k as buffer b of S
+    void put(DevState &S, int b, size_t k) const
+    {
+        char *q = base + k * stride;
+        S.x[b] = reinterpret_cast<double *>(q + o_pos);
+        S.y[b] = S.x[b] + n;
+        S.z[b] = S.y[b] + n;
+        S.rel[b] = reinterpret_cast<float4 *>(q + o_rel);
+        S.srel[b] = reinterpret_cast<float4 *>(q + o_srel);
+        S.col[b] = reinterpret_cast<int *>(q + o_int);
+        S.iz[b] = S.col[b] + n;
+        S.perm[b] = S.iz[b] + n;
+        S.siz[b] = S.perm[b] + n;
+        S.rank[b] = S.siz[b] + n;
+        S.colstart[b] = reinterpret_cast<int *>(q + o_start);
+    }
+};
 
 DiffParams diff_params(const bmxg_ctx *ctx)
 {
@@ -2230,17 +2295,14 @@ int load_pos(bmxg_ctx *ctx, const double *src)
     return BMXG_OK;
 }
 
-int dfwd_step(bmxg_ctx *ctx, double dt)
+int dfwd_step(bmxg_ctx *ctx, const DevState &S, int a, double dt)
 {
-    const DevState &S = ctx->S;
-    const int a = ctx->parity;
     const int mblk = ctx->sh_misc.block, mgrd = grid_for(ctx, ctx->sh_misc, ctx->n);
     const Shape &sh = ctx->sh_sphere[0];
     int sg, sb;
     stencil_shape(ctx, sh, ctx->n, &sg, &sb);
     LAUNCH(launch_dfwd(S, dev_params(ctx->prm), diff_params(ctx), dt, a, sg, sb, ctx->stream, sh.grid > 0));
     LAUNCH(launch_rebuild(S, a ^ 1, ctx->scan_scratch, mgrd, mblk, ctx->stream));
-    ctx->parity = a ^ 1;
     return BMXG_OK;
 }
 
@@ -2268,16 +2330,18 @@ int bmxg_forward(bmxg_ctx *ctx, double dt, int32_t nsteps, int32_t ckpt_every)
     }
     const int nseg = (nsteps + ckpt_every - 1) / ckpt_every;
     int rc;
-    if ((rc = dalloc_adj(ctx, &ctx->ckpt, (size_t)(nseg + 1) * 3 * n))) return rc;
-    if ((rc = dalloc_adj(ctx, &ctx->xT, (size_t)3 * n))) return rc;
+    double *ckpt = nullptr, *xT = nullptr;
+    if ((rc = adj_buf(ctx, kAdjCkpt, &ckpt, (size_t)(nseg + 1) * 3 * n))) return rc;
+    if ((rc = adj_buf(ctx, kAdjEnd, &xT, (size_t)3 * n))) return rc;
     const double subdt = dt / 1.0;
     CK(cudaEventRecord(ctx->ev0, ctx->stream));
     for (int t = 0; t < nsteps; ++t) {
-        if (t % ckpt_every == 0 && (rc = save_pos(ctx, ctx->parity, ctx->ckpt + (size_t)(t / ckpt_every) * 3 * n)))
+        if (t % ckpt_every == 0 && (rc = save_pos(ctx, ctx->parity, ckpt + (size_t)(t / ckpt_every) * 3 * n)))
             return rc;
-        if ((rc = dfwd_step(ctx, subdt))) return rc;
+        if ((rc = dfwd_step(ctx, ctx->S, ctx->parity, subdt))) return rc;
+        ctx->parity ^= 1;
     }
-    if ((rc = save_pos(ctx, ctx->parity, ctx->xT))) return rc;
+    if ((rc = save_pos(ctx, ctx->parity, xT))) return rc;
     CK(cudaEventRecord(ctx->ev1, ctx->stream));
     CK(cudaMemcpyAsync(ctx->h_cnt, ctx->d_cnt, sizeof(DevCounters), cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
@@ -2312,63 +2376,103 @@ int bmxg_backward(bmxg_ctx *ctx, const double *dL_dx, double *dL_dx0, double *dL
     const DevState &S = ctx->S;
     int rc;
     ctx->list_valid = false;  // the recomputation rewrites buffer 0
-    if (!ctx->lam[0]) {
-        if ((rc = dalloc_adj(ctx, &ctx->lam[0], (size_t)3 * n))) return rc;
-        if ((rc = dalloc_adj(ctx, &ctx->lam[1], (size_t)3 * n))) return rc;
-        if ((rc = dalloc_adj(ctx, &ctx->segbuf, (size_t)K * 3 * n))) return rc;
-        if ((rc = dalloc_adj(ctx, &ctx->gacc, (size_t)3 * n))) return rc;
-        if ((rc = dalloc_adj(ctx, &ctx->gadh, (size_t)n))) return rc;
-        if ((rc = dalloc_adj(ctx, &ctx->gout, 4))) return rc;
+    const size_t n3 = (size_t)3 * n;
+    double *ckpt = nullptr, *xT = nullptr, *lam[2] = {nullptr, nullptr}, *gacc = nullptr, *gout = nullptr;
+    if ((rc = adj_buf(ctx, kAdjCkpt, &ckpt, 0))) return rc;  // (the forward's)
+    if ((rc = adj_buf(ctx, kAdjEnd, &xT, 0))) return rc;
+    if ((rc = adj_buf(ctx, kAdjLam0, &lam[0], n3))) return rc;
+    if ((rc = adj_buf(ctx, kAdjLam1, &lam[1], n3))) return rc;
+    if ((rc = adj_buf(ctx, kAdjAcc, &gacc, n3 + n))) return rc;
+    if ((rc = adj_buf(ctx, kAdjOut, &gout, kReduceOut))) return rc;
+    double *gadh = gacc + n3;
+    if ((rc = ensure_io(ctx, sizeof(double) * n3))) return rc;
+    double *io = reinterpret_cast<double *>(ctx->io_buf);
+    // A segment's states, sorted, where they take at most half of the free
+    // memory (100 B per slot and step): the reverse sweep then runs one kernel
+    // per step.  Otherwise the positions alone are kept (24 B) and binned and
+    // sorted again.
+    Trail trail((size_t)n, (size_t)S.ncols_total);
+    double *segbuf = nullptr;
+    const int kseg = std::min(K, std::max(T, 1));
+    {
+        const size_t need = trail.stride * (size_t)kseg;
+        size_t free_b = 0, total_b = 0;
+        CK(cudaMemGetInfo(&free_b, &total_b));
+        if (need <= ctx->adj[kAdjTrail].bytes || need <= free_b / 2) {
+            if (adj_buf(ctx, kAdjTrail, &trail.base, need)) {
+                (void)cudaGetLastError();
+                trail.base = nullptr;
+            }
+        }
+        if (!trail.base && (rc = adj_buf(ctx, kAdjSeg, &segbuf, (size_t)kseg * n3))) return rc;
     }
     const int mblk = ctx->sh_misc.block, mgrd = grid_for(ctx, ctx->sh_misc, n);
     CK(cudaEventRecord(ctx->ev0, st));
     // dL/dx_T, caller order -> slot order
-    for (int c = 0; c < 3; ++c) {
-        CK(cudaMemcpyAsync(ctx->ud, dL_dx + (size_t)c * n, sizeof(double) * n, cudaMemcpyHostToDevice, st));
-        LAUNCH(launch_gather_d(ctx->lam[0] + (size_t)c * n, ctx->ud, S.orig, (int)n, mgrd, mblk, st));
-    }
-    CK(cudaMemsetAsync(ctx->gacc, 0, sizeof(double) * 3 * n, st));
-    CK(cudaMemsetAsync(ctx->gadh, 0, sizeof(double) * n, st));
+    CK(cudaMemcpyAsync(io, dL_dx, sizeof(double) * n3, cudaMemcpyHostToDevice, st));
+    LAUNCH(launch_gather_d(lam[0], io, S.orig, (int)n, mgrd, mblk, st, 3));
+    CK(cudaMemsetAsync(gacc, 0, sizeof(double) * (n3 + n), st));
     int cur = 0;
     const DevParams P = dev_params(ctx->prm);
     const DiffParams D = diff_params(ctx);
     const Shape &sh = ctx->sh_sphere[0];
     int ag, ab;
     stencil_shape(ctx, sh, n, &ag, &ab);
+    auto reverse = [&](const DevState &Q, int a) -> int {
+        LAUNCH(launch_dadj(Q, P, D, ctx->traj_dt, a, lam[cur], lam[cur ^ 1], gacc, gadh, ag, ab, st, sh.grid > 0));
+        cur ^= 1;
+        return BMXG_OK;
+    };
     const int nseg = (T + K - 1) / K;
     for (int seg = nseg - 1; seg >= 0; --seg) {
         const int c0 = seg * K, c1 = std::min(c0 + K, T);
-        // recompute the segment's positions from its checkpoint
-        if ((rc = load_pos(ctx, ctx->ckpt + (size_t)seg * 3 * n))) return rc;
+        const double *start = ckpt + (size_t)seg * n3;
+        if (trail.base) {
+            // recompute the segment's states from its checkpoint, entry by entry
+            DevState Q = S;
+            trail.put(Q, 0, 0);
+            CK(cudaMemcpyAsync(Q.x[0], start, sizeof(double) * n3, cudaMemcpyDeviceToDevice, st));
+            LAUNCH(launch_bin(Q, 0, mgrd, mblk, st));
+            LAUNCH(launch_rebuild(Q, 0, ctx->scan_scratch, mgrd, mblk, st));
+            for (int t = c0; t + 1 < c1; ++t) {
+                trail.put(Q, 0, (size_t)(t - c0));
+                trail.put(Q, 1, (size_t)(t - c0 + 1));
+                if ((rc = dfwd_step(ctx, Q, 0, ctx->traj_dt))) return rc;
+            }
+            for (int t = c1 - 1; t >= c0; --t) {
+                trail.put(Q, 0, (size_t)(t - c0));
+                if ((rc = reverse(Q, 0))) return rc;
+            }
+            continue;
+        }
+        if ((rc = load_pos(ctx, start))) return rc;
         for (int t = c0; t < c1; ++t) {
-            if ((rc = save_pos(ctx, ctx->parity, ctx->segbuf + (size_t)(t - c0) * 3 * n))) return rc;
-            if (t + 1 < c1 && (rc = dfwd_step(ctx, ctx->traj_dt))) return rc;
+            if ((rc = save_pos(ctx, ctx->parity, segbuf + (size_t)(t - c0) * n3))) return rc;
+            if (t + 1 < c1) {
+                if ((rc = dfwd_step(ctx, S, ctx->parity, ctx->traj_dt))) return rc;
+                ctx->parity ^= 1;
+            }
         }
         // reverse sweep through the segment
         for (int t = c1 - 1; t >= c0; --t) {
-            if ((rc = load_pos(ctx, ctx->segbuf + (size_t)(t - c0) * 3 * n))) return rc;
-            LAUNCH(launch_dadj(S, P, D, ctx->traj_dt, 0, ctx->lam[cur], ctx->lam[cur ^ 1], ctx->gacc, ctx->gadh,
-                               ag, ab, st, sh.grid > 0));
-            cur ^= 1;
+            if ((rc = load_pos(ctx, segbuf + (size_t)(t - c0) * n3))) return rc;
+            if ((rc = reverse(S, 0))) return rc;
         }
     }
-    LAUNCH(launch_dreduce(ctx->gacc, (int)n, 3, ctx->gout, st));
+    LAUNCH(launch_dreduce(gacc, (int)n, 3, gout, st));
     CK(cudaEventRecord(ctx->ev1, st));
     if (dL_dx0) {
-        for (int c = 0; c < 3; ++c) {
-            LAUNCH(launch_scatter_d(ctx->ud, ctx->lam[cur] + (size_t)c * n, S.orig, (int)n, mgrd, mblk, st));
-            CK(cudaMemcpyAsync(dL_dx0 + (size_t)c * n, ctx->ud, sizeof(double) * n, cudaMemcpyDeviceToHost, st));
-            CK(cudaStreamSynchronize(st));
-        }
+        LAUNCH(launch_scatter_d(io, lam[cur], S.orig, (int)n, mgrd, mblk, st, 3));
+        CK(cudaMemcpyAsync(dL_dx0, io, sizeof(double) * n3, cudaMemcpyDeviceToHost, st));
     }
     if (dL_dadhesion) {
-        LAUNCH(launch_scatter_d(ctx->ud, ctx->gadh, S.orig, (int)n, mgrd, mblk, st));
+        LAUNCH(launch_scatter_d(ctx->ud, gadh, S.orig, (int)n, mgrd, mblk, st));
         CK(cudaMemcpyAsync(dL_dadhesion, ctx->ud, sizeof(double) * n, cudaMemcpyDeviceToHost, st));
     }
     double g[3] = {0.0, 0.0, 0.0};
-    CK(cudaMemcpyAsync(g, ctx->gout, sizeof(g), cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(g, gout, sizeof(g), cudaMemcpyDeviceToHost, st));
     // leave the state at the end of the trajectory, as bmxg_forward did
-    if ((rc = load_pos(ctx, ctx->xT))) return rc;
+    if ((rc = load_pos(ctx, xT))) return rc;
     CK(cudaStreamSynchronize(st));
     float ms = 0.0f;
     cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);

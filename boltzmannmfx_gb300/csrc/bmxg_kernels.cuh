@@ -213,8 +213,11 @@ int launch_user_bin(const DevState &S, const double *ux, const double *uy, const
 // caller index (keys in lkey)
 int launch_user_sort(const DevState &S, const int *ucol, const int *uiz, int *colstart, int *scan_scratch,
                      int *uperm, int grid, int block, cudaStream_t st);
-int launch_gather_d(double *dst, const double *src, const int *perm, int n, int grid, int block, cudaStream_t st);
-int launch_scatter_d(double *dst, const double *src, const int *orig, int n, int grid, int block, cudaStream_t st);
+// (planes of n each)
+int launch_gather_d(double *dst, const double *src, const int *perm, int n, int grid, int block, cudaStream_t st,
+                    int planes = 1);
+int launch_scatter_d(double *dst, const double *src, const int *orig, int n, int grid, int block, cudaStream_t st,
+                     int planes = 1);
 int launch_scatter_f2d(double *dst, const float *src, const int *orig, int n, int grid, int block,
                        cudaStream_t st);
 
@@ -304,6 +307,9 @@ int launch_dfwd(const DevState &S, const DevParams &P, const DiffParams &D, doub
                 cudaStream_t st, bool pinned = false);
 int launch_dadj(const DevState &S, const DevParams &P, const DiffParams &D, double dt, int a, const double *lin,
                 double *lout, double *gacc, double *gadh, int grid, int block, cudaStream_t st, bool pinned = false);
+// out: kReduceOut values, the planes' sums first
+constexpr int kReduceBlocks = 64;
+constexpr int kReduceOut = 4 + 4 * kReduceBlocks;  // (up to four planes)
 int launch_dreduce(const double *gacc, int n, int planes, double *out, cudaStream_t st);
 
 }  // namespace bmxg

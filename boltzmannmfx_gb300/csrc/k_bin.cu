@@ -362,16 +362,20 @@ __global__ void k_user_scatter(const DevState S, const int *ucol, const int *uiz
     }
 }
 
-__global__ void k_gather_d(double *dst, const double *src, const int *perm, int n)
+__global__ void k_gather_d(double *dst, const double *src, const int *perm, int n, int planes)
 {
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x)
-        dst[s] = src[perm[s]];
+    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) {
+        const int u = perm[s];
+        for (int k = 0; k < planes; ++k) dst[(size_t)k * n + s] = src[(size_t)k * n + u];
+    }
 }
 
-__global__ void k_scatter_d(double *dst, const double *src, const int *orig, int n)
+__global__ void k_scatter_d(double *dst, const double *src, const int *orig, int n, int planes)
 {
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x)
-        dst[orig[s]] = src[s];
+    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) {
+        const int u = orig[s];
+        for (int k = 0; k < planes; ++k) dst[(size_t)k * n + u] = src[(size_t)k * n + s];
+    }
 }
 
 __global__ void k_scatter_f2d(double *dst, const float *src, const int *orig, int n)
@@ -658,17 +662,17 @@ int launch_user_sort(const DevState &S, const int *ucol, const int *uiz, int *co
     return k + 2;
 }
 
-int launch_gather_d(double *dst, const double *src, const int *perm, int n, int grid, int block,
-                     cudaStream_t st)
+int launch_gather_d(double *dst, const double *src, const int *perm, int n, int grid, int block, cudaStream_t st,
+                    int planes)
 {
-    k_gather_d<<<grid, block, 0, st>>>(dst, src, perm, n);
+    k_gather_d<<<grid, block, 0, st>>>(dst, src, perm, n, planes);
     return 1;
 }
 
-int launch_scatter_d(double *dst, const double *src, const int *orig, int n, int grid, int block,
-                      cudaStream_t st)
+int launch_scatter_d(double *dst, const double *src, const int *orig, int n, int grid, int block, cudaStream_t st,
+                     int planes)
 {
-    k_scatter_d<<<grid, block, 0, st>>>(dst, src, orig, n);
+    k_scatter_d<<<grid, block, 0, st>>>(dst, src, orig, n, planes);
     return 1;
 }
 
