@@ -1255,8 +1255,8 @@ int enqueue_step(bmxg_ctx *ctx, double dt, int precision, int a, int resync)
     } else {
         const int rg = grid_for(ctx, ctx->sh_rod, n);
         // the flat pipeline over the pairs the bookkeeping records
-        const bool pipe = S.rnb != nullptr;
-        LAUNCH(launch_rod_book(S, P, a, precision, pipe, rg, ctx->sh_rod.block, st));
+        const bool pipe = S.rwork != nullptr;
+        LAUNCH(launch_rod_book(S, P, a, pipe, rg, ctx->sh_rod.block, st));
         if (k0) cudaEventRecord(k0, st);
         if (pipe)
             LAUNCH(launch_rod_pairs(S, P, a, precision, ctx->nsm, (int)n, st));
@@ -1331,21 +1331,21 @@ int step_setup(bmxg_ctx *ctx, int32_t nsteps, int32_t precision)
         drop_graphs(ctx);
     }
     // the rod pipelines' buffers (the queue's length is an int)
-    if (ctx->S.has_rods && !ctx->S.rnb &&
+    if (ctx->S.has_rods && !ctx->S.rwork &&
         !(precision == BMXG_FP64 && (ctx->rod_walk || ctx->n > (1LL << 26)))) {
         const size_t n = (size_t)ctx->n;
-        int2 *nb = nullptr, *work = nullptr;
-        int *cnt = nullptr;
+        int4 *work = nullptr;
+        int *cnt = nullptr, *q64 = nullptr;
         double *res = nullptr;
         RodCtl *ctl = nullptr;
         const size_t held = ctx->allocs.size();
-        int rc = dalloc(ctx, &nb, n * kRodCap);
+        int rc = dalloc(ctx, &q64, n * kRodCap);
         if (!rc) rc = dalloc(ctx, &cnt, n);
         if (!rc) rc = dalloc(ctx, &res, n * kRodCap * 6);
         if (!rc) rc = dalloc(ctx, &work, n * kRodCap);
         if (!rc) rc = dalloc(ctx, &ctl, 1);
         if (rc) {
-            // no room for the lists (2 KB per segment): the FP64 form walks
+            // no room for the queues (2 KB per segment): the FP64 form walks
             while (ctx->allocs.size() > held) {
                 cudaFree(ctx->allocs.back());
                 ctx->allocs.pop_back();
@@ -1355,7 +1355,7 @@ int step_setup(bmxg_ctx *ctx, int32_t nsteps, int32_t precision)
             ctx->rod_walk = true;
             return BMXG_OK;
         }
-        ctx->S.rnb = nb;
+        ctx->S.rq64 = q64;
         ctx->S.rcnt = cnt;
         ctx->S.rres = res;
         ctx->S.rwork = work;

@@ -56,10 +56,11 @@ constexpr int kWalkWide = 400000;    // ... 128 slots per block up to here
 constexpr int kRodCap = 32;          // gated pairs per segment the rod pipelines hold (more: the
                                      // segment walks its stencil in the segment kernel)
 
-// Per-step counters of the FP32F rod pipeline (k_rod.cu).
+// Lengths of the rod pipelines' queues (k_rod.cu), emptied at the end of a step.
 struct RodCtl {
-    int kmax;   // largest number of gated pairs of a segment (at most kRodCap)
-    int nwork;  // pairs queued for FP64
+    int ncontact;  // pairs from the front of rwork
+    int nbond;     // pairs bonded by the segment's own table, from the back of rwork
+    int n64;       // FP32F: contacts that need FP64 (rq64)
 };
 
 // Device pointers of one context.  [2] arrays are ping-pong buffers indexed
@@ -107,14 +108,14 @@ struct DevState {
     float4 *axf;       // per segment, this step: FP32 axis (nx, ny, nz) and length (k_rod_book)
     double4_32a *mob;  // per segment: mobility (d0 + db, da - db, (d0 - db) / 2, 0) of its area,
                        // length and the viscosity (k_rod_mobility, on every state or parameter load)
-    // FP32F rod pipeline (null until the first FP32F rod step): the gated pairs
-    // of each segment in the reference's list order, kRodCap planes of n
-    // entries (j, stencil code: bin offsets dx, dy, dz + 1 as a base-3 number in
-    // bits 0-4, image shifts sx, sy + 1 in bits 5-8), written by k_rod_book
-    int2 *rnb;
-    int *rcnt;         // per segment: its gated pairs (may exceed kRodCap)
+    // rod pipelines (null until the first rod step): the queue of gated pairs
+    // (i, k: the pair's place in the segment's list order, j, code: bin offsets
+    // dx, dy, dz + 1 as a base-3 number in bits 0-4, image shifts sx, sy + 1 in
+    // bits 5-8, the segment's bonded site in bits 9-10), written by k_rod_book
+    int4 *rwork;       // kRodCap n entries
+    int *rq64;         // FP32F: entries of rwork left to FP64
+    int *rcnt;         // per segment: its gated pairs (more than kRodCap: it walks)
     double *rres;      // 6 x kRodCap planes of n: each pair's f1 + f2 (0-2), f1 - f2 (3-5)
-    int2 *rwork;       // the pairs evaluated in FP64: (i, k | si << 8 | sj << 12)
     RodCtl *rctl;
 
     // FP32F neighbour list with a skin (null unless the context is in list mode)
@@ -288,10 +289,9 @@ int launch_tile_step(const TileCall &C, const TileGeom &T, const DevParams &P, d
 
 // ---- rods and mixed states (k_rod.cu) ------------------------------------
 int launch_rod_mobility(const DevState &S, const DevParams &P, int grid, int block, cudaStream_t st);
-// list: also record each segment's gated pairs (the FP32F pipeline)
-int launch_rod_book(const DevState &S, const DevParams &P, int a, int precision, bool list, int grid, int block,
-                    cudaStream_t st);
-// the FP32F pipeline after the bookkeeping: FP32 pairs, FP64 pairs, per-segment sums
+// list: also queue the segments' gated pairs for the pipelines
+int launch_rod_book(const DevState &S, const DevParams &P, int a, bool list, int grid, int block, cudaStream_t st);
+// the pipelines after the bookkeeping: the queued pairs, then per-segment sums
 int launch_rod_pairs(const DevState &S, const DevParams &P, int a, int precision, int nsm, int n, cudaStream_t st);
 int launch_rod_force(const DevState &S, const DevParams &P, int a, int grid, int block, cudaStream_t st);
 int launch_rod_update(const DevState &S, double dt, int a, int grid, int block, cudaStream_t st);

@@ -210,10 +210,11 @@ struct WalkMem {
     int wsum[NS / 32];
 };
 
-// After every warp wrote its counts into end[w][slot] (more than STAGE:
-// overflow): the counts into runs, over the whole block (it synchronises).
+// After every warp wrote its counts into end[w][slot] (more than STAGE, or
+// more than `most` in all: overflow): the counts into runs, over the whole
+// block (it synchronises).
 template <int NS, int STAGE>
-__device__ __forceinline__ void walk_scan(WalkMem<NS, STAGE> &M)
+__device__ __forceinline__ void walk_scan(WalkMem<NS, STAGE> &M, int most = 0x7fffffff)
 {
     const int tid = threadIdx.x, lane = tid & 31;
     __syncthreads();
@@ -228,6 +229,7 @@ __device__ __forceinline__ void walk_scan(WalkMem<NS, STAGE> &M)
             run += c;
             M.end[w][tid] = run;
         }
+        over |= run > most;
         M.over[tid] = over ? 1 : 0;
         mine = over ? 0 : run;
         x = mine;

@@ -157,8 +157,9 @@ __device__ __forceinline__ void publish_counters(DevCounters *c, RodCtl *rctl)
     c->bond_repairs = 0ull;
     c->moved = 0ull;
     if (rctl) {
-        rctl->kmax = 0;
-        rctl->nwork = 0;
+        rctl->ncontact = 0;
+        rctl->nbond = 0;
+        rctl->n64 = 0;
     }
 }
 

@@ -169,6 +169,21 @@ __device__ void rod_site_forces(const T *r12, const T *ni, T Li, const T *nj, T 
     }
 }
 
+// The bonded spring of rod_site_forces alone (si, sj in {1, 2}): the two bonded
+// ends with its operations, the other two left out.
+__device__ __forceinline__ void rod_spring(const double *r12, const double *ni, double Li, const double *nj, double Lj,
+                                           int si, int sj, double kb, double *f1, double *f2)
+{
+    for (int d = 0; d < 3; ++d) {
+        const double hi = 0.5 * ni[d] * Li, hj = 0.5 * nj[d] * Lj;
+        const double ea = (si == 1) ? r12[d] - hi : r12[d] + hi;
+        const double eb = (sj == 1) ? -hj : hj;
+        const double f = 0.0 - kb * (ea - eb);
+        f1[d] = (si == 1) ? f : 0.0;
+        f2[d] = (si == 1) ? 0.0 : f;
+    }
+}
+
 __device__ __forceinline__ int find_in_table(const int *tb, int id, int cpu)
 {
     const int nb = min(tb[0], 4);
@@ -196,6 +211,15 @@ __device__ __forceinline__ int find_in_plane_table(const int *tab, int n, int j,
     const int nb = min(__ldg(&tab[j]), 4);
     for (int k = 0; k < nb; ++k)
         if (__ldg(&tab[(size_t)(1 + k) * n + j]) == id && __ldg(&tab[(size_t)(5 + k) * n + j]) == cpu) return k;
+    return -1;
+}
+
+// the same over a table written by this kernel
+__device__ __forceinline__ int find_in_slot_table(const int *tab, int n, int j, int id, int cpu)
+{
+    const int nb = min(tab[j], 4);
+    for (int k = 0; k < nb; ++k)
+        if (tab[(size_t)(1 + k) * n + j] == id && tab[(size_t)(5 + k) * n + j] == cpu) return k;
     return -1;
 }
 
@@ -241,119 +265,225 @@ __device__ __forceinline__ bool rod_gate(const DevState &S, const DevGeom &G, co
 }
 
 // ---- bookkeeping ----------------------------------------------------------
-// kRodList: also record the segment's gated pairs, in the order of its walk,
-// for the flat pipelines (rnb, rcnt; the step's largest count into
-// rctl->kmax).  kRodQueue (the FP64 pipeline): and queue every recorded pair
-// for k_rod_pair64, a warp's pairs together, one atomic per warp.
-enum { kRodPlain = 0, kRodList = 1, kRodQueue = 2 };
-
-template <int MODE>
-__global__ void k_rod_book(const DevState S, const DevParams P, int a)
+// The bookkeeping of segment i by a walk of its stencil: flag resets, position
+// fix-up, half-bond repair of its own table (buffer b).
+__device__ void book_slot(const DevState &S, const DevParams &P, int a, int i)
 {
-    constexpr bool LIST = MODE != kRodPlain;
     const int b = a ^ 1;
     const int n = S.n;
-    // (same trip count for every lane of a warp)
-    for (int base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
-        const int i = base + threadIdx.x;
-        int cnt = 0;
-        if (i < n) {
-        S.fflag[i] = 0;  // flag resets of bmx_pc_interaction.cpp:178-180
-        S.sflag[i] = 0;
-        S.nflag[i] = 0;
-        int tb[13];
-        for (int k = 0; k < 13; ++k) tb[k] = S.tab[a][(size_t)k * n + i];
-        {   // this step's FP32 axis and length, for the FP32F force kernel
-            const double4_32a tr = S.trig[a][i];
-            S.axf[i] = make_float4(d2f_rn(tr.y * tr.z), d2f_rn(tr.y * tr.w), d2f_rn(tr.x), d2f_rn(S.clen[i]));
-        }
-        if (S.ctype[i] == kFungi) {
-            const DevGeom &G = geom_of(S, i);
-            int bx, by;
-            col_to_bxy(G, S.col[a][i], bx, by);
-            const double xi = S.x[a][i], yi = S.y[a][i], zi = S.z[a][i];
-            const double Li = S.clen[i];
-            const float Lif = d2f_rn(Li);
-            const float4 me = S.rel[a][i];
-            const int iid = S.id[i], icpu = S.cpu[i];
-            const int fs = S.fix_site[i];
-            int pos = S.position[i];
-            bool any = false;
-            int rep = 0;
-            visit_stencil(S, G, a, i, bx, by, S.iz[a][i], [&](int j, int dxs, int dys, int dzs, int sx, int sy) {
+    S.fflag[i] = 0;  // flag resets of bmx_pc_interaction.cpp:178-180
+    S.sflag[i] = 0;
+    S.nflag[i] = 0;
+    int tb[13];
+    for (int k = 0; k < 13; ++k) tb[k] = S.tab[a][(size_t)k * n + i];
+    if (S.ctype[i] == kFungi) {
+        const DevGeom &G = geom_of(S, i);
+        int bx, by;
+        col_to_bxy(G, S.col[a][i], bx, by);
+        const double xi = S.x[a][i], yi = S.y[a][i], zi = S.z[a][i];
+        const double Li = S.clen[i];
+        const float Lif = d2f_rn(Li);
+        const float4 me = S.rel[a][i];
+        const int iid = S.id[i], icpu = S.cpu[i];
+        const int fs = S.fix_site[i];
+        int pos = S.position[i];
+        bool any = false;
+        int rep = 0;
+        visit_stencil(S, G, a, i, bx, by, S.iz[a][i], [&](int j, int dxs, int dys, int dzs, int sx, int sy) {
+            if (S.ctype[j] != kFungi) return;
+            float r12f[3];
+            if (!rod_gate(S, G, P, a, j, dxs, dys, dzs, sx, sy, me, Lif, d2f_rn(S.clen[j]), xi, yi, zi, Li, r12f))
+                return;
+            any = true;
+            const int jid = S.id[j], jcpu = S.cpu[j];
+            // position fix-up (bmx_cell_interaction_K.H:338-362); the
+            // neighbour's position is only tested against TIP, which no
+            // thread writes, so reading it while others update theirs is safe
+            if (pos == kSecond1 || pos == kSecond2) {
+                const int site = (pos == kSecond1) ? 1 : 2;
+                const int nb = min(tb[0], 4);
+                int k = 0;
+                for (; k < nb; ++k)
+                    if (tb[1 + k] == jid && tb[5 + k] == jcpu && tb[9 + k] == site) break;
+                if (k < nb && S.position[j] != kTip) pos = kInterior;
+            }
+            // half-bond repair of i (:370-467)
+            const bool i_to_j = find_in_table(tb, jid, jcpu) >= 0;
+            const bool j_to_i = find_in_plane_table(S.tab[a], n, j, iid, icpu) >= 0;
+            if (!i_to_j && j_to_i) {
+                const int nb = tb[0];
+                if (nb >= 0 && nb < 4) {
+                    const int isite = (fs == 0) ? (tb[9] == 1 ? 2 : 1) : fs;
+                    tb[1 + nb] = jid;
+                    tb[5 + nb] = jcpu;
+                    tb[9 + nb] = isite;
+                    tb[0] = nb + 1;
+                    ++rep;
+                }
+            }
+        });
+        S.position[i] = pos;
+        if (any)
+            for (int k = 0; k < 6; ++k) S.dltd[(size_t)k * n + i] = -1;
+        if (rep) atomicAdd(&S.cnt->bond_repairs, (unsigned long long)rep);
+    }
+    for (int k = 0; k < 13; ++k) S.tab[b][(size_t)k * n + i] = tb[k];
+}
+
+// this step's FP32 axis and length, for the FP32F pair math
+__device__ __forceinline__ float4 rod_axis32(const DevState &S, int a, int i)
+{
+    const double4_32a tr = S.trig[a][i];
+    return make_float4(d2f_rn(tr.y * tr.z), d2f_rn(tr.y * tr.w), d2f_rn(tr.x), d2f_rn(S.clen[i]));
+}
+
+// (contexts without room for the pipelines' queues)
+__global__ void k_rod_book_plain(const DevState S, const DevParams P, int a)
+{
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < S.n; i += gridDim.x * blockDim.x) {
+        S.axf[i] = rod_axis32(S, a, i);
+        book_slot(S, P, a, i);
+    }
+}
+
+// The bookkeeping and the queue of gated pairs, one warp per neighbour column
+// (bmxg_stencil.cuh): the walk is a chain of dependent loads (candidate, its
+// type, its ids, its bond table), which 50 000 segments on one thread each do
+// not hide.  A segment whose own table an unmutual bond will change (rare), or
+// with more candidates than the staging or kRodCap holds, takes book_slot's walk
+// for the bookkeeping; in the latter case its pairs are not queued (rcnt tells
+// the segment kernel to walk).  Every other segment's table stays as it was.
+// The block's pairs go to the queue together: contacts from the front, pairs
+// that the segment's table bonds from the back, so that the pair kernels' warps
+// run one kind.  The FP64 step of 50 000 segments, 10 steps and the load, 2.70 ->
+// 2.30 ms, FP32F, 20 steps, 3.80 -> 3.14 ms, with the pair kernels below (the
+// bookkeeping alone 54 -> 46 us).
+constexpr int kRodStage = 12;
+
+__global__ void __launch_bounds__(kWalkBlock, 3) k_rod_book(const DevState S, const DevParams P, int a)
+{
+    extern __shared__ __align__(16) unsigned char smw[];
+    auto &M = *reinterpret_cast<WalkMem<32, kRodStage> *>(smw);
+    __shared__ int tb[13][32];
+    __shared__ int repair[32], fixed[32];
+    __shared__ int nq[2], at[2];
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const int b = a ^ 1;
+    const int n = S.n;
+    const int i = blockIdx.x * 32 + lane;
+    for (int k = w; k < 13; k += kWalkCols)
+        if (i < n) tb[k][lane] = S.tab[a][(size_t)k * n + i];
+    if (w == 0) {
+        repair[lane] = 0;
+        fixed[lane] = 0;
+    }
+    if (tid < 2) nq[tid] = 0;
+    __syncthreads();
+    int cnt = 0;
+    if (i < n && S.ctype[i] == kFungi) {
+        const DevGeom &G = geom_of(S, i);
+        int bx, by;
+        col_to_bxy(G, S.col[a][i], bx, by);
+        const int izi = S.iz[a][i];
+        const double xi = S.x[a][i], yi = S.y[a][i], zi = S.z[a][i];
+        const double Li = S.clen[i];
+        const float Lif = d2f_rn(Li);
+        const float4 me = S.rel[a][i];
+        const int iid = S.id[i], icpu = S.cpu[i];
+        const int pos = S.position[i];
+        const int second = (pos == kSecond1) ? 1 : (pos == kSecond2 ? 2 : 0);
+        const int nb = min(tb[0][lane], 4);
+        int ii, jj, lo, hi, sx, sy;
+        if (walk_target(S, G, a, bx, by, w, ii, jj, lo, hi, sx, sy)) {
+            const int dxs = w / 3 - 1, dys = w % 3 - 1;
+            walk_column(S, a, lo, hi, S.rank[a][i], izi, [&](int t, const float4 q, int dzs) {
+                const int j = __ldg(&S.perm[a][t]);
                 if (S.ctype[j] != kFungi) return;
+                if ((sx | sy) && !image_in_row(S, G, a, j, ii, jj, sx, sy)) return;
                 float r12f[3];
                 if (!rod_gate(S, G, P, a, j, dxs, dys, dzs, sx, sy, me, Lif, d2f_rn(S.clen[j]), xi, yi, zi, Li, r12f))
                     return;
-                any = true;
-                if (LIST) {
-                    if (cnt < kRodCap) {
-                        const int code = ((dxs + 1) * 9 + (dys + 1) * 3 + (dzs + 1)) | (((sx + 1) * 3 + (sy + 1)) << 5);
-                        S.rnb[(size_t)cnt * n + i] = make_int2(j, code);
-                    }
-                    ++cnt;
-                }
                 const int jid = S.id[j], jcpu = S.cpu[j];
-                // position fix-up (bmx_cell_interaction_K.H:338-362); the
-                // neighbour's position is only tested against TIP, which no
-                // thread writes, so reading it while others update theirs is safe
-                if (pos == kSecond1 || pos == kSecond2) {
-                    const int site = (pos == kSecond1) ? 1 : 2;
-                    const int nb = min(tb[0], 4);
-                    int k = 0;
-                    for (; k < nb; ++k)
-                        if (tb[1 + k] == jid && tb[5 + k] == jcpu && tb[9 + k] == site) break;
-                    if (k < nb && S.position[j] != kTip) pos = kInterior;
-                }
-                // half-bond repair of i (:370-467)
-                const bool i_to_j = find_in_table(tb, jid, jcpu) >= 0;
-                const bool j_to_i = find_in_plane_table(S.tab[a], n, j, iid, icpu) >= 0;
-                if (!i_to_j && j_to_i) {
-                    const int nb = tb[0];
-                    if (nb >= 0 && nb < 4) {
-                        const int isite = (fs == 0) ? (tb[9] == 1 ? 2 : 1) : fs;
-                        tb[1 + nb] = jid;
-                        tb[5 + nb] = jcpu;
-                        tb[9 + nb] = isite;
-                        tb[0] = nb + 1;
-                        ++rep;
+                // the first entry of i's table that names j (table_site), and whether
+                // one with the position's site does (the position fix-up)
+                int site = 0;
+                bool mine = false, at_site = false;
+                for (int k = nb - 1; k >= 0; --k)
+                    if (tb[1 + k][lane] == jid && tb[5 + k][lane] == jcpu) {
+                        mine = true;
+                        site = tb[9 + k][lane];
+                        at_site |= site == second;
                     }
+                if (second && at_site && S.position[j] != kTip) fixed[lane] = 1;
+                if (!mine && find_in_plane_table(S.tab[a], n, j, iid, icpu) >= 0) repair[lane] = 1;
+                if (cnt < kRodStage) {
+                    const int code = ((dxs + 1) * 9 + (dys + 1) * 3 + (dzs + 1)) | (((sx + 1) * 3 + (sy + 1)) << 5) |
+                                     (((site == 1 || site == 2) ? site : 0) << 9);
+                    M.stage[w * 32 + lane][cnt] = make_int2(j, code);
                 }
+                ++cnt;
             });
-            S.position[i] = pos;
-            if (any)
+        }
+    }
+    M.end[w][lane] = cnt;
+    walk_scan(M, kRodCap);
+    // the slots' own records
+    if (i < n) {
+        const bool walked = M.over[lane] || repair[lane];
+        if (walked) {
+            if (w == 0) book_slot(S, P, a, i);
+        } else {
+            for (int k = w; k < 13; k += kWalkCols) S.tab[b][(size_t)k * n + i] = tb[k][lane];
+            const bool any = M.end[kWalkCols - 1][lane] > 0;
+            if (w == 4) {
+                S.fflag[i] = 0;  // flag resets of bmx_pc_interaction.cpp:178-180
+                S.sflag[i] = 0;
+                S.nflag[i] = 0;
+                if (fixed[lane]) S.position[i] = kInterior;
+            }
+            if (w == 5 && any)
                 for (int k = 0; k < 6; ++k) S.dltd[(size_t)k * n + i] = -1;
-            if (rep) atomicAdd(&S.cnt->bond_repairs, (unsigned long long)rep);
         }
-        for (int k = 0; k < 13; ++k) S.tab[b][(size_t)k * n + i] = tb[k];
-        if (LIST) {
-            // the site of i that its repaired table bonds to each recorded
-            // neighbour (1 or 2, else 0) into bits 9-10
-            for (int k = 0; k < min(cnt, kRodCap); ++k) {
-                int2 &e = S.rnb[(size_t)k * n + i];
-                const int site = table_site(tb, S.id[e.x], S.cpu[e.x]);
-                e.y |= ((site == 1 || site == 2) ? site : 0) << 9;
+        if (w == 6) S.axf[i] = rod_axis32(S, a, i);
+        if (w == 7) S.rcnt[i] = M.over[lane] ? kRodCap + 1 : M.end[kWalkCols - 1][lane];
+    }
+    // the queue: one reservation per block and end
+    __syncthreads();  // (the repaired tables, written above, are read below)
+    const int total = M.first[32];
+    for (int t0 = 0; t0 < total; t0 += kWalkBlock) {
+        const int t = t0 + tid;
+        int o = 0, kind = -1, k = 0, mine = 0;
+        int2 e = make_int2(0, 0);
+        if (t < total) {
+            e = walk_pair(M, t, o);
+            k = t - M.first[o];
+            if (repair[o]) {  // the site in the repaired table
+                const int q = blockIdx.x * 32 + o;
+                const int jb = find_in_slot_table(S.tab[b], n, q, S.id[e.x], S.cpu[e.x]);
+                const int site = jb >= 0 ? S.tab[b][(size_t)(9 + jb) * n + q] : 0;
+                e.y = (e.y & 0x1ff) | (((site == 1 || site == 2) ? site : 0) << 9);
             }
-            S.rcnt[i] = cnt;
+            kind = ((e.y >> 9) & 3) ? 1 : 0;
         }
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const unsigned m = __ballot_sync(0xffffffffu, kind == q);
+            int base = 0;
+            if (lane == 0 && m) base = atomicAdd(&nq[q], __popc(m));
+            base = __shfl_sync(0xffffffffu, base, 0);
+            if (kind == q) mine = base + __popc(m & ((1u << lane) - 1u));
         }
-        if (MODE == kRodList) {
-            const int w = __reduce_max_sync(0xffffffffu, min(cnt, kRodCap));
-            if ((threadIdx.x & 31) == 0 && w > 0) atomicMax(&S.rctl->kmax, w);
+        __syncthreads();
+        if (tid < 2) {
+            at[tid] = nq[tid] ? atomicAdd(tid ? &S.rctl->nbond : &S.rctl->ncontact, nq[tid]) : 0;
+            nq[tid] = 0;
         }
-        if (MODE == kRodQueue) {
-            const int lane = threadIdx.x & 31;
-            const int x = (cnt <= kRodCap) ? cnt : 0;  // (a longer list is walked)
-            int o = x;
-            for (int q = 1; q < 32; q <<= 1) {
-                const int v = __shfl_up_sync(0xffffffffu, o, q);
-                if (lane >= q) o += v;
-            }
-            int at = 0;
-            if (lane == 31 && o > 0) at = atomicAdd(&S.rctl->nwork, o);
-            at = __shfl_sync(0xffffffffu, at, 31) + o - x;
-            for (int k = 0; k < x; ++k) S.rwork[at + k] = make_int2(i, k);
+        __syncthreads();
+        if (kind >= 0) {
+            const size_t slot = kind ? (size_t)n * kRodCap - 1 - (size_t)(at[1] + mine) : (size_t)(at[0] + mine);
+            S.rwork[slot] = make_int4(blockIdx.x * 32 + o, k, e.x, e.y);
         }
+        if (t0 + kWalkBlock < total) __syncthreads();
     }
 }
 
@@ -671,24 +801,23 @@ __global__ void __launch_bounds__(128) k_rod_force(const DevState S, const DevPa
 }
 
 // ---- flat pipelines -----------------------------------------------------------
-// With every segment's gated pairs recorded by k_rod_book, the force gather
-// runs flat instead of one stencil walk per thread (whose lanes diverge over
-// pair counts and, in the FP32F form, over the FP32 and FP64 paths).
-// Plain FP64 form: k_rod_book queues every pair, k_rod_pair64<true> evaluates
-// one per thread in full warps, k_rod_seg64 adds a segment's pairs in list
-// order (the walk's FP64 values in the walk's order: bit-identical to it).
-// GB300 issues FP64 at 2 lanes per clock per SM whatever the mask, and the walk
-// kept 6 of 32 lanes busy: 50 000 segments in 500 trees, 10 steps and the
-// load 8.29 -> 3.35 ms.
+// With every segment's gated pairs queued by k_rod_book, the force gather runs
+// flat, one pair per thread in full warps, instead of one stencil walk per
+// thread (whose lanes diverge over pair counts and, in the FP32F form, over the
+// FP32 and FP64 paths; GB300 issues FP64 at 2 lanes per clock per SM whatever
+// the mask, and the FP64 walk kept 6 of 32 lanes busy).
+// Plain FP64 form: k_rod_pair64 evaluates every pair, k_rod_seg64 adds a
+// segment's pairs in list order (the walk's FP64 values in the walk's order:
+// bit-identical to it).  50 000 segments in 500 trees, 10 steps and the load:
+// 8.29 -> 3.35 ms when the walk became this pipeline.
 // FP32F form:
-//   k_rod_pair32  one pair per thread (pair k of segment i); evaluates it in
-//                 FP32 where the FP32F form allows, else queues it;
-//   k_rod_pair64  the queued pairs, one per thread, in FP64 (full warps on
-//                 the FP64 pipe);
+//   k_rod_pair32  contacts in FP32 where the form allows (else queued for FP64),
+//                 bonded pairs' springs in FP64;
+//   k_rod_pair64q the queued contacts in FP64;
 //   k_rod_seg32   per segment: its pairs' f1 + f2 and f1 - f2 summed in FP64 in
 //                 list order, then mobility and surface force in FP32.
-// Each pair writes its own slot, so the sums do not depend on the order in
-// which the queue filled.
+// Each pair writes its own place, so the sums do not depend on the order in
+// which the queues filled.
 
 __device__ __forceinline__ void decode_pair(int code, int &dxs, int &dys, int &dzs, int &sx, int &sy)
 {
@@ -709,122 +838,130 @@ __device__ __forceinline__ void put_pair(const DevState &S, int i, int k, const 
     }
 }
 
+// Entry t of the queue: the contacts, then the bonded pairs.
+__device__ __forceinline__ int4 rod_entry(const DevState &S, int t, int ncontact)
+{
+    return S.rwork[t < ncontact ? (size_t)t : (size_t)S.n * kRodCap - 1 - (size_t)(t - ncontact)];
+}
+
+// The bonded sites of a pair that i's repaired table bonds at isite: both when
+// j's repaired table names i too.
+__device__ __forceinline__ bool mutual_sites(const DevState &S, int b, int i, int j, int isite, int &si, int &sj)
+{
+    si = sj = 0;
+    if (!isite) return false;
+    const int jb = find_in_plane_table(S.tab[b], S.n, j, S.id[i], S.cpu[i]);
+    if (jb < 0) return false;
+    const int s2 = __ldg(&S.tab[b][(size_t)(9 + jb) * S.n + j]);
+    if (s2 != 1 && s2 != 2) return false;
+    si = isite;
+    sj = s2;
+    return true;
+}
+
+// The pair of a queue entry in FP64 (bonded: si, sj in {1, 2}).
+__device__ __forceinline__ void rod_pair_fp64(const DevState &S, const DevParams &P, int a, const int4 e, int si,
+                                              int sj)
+{
+    const int i = e.x, j = e.z;
+    int dxs, dys, dzs, sx, sy;
+    decode_pair(e.w, dxs, dys, dzs, sx, sy);
+    const DevGeom &G = geom_of(S, i);
+    double d[3];
+    sep64(S, G, a, j, sx, sy, S.x[a][i], S.y[a][i], S.z[a][i], d);
+    const double4_32a tri = S.trig[a][i], trj = S.trig[a][j];
+    const double ni[3] = {tri.y * tri.z, tri.y * tri.w, tri.x};
+    const double nj[3] = {trj.y * trj.z, trj.y * trj.w, trj.x};
+    double f1[3], f2[3], sv[3], dv[3];
+    if (si && sj) {
+        double kb = P.k_bond;  // fusing tips (bmx_cell_interaction_K.H:552-600)
+        const int itip = S.fuse_tip[i], jtip = S.fuse_tip[j];
+        if ((itip > 0 && itip == si) || (jtip > 0 && jtip == sj)) kb = S.bscale[i] * S.bscale[j] * kb;
+        rod_spring(d, ni, S.clen[i], nj, S.clen[j], si, sj, kb, f1, f2);
+    } else {
+        const double rS = S.rad[i] + S.rad[j];
+        const double rA = rS + P.bw;
+        rod_site_forces<double>(d, ni, S.clen[i], nj, S.clen[j], rS, rA, P.k, 0, 0, 0.0, f1, f2);
+    }
+    for (int c = 0; c < 3; ++c) {
+        sv[c] = f1[c] + f2[c];
+        dv[c] = f1[c] - f2[c];
+    }
+    put_pair(S, i, e.y, sv, dv);
+}
+
 __global__ void __launch_bounds__(256) k_rod_pair32(const DevState S, const DevParams P, int a)
 {
     const int b = a ^ 1;
-    const int n = S.n;
-    const long long total = (long long)n * S.rctl->kmax;
+    const int nc = S.rctl->ncontact, total = nc + S.rctl->nbond;
     const int lane = threadIdx.x & 31;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
-         t += (long long)gridDim.x * blockDim.x) {
-        const int k = (int)(t / n);
-        const int i = (int)(t - (long long)k * n);
+    for (int t0 = blockIdx.x * blockDim.x; t0 < total; t0 += gridDim.x * blockDim.x) {
+        const int t = t0 + threadIdx.x;
         bool q64 = false;
-        int si = 0, sj = 0;
-        if (k < S.rcnt[i]) {
-            const int2 e = S.rnb[(size_t)k * n + i];
-            const int j = e.x;
-            int dxs, dys, dzs, sx, sy;
-            decode_pair(e.y, dxs, dys, dzs, sx, sy);
-            const DevGeom &G = geom_of(S, i);
-            const float4 me = S.rel[a][i], q = __ldg(&S.rel[a][j]);
-            // the offsets of the gate (rod_gate), recomputed
-            float r12f[3] = {(me.x - q.x) - (float)dxs * G.dxf[0], (me.y - q.y) - (float)dys * G.dxf[1],
-                             (me.z - q.z) - (float)dzs * G.dxf[2]};
-            // bonded: i's repaired table names j (the site k_rod_book found) and
-            // j's names i
-            const int isite = (e.y >> 9) & 3;
-            if (isite) {
-                const int jb = find_in_plane_table(S.tab[b], n, j, S.id[i], S.cpu[i]);
-                if (jb >= 0) {
-                    const int s2 = __ldg(&S.tab[b][(size_t)(9 + jb) * n + j]);
-                    si = isite;
-                    sj = (s2 == 1 || s2 == 2) ? s2 : 0;
-                }
-            }
-            // FP32 unless bonded, near-parallel or touching (as rod_force_slot)
-            q64 = true;
-            const float4 axi = S.axf[i], axj = __ldg(&S.axf[j]);
-            const float nif[3] = {axi.x, axi.y, axi.z};
-            const float njf[3] = {axj.x, axj.y, axj.z};
-            const float rij = nif[0] * njf[0] + nif[1] * njf[1] + nif[2] * njf[2];
-            if (!(si && sj) && 1.0f - rij * rij >= 0.05f) {
-                const float rSf = me.w + q.w;
-                float g1[3], g2[3], rf;
-                rod_site_forces<float>(r12f, nif, axi.w, njf, axj.w, rSf, rSf + P.bw32, P.k32, 0, 0, 0.0f, g1, g2,
-                                       &rf);
-                if (rf >= 0.01f * (axi.w + axj.w)) {
-                    double sv[3], dv[3];
-                    for (int c = 0; c < 3; ++c) {
-                        sv[c] = f2d_int(g1[c] + g2[c]);
-                        dv[c] = f2d_int(g1[c] - g2[c]);
+        if (t < total) {
+            const int4 e = rod_entry(S, t, nc);
+            const int i = e.x, j = e.z;
+            int si, sj;
+            if (mutual_sites(S, b, i, j, (e.w >> 9) & 3, si, sj)) {
+                rod_pair_fp64(S, P, a, e, si, sj);
+            } else {
+                int dxs, dys, dzs, sx, sy;
+                decode_pair(e.w, dxs, dys, dzs, sx, sy);
+                const DevGeom &G = geom_of(S, i);
+                const float4 me = S.rel[a][i], q = __ldg(&S.rel[a][j]);
+                // the offsets of the gate (rod_gate), recomputed
+                float r12f[3] = {(me.x - q.x) - (float)dxs * G.dxf[0], (me.y - q.y) - (float)dys * G.dxf[1],
+                                 (me.z - q.z) - (float)dzs * G.dxf[2]};
+                // FP32 unless near-parallel or touching (as rod_force_slot)
+                q64 = true;
+                const float4 axi = S.axf[i], axj = __ldg(&S.axf[j]);
+                const float nif[3] = {axi.x, axi.y, axi.z};
+                const float njf[3] = {axj.x, axj.y, axj.z};
+                const float rij = nif[0] * njf[0] + nif[1] * njf[1] + nif[2] * njf[2];
+                if (1.0f - rij * rij >= 0.05f) {
+                    const float rSf = me.w + q.w;
+                    float g1[3], g2[3], rf;
+                    rod_site_forces<float>(r12f, nif, axi.w, njf, axj.w, rSf, rSf + P.bw32, P.k32, 0, 0, 0.0f, g1,
+                                           g2, &rf);
+                    if (rf >= 0.01f * (axi.w + axj.w)) {
+                        double sv[3], dv[3];
+                        for (int c = 0; c < 3; ++c) {
+                            sv[c] = f2d_int(g1[c] + g2[c]);
+                            dv[c] = f2d_int(g1[c] - g2[c]);
+                        }
+                        put_pair(S, i, e.y, sv, dv);
+                        q64 = false;
                     }
-                    put_pair(S, i, k, sv, dv);
-                    q64 = false;
                 }
             }
         }
-        // queue the FP64 pairs, one atomic per warp
-        const unsigned am = __activemask();
-        const unsigned qm = __ballot_sync(am, q64);
+        // queue the FP64 contacts, one atomic per warp
+        const unsigned qm = __ballot_sync(0xffffffffu, q64);
         if (qm) {
-            const int leader = __ffs(qm) - 1;
             int base = 0;
-            if (lane == leader) base = atomicAdd(&S.rctl->nwork, __popc(qm));
-            base = __shfl_sync(am, base, leader);
-            if (q64) S.rwork[base + __popc(qm & ((1u << lane) - 1u))] = make_int2(i, k | (si << 8) | (sj << 12));
+            if (lane == 0) base = atomicAdd(&S.rctl->n64, __popc(qm));
+            base = __shfl_sync(0xffffffffu, base, 0);
+            if (q64) S.rq64[base + __popc(qm & ((1u << lane) - 1u))] = t;
         }
     }
 }
 
-// ALL: the queue holds every recorded pair (k_rod_book<kRodQueue>, the plain
-// FP64 form) and the pair's bonded sites are looked up here; else they come
-// with the queue entry (k_rod_pair32).
-template <bool ALL>
-__global__ void __launch_bounds__(128) k_rod_pair64(const DevState S, const DevParams P, int a)
+__global__ void __launch_bounds__(64) k_rod_pair64q(const DevState S, const DevParams P, int a)
+{
+    const int nc = S.rctl->ncontact, nw = S.rctl->n64;
+    for (int w = blockIdx.x * blockDim.x + threadIdx.x; w < nw; w += gridDim.x * blockDim.x)
+        rod_pair_fp64(S, P, a, rod_entry(S, S.rq64[w], nc), 0, 0);
+}
+
+__global__ void __launch_bounds__(64) k_rod_pair64(const DevState S, const DevParams P, int a)
 {
     const int b = a ^ 1;
-    const int n = S.n;
-    const int nw = S.rctl->nwork;
-    for (int w = blockIdx.x * blockDim.x + threadIdx.x; w < nw; w += gridDim.x * blockDim.x) {
-        const int2 it = S.rwork[w];
-        const int i = it.x, k = it.y & 255;
-        int si = (it.y >> 8) & 15, sj = (it.y >> 12) & 15;
-        const int2 e = S.rnb[(size_t)k * n + i];
-        const int j = e.x;
-        if (ALL) {
-            const int isite = (e.y >> 9) & 3;
-            if (isite) {
-                const int jb = find_in_plane_table(S.tab[b], n, j, S.id[i], S.cpu[i]);
-                if (jb >= 0) {
-                    const int s2 = __ldg(&S.tab[b][(size_t)(9 + jb) * n + j]);
-                    si = isite;
-                    sj = (s2 == 1 || s2 == 2) ? s2 : 0;
-                }
-            }
-        }
-        int dxs, dys, dzs, sx, sy;
-        decode_pair(e.y, dxs, dys, dzs, sx, sy);
-        const DevGeom &G = geom_of(S, i);
-        double kb = P.k_bond;
-        if (si && sj) {  // fusing tips (bmx_cell_interaction_K.H:552-600)
-            const int itip = S.fuse_tip[i], jtip = S.fuse_tip[j];
-            if ((itip > 0 && itip == si) || (jtip > 0 && jtip == sj)) kb = S.bscale[i] * S.bscale[j] * kb;
-        }
-        double d[3];
-        sep64(S, G, a, j, sx, sy, S.x[a][i], S.y[a][i], S.z[a][i], d);
-        const double4_32a tri = S.trig[a][i], trj = S.trig[a][j];
-        const double ni[3] = {tri.y * tri.z, tri.y * tri.w, tri.x};
-        const double nj[3] = {trj.y * trj.z, trj.y * trj.w, trj.x};
-        const double rS = S.rad[i] + S.rad[j];
-        const double rA = rS + P.bw;
-        double f1[3], f2[3], sv[3], dv[3];
-        rod_site_forces<double>(d, ni, S.clen[i], nj, S.clen[j], rS, rA, P.k, si, sj, kb, f1, f2);
-        for (int c = 0; c < 3; ++c) {
-            sv[c] = f1[c] + f2[c];
-            dv[c] = f1[c] - f2[c];
-        }
-        put_pair(S, i, k, sv, dv);
+    const int nc = S.rctl->ncontact, total = nc + S.rctl->nbond;
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
+        const int4 e = rod_entry(S, t, nc);
+        int si, sj;
+        mutual_sites(S, b, e.x, e.z, (e.w >> 9) & 3, si, sj);
+        rod_pair_fp64(S, P, a, e, si, sj);
     }
 }
 
@@ -1112,24 +1249,22 @@ int launch_load_rods(const DevState &S, const DevParams &P, const RodFields &F, 
     return 1;
 }
 
-int launch_rod_book(const DevState &S, const DevParams &P, int a, int precision, bool list, int grid, int block,
-                    cudaStream_t st)
+int launch_rod_book(const DevState &S, const DevParams &P, int a, bool list, int grid, int block, cudaStream_t st)
 {
-    if (!list) k_rod_book<kRodPlain><<<grid, block, 0, st>>>(S, P, a);
-    else if (precision == BMXG_FP64_FORM) k_rod_book<kRodQueue><<<grid, block, 0, st>>>(S, P, a);
-    else k_rod_book<kRodList><<<grid, block, 0, st>>>(S, P, a);
+    if (list) k_rod_book<<<(S.n + 31) / 32, kWalkBlock, sizeof(WalkMem<32, kRodStage>), st>>>(S, P, a);
+    else k_rod_book_plain<<<grid, block, 0, st>>>(S, P, a);
     return 1;
 }
 
 int launch_rod_pairs(const DevState &S, const DevParams &P, int a, int precision, int nsm, int n, cudaStream_t st)
 {
     if (precision == BMXG_FP64_FORM) {
-        k_rod_pair64<true><<<nsm * 8, 64, 0, st>>>(S, P, a);
+        k_rod_pair64<<<nsm * 16, 64, 0, st>>>(S, P, a);
         k_rod_seg64<<<(n + 63) / 64, 64, 0, st>>>(S, P, a);
         return 2;
     }
-    k_rod_pair32<<<nsm * 8, 256, 0, st>>>(S, P, a);
-    k_rod_pair64<false><<<nsm * 4, 128, 0, st>>>(S, P, a);
+    k_rod_pair32<<<nsm * 4, 256, 0, st>>>(S, P, a);
+    k_rod_pair64q<<<nsm * 4, 64, 0, st>>>(S, P, a);
     k_rod_seg32<<<(n + 127) / 128, 128, 0, st>>>(S, P, a);
     return 3;
 }
