@@ -747,7 +747,8 @@ int load_state(bmxg_ctx *ctx, const bmxg_particles *p, const int64_t *colony_off
         AL(S.clen, n); AL(S.area, n); AL(S.bscale, n);
         for (int k = 0; k < 2; ++k) { AL(S.theta[k], n); AL(S.phi[k], n); AL(S.trig[k], n); AL(S.tab[k], 13 * n); }
         AL(S.id, n); AL(S.cpu, n); AL(S.fuse_tip, n); AL(S.position, n); AL(S.fix_site, n);
-        AL(S.fflag, n); AL(S.sflag, n); AL(S.nflag, n); AL(S.dltd, 6 * n); AL(S.fc, 6 * n); AL(S.axf, n); AL(S.mob, n);
+        AL(S.fflag, n); AL(S.sflag, n); AL(S.nflag, n); AL(S.dltd, 6 * n); AL(S.fc, 6 * n); AL(S.mob, n);
+        AL(S.axf[0], n); AL(S.axf[1], n);
     }
     }  // !reuse
 #undef AL
@@ -1258,12 +1259,14 @@ int enqueue_step(bmxg_ctx *ctx, double dt, int precision, int a, int resync)
         const bool pipe = S.rwork != nullptr;
         LAUNCH(launch_rod_book(S, P, a, pipe, rg, ctx->sh_rod.block, st));
         if (k0) cudaEventRecord(k0, st);
-        if (pipe)
-            LAUNCH(launch_rod_pairs(S, P, a, precision, ctx->nsm, (int)n, st));
-        else
+        if (pipe) {
+            LAUNCH(launch_rod_pairs(S, P, dt, a, precision, ctx->nsm, (int)n, st));
+            if (k1) cudaEventRecord(k1, st);
+        } else {
             LAUNCH(launch_rod_force(S, P, a, rg, ctx->sh_rod.block, st));
-        if (k1) cudaEventRecord(k1, st);
-        LAUNCH(launch_rod_update(S, dt, a, mgrd, mblk, st));
+            if (k1) cudaEventRecord(k1, st);
+            LAUNCH(launch_rod_update(S, dt, a, mgrd, mblk, st));
+        }
     }
     LAUNCH(launch_rebuild(S, b, ctx->scan_scratch, mgrd, mblk, st, true));
     return BMXG_OK;

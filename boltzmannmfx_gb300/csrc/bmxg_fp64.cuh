@@ -297,6 +297,13 @@ BMXG_HD bool le_nonneg(double a, double b)
 {
     return bits64(a) <= bits64(b) && bits64(b) <= 0x7ff0000000000000ull;
 }
+// The comparisons in either precision (templates over the pair math).
+BMXG_HD bool lt_q(float a, float b) { return a < b; }
+BMXG_HD bool lt_q(double a, double b) { return lt_bits(a, b); }
+BMXG_HD bool le_q(float a, float b) { return a <= b; }
+BMXG_HD bool le_q(double a, double b) { return le_bits(a, b); }
+BMXG_HD bool zero_q(float a) { return a == 0.0f; }
+BMXG_HD bool zero_q(double a) { return (bits64(a) << 1) == 0; }
 // x + 0.0: a negative zero becomes zero, anything else stays
 BMXG_HD double plus_zero(double x) { return (bits64(x) << 1) ? x : 0.0; }
 

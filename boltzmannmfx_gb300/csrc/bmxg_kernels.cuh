@@ -105,7 +105,7 @@ struct DevState {
     int *position, *fix_site, *fflag, *sflag, *nflag;
     int *dltd;         // 6 planes
     double *fc;        // 6 planes, force gather of the rod path
-    float4 *axf;       // per segment, this step: FP32 axis (nx, ny, nz) and length (k_rod_book)
+    float4 *axf[2];    // FP32 axis (nx, ny, nz) and length of each segment
     double4_32a *mob;  // per segment: mobility (d0 + db, da - db, (d0 - db) / 2, 0) of its area,
                        // length and the viscosity (k_rod_mobility, on every state or parameter load)
     // rod pipelines (null until the first rod step): the queue of gated pairs
@@ -291,8 +291,10 @@ int launch_tile_step(const TileCall &C, const TileGeom &T, const DevParams &P, d
 int launch_rod_mobility(const DevState &S, const DevParams &P, int grid, int block, cudaStream_t st);
 // list: also queue the segments' gated pairs for the pipelines
 int launch_rod_book(const DevState &S, const DevParams &P, int a, bool list, int grid, int block, cudaStream_t st);
-// the pipelines after the bookkeeping: the queued pairs, then per-segment sums
-int launch_rod_pairs(const DevState &S, const DevParams &P, int a, int precision, int nsm, int n, cudaStream_t st);
+// the pipelines after the bookkeeping: the queued pairs, then per segment its
+// sums, velocity and update (launch_rod_force and launch_rod_update without the queues)
+int launch_rod_pairs(const DevState &S, const DevParams &P, double dt, int a, int precision, int nsm, int n,
+                     cudaStream_t st);
 int launch_rod_force(const DevState &S, const DevParams &P, int a, int grid, int block, cudaStream_t st);
 int launch_rod_update(const DevState &S, double dt, int a, int grid, int block, cudaStream_t st);
 // one ParticleExchange substep: conc / out 3 planes (A, B, C), slot order; xpar host

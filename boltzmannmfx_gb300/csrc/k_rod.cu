@@ -37,8 +37,14 @@ namespace bmxg {
 
 namespace {
 
+// FP32 axis and length of a segment
+__device__ __forceinline__ float4 rod_axis32(const double4_32a &tr, double L)
+{
+    return make_float4(d2f_rn(tr.y * tr.z), d2f_rn(tr.y * tr.w), d2f_rn(tr.x), d2f_rn(L));
+}
+
 template <class T>
-__device__ __forceinline__ bool in01(T t) { return t >= T(0) && t <= T(1); }
+__device__ __forceinline__ bool in01(T t) { return le_q(T(0), t) && le_q(t, T(1)); }
 
 template <class T>
 __device__ __forceinline__ T sq3(T a, T b, T c) { return a * a + b * b + c * c; }
@@ -65,10 +71,10 @@ __device__ void min_distance(const T *a1, const T *a2, const T *b1, const T *b2,
     const T Bj = w[0] * rj[0] + w[1] * rj[1] + w[2] * rj[2];
     T ti = T(0), tj = T(0);
     bool search = false;
-    if (Aij == T(0)) {
+    if (zero_q(Aij)) {
         ti = qdiv(Bi, Aii);
         tj = qdiv(Bj, Ajj);
-    } else if (det == T(0)) {
+    } else if (zero_q(det)) {
         const T t0 = qdiv(Bj, Ajj);
         if (in01(t0)) { ti = T(0); tj = t0; }
         else {
@@ -80,14 +86,14 @@ __device__ void min_distance(const T *a1, const T *a2, const T *b1, const T *b2,
         ti = qdiv(Ajj * Bi - Aij * Bj, det);
         tj = qdiv(Aii * Bj - Aij * Bi, det);
         if (in01(ti)) {
-            if (tj < T(0) || tj > T(1)) {
+            if (lt_q(tj, T(0)) || lt_q(T(1), tj)) {
                 const T t0 = qdiv(Bi, Aii), t1 = qdiv(Bi + rirj, Aii);
                 if (in01(t0) && in01(t1)) {
                     const T s0 = sq3(a1[0] + t0 * ri[0] - b1[0], a1[1] + t0 * ri[1] - b1[1],
                                      a1[2] + t0 * ri[2] - b1[2]);
                     const T s1 = sq3(a1[0] + t1 * ri[0] - b2[0], a1[1] + t1 * ri[1] - b2[1],
                                      a1[2] + t1 * ri[2] - b2[2]);
-                    if (s0 < s1) { tj = T(0); ti = t0; } else { tj = T(1); ti = t1; }
+                    if (lt_q(s0, s1)) { tj = T(0); ti = t0; } else { tj = T(1); ti = t1; }
                 } else if (in01(t0)) { tj = T(0); ti = t0; }
                 else if (in01(t1)) { tj = T(1); ti = t1; }
                 else search = true;
@@ -99,7 +105,7 @@ __device__ void min_distance(const T *a1, const T *a2, const T *b1, const T *b2,
                                  b1[2] + t0 * rj[2] - a1[2]);
                 const T s1 = sq3(b1[0] + t1 * rj[0] - a2[0], b1[1] + t1 * rj[1] - a2[1],
                                  b1[2] + t1 * rj[2] - a2[2]);
-                if (s0 < s1) { ti = T(0); tj = t0; } else { ti = T(1); tj = t1; }
+                if (lt_q(s0, s1)) { ti = T(0); tj = t0; } else { ti = T(1); tj = t1; }
             } else if (in01(t0)) { ti = T(0); tj = t0; }
             else if (in01(t1)) { ti = T(1); tj = t1; }
             else search = true;
@@ -115,7 +121,7 @@ __device__ void min_distance(const T *a1, const T *a2, const T *b1, const T *b2,
         m[3] = sq3(a2[0] - b2[0], a2[1] - b2[1], a2[2] - b2[2]);
         int best = 0;
         for (int k = 1; k < 4; ++k)
-            if (m[k] < m[best]) best = k;
+            if (lt_q(m[k], m[best])) best = k;
         ti = (best >= 2) ? T(1) : T(0);
         tj = (best & 1) ? T(1) : T(0);
     }
@@ -155,13 +161,13 @@ __device__ void rod_site_forces(const T *r12, const T *ni, T Li, const T *nj, T 
     if (r_out) *r_out = r;
     // r <= 1e-8: the reference keeps the unnormalised separation (its
     // fallback direction goes to shadowing locals, :744-746); so do we.
-    if (r > T(1.0e-8)) {
+    if (lt_q(T(1.0e-8), r)) {
         dv[0] = qdiv(dv[0], r);
         dv[1] = qdiv(dv[1], r);
         dv[2] = qdiv(dv[2], r);
     }
-    const T F = (r < rA) ? -k * (r - rA) * (r - rA) * (r - rS) : T(0);
-    if (F != T(0)) {
+    const T F = lt_q(r, rA) ? -k * (r - rA) * (r - rA) * (r - rS) : T(0);
+    if (!zero_q(F)) {
         for (int d = 0; d < 3; ++d) {
             f1[d] += F * dv[d] * (T(1) - ti);
             f2[d] += F * dv[d] * ti;
@@ -264,6 +270,46 @@ __device__ __forceinline__ bool rod_gate(const DevState &S, const DevGeom &G, co
     return r2 <= (rlm - kSmall) * (rlm - kSmall);
 }
 
+// Whether two segments are certainly beyond the contact range `reach` (then the
+// contact force is exactly zero), in FP32: q = the separation at a candidate
+// (s, t) of the closest points bounds the distance from above, and since
+// |w + s u - t v|^2 is convex, its slopes at (s, t) bound it from below over
+// the whole square.  The rounding of the FP32 offsets and axes enters with 4e-6 of
+// the squared lengths, far above it.  (Segments whose axes may be exactly
+// perpendicular are never clear: the reference then takes the closest points of
+// the unbounded lines.)
+__device__ __forceinline__ bool rod_clear32(const float *r12, const float4 axi, const float4 axj, float reach)
+{
+    const float u[3] = {axi.x * axi.w, axi.y * axi.w, axi.z * axi.w};
+    const float v[3] = {axj.x * axj.w, axj.y * axj.w, axj.z * axj.w};
+    float w[3];
+    float aa = 0.0f, bb = 0.0f, cc = 0.0f, dd = 0.0f, ee = 0.0f;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        w[k] = r12[k] - 0.5f * u[k] + 0.5f * v[k];
+        aa = __fmaf_rn(u[k], u[k], aa);
+        bb = __fmaf_rn(u[k], v[k], bb);
+        cc = __fmaf_rn(v[k], v[k], cc);
+        dd = __fmaf_rn(u[k], w[k], dd);
+        ee = __fmaf_rn(v[k], w[k], ee);
+    }
+    if (!(bb * bb > 1.0e-8f * aa * cc)) return false;
+    const float det = aa * cc - bb * bb;
+    float s = (det > 1.0e-5f * aa * cc) ? __saturatef(__fdividef(bb * ee - cc * dd, det)) : 0.5f;
+    const float t = __saturatef(__fdividef(bb * s + ee, cc));
+    s = __saturatef(__fdividef(bb * t - dd, aa));
+    float f = 0.0f, gs = 0.0f, gt = 0.0f;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const float q = w[k] + s * u[k] - t * v[k];
+        f = __fmaf_rn(q, q, f);
+        gs = __fmaf_rn(2.0f * u[k], q, gs);
+        gt = __fmaf_rn(-2.0f * v[k], q, gt);
+    }
+    const float low = f - fmaxf(gs * s, -gs * (1.0f - s)) - fmaxf(gt * t, -gt * (1.0f - t)) - 4.0e-6f * (aa + cc + f);
+    return low > 1.01f * reach * reach && reach >= 0.0f;  // (not finite: not clear)
+}
+
 // ---- bookkeeping ----------------------------------------------------------
 // The bookkeeping of segment i by a walk of its stencil: flag resets, position
 // fix-up, half-bond repair of its own table (buffer b).
@@ -330,20 +376,10 @@ __device__ void book_slot(const DevState &S, const DevParams &P, int a, int i)
     for (int k = 0; k < 13; ++k) S.tab[b][(size_t)k * n + i] = tb[k];
 }
 
-// this step's FP32 axis and length, for the FP32F pair math
-__device__ __forceinline__ float4 rod_axis32(const DevState &S, int a, int i)
-{
-    const double4_32a tr = S.trig[a][i];
-    return make_float4(d2f_rn(tr.y * tr.z), d2f_rn(tr.y * tr.w), d2f_rn(tr.x), d2f_rn(S.clen[i]));
-}
-
 // (contexts without room for the pipelines' queues)
 __global__ void k_rod_book_plain(const DevState S, const DevParams P, int a)
 {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < S.n; i += gridDim.x * blockDim.x) {
-        S.axf[i] = rod_axis32(S, a, i);
-        book_slot(S, P, a, i);
-    }
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < S.n; i += gridDim.x * blockDim.x) book_slot(S, P, a, i);
 }
 
 // The bookkeeping and the queue of gated pairs, one warp per neighbour column
@@ -365,7 +401,7 @@ __global__ void __launch_bounds__(kWalkBlock, 3) k_rod_book(const DevState S, co
     extern __shared__ __align__(16) unsigned char smw[];
     auto &M = *reinterpret_cast<WalkMem<32, kRodStage> *>(smw);
     __shared__ int tb[13][32];
-    __shared__ int repair[32], fixed[32];
+    __shared__ int repair[32], fixed[32], any[32];
     __shared__ int nq[2], at[2];
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const int b = a ^ 1;
@@ -376,6 +412,7 @@ __global__ void __launch_bounds__(kWalkBlock, 3) k_rod_book(const DevState S, co
     if (w == 0) {
         repair[lane] = 0;
         fixed[lane] = 0;
+        any[lane] = 0;
     }
     if (tid < 2) nq[tid] = 0;
     __syncthreads();
@@ -387,7 +424,7 @@ __global__ void __launch_bounds__(kWalkBlock, 3) k_rod_book(const DevState S, co
         const int izi = S.iz[a][i];
         const double xi = S.x[a][i], yi = S.y[a][i], zi = S.z[a][i];
         const double Li = S.clen[i];
-        const float Lif = d2f_rn(Li);
+        const float4 axi = S.axf[a][i];
         const float4 me = S.rel[a][i];
         const int iid = S.id[i], icpu = S.cpu[i];
         const int pos = S.position[i];
@@ -401,8 +438,9 @@ __global__ void __launch_bounds__(kWalkBlock, 3) k_rod_book(const DevState S, co
                 if (S.ctype[j] != kFungi) return;
                 if ((sx | sy) && !image_in_row(S, G, a, j, ii, jj, sx, sy)) return;
                 float r12f[3];
-                if (!rod_gate(S, G, P, a, j, dxs, dys, dzs, sx, sy, me, Lif, d2f_rn(S.clen[j]), xi, yi, zi, Li, r12f))
-                    return;
+                const float4 axj = __ldg(&S.axf[a][j]);
+                if (!rod_gate(S, G, P, a, j, dxs, dys, dzs, sx, sy, me, axi.w, axj.w, xi, yi, zi, Li, r12f)) return;
+                any[lane] = 1;
                 const int jid = S.id[j], jcpu = S.cpu[j];
                 // the first entry of i's table that names j (table_site), and whether
                 // one with the position's site does (the position fix-up)
@@ -415,7 +453,10 @@ __global__ void __launch_bounds__(kWalkBlock, 3) k_rod_book(const DevState S, co
                         at_site |= site == second;
                     }
                 if (second && at_site && S.position[j] != kTip) fixed[lane] = 1;
-                if (!mine && find_in_plane_table(S.tab[a], n, j, iid, icpu) >= 0) repair[lane] = 1;
+                const bool half = !mine && find_in_plane_table(S.tab[a], n, j, iid, icpu) >= 0;
+                if (half) repair[lane] = 1;
+                // a contact out of range adds exact zeros: not queued
+                if (!half && site != 1 && site != 2 && rod_clear32(r12f, axi, axj, me.w + q.w + P.bw32)) return;
                 if (cnt < kRodStage) {
                     const int code = ((dxs + 1) * 9 + (dys + 1) * 3 + (dzs + 1)) | (((sx + 1) * 3 + (sy + 1)) << 5) |
                                      (((site == 1 || site == 2) ? site : 0) << 9);
@@ -434,17 +475,15 @@ __global__ void __launch_bounds__(kWalkBlock, 3) k_rod_book(const DevState S, co
             if (w == 0) book_slot(S, P, a, i);
         } else {
             for (int k = w; k < 13; k += kWalkCols) S.tab[b][(size_t)k * n + i] = tb[k][lane];
-            const bool any = M.end[kWalkCols - 1][lane] > 0;
             if (w == 4) {
                 S.fflag[i] = 0;  // flag resets of bmx_pc_interaction.cpp:178-180
                 S.sflag[i] = 0;
                 S.nflag[i] = 0;
                 if (fixed[lane]) S.position[i] = kInterior;
             }
-            if (w == 5 && any)
+            if (w == 5 && any[lane])
                 for (int k = 0; k < 6; ++k) S.dltd[(size_t)k * n + i] = -1;
         }
-        if (w == 6) S.axf[i] = rod_axis32(S, a, i);
         if (w == 7) S.rcnt[i] = M.over[lane] ? kRodCap + 1 : M.end[kWalkCols - 1][lane];
     }
     // the queue: one reservation per block and end
@@ -558,7 +597,9 @@ __global__ void __launch_bounds__(128) k_load_rods(const DevState S, const DevPa
         double st, ct, sp, cp;
         sincos(th, &st, &ct);
         sincos(ph, &sp, &cp);
-        S.trig[0][s] = make_trig(ct, st, cp, sp);
+        const double4_32a tr = make_trig(ct, st, cp, sp);
+        S.trig[0][s] = tr;
+        S.axf[0][s] = rod_axis32(tr, L);
         S.mob[s] = rod_mobility(S.ctype[s], L, area, P);
     }
 }
@@ -707,12 +748,12 @@ __device__ __forceinline__ void rod_force_slot(const DevState &S, const DevParam
 #pragma unroll
             for (int k = 0; k < 13; ++k) tb[k] = S.tab[b][(size_t)k * n + i];
             const float4 me = S.rel[a][i];
-            const float4 axi = S.axf[i];  // FP32 axis and length (k_rod_book)
+            const float4 axi = S.axf[a][i];  // FP32 axis and length
             double Sv[3] = {0.0, 0.0, 0.0}, Dv[3] = {0.0, 0.0, 0.0};
             float Svf[3] = {0.0f, 0.0f, 0.0f}, Dvf[3] = {0.0f, 0.0f, 0.0f};  // the FP32F pairs' sums
             visit_stencil(S, G, a, i, bx, by, izi, [&](int j, int dxs, int dys, int dzs, int sx, int sy) {
                 if (S.ctype[j] != kFungi) return;
-                const float4 axj = __ldg(&S.axf[j]);
+                const float4 axj = __ldg(&S.axf[a][j]);
                 float r12f[3];
                 if (!rod_gate(S, G, P, a, j, dxs, dys, dzs, sx, sy, me, axi.w, axj.w, xi, yi, zi, Li, r12f)) return;
                 // bonds: mutual entries in both (repaired) tables
@@ -806,7 +847,7 @@ __global__ void __launch_bounds__(128) k_rod_force(const DevState S, const DevPa
 // thread (whose lanes diverge over pair counts and, in the FP32F form, over the
 // FP32 and FP64 paths; GB300 issues FP64 at 2 lanes per clock per SM whatever
 // the mask, and the FP64 walk kept 6 of 32 lanes busy).
-// Plain FP64 form: k_rod_pair64 evaluates every pair, k_rod_seg64 adds a
+// Plain FP64 form: k_rod_pair64 evaluates every pair, k_rod_seg adds a
 // segment's pairs in list order (the walk's FP64 values in the walk's order:
 // bit-identical to it).  50 000 segments in 500 trees, 10 steps and the load:
 // 8.29 -> 3.35 ms when the walk became this pipeline.
@@ -814,8 +855,9 @@ __global__ void __launch_bounds__(128) k_rod_force(const DevState S, const DevPa
 //   k_rod_pair32  contacts in FP32 where the form allows (else queued for FP64),
 //                 bonded pairs' springs in FP64;
 //   k_rod_pair64q the queued contacts in FP64;
-//   k_rod_seg32   per segment: its pairs' f1 + f2 and f1 - f2 summed in FP64 in
-//                 list order, then mobility and surface force in FP32.
+//   k_rod_seg     per segment: its pairs' f1 + f2 and f1 - f2 summed in FP64 in
+//                 list order, then mobility and surface force in FP32, and the
+//                 update.
 // Each pair writes its own place, so the sums do not depend on the order in
 // which the queues filled.
 
@@ -914,7 +956,7 @@ __global__ void __launch_bounds__(256) k_rod_pair32(const DevState S, const DevP
                                  (me.z - q.z) - (float)dzs * G.dxf[2]};
                 // FP32 unless near-parallel or touching (as rod_force_slot)
                 q64 = true;
-                const float4 axi = S.axf[i], axj = __ldg(&S.axf[j]);
+                const float4 axi = S.axf[a][i], axj = __ldg(&S.axf[a][j]);
                 const float nif[3] = {axi.x, axi.y, axi.z};
                 const float njf[3] = {axj.x, axj.y, axj.z};
                 const float rij = nif[0] * njf[0] + nif[1] * njf[1] + nif[2] * njf[2];
@@ -965,137 +1007,132 @@ __global__ void __launch_bounds__(64) k_rod_pair64(const DevState S, const DevPa
     }
 }
 
-__global__ void __launch_bounds__(128) k_rod_seg32(const DevState S, const DevParams P, int a)
-{
-    const int n = S.n;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int cnt = S.rcnt[i];
-        if (S.ctype[i] != kFungi || cnt > kRodCap) {
-            // spheres of a mixed state, and a segment with more pairs than the
-            // lists hold: the walk
-            rod_force_slot<BMXG_FP32F_FORM>(S, P, a, i);
-            continue;
-        }
-        double Sv[3] = {0.0, 0.0, 0.0}, Dv[3] = {0.0, 0.0, 0.0};
-        for (int k = 0; k < cnt; ++k)
-            for (int c = 0; c < 3; ++c) {
-                Sv[c] += S.rres[((size_t)c * kRodCap + k) * n + i];
-                Dv[c] += S.rres[((size_t)(3 + c) * kRodCap + k) * n + i];
-            }
-        const float4 axi = S.axf[i];
-        float sv[3], dv[3], af[6];
-        for (int c = 0; c < 3; ++c) {
-            sv[c] = d2f_rn(Sv[c]);
-            dv[c] = d2f_rn(Dv[c]);
-        }
-        const float nif[3] = {axi.x, axi.y, axi.z};
-        rod_velocity32(nif, axi.w, sv, dv, S.mob[i], d2f_rn(S.z[a][i] - P.z_wall), S.rel[a][i].w, P, af);
-        for (int c = 0; c < 6; ++c) S.fc[(size_t)c * n + i] = f2d_int(af[c]);
-        S.fix_site[i] = 0;  // evaluateSurfaceForce (bmx_cell_interaction_K.H:1060)
-    }
-}
-
-// The plain FP64 form's segments: the pairs' sums in list order, as the walk
-// adds them, then mobility and surface force in FP64.
-__global__ void __launch_bounds__(64) k_rod_seg64(const DevState S, const DevParams P, int a)
-{
-    const int n = S.n;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int cnt = S.rcnt[i];
-        if (S.ctype[i] != kFungi || cnt > kRodCap) {
-            rod_force_slot<BMXG_FP64_FORM>(S, P, a, i);
-            continue;
-        }
-        double Sv[3] = {0.0, 0.0, 0.0}, Dv[3] = {0.0, 0.0, 0.0};
-        for (int k = 0; k < cnt; ++k)
-            for (int c = 0; c < 3; ++c) {
-                Sv[c] += S.rres[((size_t)c * kRodCap + k) * n + i];
-                Dv[c] += S.rres[((size_t)(3 + c) * kRodCap + k) * n + i];
-            }
-        const double4_32a tri = S.trig[a][i];
-        const double ni[3] = {tri.y * tri.z, tri.y * tri.w, tri.x};
-        double acc[6];
-        rod_velocity64(ni, S.clen[i], Sv, Dv, S.mob[i], S.x[a][i], S.y[a][i], S.z[a][i], S.rad[i], P, acc);
-        for (int c = 0; c < 6; ++c) S.fc[(size_t)c * n + i] = acc[c];
-        S.fix_site[i] = 0;  // evaluateSurfaceForce (bmx_cell_interaction_K.H:1060)
-    }
-}
-
 // ---- update ---------------------------------------------------------------
-__global__ void k_rod_update(const DevState S, double dt, int a)
+// The update of slot i from its velocity fc[0..2] and rotation fc[3..5].
+__device__ __forceinline__ void rod_update_slot(const DevState &S, double dt, int a, int i, const double *fc)
 {
     const int b = a ^ 1;
-    const int n = S.n;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const DevGeom &G = geom_of(S, i);
-        const double v[3] = {S.fc[i], S.fc[(size_t)n + i], S.fc[(size_t)2 * n + i]};
-        const double w[3] = {S.fc[(size_t)3 * n + i], S.fc[(size_t)4 * n + i], S.fc[(size_t)5 * n + i]};
-        S.vx[i] = v[0];
-        S.vy[i] = v[1];
-        S.vz[i] = v[2];
-        S.wx[i] = w[0];
-        S.wy[i] = w[1];
-        S.wz[i] = w[2];
-        double nx = S.x[a][i] + dt * v[0];
-        double ny = S.y[a][i] + dt * v[1];
-        const double nz = S.z[a][i] + dt * v[2];
-        double th = S.theta[a][i], ph = S.phi[a][i];
-        double4_32a tr = S.trig[a][i];
-        if (S.ctype[i] == kFungi) {
-            // rotate the axis by |omega| dt (bmx_pc_interaction.cpp:334-431)
-            const double ct = tr.x, st = tr.y, cp = tr.z, sp = tr.w;
-            const double R[3][3] = {{cp * st, -sp, -cp * ct}, {sp * st, cp, -sp * ct}, {ct, 0.0, st}};
-            double om[3];
-            for (int r = 0; r < 3; ++r) {
-                om[r] = 0.0;
-                for (int c = 0; c < 3; ++c) om[r] += R[c][r] * w[c];
-            }
-            const double L = S.clen[i];
-            om[0] = 0.0;
-            const double oL = div_rn(2.0, L * L);
-            om[1] *= oL;
-            om[2] *= oL;
-            Divisor by;
-            const double on = sqrt_rn(om[1] * om[1] + om[2] * om[2], &by);
-            if (on > 0.0) {
-                om[1] = div_by(om[1], by);
-                om[2] = div_by(om[2], by);
-            }
-            const double c = om[2], s = om[1];
-            const double Q[3][3] = {{1.0, 0.0, 0.0}, {0.0, c, -s}, {0.0, s, c}};
-            const double ang = on * dt;
-            double sa, ca;
-            sincos(ang, &sa, &ca);  // one argument reduction for both
-            const double u[3] = {ca, sa, 0.0};
-            double q[3], nd[3];
-            for (int r = 0; r < 3; ++r) {
-                q[r] = 0.0;
-                for (int cc = 0; cc < 3; ++cc) q[r] += Q[cc][r] * u[cc];
-            }
-            for (int r = 0; r < 3; ++r) {
-                nd[r] = 0.0;
-                for (int cc = 0; cc < 3; ++cc) nd[r] += R[r][cc] * q[cc];
-            }
-            th = acos(nd[2]);
-            const double rho = sqrt_rn(nd[0] * nd[0] + nd[1] * nd[1], &by);
-            if (rho > 0.0) nd[0] = div_by(nd[0], by);
-            ph = acos(nd[0]);
-            if (nd[1] < 0.0) ph = 2.0 * kPi - ph;
-            double st2, ct2, sp2, cp2;
-            sincos(th, &st2, &ct2);
-            sincos(ph, &sp2, &cp2);
-            tr = make_trig(ct2, st2, cp2, sp2);
+    const DevGeom &G = geom_of(S, i);
+    const double v[3] = {fc[0], fc[1], fc[2]}, w[3] = {fc[3], fc[4], fc[5]};
+    S.vx[i] = v[0];
+    S.vy[i] = v[1];
+    S.vz[i] = v[2];
+    S.wx[i] = w[0];
+    S.wy[i] = w[1];
+    S.wz[i] = w[2];
+    double nx = S.x[a][i] + dt * v[0];
+    double ny = S.y[a][i] + dt * v[1];
+    const double nz = S.z[a][i] + dt * v[2];
+    double th = S.theta[a][i], ph = S.phi[a][i];
+    double4_32a tr = S.trig[a][i];
+    if (S.ctype[i] == kFungi) {
+        // rotate the axis by |omega| dt (bmx_pc_interaction.cpp:334-431)
+        const double ct = tr.x, st = tr.y, cp = tr.z, sp = tr.w;
+        const double R[3][3] = {{cp * st, -sp, -cp * ct}, {sp * st, cp, -sp * ct}, {ct, 0.0, st}};
+        double om[3];
+        for (int r = 0; r < 3; ++r) {
+            om[r] = 0.0;
+            for (int c = 0; c < 3; ++c) om[r] += R[c][r] * w[c];
         }
-        S.theta[b][i] = th;
-        S.phi[b][i] = ph;
-        S.trig[b][i] = tr;
-        if (G.per[0]) nx = wrap1(nx, G.plo[0], G.phi[0], G.len[0]);
-        if (G.per[1]) ny = wrap1(ny, G.plo[1], G.phi[1], G.len[1]);
-        S.x[b][i] = nx;
-        S.y[b][i] = ny;
-        S.z[b][i] = nz;
-        rebin_slot(S, G, i, nx, ny, nz, S.rad[i], b);
+        const double L = S.clen[i];
+        om[0] = 0.0;
+        const double oL = div_rn(2.0, L * L);
+        om[1] *= oL;
+        om[2] *= oL;
+        Divisor by;
+        const double on = sqrt_rn(om[1] * om[1] + om[2] * om[2], &by);
+        if (on > 0.0) {
+            om[1] = div_by(om[1], by);
+            om[2] = div_by(om[2], by);
+        }
+        const double c = om[2], s = om[1];
+        const double Q[3][3] = {{1.0, 0.0, 0.0}, {0.0, c, -s}, {0.0, s, c}};
+        const double ang = on * dt;
+        double sa, ca;
+        sincos(ang, &sa, &ca);  // one argument reduction for both
+        const double u[3] = {ca, sa, 0.0};
+        double q[3], nd[3];
+        for (int r = 0; r < 3; ++r) {
+            q[r] = 0.0;
+            for (int cc = 0; cc < 3; ++cc) q[r] += Q[cc][r] * u[cc];
+        }
+        for (int r = 0; r < 3; ++r) {
+            nd[r] = 0.0;
+            for (int cc = 0; cc < 3; ++cc) nd[r] += R[r][cc] * q[cc];
+        }
+        th = acos(nd[2]);
+        const double rho = sqrt_rn(nd[0] * nd[0] + nd[1] * nd[1], &by);
+        if (rho > 0.0) nd[0] = div_by(nd[0], by);
+        ph = acos(nd[0]);
+        if (nd[1] < 0.0) ph = 2.0 * kPi - ph;
+        double st2, ct2, sp2, cp2;
+        sincos(th, &st2, &ct2);
+        sincos(ph, &sp2, &cp2);
+        tr = make_trig(ct2, st2, cp2, sp2);
     }
+    S.theta[b][i] = th;
+    S.phi[b][i] = ph;
+    S.trig[b][i] = tr;
+    S.axf[b][i] = rod_axis32(tr, S.clen[i]);
+    if (G.per[0]) nx = wrap1(nx, G.plo[0], G.phi[0], G.len[0]);
+    if (G.per[1]) ny = wrap1(ny, G.plo[1], G.phi[1], G.len[1]);
+    S.x[b][i] = nx;
+    S.y[b][i] = ny;
+    S.z[b][i] = nz;
+    rebin_slot(S, G, i, nx, ny, nz, S.rad[i], b);
+}
+
+// (contexts without room for the pipelines' queues, after k_rod_force)
+__global__ void k_rod_update(const DevState S, double dt, int a)
+{
+    const size_t n = (size_t)S.n;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < S.n; i += gridDim.x * blockDim.x) {
+        double fc[6];
+        for (int c = 0; c < 6; ++c) fc[c] = S.fc[c * n + i];
+        rod_update_slot(S, dt, a, i, fc);
+    }
+}
+
+// A segment's pairs summed in list order, as the walk adds them, then mobility,
+// surface force and update in one pass (the six force planes between a segment
+// and an update kernel never leave the registers).  Spheres of a mixed state,
+// and segments with more pairs than the queue holds: the walk.
+template <int PREC>
+__global__ void __launch_bounds__(64) k_rod_seg(const DevState S, const DevParams P, double dt, int a)
+{
+    const size_t n = (size_t)S.n;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= S.n) return;
+    double fc[6];
+    const int cnt = S.rcnt[i];
+    if (S.ctype[i] != kFungi || cnt > kRodCap) {
+        rod_force_slot<PREC>(S, P, a, i);
+        for (int c = 0; c < 6; ++c) fc[c] = S.fc[c * n + i];
+    } else {
+        double Sv[3] = {0.0, 0.0, 0.0}, Dv[3] = {0.0, 0.0, 0.0};
+        for (int k = 0; k < cnt; ++k)
+            for (int c = 0; c < 3; ++c) {
+                Sv[c] += S.rres[((size_t)c * kRodCap + k) * n + i];
+                Dv[c] += S.rres[((size_t)(3 + c) * kRodCap + k) * n + i];
+            }
+        if (PREC == BMXG_FP64_FORM) {
+            const double4_32a tri = S.trig[a][i];
+            const double ni[3] = {tri.y * tri.z, tri.y * tri.w, tri.x};
+            rod_velocity64(ni, S.clen[i], Sv, Dv, S.mob[i], S.x[a][i], S.y[a][i], S.z[a][i], S.rad[i], P, fc);
+        } else {
+            const float4 axi = S.axf[a][i];
+            float sv[3], dv[3], af[6];
+            for (int c = 0; c < 3; ++c) {
+                sv[c] = d2f_rn(Sv[c]);
+                dv[c] = d2f_rn(Dv[c]);
+            }
+            const float nif[3] = {axi.x, axi.y, axi.z};
+            rod_velocity32(nif, axi.w, sv, dv, S.mob[i], d2f_rn(S.z[a][i] - P.z_wall), S.rel[a][i].w, P, af);
+            for (int c = 0; c < 6; ++c) fc[c] = f2d_int(af[c]);
+        }
+        S.fix_site[i] = 0;  // evaluateSurfaceForce (bmx_cell_interaction_K.H:1060)
+    }
+    rod_update_slot(S, dt, a, i, fc);
 }
 
 // ---- InitBonds ---------------------------------------------------------------
@@ -1256,16 +1293,18 @@ int launch_rod_book(const DevState &S, const DevParams &P, int a, bool list, int
     return 1;
 }
 
-int launch_rod_pairs(const DevState &S, const DevParams &P, int a, int precision, int nsm, int n, cudaStream_t st)
+int launch_rod_pairs(const DevState &S, const DevParams &P, double dt, int a, int precision, int nsm, int n,
+                     cudaStream_t st)
 {
+    const int grid = (n + 63) / 64;
     if (precision == BMXG_FP64_FORM) {
-        k_rod_pair64<<<nsm * 16, 64, 0, st>>>(S, P, a);
-        k_rod_seg64<<<(n + 63) / 64, 64, 0, st>>>(S, P, a);
+        k_rod_pair64<<<nsm * 8, 64, 0, st>>>(S, P, a);
+        k_rod_seg<BMXG_FP64_FORM><<<grid, 64, 0, st>>>(S, P, dt, a);
         return 2;
     }
-    k_rod_pair32<<<nsm * 4, 256, 0, st>>>(S, P, a);
+    k_rod_pair32<<<nsm * 4, 128, 0, st>>>(S, P, a);
     k_rod_pair64q<<<nsm * 4, 64, 0, st>>>(S, P, a);
-    k_rod_seg32<<<(n + 127) / 128, 128, 0, st>>>(S, P, a);
+    k_rod_seg<BMXG_FP32F_FORM><<<grid, 64, 0, st>>>(S, P, dt, a);
     return 3;
 }
 
