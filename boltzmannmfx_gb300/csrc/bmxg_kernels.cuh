@@ -35,6 +35,10 @@ struct ListCtl {
     int max_age;           // rebuild at least this often (bounds FP32 offset drift)
     int force;             // rebuild at the next step (the state changed)
     int rebuild;           // this step's decision (read by the gated kernels)
+    int need;              // a build is due; set where none can run, the steps stall until one can
+    int active;            // the step that follows runs (there are steps left, no build is due)
+    int cur;               // ... reading the fixed-point positions of this buffer
+    int left, par;         // steps left in the call and the buffer the next one reads (set by the host)
     int builds;            // builds decided so far
     unsigned long long body_runs;  // builds actually run (counted by the first build kernel)
     unsigned long long overflow;   // slots whose list exceeded the capacity (last build)
@@ -235,28 +239,31 @@ int launch_sphere_step(const DevState &S, const DevParams &P, double dt, int a, 
                         int grid, int block, cudaStream_t st, int resync = 1, bool pinned = false);
 
 // ---- FP32F neighbour list with a skin (k_list.cu) --------------------------
-// decide: fold the last step's displacement into the bound and decide
-// whether this step rebuilds; sets the graph conditional `cond` when use_cond
-int launch_list_decide(const DevState &S, unsigned long long cond, int use_cond, cudaStream_t st);
+// decide: fold the last step's displacement into the bound and decide whether
+// this step rebuilds.  What follows it in the stream: kDecideStall no build (a
+// step that needs one does not run, nor the ones after it), kDecideCond a
+// conditional node (cond) with the build, kDecideBuild the gated build kernels.
+enum { kDecideStall = 0, kDecideCond = 1, kDecideBuild = 2 };
+int launch_list_decide(const DevState &S, unsigned long long cond, int mode, cudaStream_t st);
 // fixed-point positions of buffer a from its FP64 positions and radii (when the
 // list starts on a state), and back (whenever the FP64 positions are read)
 int launch_list_init(const DevState &S, int a, int grid, int block, cudaStream_t st);
 int launch_list_to_fp64(const DevState &S, int a, int grid, int block, cudaStream_t st);
 // axis ax (0 x, 1 y, 2 z) of it, also scattered to out in the caller's order (out[orig[i]])
 int launch_list_to_fp64_axis(const DevState &S, int a, int ax, double *out, int block, cudaStream_t st);
-// rebuild (gated on lctl->rebuild): bins of buffer a's positions into the
+// rebuild (gated on lctl->rebuild): bins of buffer lctl->cur's positions into the
 // list bins, column lists, and the list itself
 // (returns the kernels it enqueues, kListBodyKernels)
-int launch_list_rebuild(const DevState &S, const DevParams &P, int a, int *scan_scratch, int grid, int block,
+int launch_list_rebuild(const DevState &S, const DevParams &P, int *scan_scratch, int grid, int block,
                         int build_block, cudaStream_t st);
 // the list build kernel alone (gated on lctl->rebuild), build_block threads per block
 int launch_list_build(const DevState &S, const DevParams &P, int build_block, cudaStream_t st);
 constexpr int kListBodyKernels = 12;
-// force + wall + update over the list, reading buffer a and writing buffer b
-// (grid = the SM count; passes of the block per chunk of slots, <= 0: a rule;
+// force + wall + update over the list, reading buffer lctl->cur and writing the
+// other, or nothing when the step is not active (grid = the SM count; passes of the block per chunk of slots, <= 0: a rule;
 // persistent: one wave of blocks taking chunks from a counter, else one block
 // per chunk)
-int launch_list_step(const DevState &S, const DevParams &P, double dt, int a, int grid, int block, int passes,
+int launch_list_step(const DevState &S, const DevParams &P, double dt, int grid, int block, int passes,
                      cudaStream_t st, bool persistent = false);
 
 // ---- one tile with the caller's ghosts (k_tile.cu) -------------------------

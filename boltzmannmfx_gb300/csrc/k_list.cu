@@ -94,42 +94,61 @@ __device__ __forceinline__ long long fx_inc(float f, float c, float cl, bool &bi
 // drift common to all slots (here: the rise of the slots below the growth
 // surface).  Each step adds eps_step per component for the FP32 rounding of
 // the pair offsets the gate sees.
-// It also clears the per-step counters (no memset nodes in the step).
-__global__ void k_list_decide(ListCtl *c, DevCounters *cnt, cudaGraphConditionalHandle h, int use_h)
+// It also clears the per-step counters (no memset nodes in the step), counts
+// the call's steps down and names the buffer the step reads, so that steps can
+// be enqueued without knowing which of them will run: see kDecideStall.
+__global__ void k_list_decide(ListCtl *c, DevCounters *cnt, cudaGraphConditionalHandle h, int mode)
 {
-    cnt->out_of_domain = 0ull;
-    cnt->edge_ghost = 0ull;
-    cnt->pairs = 0ull;
-    cnt->bond_repairs = 0ull;
-    cnt->moved = 0ull;
-    float r2 = 0.0f;
-    float rg[3];
-    for (int k = 0; k < 3; ++k) {
-        const unsigned lo = c->inc_min[k], hi = c->inc_max[k];
-        // no slot reported (empty state): no spread
-        const float spread = (hi >= lo) ? (funkey(hi) - funkey(lo)) : 0.0f;
-        rg[k] = c->range[k] + spread * 1.000001f + c->eps_step;
-        r2 += rg[k] * rg[k];
-        c->inc_min[k] = kKeyPosInf;
-        c->inc_max[k] = kKeyNegInf;
+    bool run = c->left > 0;
+    bool rb = false;
+    if (run) {
+        bool need = c->need != 0;
+        if (!need) {
+            float r2 = 0.0f;
+            float rg[3];
+            for (int k = 0; k < 3; ++k) {
+                const unsigned lo = c->inc_min[k], hi = c->inc_max[k];
+                // no slot reported (empty state): no spread
+                const float spread = (hi >= lo) ? (funkey(hi) - funkey(lo)) : 0.0f;
+                rg[k] = c->range[k] + spread * 1.000001f + c->eps_step;
+                r2 += rg[k] * rg[k];
+                c->inc_min[k] = kKeyPosInf;
+                c->inc_max[k] = kKeyNegInf;
+                c->range[k] = rg[k];
+            }
+            const float acc = sqrtf(r2);
+            const int age = c->age + 1;
+            need = c->force != 0 || !(acc <= c->skin) || age > c->max_age;
+            c->acc = acc;
+            c->age = age;
+        }
+        if (need && mode != kDecideStall) {
+            rb = true;
+            need = false;
+            for (int k = 0; k < 3; ++k) c->range[k] = 0.0f;
+            c->acc = 0.0f;
+            c->age = 0;
+            c->force = 0;
+            c->builds += 1;
+            c->overflow = 0ull;
+        }
+        c->need = need ? 1 : 0;
+        run = !need;
+        if (run) {
+            cnt->out_of_domain = 0ull;
+            cnt->edge_ghost = 0ull;
+            cnt->pairs = 0ull;
+            cnt->bond_repairs = 0ull;
+            cnt->moved = 0ull;
+            c->left -= 1;
+            const int par = c->par;
+            c->cur = par;
+            c->par = par ^ 1;
+        }
     }
-    const float acc = sqrtf(r2);
-    const int age = c->age + 1;
-    const bool rb = c->force != 0 || !(acc <= c->skin) || age > c->max_age;
-    if (rb) {
-        for (int k = 0; k < 3; ++k) c->range[k] = 0.0f;
-        c->acc = 0.0f;
-        c->age = 0;
-        c->force = 0;
-        c->builds += 1;
-        c->overflow = 0ull;
-    } else {
-        for (int k = 0; k < 3; ++k) c->range[k] = rg[k];
-        c->acc = acc;
-        c->age = age;
-    }
+    c->active = run ? 1 : 0;
     c->rebuild = rb ? 1 : 0;
-    if (use_h) cudaGraphSetConditional(h, rb ? 1u : 0u);
+    if (mode == kDecideCond) cudaGraphSetConditional(h, rb ? 1u : 0u);
 }
 
 // Colony of index i for a kernel whose blocks take consecutive indices, one
@@ -159,11 +178,12 @@ __device__ __forceinline__ int fx_bin(unsigned h, int nb, int per)
     return (b >= nb) ? nb : (int)b + 1;
 }
 
-// Bins of buffer a's fixed-point positions into the list bins (kListBins
+// Bins of the step's fixed-point positions (buffer lctl->cur) into the list bins (kListBins
 // buffer) and the column counts.
-__global__ void k_list_rebin(const DevState S, int a)
+__global__ void k_list_rebin(const DevState S)
 {
     if (!S.lctl->rebuild) return;
+    const int a = S.lctl->cur;
     constexpr int B = kListBins;
     if (blockIdx.x == 0 && threadIdx.x == 0) S.lctl->body_runs += 1ull;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -208,9 +228,10 @@ __global__ void k_list_scatter(const DevState S)
 // deterministic order inside a column (z bin, then ascending original index:
 // the slot's rank among its column's keys), and the sorted copies the build
 // walks: the position record, z bin, slot, and each slot's rank
-__global__ void k_list_canon(const DevState S, int a)
+__global__ void k_list_canon(const DevState S)
 {
     if (!S.lctl->rebuild) return;
+    const int a = S.lctl->cur;
     constexpr int B = kListBins;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < S.n) {
@@ -441,10 +462,11 @@ __global__ void k_list_xcopy(const DevState S)
 // few sectors per warp, not one per entry as a plane per list position would
 // cost.
 template <bool CAP, bool PERSIST>
-__global__ void __launch_bounds__(256, 6) k_list_step(const DevState S, const DevParams P, float dtf, int a, int chunk)
+__global__ void __launch_bounds__(256, 6) k_list_step(const DevState S, const DevParams P, float dtf, int chunk)
 {
+    if (!S.lctl->active) return;  // (a stalled step, or one past the call's last)
     constexpr int B = kListBins;
-    const int b = a ^ 1;
+    const int a = S.lctl->cur, b = a ^ 1;
     const int n = S.n;
     const float bwf = P.bw32, kf = P.k32;
     const float zkf = P.z_k32, zbwf = P.z_bw32, zgf = P.z_g32;
@@ -751,9 +773,9 @@ __global__ void k_list_to_fp64_axis(const DevState S, int a, int ax, double *out
 
 }  // namespace
 
-int launch_list_decide(const DevState &S, unsigned long long cond, int use_cond, cudaStream_t st)
+int launch_list_decide(const DevState &S, unsigned long long cond, int mode, cudaStream_t st)
 {
-    k_list_decide<<<1, 1, 0, st>>>(S.lctl, S.cnt, (cudaGraphConditionalHandle)cond, use_cond);
+    k_list_decide<<<1, 1, 0, st>>>(S.lctl, S.cnt, (cudaGraphConditionalHandle)cond, mode);
     return 1;
 }
 
@@ -783,16 +805,16 @@ int launch_list_build(const DevState &S, const DevParams &P, int build_block, cu
     return 1;
 }
 
-int launch_list_rebuild(const DevState &S, const DevParams &P, int a, int *scan_scratch, int grid, int block,
+int launch_list_rebuild(const DevState &S, const DevParams &P, int *scan_scratch, int grid, int block,
                         int build_block, cudaStream_t st)
 {
     const int *gate = &S.lctl->rebuild;
     // one slot per thread (a block's colonies from one search)
     const int g1 = (S.n + block - 1) / block;
-    k_list_rebin<<<g1, block, 0, st>>>(S, a);
+    k_list_rebin<<<g1, block, 0, st>>>(S);
     int k = 1 + launch_scan(S.colcnt, S.colstart[kListBins], S.ncols_total, scan_scratch, st, gate);
     k_list_scatter<<<g1, block, 0, st>>>(S);
-    k_list_canon<<<g1, block, 0, st>>>(S, a);
+    k_list_canon<<<g1, block, 0, st>>>(S);
     // the cell offsets: a block per kCellsBlock columns of the largest colony
     const dim3 gc(S.ncol, std::max(1, std::min(65535, (S.cols_max + kCellsBlock - 1) / kCellsBlock)));
     k_list_cells<<<gc, kCellsBlock, 0, st>>>(S);
@@ -807,7 +829,7 @@ int launch_list_rebuild(const DevState &S, const DevParams &P, int a, int *scan_
     return k + 5;
 }
 
-int launch_list_step(const DevState &S, const DevParams &P, double dt, int a, int grid, int block, int passes,
+int launch_list_step(const DevState &S, const DevParams &P, double dt, int grid, int block, int passes,
                      cudaStream_t st, bool persistent)
 {
     // passes of the block per chunk (passes <= 0: the rule): short enough that
@@ -825,11 +847,11 @@ int launch_list_step(const DevState &S, const DevParams &P, double dt, int a, in
     if (persistent) {
         // one wave: the blocks that fit on the SMs at once (1536 threads per SM)
         const int wave = std::max(1, std::min(nb, grid * (1536 / block)));
-        if (S.pcap) k_list_step<true, true><<<wave, block, 0, st>>>(S, P, (float)dt, a, chunk);
-        else k_list_step<false, true><<<wave, block, 0, st>>>(S, P, (float)dt, a, chunk);
+        if (S.pcap) k_list_step<true, true><<<wave, block, 0, st>>>(S, P, (float)dt, chunk);
+        else k_list_step<false, true><<<wave, block, 0, st>>>(S, P, (float)dt, chunk);
     } else {
-        if (S.pcap) k_list_step<true, false><<<nb, block, 0, st>>>(S, P, (float)dt, a, chunk);
-        else k_list_step<false, false><<<nb, block, 0, st>>>(S, P, (float)dt, a, chunk);
+        if (S.pcap) k_list_step<true, false><<<nb, block, 0, st>>>(S, P, (float)dt, chunk);
+        else k_list_step<false, false><<<nb, block, 0, st>>>(S, P, (float)dt, chunk);
     }
     return 1;
 }
