@@ -1248,7 +1248,8 @@ int enqueue_list_step(bmxg_ctx *ctx, double dt, bool build)
     cudaEvent_t k0, k1;
     prof_events(ctx, &k0, &k1);
     if (k0) cudaEventRecord(k0, st);
-    launch_list_step(S, P, dt, ctx->nsm, ctx->ls_block, ctx->ls_passes, st, ctx->ls_persist);
+    launch_list_step(S, P, dt, ctx->nsm, ctx->ls_block, ctx->ls_passes, st, ctx->ls_persist,
+                     ctx->capturing && !build);
     if (k1) cudaEventRecord(k1, st);
     const cudaError_t le = cudaPeekAtLastError();
     if (le != cudaSuccess) return fail(ctx, BMXG_ERR_CUDA, std::string("list step: ") + cudaGetErrorString(le));

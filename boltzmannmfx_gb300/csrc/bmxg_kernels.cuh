@@ -262,9 +262,9 @@ constexpr int kListBodyKernels = 12;
 // force + wall + update over the list, reading buffer lctl->cur and writing the
 // other, or nothing when the step is not active (grid = the SM count; passes of the block per chunk of slots, <= 0: a rule;
 // persistent: one wave of blocks taking chunks from a counter, else one block
-// per chunk)
+// per chunk; chained: right after the decision kernel, no build between)
 int launch_list_step(const DevState &S, const DevParams &P, double dt, int grid, int block, int passes,
-                     cudaStream_t st, bool persistent = false);
+                     cudaStream_t st, bool persistent = false, bool chained = false);
 
 // ---- one tile with the caller's ghosts (k_tile.cu) -------------------------
 // The level's domain and the tile: cells are the domain's (1-based bins of

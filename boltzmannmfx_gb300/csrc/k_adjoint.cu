@@ -20,6 +20,7 @@
 // and reduced once at the end.
 #include <algorithm>
 
+#include "bmxg_pdl.cuh"
 #include "bmxg_stencil.cuh"
 
 namespace bmxg {
@@ -187,7 +188,7 @@ __device__ __forceinline__ bool dfwd_term(const DevState &S, const DevGeom &G, c
 // gathered J w (t[0..2]) and to the stiffness, damping, drag and adhesion
 // slopes (t[3..6]) (false: no contribution).
 __device__ __forceinline__ bool dadj_term(const DevState &S, const DevGeom &G, const DevParams &P,
-                                          const DiffParams &D, int a, const double *__restrict__ lin, int n,
+                                          const DiffParams &D, int a, const double *lin, int n,
                                           const double *o, int j, int sx, int sy, double *t)
 {
     // o: xk, yk, zk, rk, mk, dmk, ak, lk[3]
@@ -424,6 +425,7 @@ __global__ void __launch_bounds__(kWalkBlock, 3) k_dfwdw(const DevState S, const
     __shared__ unsigned char opass[kWalkBlock];
     const int tid = threadIdx.x;
     const int b = a ^ 1;
+    chain_wait();
     walk_block(S, a, P.bw32, M, [&](int s, int i, int col) {
         const double ri = S.rad[i];
         own[0][s] = S.x[a][i];
@@ -482,9 +484,7 @@ __global__ void __launch_bounds__(kWalkBlock, 3) k_dfwdw(const DevState S, const
 
 template <int NS, int STAGE>
 __global__ void __launch_bounds__(kWalkBlock, 2) k_dadjw(const DevState S, const DevParams P, DiffParams D, double dt,
-                                                         int a, const double *__restrict__ lin,
-                                                         double *__restrict__ lout, double *__restrict__ gacc,
-                                                         double *__restrict__ gadh)
+                                                         int a, const double *lin, double *lout, double *gacc, double *gadh)
 {
     constexpr int NO = 10, NT = 7;
     extern __shared__ __align__(16) unsigned char smw[];
@@ -495,6 +495,7 @@ __global__ void __launch_bounds__(kWalkBlock, 2) k_dadjw(const DevState S, const
     __shared__ unsigned char opass[kWalkBlock];
     const int tid = threadIdx.x;
     const int n = S.n;
+    chain_wait();
     walk_block(S, a, P.bw32, M, [&](int s, int k, int col) {
         double *o = own[s];
         const double rk = S.rad[k];
@@ -601,7 +602,7 @@ int launch_dfwd(const DevState &S, const DevParams &P, const DiffParams &D, doub
     // with recomputation, one thread per slot -> a warp per column: 1000 spheres 57 -> 23 / 144 -> 77, 20 000
     // 79 -> 40 / 195 -> 129, 40 000 82 -> 61 / 207 -> 192)
     if (S.srel[a] && !pinned && S.n <= kWalkNarrow) {
-        k_dfwdw<32, 6><<<(S.n + 31) / 32, kWalkBlock, sizeof(WalkMem<32, 6>), st>>>(S, P, D, dt, a);
+        launch_after(k_dfwdw<32, 6>, (S.n + 31) / 32, kWalkBlock, sizeof(WalkMem<32, 6>), st, S, P, D, dt, a);
     } else if (S.srel[a]) {
         allow_smem(k_dfwd<true>, smem);
         k_dfwd<true><<<grid, block, smem, st>>>(S, P, D, dt, a);
@@ -617,8 +618,8 @@ int launch_dadj(const DevState &S, const DevParams &P, const DiffParams &D, doub
 {
     const size_t smem = staged_smem(block, 10, 7);
     if (S.srel[a] && !pinned && S.n <= kWalkNarrow) {
-        k_dadjw<32, 6><<<(S.n + 31) / 32, kWalkBlock, sizeof(WalkMem<32, 6>), st>>>(S, P, D, dt, a, lin, lout, gacc,
-                                                                                     gadh);
+        launch_after(k_dadjw<32, 6>, (S.n + 31) / 32, kWalkBlock, sizeof(WalkMem<32, 6>), st, S, P, D, dt, a, lin,
+                     lout, gacc, gadh);
     } else if (S.srel[a]) {
         allow_smem(k_dadj<true>, smem);
         k_dadj<true><<<grid, block, smem, st>>>(S, P, D, dt, a, lin, lout, gacc, gadh);

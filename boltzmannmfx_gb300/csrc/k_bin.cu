@@ -13,6 +13,7 @@
 
 #include <cooperative_groups.h>
 
+#include "bmxg_pdl.cuh"
 #include "bmxg_stencil.cuh"
 
 namespace bmxg {
@@ -253,6 +254,7 @@ __global__ void __launch_bounds__(kSortBlock) k_sort_cluster(const SortJob J)
     const int nb = (int)cl.num_blocks(), rank = (int)cl.block_rank();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int T = nb * kSortBlock, g = rank * kSortBlock + tid;
+    chain_wait();
     if (J.publish && g == 0) publish_counters(J.cnt, J.rctl);
     // this thread's slots, loaded while the scan runs
     int c[kSortItems], z[kSortItems], o[kSortItems];
@@ -620,15 +622,17 @@ static bool sort_in_cluster(const SortJob &J, cudaStream_t st)
     int use = c;
     while (use > 1 && J.n <= (use / 2) * kSortBlock && J.ncols <= (use / 2) * kSortBlock * 4) use /= 2;
     cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = (unsigned)use;
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // (launch_after)
+    at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.gridDim = dim3((unsigned)use);
     cfg.blockDim = dim3(kSortBlock);
     cfg.stream = st;
     cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
     cudaLaunchKernelEx(&cfg, k_sort_cluster, J);  // (an error is the launch status the caller reads)
     return true;
 }

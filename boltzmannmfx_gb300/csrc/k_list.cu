@@ -42,6 +42,7 @@
 #include <algorithm>
 
 #include "bmxg_fx.cuh"
+#include "bmxg_pdl.cuh"
 #include "bmxg_stencil.cuh"
 
 namespace bmxg {
@@ -99,6 +100,7 @@ __device__ __forceinline__ long long fx_inc(float f, float c, float cl, bool &bi
 // be enqueued without knowing which of them will run: see kDecideStall.
 __global__ void k_list_decide(ListCtl *c, DevCounters *cnt, cudaGraphConditionalHandle h, int mode)
 {
+    chain_wait();
     bool run = c->left > 0;
     bool rb = false;
     if (run) {
@@ -464,6 +466,7 @@ __global__ void k_list_xcopy(const DevState S)
 template <bool CAP, bool PERSIST>
 __global__ void __launch_bounds__(256, 6) k_list_step(const DevState S, const DevParams P, float dtf, int chunk)
 {
+    chain_wait();
     if (!S.lctl->active) return;  // (a stalled step, or one past the call's last)
     constexpr int B = kListBins;
     const int a = S.lctl->cur, b = a ^ 1;
@@ -775,7 +778,7 @@ __global__ void k_list_to_fp64_axis(const DevState S, int a, int ax, double *out
 
 int launch_list_decide(const DevState &S, unsigned long long cond, int mode, cudaStream_t st)
 {
-    k_list_decide<<<1, 1, 0, st>>>(S.lctl, S.cnt, (cudaGraphConditionalHandle)cond, mode);
+    launch_after(k_list_decide, 1, 1, 0, st, S.lctl, S.cnt, (cudaGraphConditionalHandle)cond, mode);
     return 1;
 }
 
@@ -830,7 +833,7 @@ int launch_list_rebuild(const DevState &S, const DevParams &P, int *scan_scratch
 }
 
 int launch_list_step(const DevState &S, const DevParams &P, double dt, int grid, int block, int passes,
-                     cudaStream_t st, bool persistent)
+                     cudaStream_t st, bool persistent, bool chained)
 {
     // passes of the block per chunk (passes <= 0: the rule): short enough that
     // the block scheduler evens out the uneven list lengths of the colonies
@@ -850,7 +853,8 @@ int launch_list_step(const DevState &S, const DevParams &P, double dt, int grid,
         if (S.pcap) k_list_step<true, true><<<wave, block, 0, st>>>(S, P, (float)dt, chunk);
         else k_list_step<false, true><<<wave, block, 0, st>>>(S, P, (float)dt, chunk);
     } else {
-        if (S.pcap) k_list_step<true, false><<<nb, block, 0, st>>>(S, P, (float)dt, chunk);
+        if (chained && !S.pcap) launch_after(k_list_step<false, false>, nb, block, 0, st, S, P, (float)dt, chunk);
+        else if (S.pcap) k_list_step<true, false><<<nb, block, 0, st>>>(S, P, (float)dt, chunk);
         else k_list_step<false, false><<<nb, block, 0, st>>>(S, P, (float)dt, chunk);
     }
     return 1;

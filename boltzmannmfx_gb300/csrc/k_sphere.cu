@@ -27,6 +27,7 @@
 // Roofline: HBM / L2 bound gather; no dense contraction, so no tensor cores.
 #include <atomic>
 
+#include "bmxg_pdl.cuh"
 #include "bmxg_stencil.cuh"
 
 namespace bmxg {
@@ -228,6 +229,7 @@ __global__ void __launch_bounds__(kWalkBlock, 3) k_sphere64w(const DevState S, c
     __shared__ unsigned char opass[kWalkBlock];
     const int tid = threadIdx.x;
     const int b = a ^ 1;
+    chain_wait();
     walk_block(S, a, P.bw32, M, [&](int s, int i, int col) {
         opos[s][0] = S.x[a][i];
         opos[s][1] = S.y[a][i];
@@ -406,13 +408,13 @@ int launch_sphere_step(const DevState &S, const DevParams &P, double dt, int a, 
     if (precision == BMXG_FP64_FORM) {
         const int ns = (sorted && !pinned) ? sphere64_slots(S.n) : 0;
         if (ns == 32) {
-            k_sphere64w<32, 6><<<(S.n + 31) / 32, kWalkBlock, sizeof(WalkMem<32, 6>), st>>>(S, P, dt, a);
+            launch_after(k_sphere64w<32, 6>, (S.n + 31) / 32, kWalkBlock, sizeof(WalkMem<32, 6>), st, S, P, dt, a);
             return 1;
         }
         if (ns == 128) {
             static std::atomic<unsigned long long> known{0};
             allow_smem_once(k_sphere64w<128, 4>, sizeof(WalkMem<128, 4>), known);
-            k_sphere64w<128, 4><<<(S.n + 127) / 128, kWalkBlock, sizeof(WalkMem<128, 4>), st>>>(S, P, dt, a);
+            launch_after(k_sphere64w<128, 4>, (S.n + 127) / 128, kWalkBlock, sizeof(WalkMem<128, 4>), st, S, P, dt, a);
             return 1;
         }
         // (block a multiple of 32, at most 256: the block stages and evaluates its pairs together)
