@@ -27,12 +27,14 @@ struct GraphKey {
     int precision;
     int parity;
     int single;  // -1: kResyncEvery steps; 0 / 1: one step without / with the FP32F re-sync
+    bool list;   // list steps (their kernels read the parity from the control block)
     bool operator<(const GraphKey &o) const
     {
         if (dt != o.dt) return dt < o.dt;
         if (precision != o.precision) return precision < o.precision;
         if (parity != o.parity) return parity < o.parity;
-        return single < o.single;
+        if (single != o.single) return single < o.single;
+        return list < o.list;
     }
 };
 
@@ -127,6 +129,10 @@ struct bmxg_ctx {
     int64_t ncells_total = 0;     // 3D cells over all colonies
     int *cell_scratch = nullptr;  // scan scratch of the list build (column counts, group entries)
     float skin_cur = 0.0f;        // skin of the list control block
+    int list_prec = BMXG_FP32F;   // the form whose steps the list follows
+    bool list_room = true;        // (false: no room for the list, FP64 steps go without)
+    bool list64_bail = false;     // the loaded state left what FP64 list steps cover
+    int64_t plain64 = 0;          // FP64 steps of this state's size that went without a list
     float list_period = 16.0f;    // steps per list build, from the calls so far
     int *h_run = nullptr;         // pinned: steps and buffer of a list call
     ListCtl *h_lctl = nullptr;    // pinned copy of the control block
@@ -260,6 +266,8 @@ void free_state(bmxg_ctx *ctx)
     ctx->allocs.clear();
     ctx->S = DevState{};
     ctx->rod_walk = false;
+    ctx->list_room = true;
+    ctx->plain64 = 0;
     ctx->d_geoms = nullptr;
     ctx->d_cbase = nullptr;
     ctx->scan_scratch = nullptr;
@@ -829,6 +837,7 @@ int load_state(bmxg_ctx *ctx, const bmxg_particles *p, const int64_t *colony_off
     ctx->vel32 = false;
     ctx->vel64_zero = !p->velx && !p->vely && !p->velz && !p->wx && !p->wy && !p->wz;
     ctx->step_count = 0;
+    ctx->list64_bail = false;
     ctx->parity = 0;
     ctx->rmax = rmax;
     ctx->list_valid = false;
@@ -1081,6 +1090,17 @@ void prof_events(bmxg_ctx *ctx, cudaEvent_t *k0, cudaEvent_t *k1)
 
 // ---- FP32F neighbour list with a skin ---------------------------------------
 constexpr int kListMaxAge = 64;      // builds at least this often
+// FP64 spheres step over the list where it is the faster path, per-step path / list:
+// 10 000 slots 19 / 22 us a step, 20 000 29 / 22, 40 000 40 / 24, 160 000 84 / 48,
+// 400 000 155 / 96, 688 000 in 64 colonies 430 / 245 (up to 16 384 slots the
+// per-step path's sort is one cluster and its step little more than two launches).
+// From a load on, with the build: 6 steps of 20 000 slots 387 / 370 us, 400 000
+// 1294 / 1031; fewer steps keep the per-step path.  The list's buffers and graphs
+// cost 0.6-0.7 ms once, which 7 + 1.6e6 / slots steps pay back (fresh context, 20
+// steps: 40 000 slots 2294 / 2439, 160 000 4192 / 4180, 400 000 6590 / 6254).
+constexpr int kList64Slots = 16384;
+constexpr int kList64MinSteps = 6;
+constexpr double kList64Pay = 1.6e6;
 constexpr int kListSingles = 4;      // so few steps: a graph (with its conditional node) for each
 constexpr int kListMinSteps = 2;     // a shorter first call after a load runs the per-step path
 
@@ -1108,9 +1128,27 @@ float list_skin(const bmxg_ctx *ctx)
     return (float)skin;
 }
 
+// Whether FP64 steps go over the list (which covers the state: list_skin).
+bool list64_pays(const bmxg_ctx *ctx, int32_t nsteps)
+{
+    if (!ctx->list_room || ctx->list64_bail || ctx->n <= kList64Slots) return false;
+    if (ctx->list_valid && ctx->list_prec == BMXG_FP64) return true;
+    if (ctx->step_count + nsteps < kList64MinSteps) return false;
+    if (ctx->S.nbr) return true;
+    if ((double)(ctx->plain64 + nsteps) < 7.0 + kList64Pay / (double)ctx->n) return false;
+    // (and leaves three quarters of the free memory)
+    size_t room = 0, all = 0;
+    const size_t need = (size_t)ctx->n * 320 + (size_t)ctx->ncells_total * sizeof(int);
+    if (cudaMemGetInfo(&room, &all) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return false;
+    }
+    return need <= room / 4;
+}
+
 // Allocate the list on first use; (re)initialise its control block when the
 // state or the skin changed, asking the next step for a build.
-int ensure_list(bmxg_ctx *ctx, float skin)
+int ensure_list(bmxg_ctx *ctx, float skin, int precision)
 {
     DevState &S = ctx->S;
     if (!S.nbr) {
@@ -1138,7 +1176,10 @@ int ensure_list(bmxg_ctx *ctx, float skin)
         ctx->list_valid = false;
         drop_graphs(ctx);  // captured kernels hold the state's pointers by value
     }
-    if (ctx->list_valid && skin == ctx->skin_cur) return BMXG_OK;
+    if (ctx->list_valid && skin == ctx->skin_cur && ctx->list_prec == precision) return BMXG_OK;
+    // (the other form's steps left their own positions ahead)
+    if (int rc = sync_fp64(ctx)) return rc;
+    ctx->list_prec = precision;
     double dmax = 0.0;
     for (const DevGeom &g : ctx->h_geoms) dmax = std::max(dmax, std::max(g.dx[0], std::max(g.dx[1], g.dx[2])));
     ListCtl h;
@@ -1150,11 +1191,19 @@ int ensure_list(bmxg_ctx *ctx, float skin)
         h.inc_max[k] = 0x007fffffu;
     }
     h.max_age = kListMaxAge;
+    h.whole = precision == BMXG_FP64;
     h.force = 1;
-    // the fixed-point positions start from the FP64 ones
-    LAUNCH(launch_list_init(S, ctx->parity, grid_for(ctx, ctx->sh_misc, ctx->n), ctx->sh_misc.block, ctx->stream));
-    ctx->fx_ahead = false;
     CK(cudaMemcpyAsync(S.lctl, &h, sizeof(h), cudaMemcpyHostToDevice, ctx->stream));
+    // the fixed-point positions (FP64 form: the screen's coordinates) start from
+    // the FP64 ones
+    if (precision == BMXG_FP32F)
+        LAUNCH(launch_list_init(S, ctx->parity, grid_for(ctx, ctx->sh_misc, ctx->n), ctx->sh_misc.block,
+                                ctx->stream));
+    else {
+        LAUNCH(launch_list64_begin(S, ctx->parity, ctx->stream));
+        ctx->bins_exact = false;  // (in place of the offsets from the bins' corners)
+    }
+    ctx->fx_ahead = false;
     CK(cudaStreamSynchronize(ctx->stream));
     ctx->skin_cur = skin;
     ctx->body_runs_seen = 0;
@@ -1202,7 +1251,7 @@ int set_list_run(bmxg_ctx *ctx, int steps)
 // where `build`, else the step stalls), then the force / update kernel.  What
 // ran is counted after the call (two kernels a step, the build's when it ran):
 // a kernel of a step that did not run returns at once.
-int enqueue_list_step(bmxg_ctx *ctx, double dt, bool build)
+int enqueue_list_step(bmxg_ctx *ctx, double dt, int precision, bool build)
 {
     const DevState &S = ctx->S;
     cudaStream_t st = ctx->stream;
@@ -1232,6 +1281,7 @@ int enqueue_list_step(bmxg_ctx *ctx, double dt, bool build)
         CK(cudaStreamUpdateCaptureDependencies(st, &cn, nullptr, 1, cudaStreamSetCaptureDependencies));
         CK(cudaStreamBeginCaptureToGraph(ctx->body_stream, cp.conditional.phGraph_out[0], nullptr, nullptr, 0,
                                          cudaStreamCaptureModeRelaxed));
+        if (precision == BMXG_FP64) launch_list64_fx(S, ctx->body_stream);
         launch_list_rebuild(S, P, ctx->cell_scratch, mgrd, mblk, ctx->lb_block, ctx->body_stream);
         const cudaError_t e1 = cudaPeekAtLastError();
         cudaGraph_t body = nullptr;
@@ -1241,6 +1291,7 @@ int enqueue_list_step(bmxg_ctx *ctx, double dt, bool build)
                         std::string("list build capture: ") + cudaGetErrorString(e1 != cudaSuccess ? e1 : e2));
     } else {
         launch_list_decide(S, 0, kDecideBuild, st);
+        if (precision == BMXG_FP64) launch_list64_fx(S, st);
         launch_list_rebuild(S, P, ctx->cell_scratch, mgrd, mblk, ctx->lb_block, st);
         const cudaError_t e = cudaPeekAtLastError();
         if (e != cudaSuccess) return fail(ctx, BMXG_ERR_CUDA, std::string("list build: ") + cudaGetErrorString(e));
@@ -1248,8 +1299,9 @@ int enqueue_list_step(bmxg_ctx *ctx, double dt, bool build)
     cudaEvent_t k0, k1;
     prof_events(ctx, &k0, &k1);
     if (k0) cudaEventRecord(k0, st);
-    launch_list_step(S, P, dt, ctx->nsm, ctx->ls_block, ctx->ls_passes, st, ctx->ls_persist,
-                     ctx->capturing && !build);
+    const bool chained = ctx->capturing && !build;
+    if (precision == BMXG_FP64) launch_list64_step(S, P, dt, st, chained);
+    else launch_list_step(S, P, dt, ctx->nsm, ctx->ls_block, ctx->ls_passes, st, ctx->ls_persist, chained);
     if (k1) cudaEventRecord(k1, st);
     const cudaError_t le = cudaPeekAtLastError();
     if (le != cudaSuccess) return fail(ctx, BMXG_ERR_CUDA, std::string("list step: ") + cudaGetErrorString(le));
@@ -1258,7 +1310,7 @@ int enqueue_list_step(bmxg_ctx *ctx, double dt, bool build)
 
 int enqueue_step(bmxg_ctx *ctx, double dt, int precision, int a, int resync)
 {
-    if (ctx->list_on) return enqueue_list_step(ctx, dt, resync != 0);  // (list steps take no re-sync: a build)
+    if (ctx->list_on) return enqueue_list_step(ctx, dt, precision, resync != 0);  // (list steps take no re-sync: a build)
     const DevState &S = ctx->S;
     cudaStream_t st = ctx->stream;
     const DevParams P = dev_params(ctx->prm);
@@ -1305,7 +1357,7 @@ int get_graph(bmxg_ctx *ctx, double dt, int precision, int parity, cudaGraphExec
         parity = 0;
         if (single >= 0) single = 1;
     }
-    GraphKey key{dt, precision, parity, single};
+    GraphKey key{dt, precision, parity, single, ctx->list_on};
     auto it = ctx->graphs.find(key);
     if (it != ctx->graphs.end()) {
         *out = it->second;
@@ -1343,10 +1395,11 @@ int get_graph(bmxg_ctx *ctx, double dt, int precision, int parity, cudaGraphExec
     return BMXG_OK;
 }
 
-// nsteps list steps, to the end (the stream is synchronised, h_cnt and h_lctl
+// nsteps list steps, to the end or (FP64 form) until a slot left the range the
+// list covers: *done of them ran (the stream is synchronised, h_cnt and h_lctl
 // read back).  Graphs are launched for the steps left and for those that the
 // builds due by then will stall, and again for what is still left.
-int list_steps(bmxg_ctx *ctx, double dt, int32_t nsteps)
+int list_steps(bmxg_ctx *ctx, double dt, int32_t nsteps, int precision, int32_t *done)
 {
     cudaStream_t st = ctx->stream;
     if (int rc = set_list_run(ctx, nsteps)) return rc;
@@ -1355,12 +1408,12 @@ int list_steps(bmxg_ctx *ctx, double dt, int32_t nsteps)
         cudaGraphExec_t g = nullptr;
         if (ctx->profiling) {  // launched one by one, with events around the force kernel
             for (int k = 0; k < left; ++k)
-                if (int rc = enqueue_list_step(ctx, dt, true)) return rc;
+                if (int rc = enqueue_list_step(ctx, dt, precision, true)) return rc;
         } else if (left <= kListSingles) {
-            if (int rc = get_graph(ctx, dt, BMXG_FP32F, 0, &g, 1)) return rc;
+            if (int rc = get_graph(ctx, dt, precision, 0, &g, 1)) return rc;
             for (int k = 0; k < left; ++k) CK(cudaGraphLaunch(g, st));
         } else {
-            if (int rc = get_graph(ctx, dt, BMXG_FP32F, 0, &g)) return rc;
+            if (int rc = get_graph(ctx, dt, precision, 0, &g)) return rc;
             const float stalled = 0.5f * (kResyncEvery - 1) * (float)left / std::max(ctx->list_period, 1.0f);
             const int graphs = std::max(1, (int)(((float)left + stalled) / (float)kResyncEvery));
             for (int k = 0; k < graphs; ++k) CK(cudaGraphLaunch(g, st));
@@ -1370,11 +1423,28 @@ int list_steps(bmxg_ctx *ctx, double dt, int32_t nsteps)
         CK(cudaMemcpyAsync(ctx->h_lctl, ctx->S.lctl, sizeof(ListCtl), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
         const int now = ctx->h_lctl->left;
+        const bool over = precision == BMXG_FP64 && ctx->h_lctl->overflow;  // (the step of that build did not run)
+        if (over || ctx->h_lctl->bail) {
+            ctx->list64_bail = true;
+            left = now + (over ? 1 : 0);
+            break;
+        }
         if (now >= left || now < 0) return fail(ctx, BMXG_ERR_STATE, "internal: list steps made no progress");
         left = now;
     }
-    ctx->parity ^= nsteps & 1;
-    ctx->step_count += nsteps;
+    *done = nsteps - left;
+    ctx->parity ^= *done & 1;
+    ctx->step_count += *done;
+    const unsigned long long runs = ctx->h_lctl->body_runs - ctx->body_runs_seen;
+    ctx->body_runs_seen = ctx->h_lctl->body_runs;
+    ctx->launches += (int64_t)runs * (kListBodyKernels + (precision == BMXG_FP64 ? 1 : 0)) + 2 * (int64_t)*done;
+    if (runs > 0) ctx->list_period = 0.5f * (ctx->list_period + (float)*done / (float)runs);
+    ctx->stats.n_rebins += (int64_t)runs;
+    if (*done > 0) {
+        ctx->bins_exact = false;
+        if (precision == BMXG_FP32F) ctx->fx_ahead = true;
+    }
+    if (precision == BMXG_FP64 && ctx->list64_bail) ctx->list_valid = false;
     return BMXG_OK;
 }
 
@@ -1383,19 +1453,34 @@ int list_steps(bmxg_ctx *ctx, double dt, int32_t nsteps)
 // before an allocation are dropped: they hold the state's pointers by value).
 int step_setup(bmxg_ctx *ctx, int32_t nsteps, int32_t precision)
 {
-    float skin = (precision == BMXG_FP32F && ctx->list_mode) ? list_skin(ctx) : 0.0f;
-    if (skin > 0.0f && !ctx->list_valid && nsteps < kListMinSteps && ctx->step_count == 0) skin = 0.0f;
-    if (skin > 0.0f) {
-        int rc = ensure_list(ctx, skin);
+    float skin = (ctx->list_mode && (precision == BMXG_FP32F || list64_pays(ctx, nsteps))) ? list_skin(ctx) : 0.0f;
+    if (skin > 0.0f && precision == BMXG_FP32F && !ctx->list_valid && nsteps < kListMinSteps && ctx->step_count == 0)
+        skin = 0.0f;
+    if (skin > 0.0f && precision == BMXG_FP64) {
+        const size_t held = ctx->allocs.size();
+        int rc = ensure_list(ctx, skin, precision);
+        if (rc == BMXG_ERR_OOM) {  // no room for the list: FP64 steps go without
+            while (ctx->allocs.size() > held) {
+                cudaFree(ctx->allocs.back());
+                ctx->allocs.pop_back();
+            }
+            (void)cudaGetLastError();
+            ctx->S.nbr = nullptr;
+            ctx->list_room = false;
+            skin = 0.0f;
+            rc = ensure_exact(ctx);
+        }
+        if (rc) return rc;
+    } else if (skin > 0.0f) {
+        int rc = ensure_list(ctx, skin, precision);
         if (rc) return rc;
     } else {
         int rc = ensure_exact(ctx);
         if (rc) return rc;
     }
-    if ((skin > 0.0f) != ctx->list_on) drop_graphs(ctx);
     ctx->list_on = skin > 0.0f;
     ctx->pcap_valid = false;
-    if (ctx->list_on && ctx->pair_capture && !ctx->S.pcap) {
+    if (ctx->list_on && precision == BMXG_FP32F && ctx->pair_capture && !ctx->S.pcap) {
         int rc = dalloc(ctx, &ctx->S.pcap, (size_t)(kPairCap + 1) * ctx->n);
         if (rc) return rc;
         drop_graphs(ctx);
@@ -1486,9 +1571,16 @@ int bmxg_step(bmxg_ctx *ctx, double dt, int32_t nsteps, int32_t precision)
     int32_t left = nsteps;
     ctx->kev_used = 0;
     if (ctx->list_on) {
-        if (int rc = list_steps(ctx, subdt, nsteps)) return rc;
-        left = 0;
+        int32_t done = 0;
+        if (int rc = list_steps(ctx, subdt, nsteps, precision, &done)) return rc;
+        left -= done;
+        if (left > 0) {  // (FP64, out of the list's range) the rest on the per-step path
+            if (int rc = ensure_exact(ctx)) return rc;
+            ctx->list_on = false;
+        }
     }
+    const bool by_list = ctx->list_on;
+    const int32_t per_step = left;
     auto eager = [&]() -> int {  // one step on the re-sync schedule
         // re-sync on the last step of each kResyncEvery (not right after a load,
         // whose offsets are exact)
@@ -1533,23 +1625,14 @@ int bmxg_step(bmxg_ctx *ctx, double dt, int32_t nsteps, int32_t precision)
         if (rc) return rc;
     }
     ctx->vel32 = (precision == BMXG_FP32F) && !ctx->S.has_rods;
-    ctx->pcap_valid = ctx->list_on && ctx->S.pcap != nullptr;
-    if (!ctx->list_on) {
+    ctx->pcap_valid = by_list && precision == BMXG_FP32F && ctx->S.pcap != nullptr;
+    if (!by_list) {
         CK(cudaGetLastError());
         CK(cudaEventRecord(ctx->ev1, ctx->stream));
         CK(cudaMemcpyAsync(ctx->h_cnt, ctx->d_cnt, sizeof(DevCounters), cudaMemcpyDeviceToHost, ctx->stream));
         CK(cudaStreamSynchronize(ctx->stream));
-    }
-    if (ctx->list_on) {
-        ctx->fx_ahead = true;
-        const unsigned long long runs = ctx->h_lctl->body_runs - ctx->body_runs_seen;
-        ctx->body_runs_seen = ctx->h_lctl->body_runs;
-        ctx->launches += (int64_t)runs * kListBodyKernels + 2 * (int64_t)nsteps;
-        if (runs > 0) ctx->list_period = 0.5f * (ctx->list_period + (float)nsteps / (float)runs);
-        ctx->stats.n_rebins += (int64_t)runs;
-        ctx->bins_exact = false;
-    } else {
-        ctx->stats.n_rebins += nsteps;
+        ctx->stats.n_rebins += per_step;
+        if (precision == BMXG_FP64) ctx->plain64 += per_step;
         ctx->list_valid = false;
     }
     ctx->stepped = true;
@@ -1566,9 +1649,9 @@ int bmxg_step(bmxg_ctx *ctx, double dt, int32_t nsteps, int32_t precision)
     ctx->kev_used = 0;
     ctx->stats.n_kernel_launches = ctx->launches;
     const DevCounters &hc = *ctx->h_cnt;
-    ctx->stats.n_out_of_domain = (int64_t)(ctx->list_on ? hc.out_of_domain : hc.last_out_of_domain);
-    ctx->stats.n_edge_ghost = (int64_t)(ctx->list_on ? hc.edge_ghost : hc.last_edge_ghost);
-    ctx->stats.n_bond_repairs = (int64_t)(ctx->list_on ? hc.bond_repairs : hc.last_bond_repairs);
+    ctx->stats.n_out_of_domain = (int64_t)(by_list ? hc.out_of_domain : hc.last_out_of_domain);
+    ctx->stats.n_edge_ghost = (int64_t)(by_list ? hc.edge_ghost : hc.last_edge_ghost);
+    ctx->stats.n_bond_repairs = (int64_t)(by_list ? hc.bond_repairs : hc.last_bond_repairs);
     if (ctx->h_cnt->bad_index) return fail(ctx, BMXG_ERR_STATE, "internal: inconsistent bin counts");
     if (ctx->h_cnt->nonfinite) return fail(ctx, BMXG_ERR_NONFINITE, "a step produced a non-finite position");
     if (ctx->h_cnt->range)
@@ -2157,7 +2240,7 @@ int bmxg_autotune(bmxg_ctx *ctx, const char *cache_path)
             // buffer a and write buffer b (dt = 0), and the build launches
             // rewrite the same list: the loaded state is untouched, and the
             // list path starts afresh at the next step (list_valid = false)
-            if (int rc = ensure_list(ctx, skin)) return rc;
+            if (int rc = ensure_list(ctx, skin, BMXG_FP32F)) return rc;
             cudaStream_t st = ctx->stream;
             if (int rc = set_list_run(ctx, 1)) return rc;  // (the timed launches repeat that step)
             const int mblk = ctx->sh_misc.block, mgrd = grid_for(ctx, ctx->sh_misc, n);

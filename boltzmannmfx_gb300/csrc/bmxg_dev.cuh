@@ -171,6 +171,15 @@ __device__ __forceinline__ int bin_of_fast(double x, double plo, double dxi, flo
     return bin_of(x, plo, dxi, lo_c, hi_c);
 }
 
+// The coordinate x of a particle's image s (-1, 1) domain lengths away along
+// axis d, and the bin (0..n + 1) it is in: x + s len in FP64 (s len is exact), the
+// bin as bin_of's.
+__device__ __forceinline__ double image_coord(double x, double len, int s) { return __dadd_rn(x, s < 0 ? -len : len); }
+__device__ __forceinline__ int image_bin(const DevGeom &G, int d, double gx)
+{
+    return bin_of_fast(gx, G.plo[d], G.dxi[d], G.plof[d], G.dxif[d], 0, G.n[d] + 1);
+}
+
 // Round-to-nearest double -> float from the bits (no FP64 instruction) where
 // the result is a normal float, the FP32 conversion otherwise; equal to it.
 __device__ __forceinline__ float d2f_rn(double x)

@@ -39,6 +39,8 @@ struct ListCtl {
     int active;            // the step that follows runs (there are steps left, no build is due)
     int cur;               // ... reading the fixed-point positions of this buffer
     int left, par;         // steps left in the call and the buffer the next one reads (set by the host)
+    int whole;             // the steps take no overflowed list (FP64 form)
+    int bail;              // FP64 list steps: a slot left the range the list covers; no step runs any more
     int builds;            // builds decided so far
     unsigned long long body_runs;  // builds actually run (counted by the first build kernel)
     unsigned long long overflow;   // slots whose list exceeded the capacity (last build)
@@ -263,6 +265,12 @@ constexpr int kListBodyKernels = 12;
 // other, or nothing when the step is not active (grid = the SM count; passes of the block per chunk of slots, <= 0: a rule;
 // persistent: one wave of blocks taking chunks from a counter, else one block
 // per chunk; chained: right after the decision kernel, no build between)
+// FP64 form of the path: the FP32 coordinates the steps screen with (in rel) from
+// buffer a's positions; the fixed-point positions of the build (first kernel of
+// the build's body); the step.
+int launch_list64_begin(const DevState &S, int a, cudaStream_t st);
+int launch_list64_fx(const DevState &S, cudaStream_t st);
+int launch_list64_step(const DevState &S, const DevParams &P, double dt, cudaStream_t st, bool chained);
 int launch_list_step(const DevState &S, const DevParams &P, double dt, int grid, int block, int passes,
                      cudaStream_t st, bool persistent = false, bool chained = false);
 

@@ -14,12 +14,10 @@ __device__ __forceinline__ bool image_in_row(const DevState &S, const DevGeom &G
                                              int ii, int jj, int sx, int sy)
 {
     if (sx) {
-        double gx = S.x[a][j] + (double)sx * G.len[0];
-        if (bin_of(gx, G.plo[0], G.dxi[0], 0, G.n[0] + 1) != ii) return false;
+        if (image_bin(G, 0, image_coord(S.x[a][j], G.len[0], sx)) != ii) return false;
     }
     if (sy) {
-        double gy = S.y[a][j] + (double)sy * G.len[1];
-        if (bin_of(gy, G.plo[1], G.dxi[1], 0, G.n[1] + 1) != jj) return false;
+        if (image_bin(G, 1, image_coord(S.y[a][j], G.len[1], sy)) != jj) return false;
     }
     return true;
 }
@@ -374,6 +372,32 @@ __device__ __forceinline__ void walk_pairs(const WalkMem<NS, STAGE> &M, double *
     }
 }
 
+// Counters of a slot at (x, y, z) in bins bx, by: out-of-domain z, non-finite
+// positions, images that leave their halo cell.
+__device__ __forceinline__ void count_slot(const DevState &S, const DevGeom &G, double x, double y, double z, int bx,
+                                           int by, bool count_domain)
+{
+    if (count_domain) {
+        // inside for certain from the FP32 values (truncated z within 2^-21 of the
+        // magnitudes), else the FP64 test
+        const float zf = d2f_trunc(z);
+        const float m = 4.8e-7f * (fabsf(zf) + fabsf(G.plof[2]) + fabsf(G.phif[2]));
+        const bool sure = G.phif[2] > G.plof[2] && zf - m > G.plof[2] && zf + m < G.phif[2];
+        if (!sure && !(z >= G.plo[2] && z < G.phi[2])) atomicAdd(&S.cnt->out_of_domain, 1ULL);
+    }
+    if (!finite_bits(x) || !finite_bits(y) || !finite_bits(z)) atomicAdd(&S.cnt->nonfinite, 1ULL);
+    if (G.per[0] && (bx == 1 || bx == G.n[0])) {
+        const int sx = (bx == 1) ? 1 : -1;
+        const int gb = image_bin(G, 0, image_coord(x, G.len[0], sx));
+        if (gb != (sx > 0 ? G.n[0] + 1 : 0)) atomicAdd(&S.cnt->edge_ghost, 1ULL);
+    }
+    if (G.per[1] && (by == 1 || by == G.n[1])) {
+        const int sy = (by == 1) ? 1 : -1;
+        const int gb = image_bin(G, 1, image_coord(y, G.len[1], sy));
+        if (gb != (sy > 0 ? G.n[1] + 1 : 0)) atomicAdd(&S.cnt->edge_ghost, 1ULL);
+    }
+}
+
 // Bin a slot at position (x, y, z): column and z bin into buffer bb, FP32
 // offsets from the bin corner into buffer rb, column count; flag
 // out-of-domain z, images that leave their halo cell, and non-finite positions.
@@ -395,25 +419,7 @@ __device__ __forceinline__ void place_slot(const DevState &S, const DevGeom &G, 
     const double cx = corner(0, bx), cy = corner(1, by), cz = corner(2, bz);
     S.rel[rb][i] = make_float4(d2f_rn(x - cx), d2f_rn(y - cy), d2f_rn(z - cz), d2f_rn(r));
     if (count_col) atomicAdd(&S.colcnt[c], 1);
-    if (count_domain) {
-        // inside for certain from the FP32 values (truncated z within 2^-21 of the
-        // magnitudes), else the FP64 test
-        const float zf = d2f_trunc(z);
-        const float m = 4.8e-7f * (fabsf(zf) + fabsf(G.plof[2]) + fabsf(G.phif[2]));
-        const bool sure = G.phif[2] > G.plof[2] && zf - m > G.plof[2] && zf + m < G.phif[2];
-        if (!sure && !(z >= G.plo[2] && z < G.phi[2])) atomicAdd(&S.cnt->out_of_domain, 1ULL);
-    }
-    if (!finite_bits(x) || !finite_bits(y) || !finite_bits(z)) atomicAdd(&S.cnt->nonfinite, 1ULL);
-    if (G.per[0] && (bx == 1 || bx == G.n[0])) {
-        const int sx = (bx == 1) ? 1 : -1;
-        const int gb = bin_of(x + (double)sx * G.len[0], G.plo[0], G.dxi[0], 0, G.n[0] + 1);
-        if (gb != (sx > 0 ? G.n[0] + 1 : 0)) atomicAdd(&S.cnt->edge_ghost, 1ULL);
-    }
-    if (G.per[1] && (by == 1 || by == G.n[1])) {
-        const int sy = (by == 1) ? 1 : -1;
-        const int gb = bin_of(y + (double)sy * G.len[1], G.plo[1], G.dxi[1], 0, G.n[1] + 1);
-        if (gb != (sy > 0 ? G.n[1] + 1 : 0)) atomicAdd(&S.cnt->edge_ghost, 1ULL);
-    }
+    count_slot(S, G, x, y, z, bx, by, count_domain);
 }
 
 __device__ __forceinline__ void rebin_slot_into(const DevState &S, const DevGeom &G, int i, double x, double y,

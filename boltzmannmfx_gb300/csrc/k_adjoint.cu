@@ -162,8 +162,8 @@ __device__ __forceinline__ bool dfwd_term(const DevState &S, const DevGeom &G, c
                                           const DiffParams &D, int a, double xi, double yi, double zi, double ri,
                                           double mi, double ai, int j, int sx, int sy, double *t)
 {
-    const double xj = sx ? S.x[a][j] + (double)sx * G.len[0] : S.x[a][j];
-    const double yj = sy ? S.y[a][j] + (double)sy * G.len[1] : S.y[a][j];
+    const double xj = sx ? image_coord(S.x[a][j], G.len[0], sx) : S.x[a][j];
+    const double yj = sy ? image_coord(S.y[a][j], G.len[1], sy) : S.y[a][j];
     const double dx = xi - xj, dy = yi - yj, dz = zi - S.z[a][j];
     const double r2 = dx * dx + dy * dy + dz * dz;
     if (!G.nbh_trivial && !(r2 <= P.nbh)) return false;
@@ -194,8 +194,8 @@ __device__ __forceinline__ bool dadj_term(const DevState &S, const DevGeom &G, c
     // o: xk, yk, zk, rk, mk, dmk, ak, lk[3]
     const double xk = o[0], yk = o[1], zk = o[2], rk = o[3], mk = o[4], dmk = o[5], ak = o[6];
     const double lk[3] = {o[7], o[8], o[9]};
-    const double xj = sx ? S.x[a][j] + (double)sx * G.len[0] : S.x[a][j];
-    const double yj = sy ? S.y[a][j] + (double)sy * G.len[1] : S.y[a][j];
+    const double xj = sx ? image_coord(S.x[a][j], G.len[0], sx) : S.x[a][j];
+    const double yj = sy ? image_coord(S.y[a][j], G.len[1], sy) : S.y[a][j];
     const double d[3] = {xk - xj, yk - yj, zk - S.z[a][j]};
     const double r2 = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
     if (!G.nbh_trivial && !(r2 <= P.nbh)) return false;

@@ -1,4 +1,5 @@
-// k_list.cu -- FP32F sphere step over a neighbour list with a skin.
+// k_list.cu -- sphere steps over a neighbour list with a skin: the FP32F form, and
+// FP64 steps on the same list (k_list64_step).
 //
 // The force acts only on pairs closer than rA = r_i + r_j + bw
 // (maxInteractionDistance and the gate r^2 <= (r_lm - 1e-15)^2,
@@ -101,7 +102,7 @@ __device__ __forceinline__ long long fx_inc(float f, float c, float cl, bool &bi
 __global__ void k_list_decide(ListCtl *c, DevCounters *cnt, cudaGraphConditionalHandle h, int mode)
 {
     chain_wait();
-    bool run = c->left > 0;
+    bool run = c->left > 0 && !c->bail && !(c->whole && c->overflow);
     bool rb = false;
     if (run) {
         bool need = c->need != 0;
@@ -723,6 +724,312 @@ __device__ __forceinline__ unsigned long long to_fx(double x, const FxGeom &F, i
     return over ? ~0ull : X;
 }
 
+// ---- FP64 steps over the list ------------------------------------------------
+// The plain form on the same list: the list is a superset of the pairs within the
+// cutoff for as long as the bound holds, whoever moves the slots, so an FP64 step
+// needs no re-binning, sort and stencil walk either.  What it must keep is the
+// reference's summation order, which follows the CURRENT bins (27 bins around
+// the slot's own in walk order, ascending caller index within one): each pair
+// that passes the FP64 gate gets that order as its key, from its bins
+// re-derived out of the FP64 positions (bin_of_fast: exact, no FP64 arithmetic),
+// and a slot adds its terms by ascending key.  The keys of a list ascend as it was
+// built and rarely stop doing so between builds; then the slot selects by key.
+// Image membership is the reference's (the image's bin from its shifted FP64
+// position).  So the result is bit-identical to the per-step path's.
+// Each step also writes the slots' coordinates above the domain's corner in
+// FP32 (rel; c = plo + coordinate within 2^-23 of the magnitudes), which the next
+// step screens its entries with.
+// Bound: FP64 issue (2 lanes a clock per SM) of the pairs that pass the screen and
+// of the update, then the screen's loads; 688 000 slots in 64 colonies step in 190 us
+// (per-step path 430 with its rebuild), 400 000 in 80.  Blocks of 64 slots: the
+// pairs of a block spread evenly over its threads, and eight blocks fit an SM.  The
+// staging holds a whole list: with room for 12 entries and a serial way out the few
+// slots beyond it (2 % of a dense colony's blocks held one) kept the kernel for
+// 520 us.  A state with an overflowed list (over 32 slots within the cutoff and the
+// skin of one) steps on the per-step path, whose walk is one thread's or warp's.
+constexpr int kList64Block = 64;
+constexpr int kList64Pairs = 4;  // evaluated at once, per slot on average (more: in batches of slots)
+
+// FP32 coordinates of a position; false when the list does not cover it: a
+// closed axis more than 0.7 of a length outside the domain, or not finite.
+__device__ __forceinline__ bool coords32(const DevGeom &G, double x, double y, double z, float &cx, float &cy,
+                                         float &cz)
+{
+    cx = d2f_rn(x) - G.plof[0];
+    cy = d2f_rn(y) - G.plof[1];
+    cz = d2f_rn(z) - G.plof[2];
+    bool in = finite_bits(x) && finite_bits(y) && finite_bits(z);
+    const float c[3] = {cx, cy, cz};
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        const float len = G.dxf[d] * (float)G.n[d];
+        in = in && c[d] > -0.7f * len && c[d] < 1.7f * len;
+    }
+    return in;
+}
+
+// Whether the state's positions resolve in FP32 coordinates, and those coordinates.
+__global__ void k_list64_begin(const DevState S, int a)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int col = block_colony(S, i);
+    if (i < S.n) {
+        float cx, cy, cz;
+        if (!coords32(S.geoms[col], S.x[a][i], S.y[a][i], S.z[a][i], cx, cy, cz)) S.lctl->bail = 1;
+        S.rel[a][i] = make_float4(cx, cy, cz, d2f_rn(S.rad[i]));
+    }
+}
+
+// Sum of the terms t0 .. t0 + m - 1 by ascending key (the keys of a slot's
+// pairs differ; ~0: no term).
+__device__ __forceinline__ void add_by_key(const unsigned long long *key, const double *term, int pitch, int t0, int m,
+                                           double &fx, double &fy, double &fz)
+{
+    unsigned long long last = 0ull;
+    bool ordered = true;
+    for (int k = t0; k < t0 + m; ++k) {
+        const unsigned long long q = key[k];
+        if (q == ~0ull) continue;
+        ordered = ordered && q >= last;
+        last = q;
+    }
+    if (ordered) {
+        for (int k = t0; k < t0 + m; ++k) {
+            if (key[k] == ~0ull) continue;
+            fx += term[k];
+            fy += term[pitch + k];
+            fz += term[2 * pitch + k];
+        }
+        return;
+    }
+    last = 0ull;
+    for (int r = 0; r < m; ++r) {
+        unsigned long long best = ~0ull;
+        int at = -1;
+        for (int k = t0; k < t0 + m; ++k)
+            if (key[k] < best && (r == 0 || key[k] > last)) {
+                best = key[k];
+                at = k;
+            }
+        if (at < 0) break;
+        last = best;
+        fx += term[at];
+        fy += term[pitch + at];
+        fz += term[2 * pitch + at];
+    }
+}
+
+// The FP64 term of a slot (position and radius o, bins ob, colony geometry Q) on
+// j, and the pair's place in the reference's order (~0: not in the list or
+// beyond the cutoff).
+__device__ __forceinline__ unsigned long long pair_by_list64(const DevState &S, const DevParams &P, int a,
+                                                             const double *o, const int4 ob, const DevGeom &Q, int j,
+                                                             int code, double *t)
+{
+    const int sx = code / 3 - 1, sy = code % 3 - 1;
+    const double x = S.x[a][j], y = S.y[a][j], z = S.z[a][j];
+    const double xj = sx ? image_coord(x, Q.len[0], sx) : x;
+    const double yj = sy ? image_coord(y, Q.len[1], sy) : y;
+    if (!sphere_pair64(P, 1, o[0] - xj, o[1] - yj, o[2] - z, o[3], S.rad[j], t)) return ~0ull;
+    // (an image's bin is the halo cell its shifted position is in, or it is not listed)
+    int jx, jy;
+    if (sx) {
+        jx = sx < 0 ? 0 : Q.n[0] + 1;
+        if (image_bin(Q, 0, xj) != jx) return ~0ull;
+    } else {
+        jx = bin_of_fast(x, Q.plo[0], Q.dxi[0], Q.plof[0], Q.dxif[0], 1, Q.n[0]);
+    }
+    if (sy) {
+        jy = sy < 0 ? 0 : Q.n[1] + 1;
+        if (image_bin(Q, 1, yj) != jy) return ~0ull;
+    } else {
+        jy = bin_of_fast(y, Q.plo[1], Q.dxi[1], Q.plof[1], Q.dxif[1], 1, Q.n[1]);
+    }
+    const int jz = bin_of_fast(z, Q.plo[2], Q.dxi[2], Q.plof[2], Q.dxif[2], 1, Q.n[2]);
+    const int d0 = jx - ob.x + 1, d1 = jy - ob.y + 1, d2 = jz - ob.z + 1;
+    if ((unsigned)d0 > 2u || (unsigned)d1 > 2u || (unsigned)d2 > 2u) return ~0ull;  // not a stencil pair
+    return ((unsigned long long)(d0 * 9 + d1 * 3 + d2) << 32) | (unsigned)S.orig[j];
+}
+
+__global__ void __launch_bounds__(kList64Block, 8) k_list64_step(const DevState S, const DevParams P, double dt)
+{
+    constexpr int B = kList64Block, cap = B * kList64Pairs;
+    static_assert(kNbrCap <= cap, "a slot's pairs fit a batch");
+    chain_wait();
+    // (a stalled step, or one past the call's last; an overflowed list)
+    if (!S.lctl->active || S.lctl->overflow) return;
+    const int a = S.lctl->cur, b = a ^ 1;
+    __shared__ int stage[kNbrCap][B];
+    __shared__ unsigned char codes[kNbrCap][B];
+    __shared__ double opos[B][4];
+    __shared__ int4 obin[B];
+    __shared__ double term[3 * cap];
+    __shared__ unsigned long long key[cap];
+    __shared__ int orun[B + 1], wsum[B / 32];
+    __shared__ unsigned wmin[B / 32][3], wmax[B / 32][3];
+    const int n = S.n;
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const int i = blockIdx.x * B + tid;
+    const bool act = i < n;
+    const int colony = block_colony(S, i);
+    const float4 *__restrict__ ca = S.rel[a];
+    double xi = 0.0, yi = 0.0, zi = 0.0, ri = 0.0;
+    int xl = 0, bx = 1, by = 1, bz = 1;
+    const DevGeom &G = S.geoms[act ? colony : 0];
+    if (act) {
+        const int4 rec = __ldg(&S.lrec[i]);
+        const float4 me = ca[i];
+        xi = S.x[a][i];
+        yi = S.y[a][i];
+        zi = S.z[a][i];
+        ri = S.rad[i];
+        bx = bin_of_fast(xi, G.plo[0], G.dxi[0], G.plof[0], G.dxif[0], 1, G.n[0]);
+        by = bin_of_fast(yi, G.plo[1], G.dxi[1], G.plof[1], G.dxif[1], 1, G.n[1]);
+        bz = bin_of_fast(zi, G.plo[2], G.dxi[2], G.plof[2], G.dxif[2], 1, G.n[2]);
+        const float lenx = G.dxf[0] * (float)G.n[0], leny = G.dxf[1] * (float)G.n[1];
+        // the FP32 coordinates' rounding (2^-23 of the magnitudes each, four of them per
+        // axis with the subtraction's) and 2e-6 of the bound's own
+        const float mag = fabsf(G.plof[0]) + fabsf(G.plof[1]) + fabsf(G.plof[2]) +
+                          2.0f * (lenx + leny + G.dxf[2] * (float)G.n[2]);
+        const float ci = (me.w + P.bw32) * 1.000002f + 2.0e-6f * (G.dxf[0] + G.dxf[1] + G.dxf[2]) + 4.8e-7f * mag;
+        auto entry = [&](int j) {
+            const float4 q = __ldg(&ca[j]);
+            float ex = me.x - q.x, ey = me.y - q.y;
+            const float ez = me.z - q.z;
+            int sx = 0, sy = 0;
+            if (G.per[0] && fabsf(ex) > 0.5f * lenx) {
+                sx = ex < 0.0f ? -1 : 1;
+                ex -= (float)sx * lenx;
+            }
+            if (G.per[1] && fabsf(ey) > 0.5f * leny) {
+                sy = ey < 0.0f ? -1 : 1;
+                ey -= (float)sy * leny;
+            }
+            const float r2f = __fmaf_rn(ex, ex, __fmaf_rn(ey, ey, __fmul_rn(ez, ez)));
+            const float lim = q.w + ci;
+            if (!(r2f > lim * lim)) {
+                stage[xl][tid] = j;
+                codes[xl][tid] = (unsigned char)((sx + 1) * 3 + (sy + 1));
+                ++xl;
+            }
+        };
+        const int len = rec.x & 0xff;
+        if (len > 0) entry(rec.y);
+        if (len > 1) entry(rec.z);
+        if (len > 2) entry(rec.w);
+        const int m = list_extra(len);
+        const int *xs = S.xlist + (m ? __ldg(&S.xoff[i >> 5]) + ((rec.x >> 8) & 0x3ff) : 0);
+        for (int k = 0; k < m; ++k) entry(__ldg(xs + k));
+    }
+    opos[tid][0] = xi;
+    opos[tid][1] = yi;
+    opos[tid][2] = zi;
+    opos[tid][3] = ri;
+    obin[tid] = make_int4(bx, by, bz, colony);
+    // the block's run of staged pairs: slot by slot in thread order
+    int xo = xl;
+    for (int d = 1; d < 32; d <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, xo, d);
+        if (lane >= d) xo += v;
+    }
+    if (lane == 31) wsum[w] = xo;
+    __syncthreads();
+    for (int v = 0; v < w; ++v) xo += wsum[v];
+    orun[tid + 1] = xo;
+    if (tid == 0) orun[0] = 0;
+    __syncthreads();
+    xo -= xl;
+    double fx = 0.0, fy = 0.0, fz = 0.0;
+    // one pair per thread, a slot's terms added by its thread; in batches of
+    // slots when the block's pairs are more than the terms' room
+    for (int s0 = 0; s0 < B;) {
+        const int t0 = orun[s0];
+        int s1 = B;
+        if (orun[B] - t0 > cap)
+            for (s1 = s0 + 1; orun[s1 + 1] - t0 <= cap;) ++s1;
+        const int t1 = orun[s1];
+        for (int t = t0 + tid; t < t1; t += B) {
+            int o = 0;  // the slot that owns pair t
+#pragma unroll
+            for (int s2 = B / 2; s2 >= 1; s2 >>= 1)
+                if (orun[o + s2] <= t) o += s2;
+            const int k = t - orun[o];
+            double tt[3] = {0.0, 0.0, 0.0};
+            key[t - t0] = pair_by_list64(S, P, a, opos[o], obin[o], S.geoms[obin[o].w], stage[k][o], codes[k][o], tt);
+            term[t - t0] = tt[0];
+            term[cap + t - t0] = tt[1];
+            term[2 * cap + t - t0] = tt[2];
+        }
+        __syncthreads();
+        if (tid >= s0 && tid < s1) add_by_key(key, term, cap, xo - t0, xl, fx, fy, fz);
+        __syncthreads();
+        s0 = s1;
+    }
+    unsigned lo[3] = {kKeyPosInf, kKeyPosInf, kKeyPosInf}, hi[3] = {kKeyNegInf, kKeyNegInf, kKeyNegInf};
+    if (act) {
+        // evaluateSurfaceForce, sphere branch, the update and the wrap, as k_sphere64
+        const double vx = plus_zero(fx);
+        const double vy = plus_zero(fy);
+        const double vz = fz + wall_law(zi, ri, P);
+        const double ix = dt * vx, iy = dt * vy, iz = dt * vz;
+        double nx = xi + ix;
+        double ny = yi + iy;
+        const double nz = zi + iz;
+        if (G.per[0]) nx = wrap1(nx, G.plo[0], G.phi[0], G.len[0]);
+        if (G.per[1]) ny = wrap1(ny, G.plo[1], G.phi[1], G.len[1]);
+        S.x[b][i] = nx;
+        S.y[b][i] = ny;
+        S.z[b][i] = nz;
+        S.vx[i] = vx;
+        S.vy[i] = vy;
+        S.vz[i] = vz;
+        float cx, cy, cz;
+        if (!coords32(G, nx, ny, nz, cx, cy, cz)) S.lctl->bail = 1;
+        S.rel[b][i] = make_float4(cx, cy, cz, d2f_rn(ri));
+        count_slot(S, G, nx, ny, nz,
+                   bin_of_fast(nx, G.plo[0], G.dxi[0], G.plof[0], G.dxif[0], 1, G.n[0]),
+                   bin_of_fast(ny, G.plo[1], G.dxi[1], G.plof[1], G.dxif[1], 1, G.n[1]), true);
+        lo[0] = hi[0] = fkey(d2f_rn(ix));
+        lo[1] = hi[1] = fkey(d2f_rn(iy));
+        lo[2] = hi[2] = fkey(d2f_rn(iz));
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        lo[k] = __reduce_min_sync(0xffffffffu, lo[k]);
+        hi[k] = __reduce_max_sync(0xffffffffu, hi[k]);
+        if (lane == 0) {
+            wmin[w][k] = lo[k];
+            wmax[w][k] = hi[k];
+        }
+    }
+    __syncthreads();
+    if (tid < 3) {
+        unsigned l = kKeyPosInf, h = kKeyNegInf;
+        for (int v = 0; v < B / 32; ++v) {
+            l = min(l, wmin[v][tid]);
+            h = max(h, wmax[v][tid]);
+        }
+        if (h >= l) {
+            atomicMin(&S.lctl->inc_min[tid], l);
+            atomicMax(&S.lctl->inc_max[tid], h);
+        }
+    }
+}
+
+// The build's fixed-point positions from the FP64 ones (the high words alone).
+__global__ void k_list64_fx(const DevState S)
+{
+    if (!S.lctl->rebuild) return;
+    const int a = S.lctl->cur;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int col = block_colony(S, i);
+    if (i < S.n) {
+        const FxGeom &F = S.fxg[col];
+        S.fxh[a][i] = make_int4((int)(to_fx(S.x[a][i], F, 0) >> 32), (int)(to_fx(S.y[a][i], F, 1) >> 32),
+                                (int)(to_fx(S.z[a][i], F, 2) >> 32), __float_as_int(d2f_rn(S.rad[i])));
+    }
+}
+
 // Fixed-point positions of buffer a from its FP64 positions and the radii
 __global__ void k_list_init(const DevState S, int a)
 {
@@ -779,6 +1086,26 @@ __global__ void k_list_to_fp64_axis(const DevState S, int a, int ax, double *out
 int launch_list_decide(const DevState &S, unsigned long long cond, int mode, cudaStream_t st)
 {
     launch_after(k_list_decide, 1, 1, 0, st, S.lctl, S.cnt, (cudaGraphConditionalHandle)cond, mode);
+    return 1;
+}
+
+int launch_list64_begin(const DevState &S, int a, cudaStream_t st)
+{
+    k_list64_begin<<<(S.n + 255) / 256, 256, 0, st>>>(S, a);
+    return 1;
+}
+
+int launch_list64_fx(const DevState &S, cudaStream_t st)
+{
+    k_list64_fx<<<(S.n + 255) / 256, 256, 0, st>>>(S);
+    return 1;
+}
+
+int launch_list64_step(const DevState &S, const DevParams &P, double dt, cudaStream_t st, bool chained)
+{
+    const int grid = (S.n + kList64Block - 1) / kList64Block;
+    if (chained) launch_after(k_list64_step, grid, kList64Block, 0, st, S, P, dt);
+    else k_list64_step<<<grid, kList64Block, 0, st>>>(S, P, dt);
     return 1;
 }
 

@@ -40,8 +40,8 @@ __device__ __forceinline__ bool sphere_term64(const DevState &S, const DevGeom &
                                               double xi, double yi, double zi, double ri, int j, int sx, int sy,
                                               double *t)
 {
-    const double xj = sx ? S.x[a][j] + (double)sx * G.len[0] : S.x[a][j];
-    const double yj = sy ? S.y[a][j] + (double)sy * G.len[1] : S.y[a][j];
+    const double xj = sx ? image_coord(S.x[a][j], G.len[0], sx) : S.x[a][j];
+    const double yj = sy ? image_coord(S.y[a][j], G.len[1], sy) : S.y[a][j];
     return sphere_pair64(P, G.nbh_trivial, xi - xj, yi - yj, zi - S.z[a][j], ri, S.rad[j], t);
 }
 

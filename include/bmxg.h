@@ -136,7 +136,7 @@ typedef struct bmxg_stats {
     int64_t n_edge_ghost;       /* periodic images whose bin left the halo cell   */
     int64_t n_bond_repairs;     /* half-bonds repaired (rods)                      */
     int64_t n_rebins;           /* bin-order rebuilds: one per step, or one per
-                                   list build in the FP32F list mode (cumulative) */
+                                   list build in the list mode (cumulative) */
     int64_t n_kernel_launches;  /* kernels this context enqueued, graph nodes counted */
     int64_t main_kernel_launches; /* force-kernel launches timed while profiling     */
     double  main_kernel_ms;     /* their summed device time (profiling mode)        */
@@ -439,8 +439,10 @@ int  bmxg_get_step_pairs(bmxg_ctx *ctx, int64_t *offs, int32_t *idx, int64_t cap
 
 /* ---- tuning ------------------------------------------------------------- */
 
-/* FP32F sphere steps keep a neighbour list with a skin between builds when it
- * reproduces the reference's pair set exactly: the largest force cutoff
+/* Sphere steps keep a neighbour list with a skin between builds when it
+ * reproduces the reference's pair set exactly (FP64 steps: and when there are
+ * enough slots and steps for it to be the faster path; their results are the
+ * per-step path's, bit for bit): the largest force cutoff
  * 2 r_max + bndry_width plus the skin fits inside the smallest bin width, and
  * BMXCheckPair holds for every stencil pair.  mode 1 (default) uses it there,
  * mode 0 never (every step re-bins and walks the stencil).  The reference
