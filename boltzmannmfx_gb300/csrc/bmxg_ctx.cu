@@ -1109,7 +1109,8 @@ constexpr int kListMinSteps = 2;     // a shorter first call after a load runs t
 // 2 r_max + bw plus the skin must stay within the smallest bin width (so
 // that every pair inside the cutoff is a stencil pair whatever the bins),
 // BMXCheckPair must hold for every stencil pair, and the fixed point's high
-// word must resolve offsets to 2^-20 of a bin.
+// word must resolve offsets to 2^-20 of a bin (and its unit squared be a normal
+// FP32 number: the step takes r^2 for one).
 float list_skin(const bmxg_ctx *ctx)
 {
     if (ctx->S.has_rods || ctx->n == 0 || ctx->n >= (1LL << kNbrShift)) return 0.0f;
@@ -1121,8 +1122,10 @@ float list_skin(const bmxg_ctx *ctx)
         const double rcut = 2.0 * ctx->rmax + ctx->prm.bndry_width;
         const double sk = std::min(0.25 * dmin, 0.95 * (dmin - rcut));
         if (!(sk >= 0.02 * dmin)) return 0.0f;
-        for (int d = 0; d < 3; ++d)
-            if (!(std::ldexp((g.per[d] ? 1.0 : 4.0) * g.len[d], -32) <= std::ldexp(dmin, -20))) return 0.0f;
+        for (int d = 0; d < 3; ++d) {
+            const double unit = std::ldexp((g.per[d] ? 1.0 : 4.0) * g.len[d], -32);
+            if (!(unit <= std::ldexp(dmin, -20) && unit >= std::ldexp(1.0, -62))) return 0.0f;
+        }
         skin = std::min(skin, sk);
     }
     return (float)skin;
