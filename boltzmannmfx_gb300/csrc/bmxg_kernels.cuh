@@ -57,8 +57,7 @@ constexpr int kListBins = 0;         // list mode keeps its frozen bins in buffe
 constexpr int kListStepBlock = 128;  // k_list_step's default block (at most 256; autotuned)
 constexpr int kListBuildBlock = 128; // k_list_build's default block (one slot per thread; at most 256)
 constexpr int kSphereBlock = 64;     // per-step sphere kernels' block (one slot per thread)
-constexpr int kWalkNarrow = 65536;   // FP64 steps: 32 slots per block, a warp per neighbour column, up to here
-constexpr int kWalkWide = 400000;    // ... 128 slots per block up to here
+constexpr int kWalkNarrow = 65536;   // adjoint, tile: 32 slots per block, a warp per neighbour column, up to here
 constexpr int kRodCap = 32;          // gated pairs per segment the rod pipelines hold (more: the
                                      // segment walks its stencil in the segment kernel)
 

@@ -55,9 +55,15 @@ __device__ __forceinline__ bool sphere_term64(const DevState &S, const DevGeom &
 // and a warp whose share of a round is empty skips it.  Each slot then adds
 // its pairs' terms in walk order -- the same FP64 values in the same order as
 // a walk that evaluates each pair when it meets it, so the result stays
-// bit-identical to the oracle.  A slot with more than kStage64 staged
-// candidates evaluates them itself, in order, as it walks.
-constexpr int kStage64 = 16;
+// bit-identical to the oracle.  A slot with more than kStage64 candidates walks
+// again and evaluates them itself, in order.
+// Bound: the walk's loads and instructions (FP64 pipe 37 % busy).  The walk over
+// the sorted copies takes a column at a time, four entries in flight, and three blocks of
+// 256 threads fit an SM (80 registers): 500 000 slots 223 -> 172 us, 2 million 687 -> 507,
+// 688 000 in 64 colonies 379 -> 245 against entry by entry with the crowded slots'
+// evaluation inside the walk (128 registers).  64 registers: 183; a stage of 16: 174;
+// the next column's bounds a column ahead: 179; three columns unrolled: 216.
+constexpr int kStage64 = 12;
 
 // dynamic shared memory of k_sphere64 for a block of `block` threads
 __host__ __device__ constexpr size_t sphere64_smem(int block)
@@ -67,7 +73,7 @@ __host__ __device__ constexpr size_t sphere64_smem(int block)
 }
 
 template <bool SORTED>
-__global__ void __launch_bounds__(256) k_sphere64(const DevState S, const DevParams P, double dt, int a)
+__global__ void __launch_bounds__(256, 3) k_sphere64(const DevState S, const DevParams P, double dt, int a)
 {
     // per thread: its staged candidates (j, image code); its slot's position,
     // radius, colony and run of staged pairs (for the block's evaluation);
@@ -85,6 +91,7 @@ __global__ void __launch_bounds__(256) k_sphere64(const DevState S, const DevPar
     int *wsum = opass + B;  // per warp: staged pairs, then their exclusive scan
     const int b = a ^ 1;
     const float bwf = P.bw32;
+    if (SORTED) chain_wait();
     for (int base = blockIdx.x * B; base < S.n; base += gridDim.x * B) {
         const int i = base + tid;
         const bool act = i < S.n;
@@ -102,36 +109,44 @@ __global__ void __launch_bounds__(256) k_sphere64(const DevState S, const DevPar
             zi = S.z[a][i];
             ri = S.rad[i];
             const float4 me = S.rel[a][i];
-            const float dxb = G.dxf[0], dyb = G.dxf[1], dzb = G.dxf[2];
-            // absolute slack bounding the FP32 distance error (offsets + bin widths)
-            const float slack = 8.0f * 1.1920929e-7f * fmaxf(dxb, fmaxf(dyb, dzb));
+            const float slack = screen_slack(G), dzb = G.dxf[2];
             int2 *mine = stage + (size_t)tid * kStage64;
-            auto eval = [&](int j, int sx, int sy) {
-                double t[3];
-                if (sphere_term64(S, G, P, a, xi, yi, zi, ri, j, sx, sy, t)) {
-                    fx += t[0];
-                    fy += t[1];
-                    fz += t[2];
-                }
-            };
-            walk<SORTED>(S, G, a, i, bx, by, izi, [&](const float4 q, auto slot, int dxs, int dys, int dzs, int sx,
-                                                      int sy) {
-                const float ex = (me.x - q.x) - (float)dxs * dxb;
-                const float ey = (me.y - q.y) - (float)dys * dyb;
-                const float ez = (me.z - q.z) - (float)dzs * dzb;
-                const float r2f = __fmaf_rn(ex, ex, __fmaf_rn(ey, ey, __fmul_rn(ez, ez)));
-                const float lim = __fadd_rn(__fadd_rn(__fadd_rn(me.w, q.w), bwf), slack);
-                if (r2f > __fmul_rn(lim, lim)) return;
-                const int j = slot();
-                if (cnt < kStage64) {
-                    mine[cnt] = make_int2(j, (sx + 1) * 3 + (sy + 1));
-                } else {
-                    if (cnt == kStage64)  // too many for the stage: the staged ones first, in order
-                        for (int k = 0; k < kStage64; ++k) eval(mine[k].x, mine[k].y / 3 - 1, mine[k].y % 3 - 1);
-                    eval(j, sx, sy);
-                }
+            auto take = [&](int j, int sx, int sy) {
+                if (cnt < kStage64) mine[cnt] = make_int2(j, (sx + 1) * 3 + (sy + 1));
                 ++cnt;
-            });
+            };
+            if constexpr (SORTED) {
+                const int self_t = S.rank[a][i];
+                for (int c = 0; c < kWalkCols; ++c) {
+                    const float ox = (float)(c / 3 - 1) * G.dxf[0], oy = (float)(c % 3 - 1) * G.dxf[1];
+                    int ii, jj, lo, hi, sx, sy;
+                    if (!walk_target(S, G, a, bx, by, c, ii, jj, lo, hi, sx, sy)) continue;
+                    walk_column(S, a, lo, hi, self_t, izi, [&](int t, const float4 q, int dzs) {
+                        if (!near_pair32(me, q, ox, oy, (float)dzs * dzb, bwf, slack)) return;
+                        const int j = __ldg(&S.perm[a][t]);
+                        if ((sx | sy) && !image_in_row(S, G, a, j, ii, jj, sx, sy)) return;
+                        take(j, sx, sy);
+                    });
+                }
+            } else {
+                walk<false>(S, G, a, i, bx, by, izi, [&](const float4 q, auto slot, int dxs, int dys, int dzs, int sx,
+                                                         int sy) {
+                    if (near_pair32(me, q, (float)dxs * G.dxf[0], (float)dys * G.dxf[1], (float)dzs * dzb, bwf, slack))
+                        take(slot(), sx, sy);
+                });
+            }
+            if (cnt > kStage64)  // too many for the stage: the whole walk, each pair evaluated as it is met
+                walk<SORTED>(S, G, a, i, bx, by, izi, [&](const float4 q, auto slot, int dxs, int dys, int dzs, int sx,
+                                                          int sy) {
+                    if (!near_pair32(me, q, (float)dxs * G.dxf[0], (float)dys * G.dxf[1], (float)dzs * dzb, bwf, slack))
+                        return;
+                    double t[3];
+                    if (sphere_term64(S, G, P, a, xi, yi, zi, ri, slot(), sx, sy, t)) {
+                        fx += t[0];
+                        fy += t[1];
+                        fz += t[2];
+                    }
+                });
         }
         // the block's run of staged pairs: slot by slot in thread order
         const int xl = (cnt <= kStage64) ? cnt : 0;
@@ -389,32 +404,21 @@ static void allow_smem_once(K kernel, size_t bytes, std::atomic<unsigned long lo
 }
 
 // Which FP64 kernel a sorted state takes: one warp per neighbour column where
-// the slots are too few for a thread each to hide the walk's dependent loads
-// (32 slots per block up to kWalkNarrow slots, 128 up to kWalkWide), one thread
-// per slot above, where the walk's instructions count and not its latency.
-// Measured, us per step with the re-binning, one thread per slot / 32 / 128
-// slots per block: 1000 spheres 39 / 17 / -, 20 000 50 / 30 / 44, 40 000 54 / 41 / 48,
-// 80 000 69 / 65 / 59, 160 000 96 / 109 / 77, 500 000 (host load and store
-// included) 698 / 814 / 698, 688 000 in 64 colonies 445 / 552 / 483.
-static int sphere64_slots(int n)
-{
-    return n <= kWalkNarrow ? 32 : (n <= kWalkWide ? 128 : 0);
-}
+// the slots are too few for a thread each to hide the walk's dependent loads,
+// one thread per slot above, where the walk's instructions count and not its
+// latency.  Measured, us a step of the kernel alone, one thread per slot / one warp
+// per column, on a sparse and a dense monolayer: 10 000 slots 36, 35 / 28, 21,
+// 20 000 25, 36 / 23, 27, 40 000 27, 42 / 31, 45, 100 000 34, 53 / 62, 87, 400 000
+// 105, 167 / 226, 276.
+constexpr int kColumnSlots64 = 32768;
 
 int launch_sphere_step(const DevState &S, const DevParams &P, double dt, int a, int precision, int grid,
                        int block, cudaStream_t st, int resync, bool pinned)
 {
     const bool sorted = S.srel[a] != nullptr;  // the context keeps sorted copies; bare callers do not
     if (precision == BMXG_FP64_FORM) {
-        const int ns = (sorted && !pinned) ? sphere64_slots(S.n) : 0;
-        if (ns == 32) {
+        if (sorted && !pinned && S.n <= kColumnSlots64) {
             launch_after(k_sphere64w<32, 6>, (S.n + 31) / 32, kWalkBlock, sizeof(WalkMem<32, 6>), st, S, P, dt, a);
-            return 1;
-        }
-        if (ns == 128) {
-            static std::atomic<unsigned long long> known{0};
-            allow_smem_once(k_sphere64w<128, 4>, sizeof(WalkMem<128, 4>), known);
-            launch_after(k_sphere64w<128, 4>, (S.n + 127) / 128, kWalkBlock, sizeof(WalkMem<128, 4>), st, S, P, dt, a);
             return 1;
         }
         // (block a multiple of 32, at most 256: the block stages and evaluates its pairs together)
@@ -422,7 +426,7 @@ int launch_sphere_step(const DevState &S, const DevParams &P, double dt, int a, 
         if (sorted) {
             static std::atomic<unsigned long long> known{0};
             allow_smem_once(k_sphere64<true>, sphere64_smem(256), known);
-            k_sphere64<true><<<grid, block, smem, st>>>(S, P, dt, a);
+            launch_after(k_sphere64<true>, grid, block, smem, st, S, P, dt, a);
         } else {
             static std::atomic<unsigned long long> known{0};
             allow_smem_once(k_sphere64<false>, sphere64_smem(256), known);

@@ -194,7 +194,7 @@ int launch_tile_step(const TileCall &C, const TileGeom &T, const DevParams &P, d
     const int n = C.S.n, blk = 128;
     k_tile_bin<<<(n + blk - 1) / blk, blk, 0, st>>>(C, T);
     int k = 1 + launch_rebuild(C.S, 0, scan_scratch, (n + blk - 1) / blk, blk, st);
-    // 32 or 128 slots per block: the whole-domain step's rule
+    // 32 slots per block while that leaves SMs without work, then 128
     if (n <= kWalkNarrow) {
         k_tile_step<32, 6><<<(n + 31) / 32, kWalkBlock, sizeof(WalkMem<32, 6>), st>>>(C, T, P, dt);
     } else {
