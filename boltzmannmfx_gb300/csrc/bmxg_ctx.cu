@@ -1091,16 +1091,17 @@ void prof_events(bmxg_ctx *ctx, cudaEvent_t *k0, cudaEvent_t *k1)
 // ---- FP32F neighbour list with a skin ---------------------------------------
 constexpr int kListMaxAge = 64;      // builds at least this often
 // FP64 spheres step over the list where it is the faster path, per-step path / list:
-// 10 000 slots 19 / 22 us a step, 20 000 29 / 22, 40 000 40 / 24, 160 000 84 / 48,
-// 400 000 155 / 96, 688 000 in 64 colonies 430 / 245 (up to 16 384 slots the
+// 10 000 slots 19 / 22 us a step, 20 000 29 / 22, 40 000 37 / 24, 160 000 69 / 48,
+// 400 000 128 / 95, 688 000 in 64 colonies 295 / 236 (up to 16 384 slots the
 // per-step path's sort is one cluster and its step little more than two launches).
-// From a load on, with the build: 6 steps of 20 000 slots 387 / 370 us, 400 000
-// 1294 / 1031; fewer steps keep the per-step path.  The list's buffers and graphs
-// cost 0.6-0.7 ms once, which 7 + 1.6e6 / slots steps pay back (fresh context, 20
-// steps: 40 000 slots 2294 / 2439, 160 000 4192 / 4180, 400 000 6590 / 6254).
+// From a load on, with the build: 6 steps of 40 000 slots 446 / 444 us, 400 000
+// 1180 / 1047; fewer steps keep the per-step path.  The list's buffers and graphs
+// cost 0.6-0.7 ms once, which 12 + 2.4e6 / slots steps pay back, above 300 000 slots
+// 6e6 / slots (fresh context, 20 steps: 40 000 slots 2086 / 2335, 160 000 3943 / 4145,
+// 400 000 6159 / 6245; 100 steps: 4726 / 4289, 9066 / 7385, 15 604 / 12 924; the 64
+// colonies, 10 steps: 4702 / 4412).
 constexpr int kList64Slots = 16384;
 constexpr int kList64MinSteps = 6;
-constexpr double kList64Pay = 1.6e6;
 constexpr int kListSingles = 4;      // so few steps: a graph (with its conditional node) for each
 constexpr int kListMinSteps = 2;     // a shorter first call after a load runs the per-step path
 
@@ -1138,7 +1139,8 @@ bool list64_pays(const bmxg_ctx *ctx, int32_t nsteps)
     if (ctx->list_valid && ctx->list_prec == BMXG_FP64) return true;
     if (ctx->step_count + nsteps < kList64MinSteps) return false;
     if (ctx->S.nbr) return true;
-    if ((double)(ctx->plain64 + nsteps) < 7.0 + kList64Pay / (double)ctx->n) return false;
+    const double steps = (double)(ctx->plain64 + nsteps), n = (double)ctx->n;
+    if (steps < 12.0 + 2.4e6 / n && steps < 6.0e6 / n) return false;
     // (and leaves three quarters of the free memory)
     size_t room = 0, all = 0;
     const size_t need = (size_t)ctx->n * 320 + (size_t)ctx->ncells_total * sizeof(int);

@@ -770,7 +770,7 @@ __device__ __forceinline__ unsigned long long to_fx(double x, const FxGeom &F, i
 // step screens its entries with.
 // Bound: FP64 issue (2 lanes a clock per SM) of the pairs that pass the screen and
 // of the update, then the screen's loads; 688 000 slots in 64 colonies step in 190 us
-// (per-step path 430 with its rebuild), 400 000 in 80.  Blocks of 64 slots: the
+// (per-step path 295 with its rebuild), 400 000 in 80.  Blocks of 64 slots: the
 // pairs of a block spread evenly over its threads, and eight blocks fit an SM.  The
 // staging holds a whole list: with room for 12 entries and a serial way out the few
 // slots beyond it (2 % of a dense colony's blocks held one) kept the kernel for

@@ -67,11 +67,11 @@ def test_list_steps_equal_per_step_path(gpu_lib, oracle_lib, sizes, side, crowd,
     B.set_list_mode(0)
     for c in (A, B):
         c.set_state(P, off)
-        c.step(0.25, 128, BMXG_FP64)  # (enough steps for the rule to take the list)
+        c.step(0.25, 160, BMXG_FP64)  # (enough steps for the rule to take the list)
     same(A, B, P)
     over = crowd > 32  # some list overflows: one build, then the per-step path
-    assert (A.stats()["n_rebins"] == 129 if over else A.stats()["n_rebins"] < 128)
-    assert B.stats()["n_rebins"] == 128
+    assert (A.stats()["n_rebins"] == 161 if over else A.stats()["n_rebins"] < 160)
+    assert B.stats()["n_rebins"] == 160
     for k in (3, 1, 9):
         A.step(0.25, k, BMXG_FP64)
         B.step(0.25, k, BMXG_FP64)
@@ -110,7 +110,7 @@ def test_range_left_in_mid_call(gpu_lib):
     A, B = Context(PRM, g), Context(PRM, g)
     B.set_list_mode(0)
     A.set_state(warm)
-    A.step(0.25, 128, BMXG_FP64)
+    A.step(0.25, 160, BMXG_FP64)
     for c in (A, B):
         c.set_state(P)
     r0 = A.stats()["n_rebins"]
@@ -135,7 +135,7 @@ def test_form_changes_between_calls(gpu_lib):
     A, B = Context(PRM, g), Context(PRM, g)
     B.set_list_mode(0)
     A.set_state(P)
-    A.step(0.25, 128, BMXG_FP64)
+    A.step(0.25, 160, BMXG_FP64)
     A.step(0.25, 8, BMXG_FP32F)
     B.set_state(state(A, P))
     A.step(0.25, 7, BMXG_FP64)
@@ -160,7 +160,7 @@ def test_prepared_and_profiled_calls(gpu_lib, nsteps):
     A, B = Context(PRM, g), Context(PRM, g)
     for c in (A, B):
         c.set_state(P)
-        c.step(0.25, 128, BMXG_FP64)
+        c.step(0.25, 160, BMXG_FP64)
         c.set_state(P)
     A.prepare(0.25, BMXG_FP64)
     B.set_profiling(True)
@@ -182,7 +182,7 @@ def test_non_finite_positions_are_reported(gpu_lib, field, bad):
     B.set_list_mode(0)
     for c in (A, B):
         c.set_state(P)
-        c.step(0.25, 128, BMXG_FP64)
+        c.step(0.25, 160, BMXG_FP64)
         c.set_state(N)
         with pytest.raises(BmxgError) as e:
             c.step(0.25, 8, BMXG_FP64)
