@@ -163,6 +163,22 @@ __device__ __forceinline__ void col_to_bxy(const DevGeom &G, int col, int &bx, i
 constexpr int kWalkCols = 9;
 constexpr int kWalkBlock = 32 * kWalkCols;
 
+// Blocks an SM a launch of `blocks` is compiled for, `least` to 5: as few (as many
+// registers a thread, as few spills) as hold the grid in the fewest waves.  The
+// blocks do about the same work, so a wave that is nearly empty costs as much
+// as a full one.  Measured, us: k_sphere64w, 3 / 4 / 5 blocks an SM: 10 000 slots (3 blocks for
+// each SM) 14.7 / 14.9 / 15.1, 15 000 (4) 22.7 / 15.3 / 16.9, 20 000 (5) 22.8 / 22.2 / 16.8, 25 000
+// (6) 22.7 / 22.8 / 23.9, 32 768 (7) 29.5 / 23.1 / 25.1; the adjoint's two kernels with 3 and 2 / 3 and
+// 3 / 5 and 5, forward and backward of 40 steps: 9000 slots 2634 / 2686 / 2923, 14 000 3171 / 2767 /
+// 3252, 24 000 4651 / 4307 / 3595, 48 000 7500 / 7120 / 5794.
+inline int wave_fit(int blocks, int least)
+{
+    int best = least;
+    for (int k = least + 1; k <= 5; ++k)
+        if ((blocks + kSMs * k - 1) / (kSMs * k) < (blocks + kSMs * best - 1) / (kSMs * best)) best = k;
+    return best;
+}
+
 // One column of one slot: up to four entries are loaded before any is used.
 // f(t, dzs) for every entry of z bins izi - 1 .. izi + 1 but the slot itself.
 template <class F>

@@ -413,8 +413,8 @@ __global__ void __launch_bounds__(256) k_dadj(const DevState S, const DevParams 
 // The same two kernels with one warp per neighbour column (bmxg_stencil.cuh),
 // for sizes whose walks are bound by their dependent loads: same pairs, same
 // FP64 operations, same order of the sums.
-template <int NS, int STAGE>
-__global__ void __launch_bounds__(kWalkBlock, 3) k_dfwdw(const DevState S, const DevParams P, DiffParams D, double dt,
+template <int NS, int STAGE, int RESIDENT>
+__global__ void __launch_bounds__(kWalkBlock, RESIDENT) k_dfwdw(const DevState S, const DevParams P, DiffParams D, double dt,
                                                          int a)
 {
     extern __shared__ __align__(16) unsigned char smw[];
@@ -482,8 +482,8 @@ __global__ void __launch_bounds__(kWalkBlock, 3) k_dfwdw(const DevState S, const
     rebin_slot(S, G, i, nx, ny, nz, ri, b);
 }
 
-template <int NS, int STAGE>
-__global__ void __launch_bounds__(kWalkBlock, 2) k_dadjw(const DevState S, const DevParams P, DiffParams D, double dt,
+template <int NS, int STAGE, int RESIDENT>
+__global__ void __launch_bounds__(kWalkBlock, RESIDENT) k_dadjw(const DevState S, const DevParams P, DiffParams D, double dt,
                                                          int a, const double *lin, double *lout, double *gacc, double *gadh)
 {
     constexpr int NO = 10, NT = 7;
@@ -602,7 +602,9 @@ int launch_dfwd(const DevState &S, const DevParams &P, const DiffParams &D, doub
     // with recomputation, one thread per slot -> a warp per column: 1000 spheres 57 -> 23 / 144 -> 77, 20 000
     // 79 -> 40 / 195 -> 129, 40 000 82 -> 61 / 207 -> 192)
     if (S.srel[a] && !pinned && S.n <= kWalkNarrow) {
-        launch_after(k_dfwdw<32, 6>, (S.n + 31) / 32, kWalkBlock, sizeof(WalkMem<32, 6>), st, S, P, D, dt, a);
+        const int blocks = (S.n + 31) / 32, fit = wave_fit(blocks, 3);
+        launch_after(fit == 3 ? k_dfwdw<32, 6, 3> : (fit == 4 ? k_dfwdw<32, 6, 4> : k_dfwdw<32, 6, 5>), blocks,
+                     kWalkBlock, sizeof(WalkMem<32, 6>), st, S, P, D, dt, a);
     } else if (S.srel[a]) {
         allow_smem(k_dfwd<true>, smem);
         k_dfwd<true><<<grid, block, smem, st>>>(S, P, D, dt, a);
@@ -618,8 +620,10 @@ int launch_dadj(const DevState &S, const DevParams &P, const DiffParams &D, doub
 {
     const size_t smem = staged_smem(block, 10, 7);
     if (S.srel[a] && !pinned && S.n <= kWalkNarrow) {
-        launch_after(k_dadjw<32, 6>, (S.n + 31) / 32, kWalkBlock, sizeof(WalkMem<32, 6>), st, S, P, D, dt, a, lin,
-                     lout, gacc, gadh);
+        const int blocks = (S.n + 31) / 32, fit = wave_fit(blocks, 2);
+        launch_after(fit == 2 ? k_dadjw<32, 6, 2>
+                              : (fit == 3 ? k_dadjw<32, 6, 3> : (fit == 4 ? k_dadjw<32, 6, 4> : k_dadjw<32, 6, 5>)),
+                     blocks, kWalkBlock, sizeof(WalkMem<32, 6>), st, S, P, D, dt, a, lin, lout, gacc, gadh);
     } else if (S.srel[a]) {
         allow_smem(k_dadj<true>, smem);
         k_dadj<true><<<grid, block, smem, st>>>(S, P, D, dt, a, lin, lout, gacc, gadh);

@@ -233,8 +233,8 @@ __global__ void __launch_bounds__(256, 3) k_sphere64(const DevState S, const Dev
 // The same step with one warp per neighbour column (bmxg_stencil.cuh): the
 // staged pairs one per thread over the block, the sums and the slots' updates
 // in its first warps.  Same pairs, same FP64 operations, same order of the sums.
-template <int NS, int STAGE>
-__global__ void __launch_bounds__(kWalkBlock, 3) k_sphere64w(const DevState S, const DevParams P, double dt, int a)
+template <int NS, int STAGE, int RESIDENT>
+__global__ void __launch_bounds__(kWalkBlock, RESIDENT) k_sphere64w(const DevState S, const DevParams P, double dt, int a)
 {
     extern __shared__ __align__(16) unsigned char smw[];
     auto &M = *reinterpret_cast<WalkMem<NS, STAGE> *>(smw);
@@ -418,7 +418,9 @@ int launch_sphere_step(const DevState &S, const DevParams &P, double dt, int a, 
     const bool sorted = S.srel[a] != nullptr;  // the context keeps sorted copies; bare callers do not
     if (precision == BMXG_FP64_FORM) {
         if (sorted && !pinned && S.n <= kColumnSlots64) {
-            launch_after(k_sphere64w<32, 6>, (S.n + 31) / 32, kWalkBlock, sizeof(WalkMem<32, 6>), st, S, P, dt, a);
+            const int blocks = (S.n + 31) / 32, fit = wave_fit(blocks, 3);
+            launch_after(fit == 3 ? k_sphere64w<32, 6, 3> : (fit == 4 ? k_sphere64w<32, 6, 4> : k_sphere64w<32, 6, 5>),
+                         blocks, kWalkBlock, sizeof(WalkMem<32, 6>), st, S, P, dt, a);
             return 1;
         }
         // (block a multiple of 32, at most 256: the block stages and evaluates its pairs together)
