@@ -22,11 +22,19 @@ using namespace bmxg;
 
 namespace {
 
+// What a step call reads back, in one copy.
+struct StepBlock {
+    DevCounters cnt;
+    alignas(256) ListCtl ctl;  // (its atomics in lines of their own)
+};
+
 struct GraphKey {
     double dt;
     int precision;
     int parity;
-    int single;  // -1: kResyncEvery steps; 0 / 1: one step without / with the FP32F re-sync
+    // -1: kResyncEvery steps; 0 / 1: one step without / with the FP32F re-sync (list steps:
+    // 1 one that adds itself to the call's steps, 2 one of those set before)
+    int single;
     bool list;   // list steps (their kernels read the parity from the control block)
     bool operator<(const GraphKey &o) const
     {
@@ -81,7 +89,8 @@ struct bmxg_ctx {
     std::vector<int> h_cbase;
     std::vector<DevGeom> h_geoms;
     DevCounters *d_cnt = nullptr;
-    DevCounters *h_cnt = nullptr;  // pinned
+    DevCounters *h_cnt = nullptr;  // pinned (h_step's)
+    StepBlock *d_step = nullptr, *h_step = nullptr;
     int *scan_scratch = nullptr;
     // staging in caller order
     double *ud = nullptr;  // n doubles
@@ -120,8 +129,8 @@ struct bmxg_ctx {
                               // and no kernel that writes them ran since
     int64_t step_count = 0;   // steps since set_state (FP32F re-sync schedule)
 
-    // FP32F neighbour list with a skin (k_list.cu)
-    int list_mode = 1;            // 1: FP32F sphere steps use the list where it is exact; 0: never
+    // neighbour list with a skin (k_list.cu)
+    int list_mode = 1;            // 1: sphere steps use the list where it is exact (FP64: and pays); 0: never
     bool list_on = false;         // the steps being enqueued use the list
     bool list_valid = false;      // the list and its frozen bins describe the state
     bool bins_exact = true;       // bins of buffer `parity` are the reference's (list steps freeze them)
@@ -135,9 +144,10 @@ struct bmxg_ctx {
     int64_t plain64 = 0;          // FP64 steps of this state's size that went without a list
     float list_period = 16.0f;    // steps per list build, from the calls so far
     int *h_run = nullptr;         // pinned: steps and buffer of a list call
-    ListCtl *h_lctl = nullptr;    // pinned copy of the control block
+    ListCtl *h_lctl = nullptr;    // pinned copy of the control block (h_step's)
     unsigned long long body_runs_seen = 0;  // list builds already counted as launches
     bool capturing = false;       // enqueue_step runs inside a graph capture
+    bool list_one = false;        // ... of a list step that adds itself to the call's steps
     bool pair_capture = false;    // list steps record their gated pairs (S.pcap)
     bool pcap_valid = false;      // S.pcap holds the last step's gated pairs
     bool fx_ahead = false;        // list steps moved the fixed-point positions past the FP64 ones
@@ -470,8 +480,11 @@ int bmxg_create(const bmxg_params *params, int32_t ncolonies, const bmxg_geometr
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->own_stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreate(&ctx->ev0);
     if (e == cudaSuccess) e = cudaEventCreate(&ctx->ev1);
-    if (e == cudaSuccess) e = cudaMallocHost(&ctx->h_cnt, sizeof(DevCounters));
-    if (e == cudaSuccess) e = cudaMallocHost(&ctx->h_lctl, sizeof(ListCtl));
+    if (e == cudaSuccess) e = cudaMallocHost(&ctx->h_step, sizeof(StepBlock));
+    if (e == cudaSuccess) {
+        ctx->h_cnt = &ctx->h_step->cnt;
+        ctx->h_lctl = &ctx->h_step->ctl;
+    }
     if (e == cudaSuccess) e = cudaMallocHost(&ctx->h_run, 2 * sizeof(int));
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->body_stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->io_stream, cudaStreamNonBlocking);
@@ -498,8 +511,7 @@ void bmxg_destroy(bmxg_ctx *ctx)
     if (!ctx) return;
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     free_state(ctx);
-    if (ctx->h_cnt) cudaFreeHost(ctx->h_cnt);
-    if (ctx->h_lctl) cudaFreeHost(ctx->h_lctl);
+    if (ctx->h_step) cudaFreeHost(ctx->h_step);
     if (ctx->h_run) cudaFreeHost(ctx->h_run);
     if (ctx->body_stream) cudaStreamDestroy(ctx->body_stream);
     if (ctx->io_stream) {
@@ -742,7 +754,8 @@ int load_state(bmxg_ctx *ctx, const bmxg_particles *p, const int64_t *colony_off
     AL(ctx->d_geoms, ctx->ncol);
     AL(ctx->d_fxg, ctx->ncol);
     AL(ctx->d_cbase, ctx->ncol + 1);
-    AL(ctx->d_cnt, 1);
+    AL(ctx->d_step, 1);
+    ctx->d_cnt = &ctx->d_step->cnt;
     for (int k = 0; k < 2; ++k) {
         AL(S.x[k], n); AL(S.y[k], n); AL(S.z[k], n);
         AL(S.rel[k], n); AL(S.col[k], n); AL(S.iz[k], n);
@@ -1088,7 +1101,7 @@ void prof_events(bmxg_ctx *ctx, cudaEvent_t *k0, cudaEvent_t *k1)
     }
 }
 
-// ---- FP32F neighbour list with a skin ---------------------------------------
+// ---- neighbour list with a skin ---------------------------------------
 constexpr int kListMaxAge = 64;      // builds at least this often
 // FP64 spheres step over the list where it is the faster path, per-step path / list:
 // 10 000 slots 19 / 22 us a step, 20 000 29 / 22, 40 000 37 / 24, 160 000 69 / 48,
@@ -1102,7 +1115,11 @@ constexpr int kListMaxAge = 64;      // builds at least this often
 // colonies, 10 steps: 4702 / 4412).
 constexpr int kList64Slots = 16384;
 constexpr int kList64MinSteps = 6;
-constexpr int kListSingles = 4;      // so few steps: a graph (with its conditional node) for each
+// So few list steps go as a graph (with its conditional node) for each, more as graphs of
+// kResyncEvery whose surplus steps return at once: the node costs 7 us, a surplus step its
+// blocks' launch.  3 / 4 steps as singles and as one graph, us: 20 000 slots 66, 81 and 53, 63;
+// 200 000 79, 93 and 68, 77; 1 million 128, 167 and 163, 177.
+inline int list_singles(int64_t n) { return n <= 400000 ? 2 : 4; }
 constexpr int kListMinSteps = 2;     // a shorter first call after a load runs the per-step path
 
 // Skin of the list for the loaded state and parameters, or 0 where the list
@@ -1172,7 +1189,7 @@ int ensure_list(bmxg_ctx *ctx, float skin, int precision)
         // (the scratch serves the scan of the column counts and that of the groups' entries)
         const int nscan = (int)std::max<int64_t>(S.ncols_total, ((int64_t)ctx->n + 31) / 32);
         if ((rc = dalloc(ctx, &ctx->cell_scratch, scan_scratch_ints(nscan)))) return rc;
-        if ((rc = dalloc(ctx, &S.lctl, 1))) return rc;
+        S.lctl = &ctx->d_step->ctl;
         S.ncells_total = (int)ctx->ncells_total;
         S.cols_max = 0;
         for (const DevGeom &g : ctx->h_geoms) S.cols_max = std::max(S.cols_max, g.n[0] * g.n[1]);
@@ -1198,6 +1215,7 @@ int ensure_list(bmxg_ctx *ctx, float skin, int precision)
     h.max_age = kListMaxAge;
     h.whole = precision == BMXG_FP64;
     h.force = 1;
+    h.par = ctx->parity;
     CK(cudaMemcpyAsync(S.lctl, &h, sizeof(h), cudaMemcpyHostToDevice, ctx->stream));
     // the fixed-point positions (FP64 form: the screen's coordinates) start from
     // the FP64 ones
@@ -1252,7 +1270,7 @@ int set_list_run(bmxg_ctx *ctx, int steps)
     return BMXG_OK;
 }
 
-// One FP32F list step: decide, build when needed (capturing: a conditional node
+// One list step: decide, build when needed (capturing: a conditional node
 // where `build`, else the step stalls), then the force / update kernel.  What
 // ran is counted after the call (two kernels a step, the build's when it ran):
 // a kernel of a step that did not run returns at once.
@@ -1275,7 +1293,7 @@ int enqueue_list_step(bmxg_ctx *ctx, double dt, int precision, bool build)
         CK(cudaStreamGetCaptureInfo(st, &cs, nullptr, &cg, &deps, &ed, &nd));
         cudaGraphConditionalHandle h;
         CK(cudaGraphConditionalHandleCreate(&h, cg, 0, 0));
-        launch_list_decide(S, (unsigned long long)h, kDecideCond, st);
+        launch_list_decide(S, (unsigned long long)h, ctx->list_one ? kDecideOne : kDecideCond, st);
         CK(cudaStreamGetCaptureInfo(st, &cs, nullptr, &cg, &deps, &ed, &nd));
         cudaGraphNodeParams cp = {cudaGraphNodeTypeConditional};
         cp.conditional.handle = h;
@@ -1360,7 +1378,7 @@ int get_graph(bmxg_ctx *ctx, double dt, int precision, int parity, cudaGraphExec
 {
     if (ctx->list_on) {
         parity = 0;
-        if (single >= 0) single = 1;
+        if (single >= 0) single = std::max(single, 1);
     }
     GraphKey key{dt, precision, parity, single, ctx->list_on};
     auto it = ctx->graphs.find(key);
@@ -1376,7 +1394,11 @@ int get_graph(bmxg_ctx *ctx, double dt, int precision, int parity, cudaGraphExec
     int rc2 = BMXG_OK;
     ctx->capturing = true;
     if (single >= 0)
+    {
+        ctx->list_one = ctx->list_on && single == 1;
         rc2 = enqueue_step(ctx, dt, precision, parity, single);
+        ctx->list_one = false;
+    }
     else
         for (int s = 0; s < kResyncEvery && !rc2; ++s)
             rc2 = enqueue_step(ctx, dt, precision, parity ^ (s & 1),
@@ -1407,15 +1429,20 @@ int get_graph(bmxg_ctx *ctx, double dt, int precision, int parity, cudaGraphExec
 int list_steps(bmxg_ctx *ctx, double dt, int32_t nsteps, int precision, int32_t *done)
 {
     cudaStream_t st = ctx->stream;
-    if (int rc = set_list_run(ctx, nsteps)) return rc;
+    // a call of few steps sets nothing before them (the copy costs 3-6 us): none are
+    // left over from the last, and the buffer is where that ended
+    const bool few = !ctx->profiling && nsteps <= list_singles(ctx->n);
+    if (!few)
+        if (int rc = set_list_run(ctx, nsteps)) return rc;
+    ctx->list_valid = false;  // until the steps have run
     int left = nsteps;
     while (left > 0) {
         cudaGraphExec_t g = nullptr;
         if (ctx->profiling) {  // launched one by one, with events around the force kernel
             for (int k = 0; k < left; ++k)
                 if (int rc = enqueue_list_step(ctx, dt, precision, true)) return rc;
-        } else if (left <= kListSingles) {
-            if (int rc = get_graph(ctx, dt, precision, 0, &g, 1)) return rc;
+        } else if (few || (left < nsteps && left <= 4)) {  // (the last ones: none can stall)
+            if (int rc = get_graph(ctx, dt, precision, 0, &g, few ? 1 : 2)) return rc;
             for (int k = 0; k < left; ++k) CK(cudaGraphLaunch(g, st));
         } else {
             if (int rc = get_graph(ctx, dt, precision, 0, &g)) return rc;
@@ -1424,8 +1451,7 @@ int list_steps(bmxg_ctx *ctx, double dt, int32_t nsteps, int precision, int32_t 
             for (int k = 0; k < graphs; ++k) CK(cudaGraphLaunch(g, st));
         }
         CK(cudaEventRecord(ctx->ev1, st));
-        CK(cudaMemcpyAsync(ctx->h_cnt, ctx->d_cnt, sizeof(DevCounters), cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(ctx->h_lctl, ctx->S.lctl, sizeof(ListCtl), cudaMemcpyDeviceToHost, st));
+        CK(cudaMemcpyAsync(ctx->h_step, ctx->d_step, sizeof(StepBlock), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
         const int now = ctx->h_lctl->left;
         const bool over = precision == BMXG_FP64 && ctx->h_lctl->overflow;  // (the step of that build did not run)
@@ -1449,7 +1475,7 @@ int list_steps(bmxg_ctx *ctx, double dt, int32_t nsteps, int precision, int32_t 
         ctx->bins_exact = false;
         if (precision == BMXG_FP32F) ctx->fx_ahead = true;
     }
-    if (precision == BMXG_FP64 && ctx->list64_bail) ctx->list_valid = false;
+    ctx->list_valid = !(precision == BMXG_FP64 && ctx->list64_bail);
     return BMXG_OK;
 }
 
@@ -1546,7 +1572,7 @@ int bmxg_prepare(bmxg_ctx *ctx, double dt, int32_t precision)
     for (int parity = 0; parity < 2; ++parity) {
         cudaGraphExec_t g = nullptr;
         if (int rc = get_graph(ctx, subdt, precision, parity, &g)) return rc;
-        for (int resync = 0; resync < 2; ++resync)
+        for (int resync = 0; resync < (ctx->list_on ? 3 : 2); ++resync)
             if (int rc = get_graph(ctx, subdt, precision, parity, &g, resync)) return rc;
     }
     return BMXG_OK;
@@ -1571,7 +1597,8 @@ int bmxg_step(bmxg_ctx *ctx, double dt, int32_t nsteps, int32_t precision)
     // load-step-store caller never reuses a list); later calls build one
     if (int rc = step_setup(ctx, nsteps, precision)) return rc;
     // the per-step counters (the end of each step clears them for the next)
-    CK(cudaMemsetAsync(ctx->d_cnt, 0, kStepCounters * sizeof(unsigned long long), ctx->stream));
+    // (list steps clear them first)
+    if (!ctx->list_on) CK(cudaMemsetAsync(ctx->d_cnt, 0, kStepCounters * sizeof(unsigned long long), ctx->stream));
     CK(cudaEventRecord(ctx->ev0, ctx->stream));
     int32_t left = nsteps;
     ctx->kev_used = 0;
@@ -1582,6 +1609,7 @@ int bmxg_step(bmxg_ctx *ctx, double dt, int32_t nsteps, int32_t precision)
         if (left > 0) {  // (FP64, out of the list's range) the rest on the per-step path
             if (int rc = ensure_exact(ctx)) return rc;
             ctx->list_on = false;
+            CK(cudaMemsetAsync(ctx->d_cnt, 0, kStepCounters * sizeof(unsigned long long), ctx->stream));
         }
     }
     const bool by_list = ctx->list_on;

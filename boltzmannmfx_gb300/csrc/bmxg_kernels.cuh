@@ -245,7 +245,9 @@ int launch_sphere_step(const DevState &S, const DevParams &P, double dt, int a, 
 // this step rebuilds.  What follows it in the stream: kDecideStall no build (a
 // step that needs one does not run, nor the ones after it), kDecideCond a
 // conditional node (cond) with the build, kDecideBuild the gated build kernels.
-enum { kDecideStall = 0, kDecideCond = 1, kDecideBuild = 2 };
+// kDecideOne: as kDecideCond, and the call's steps are one more (a call of few steps sets
+// none before it).
+enum { kDecideStall = 0, kDecideCond = 1, kDecideBuild = 2, kDecideOne = 3 };
 int launch_list_decide(const DevState &S, unsigned long long cond, int mode, cudaStream_t st);
 // fixed-point positions of buffer a from its FP64 positions and radii (when the
 // list starts on a state), and back (whenever the FP64 positions are read)

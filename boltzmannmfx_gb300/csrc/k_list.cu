@@ -108,6 +108,7 @@ __device__ __forceinline__ long long fx_inc_small(float f, float c, float cl, fl
 __global__ void k_list_decide(ListCtl *c, DevCounters *cnt, cudaGraphConditionalHandle h, int mode)
 {
     chain_wait();
+    if (mode == kDecideOne) c->left += 1;
     bool run = c->left > 0 && !c->bail && !(c->whole && c->overflow);
     bool rb = false;
     if (run) {
@@ -157,7 +158,7 @@ __global__ void k_list_decide(ListCtl *c, DevCounters *cnt, cudaGraphConditional
     }
     c->active = run ? 1 : 0;
     c->rebuild = rb ? 1 : 0;
-    if (mode == kDecideCond) cudaGraphSetConditional(h, rb ? 1u : 0u);
+    if (mode == kDecideCond || mode == kDecideOne) cudaGraphSetConditional(h, rb ? 1u : 0u);
 }
 
 // Colony of index i for a kernel whose blocks take consecutive indices, one
