@@ -558,10 +558,14 @@ def run_ours(args):
     achieved = alg / (k_ms / 1e3) / 1e9
     if list_mode:
         kname = "k_list_step"
+    elif kind == "sphere" and prec == BMXG_FP64 and rebins < args.steps:
+        kname = "k_list64_step"
     elif kind == "rod" and prec == BMXG_FP32F:  # the events bracket the three kernels of the rod pipeline
-        kname = "k_rod_pair32 + k_rod_pair64 + k_rod_seg32"
+        kname = "k_rod_pair32 + k_rod_pair64q + k_rod_seg"
+    elif kind == "rod":
+        kname = "k_rod_pair64 + k_rod_seg"
     else:
-        kname = ("k_sphere" if kind == "sphere" else "k_rod_force") + ("<FP32F>" if prec == BMXG_FP32F else "<FP64>")
+        kname = "k_sphere" + ("<FP32F>" if prec == BMXG_FP32F else "<FP64>")
     roof = {"bound": "hbm", "kernel": kname, "achieved": achieved, "peak": peak, "unit": "GB/s",
             "frac": achieved / peak, "peak_kind": peak_kind, "kernel_ms": k_ms,
             "algorithmic_bytes_per_launch": alg,

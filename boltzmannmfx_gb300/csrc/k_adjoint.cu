@@ -598,9 +598,10 @@ int launch_dfwd(const DevState &S, const DevParams &P, const DiffParams &D, doub
                 cudaStream_t st, bool pinned)
 {
     const size_t smem = staged_smem(block, 6, 3);
-    // (the FP64 step's rule, launch_sphere_step.  Measured, us per step of the forward / the backward sweep
+    // (a warp per column up to kWalkNarrow slots.  Measured, us per step of the forward / the backward sweep
     // with recomputation, one thread per slot -> a warp per column: 1000 spheres 57 -> 23 / 144 -> 77, 20 000
-    // 79 -> 40 / 195 -> 129, 40 000 82 -> 61 / 207 -> 192)
+    // 79 -> 40 / 195 -> 129, 40 000 82 -> 61 / 207 -> 192; with the resident blocks chosen by wave_fit
+    // 20 000 spheres take 35 / 82)
     if (S.srel[a] && !pinned && S.n <= kWalkNarrow) {
         const int blocks = (S.n + 31) / 32, fit = wave_fit(blocks, 3);
         launch_after(fit == 3 ? k_dfwdw<32, 6, 3> : (fit == 4 ? k_dfwdw<32, 6, 4> : k_dfwdw<32, 6, 5>), blocks,
