@@ -770,9 +770,11 @@ __device__ __forceinline__ unsigned long long to_fx(double x, const FxGeom &F, i
 // FP32 (rel; c = plo + coordinate within 2^-23 of the magnitudes), which the next
 // step screens its entries with.
 // Bound: FP64 issue (2 lanes a clock per SM) of the pairs that pass the screen and
-// of the update, then the screen's loads; 688 000 slots in 64 colonies step in 190 us
-// (per-step path 295 with its rebuild), 400 000 in 80.  Blocks of 64 slots: the
-// pairs of a block spread evenly over its threads, and eight blocks fit an SM.  The
+// of the update, then the screen's loads; 688 000 slots in 64 colonies step in 187 us
+// (per-step path 295 with its rebuild), 400 000 in 81.  Blocks of 64 slots: the
+// pairs of a block spread evenly over its threads; ten blocks fit an SM (96 registers:
+// 2 million slots 372 us; eight at 119 386, twelve at 80 381; the entries' gathers four at
+// a time 373).  The
 // staging holds a whole list: with room for 12 entries and a serial way out the few
 // slots beyond it (2 % of a dense colony's blocks held one) kept the kernel for
 // 520 us.  A state with an overflowed list (over 32 slots within the cutoff and the
@@ -881,7 +883,7 @@ __device__ __forceinline__ unsigned long long pair_by_list64(const DevState &S, 
     return ((unsigned long long)(d0 * 9 + d1 * 3 + d2) << 32) | (unsigned)S.orig[j];
 }
 
-__global__ void __launch_bounds__(kList64Block, 8) k_list64_step(const DevState S, const DevParams P, double dt)
+__global__ void __launch_bounds__(kList64Block, 10) k_list64_step(const DevState S, const DevParams P, double dt)
 {
     constexpr int B = kList64Block, cap = B * kList64Pairs;
     static_assert(kNbrCap <= cap, "a slot's pairs fit a batch");
