@@ -863,19 +863,20 @@ __device__ __forceinline__ unsigned long long pair_by_list64(const DevState &S, 
     const double xj = sx ? image_coord(x, Q.len[0], sx) : x;
     const double yj = sy ? image_coord(y, Q.len[1], sy) : y;
     if (!sphere_pair64(P, 1, o[0] - xj, o[1] - yj, o[2] - z, o[3], S.rad[j], t)) return ~0ull;
-    // (an image's bin is the halo cell its shifted position is in, or it is not listed)
-    int jx, jy;
+    // (an image is listed when its source's own bin is the face's and its shifted
+    // position is in the halo cell; image_bin clamps, and a position beyond a face,
+    // as a load may hold, has partners farther in than the face's bin)
+    int jx = bin_of_fast(x, Q.plo[0], Q.dxi[0], Q.plof[0], Q.dxif[0], 1, Q.n[0]);
+    int jy = bin_of_fast(y, Q.plo[1], Q.dxi[1], Q.plof[1], Q.dxif[1], 1, Q.n[1]);
     if (sx) {
+        if (jx != (sx < 0 ? Q.n[0] : 1)) return ~0ull;
         jx = sx < 0 ? 0 : Q.n[0] + 1;
         if (image_bin(Q, 0, xj) != jx) return ~0ull;
-    } else {
-        jx = bin_of_fast(x, Q.plo[0], Q.dxi[0], Q.plof[0], Q.dxif[0], 1, Q.n[0]);
     }
     if (sy) {
+        if (jy != (sy < 0 ? Q.n[1] : 1)) return ~0ull;
         jy = sy < 0 ? 0 : Q.n[1] + 1;
         if (image_bin(Q, 1, yj) != jy) return ~0ull;
-    } else {
-        jy = bin_of_fast(y, Q.plo[1], Q.dxi[1], Q.plof[1], Q.dxif[1], 1, Q.n[1]);
     }
     const int jz = bin_of_fast(z, Q.plo[2], Q.dxi[2], Q.plof[2], Q.dxif[2], 1, Q.n[2]);
     const int d0 = jx - ob.x + 1, d1 = jy - ob.y + 1, d2 = jz - ob.z + 1;
