@@ -26,14 +26,9 @@ struct ListCtl {
     // per component, the smallest and largest position increment of the last
     // step over all slots (order-preserving integer keys of the floats); the
     // change of any pair's separation since the build is bounded per
-    // component by the sum over steps of (largest - smallest).  In lines of their
-    // own: every block of a step ends with an atomic on each of them, and every block
-    // begins by reading `active` and `cur`, which waited behind those atomics where the
-    // line was the same.  1.1 million slots, calls of 1 / 12 FP32F steps 63.7 / 703 -> 55.2 /
-    // 611 us (56.5 / 652 with the buffer a kernel argument), 1.6 million 77.9 / 948 -> 64.6 / 824,
-    // 500 000 51.0 / 407 -> 42.1 / 369, 480 000 in 64 colonies, 40 steps, 1297 -> 1197.
+    // component by the sum over steps of (largest - smallest)
     unsigned inc_min[3], inc_max[3];
-    alignas(256) float range[3];  // those sums since the last build
+    float range[3];        // those sums since the last build
     float acc;             // |range|: the bound on any pair's separation change
     float skin;            // list skin (cm)
     float eps_step;        // FP32 rounding of one position update, added per step
@@ -42,8 +37,6 @@ struct ListCtl {
     int force;             // rebuild at the next step (the state changed)
     int rebuild;           // this step's decision (read by the gated kernels)
     int need;              // a build is due; set where none can run, the steps stall until one can
-    int active;            // the step that follows runs (there are steps left, no build is due)
-    int cur;               // ... reading the fixed-point positions of this buffer
     int left, par;         // steps left in the call and the buffer the next one reads (set by the host)
     int whole;             // the steps take no overflowed list (FP64 form)
     int bail;              // FP64 list steps: a slot left the range the list covers; no step runs any more
@@ -53,6 +46,14 @@ struct ListCtl {
     // the persistent list step's chunk dispenser: the next chunk to hand out
     // and the blocks that found none left; the last of them resets both
     unsigned next_chunk, done_blocks;
+    // Whether the step that follows runs (there are steps left, no build is due), and the
+    // buffer it reads.  In a line of their own: every block of a step begins by reading
+    // them and ends with an atomic on each of inc_min and inc_max, and the reads waited
+    // behind those atomics where the line was the same.  1.1 million slots, calls of 1 / 12
+    // FP32F steps 63.7 / 703 -> 55.2 / 611 us (56.5 / 652 with the buffer a kernel argument),
+    // 1.6 million 77.9 / 948 -> 64.6 / 824, 500 000 51.0 / 407 -> 42.1 / 369.
+    alignas(256) int active;
+    int cur;
 };
 static_assert(offsetof(ListCtl, active) / 256 != offsetof(ListCtl, inc_max) / 256 &&
                   offsetof(ListCtl, cur) / 256 != offsetof(ListCtl, inc_max) / 256,

@@ -9,6 +9,7 @@
 // (src/des/bmx_pc.H:55-82), periodic images come from a one-cell halo
 // (src/des/bmx_pc.cpp:23).  All of it is integer / byte work bounded by HBM
 // and L2 bandwidth; nothing here is a contraction.
+#include <algorithm>
 #include <atomic>
 
 #include <cooperative_groups.h>
@@ -164,6 +165,67 @@ __device__ __forceinline__ void publish_counters(DevCounters *c, RodCtl *rctl)
     }
 }
 
+// ---- long columns ------------------------------------------------------------
+// A slot's rank in its column counted over all of the column's keys is work of the
+// square of its length: columns of tall domains.  Their keys are first put into
+// ascending order kRun at a time (one warp per run of them from the column's start),
+// then a rank is a binary search per run, eight reads for 128 keys.  In the cluster sort,
+// whose 16 SMs counted slower than the separate kernels' blocks do, 60 000 FP64 spheres in
+// 1 / 4 / 16 / 64 columns, 5 steps: 54.4 / 16.2 / 5.35 / 2.12 -> 12.7 / 4.5 / 1.90 / 1.29 ms
+// (separate kernels, every key counted: 16.6 / 5.21 / 2.25 / 1.37); runs of 32: 33.9 / 10.4 /
+// 3.32 / 1.46.  In a tile of 50 451 + 62 038 in 36 columns 2006 -> 1653 us (cell by cell 1791).
+// Where it starts: 65 000 spheres at 253 / 112 a column, 5 steps, from 128 slots on 980 / 836, from
+// 512 on 1075 / 786 us.
+constexpr int kLongColumn = 160;  // slots of a column above which its runs are sorted
+constexpr int kRun = 128;
+
+// The warp sorts the run at t (keys t .. end - 1, at most kRun of them): a bitonic
+// network over four keys a lane, key e of the run in lane e & 31.
+__device__ __forceinline__ void sort_run(unsigned long long *lkey, int t, int end)
+{
+    constexpr int M = kRun / 32;
+    const int lane = threadIdx.x & 31;
+    unsigned long long v[M];
+#pragma unroll
+    for (int j = 0; j < M; ++j) v[j] = (t + lane + 32 * j < end) ? lkey[t + lane + 32 * j] : ~0ull;
+#pragma unroll
+    for (int k = 2; k <= kRun; k <<= 1)
+#pragma unroll
+        for (int d = k >> 1; d > 0; d >>= 1)
+#pragma unroll
+            for (int j = 0; j < M; ++j) {
+                const bool up = ((lane + 32 * j) & k) == 0;
+                if (d >= 32) {
+                    const int q = j | (d >> 5);
+                    if (q == j) continue;
+                    const unsigned long long lo = min(v[j], v[q]), hi = max(v[j], v[q]);
+                    v[j] = up ? lo : hi;
+                    v[q] = up ? hi : lo;
+                } else {
+                    const unsigned long long o = __shfl_xor_sync(0xffffffffu, v[j], d);
+                    v[j] = (up == ((lane & d) == 0)) ? min(v[j], o) : max(v[j], o);
+                }
+            }
+#pragma unroll
+    for (int j = 0; j < M; ++j)
+        if (t + lane + 32 * j < end) lkey[t + lane + 32 * j] = v[j];
+}
+
+// Keys below `key` among s0 .. s1 - 1, the runs from s0 in order.
+__device__ __forceinline__ int rank_in_runs(const unsigned long long *lkey, int s0, int s1, unsigned long long key)
+{
+    int rank = 0;
+    for (int t = s0; t < s1; t += kRun) {
+        const int m = min(kRun, s1 - t);
+        int c = 0;
+#pragma unroll
+        for (int d = kRun; d > 0; d >>= 1)
+            if (c + d <= m && lkey[t + c + d - 1] < key) c += d;
+        rank += c;
+    }
+    return rank;
+}
+
 // ---- scatter into columns, then the deterministic in-column order --------
 // Arrival order from the atomics is arbitrary; k_canon ranks every slot by
 // its (z bin, original index) key among the members of its column, which is
@@ -187,7 +249,15 @@ __global__ void k_scatter(const DevState S, int b)
     }
 }
 
-__global__ void k_canon(const DevState S, int b, int publish)
+// (one column per blockIdx.x; the warps of blockIdx.y's blocks take its runs in turn)
+__global__ void __launch_bounds__(256) k_sort_runs(const DevState S, int b)
+{
+    const int s0 = max(S.colstart[b][blockIdx.x], 0), s1 = min(S.colstart[b][blockIdx.x + 1], S.n);
+    const int w = (blockIdx.y * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.y * blockDim.x) >> 5;
+    for (int t = s0 + w * kRun; t < s1; t += nw * kRun) sort_run(S.lkey, t, s1);
+}
+
+__global__ void k_canon(const DevState S, int b, int publish, int runs)
 {
     if (publish && blockIdx.x == 0 && threadIdx.x == 0) publish_counters(S.cnt, S.rctl);
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < S.n; i += gridDim.x * blockDim.x) {
@@ -196,7 +266,9 @@ __global__ void k_canon(const DevState S, int b, int publish)
         const int izi = S.iz[b][i];
         const unsigned long long key = col_key(izi, S.orig ? S.orig[i] : i);
         int rank = 0;
-        if (S.lkey) {
+        if (runs) {
+            rank = rank_in_runs(S.lkey, s0, s1, key);
+        } else if (S.lkey) {
             for (int t = s0; t < s1; ++t) rank += (__ldg(&S.lkey[t]) < key);
         } else {
             for (int t = s0; t < s1; ++t) {
@@ -245,19 +317,62 @@ constexpr int kSortItems = 4;    // slots per thread
 constexpr int kSortCols = 16;    // columns per thread
 constexpr int kSortCluster = 16; // blocks (non-portable size; 8 where the device refuses it)
 
+// The rest of k_sort_cluster, after the keys' scatter, for a state with a long
+// column; at: the places the thread's slots drew.  (Out of line, and found out from
+// the scatter: with the columns' lengths looked at in the scan and this in line the sort of
+// 50 000 segments in 65 536 columns took 2 us more; so, 1 us.)
+__device__ __noinline__ void rank_long(const SortJob &J, int g, int T, int4 at)
+{
+    for (int k = 0; k < kSortItems; ++k) {  // a run is sorted by the warp whose slot drew its first place
+        const int i = g + k * T;
+        int t = k == 0 ? at.x : (k == 1 ? at.y : (k == 2 ? at.z : at.w)), end = 0;
+        if (i < J.n) {
+            const int c = J.col[i];
+            const int s0 = max(J.colstart[c], 0);
+            end = min(J.colstart[c + 1], J.n);
+            if (end - s0 <= kLongColumn || ((t - s0) & (kRun - 1)) || t < s0 || t >= end) end = 0;
+        }
+        for (unsigned m = __ballot_sync(0xffffffffu, end > 0); m; m &= m - 1) {
+            const int from = __ffs(m) - 1;
+            sort_run(J.lkey, __shfl_sync(0xffffffffu, t, from), __shfl_sync(0xffffffffu, end, from));
+        }
+    }
+    cooperative_groups::this_cluster().sync();
+    for (int i = g; i < J.n; i += T) {
+        const int c = J.col[i], z = J.iz[i];
+        const int s0 = max(J.colstart[c], 0), s1 = min(J.colstart[c + 1], J.n);
+        const unsigned long long key = col_key(z, J.orig ? J.orig[i] : i);
+        int r = 0;
+        if (s1 - s0 > kLongColumn) r = rank_in_runs(J.lkey, s0, s1, key);
+        else
+            for (int t = s0; t < s1; ++t) r += (J.lkey[t] < key);
+        const int t = s0 + r;
+        if (t >= s1) {  // i is not among its column's members: inconsistent counts
+            atomicAdd(&J.cnt->bad_index, 1ULL);
+            continue;
+        }
+        J.perm[t] = i;
+        if (J.srel) {
+            J.srel[t] = J.rel[i];
+            J.siz[t] = z;
+            J.rank[i] = t;
+        }
+    }
+}
+
 __global__ void __launch_bounds__(kSortBlock) k_sort_cluster(const SortJob J)
 {
     namespace cg = cooperative_groups;
     cg::cluster_group cl = cg::this_cluster();
     __shared__ int warp_sums[kSortBlock / 32];
-    __shared__ int block_sum;
+    __shared__ int block_sum, some_long;
     const int nb = (int)cl.num_blocks(), rank = (int)cl.block_rank();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int T = nb * kSortBlock, g = rank * kSortBlock + tid;
     chain_wait();
     if (J.publish && g == 0) publish_counters(J.cnt, J.rctl);
     // this thread's slots, loaded while the scan runs
-    int c[kSortItems], z[kSortItems], o[kSortItems];
+    int c[kSortItems], z[kSortItems], o[kSortItems], at[kSortItems];
 #pragma unroll
     for (int k = 0; k < kSortItems; ++k) {
         const int i = g + k * T;
@@ -280,6 +395,7 @@ __global__ void __launch_bounds__(kSortBlock) k_sort_cluster(const SortJob J)
         if (lane >= d) x += y;
     }
     if (lane == 31) warp_sums[warp] = x;
+    if (tid == 0) some_long = 0;
     __syncthreads();
     if (warp == 0) {
         int w = warp_sums[lane];
@@ -311,8 +427,15 @@ __global__ void __launch_bounds__(kSortBlock) k_sort_cluster(const SortJob J)
         const int t = J.colstart[c[k]] + r;
         if (t >= 0 && t < J.n) J.lkey[t] = col_key(z[k], o[k]);
         else atomicAdd(&J.cnt->bad_index, 1ULL);
+        at[k] = t;
+        if (r == kLongColumn)  // (one slot of each long column: every block learns of it)
+            for (int v = 0; v < nb; ++v) *cl.map_shared_rank(&some_long, v) = 1;
     }
     cl.sync();
+    if (some_long) {  // (the same in every block)
+        rank_long(J, g, T, make_int4(at[0], at[1], at[2], at[3]));
+        return;
+    }
 #pragma unroll
     for (int k = 0; k < kSortItems; ++k) {
         if (c[k] < 0) continue;
@@ -644,8 +767,12 @@ int launch_rebuild(const DevState &S, int b, int *scan_scratch, int grid, int bl
     if (sort_in_cluster(J, st)) return 1;
     const int k = launch_scan(S.colcnt, S.colstart[b], S.ncols_total, scan_scratch, st);
     k_scatter<<<grid, block, 0, st>>>(S, b);
-    k_canon<<<grid, block, 0, st>>>(S, b, publish ? 1 : 0);
-    return k + 2;
+    // (the host knows the columns' average alone)
+    const bool runs = S.lkey && S.n / std::max(S.ncols_total, 1) > kLongColumn;
+    if (runs)
+        k_sort_runs<<<dim3(S.ncols_total, std::max(1, std::min(64, S.n / S.ncols_total / 256))), 256, 0, st>>>(S, b);
+    k_canon<<<grid, block, 0, st>>>(S, b, publish ? 1 : 0, runs ? 1 : 0);
+    return k + 2 + (runs ? 1 : 0);
 }
 
 int launch_user_bin(const DevState &S, const double *ux, const double *uy, const double *uz, int *ucol,
