@@ -32,8 +32,9 @@ struct GraphKey {
     double dt;
     int precision;
     int parity;
-    // -1: kResyncEvery steps; 0 / 1: one step without / with the FP32F re-sync (list steps:
-    // 1 one that adds itself to the call's steps, 2 one of those set before)
+    // -1: kResyncEvery steps (list steps: -2 with a build possible before each, -1 before the
+    // first); 0 / 1: one step without / with the FP32F re-sync (list steps: 1 one that adds
+    // itself to the call's steps, 2 one of those set before)
     int single;
     bool list;   // list steps (their kernels read the parity from the control block)
     bool operator<(const GraphKey &o) const
@@ -142,7 +143,10 @@ struct bmxg_ctx {
     bool list_room = true;        // (false: no room for the list, FP64 steps go without)
     bool list64_bail = false;     // the loaded state left what FP64 list steps cover
     int64_t plain64 = 0;          // FP64 steps of this state's size that went without a list
-    float list_period = 16.0f;    // steps per list build, from the calls so far
+    // list steps and the builds that fell due among them, over the last calls
+    // (16 steps a build to begin with)
+    double period_steps = 4.0, period_builds = 0.25;
+    bool list_begun = false;      // the next build is the list's first (not one that fell due)
     int *h_run = nullptr;         // pinned: steps and buffer of a list call
     ListCtl *h_lctl = nullptr;    // pinned copy of the control block (h_step's)
     unsigned long long body_runs_seen = 0;  // list builds already counted as launches
@@ -1120,6 +1124,12 @@ constexpr int kList64MinSteps = 6;
 // blocks' launch.  3 / 4 steps as singles and as one graph, us: 20 000 slots 66, 81 and 53, 63;
 // 200 000 79, 93 and 68, 77; 1 million 128, 167 and 163, 177.
 inline int list_singles(int64_t n) { return n <= 400000 ? 2 : 4; }
+// Fewer steps a build than this: graphs with a conditional node before every step, where
+// none stalls.  48 FP32F steps with one node per graph / one per step, by steps a build, us:
+// 2000 slots 5: 1033 / 1200, 4: 1203 / 1287, 3: 1474 / 1472, 2: 2108 / 1865, 1.2: 3201 / 2517;
+// 200 000 slots 5: 1529 / 1681, 3: 2151 / 2058, 1.2: 4548 / 3658; 1 million 5: 3977 / 4018,
+// 3: 5676 / 5092, 1.2: 12 479 / 9857.
+constexpr double kStallPeriod = 4.0;
 constexpr int kListMinSteps = 2;     // a shorter first call after a load runs the per-step path
 
 // Skin of the list for the loaded state and parameters, or 0 where the list
@@ -1230,6 +1240,7 @@ int ensure_list(bmxg_ctx *ctx, float skin, int precision)
     CK(cudaStreamSynchronize(ctx->stream));
     ctx->skin_cur = skin;
     ctx->body_runs_seen = 0;
+    ctx->list_begun = true;
     ctx->list_valid = true;
     return BMXG_OK;
 }
@@ -1373,7 +1384,9 @@ int enqueue_step(bmxg_ctx *ctx, double dt, int precision, int a, int resync)
 // kResyncEvery list steps has one, before its first step; a step that finds a
 // build due stalls, with the rest of the graph, until the next graph's.  200 000
 // spheres, 100 steps, load and store: 2.19 -> 1.70 ms; 2.73 M in 256 colonies the
-// same within noise, where a stalled launch of 10 700 blocks costs what it saves)
+// same within noise, where a stalled launch of 10 700 blocks costs what it saves.
+// Where builds fall due every few steps the stalls cost more than the nodes: see
+// kStallPeriod)
 int get_graph(bmxg_ctx *ctx, double dt, int precision, int parity, cudaGraphExec_t *out, int single = -1)
 {
     if (ctx->list_on) {
@@ -1402,7 +1415,7 @@ int get_graph(bmxg_ctx *ctx, double dt, int precision, int parity, cudaGraphExec
     else
         for (int s = 0; s < kResyncEvery && !rc2; ++s)
             rc2 = enqueue_step(ctx, dt, precision, parity ^ (s & 1),
-                               ctx->list_on ? s == 0 : s == kResyncEvery - 1);
+                               ctx->list_on ? s == 0 || single == -2 : s == kResyncEvery - 1);
     ctx->capturing = false;
     cudaError_t e = cudaStreamEndCapture(ctx->stream, &g);
     if (rc2) {
@@ -1436,8 +1449,10 @@ int list_steps(bmxg_ctx *ctx, double dt, int32_t nsteps, int precision, int32_t 
         if (int rc = set_list_run(ctx, nsteps)) return rc;
     ctx->list_valid = false;  // until the steps have run
     int left = nsteps;
+    double due = 0.0;  // builds of this call that fell due
     while (left > 0) {
         cudaGraphExec_t g = nullptr;
+        const double period = (ctx->period_steps + (nsteps - left)) / (ctx->period_builds + due);
         if (ctx->profiling) {  // launched one by one, with events around the force kernel
             for (int k = 0; k < left; ++k)
                 if (int rc = enqueue_list_step(ctx, dt, precision, true)) return rc;
@@ -1445,15 +1460,17 @@ int list_steps(bmxg_ctx *ctx, double dt, int32_t nsteps, int precision, int32_t 
             if (int rc = get_graph(ctx, dt, precision, 0, &g, few ? 1 : 2)) return rc;
             for (int k = 0; k < left; ++k) CK(cudaGraphLaunch(g, st));
         } else {
-            if (int rc = get_graph(ctx, dt, precision, 0, &g)) return rc;
-            const float stalled = 0.5f * (kResyncEvery - 1) * (float)left / std::max(ctx->list_period, 1.0f);
-            const int graphs = std::max(1, (int)(((float)left + stalled) / (float)kResyncEvery));
+            const bool each = period < kStallPeriod;
+            if (int rc = get_graph(ctx, dt, precision, 0, &g, each ? -2 : -1)) return rc;
+            const double stalled = each ? 0.0 : 0.5 * (kResyncEvery - 1) * left / std::max(period, 1.0);
+            const int graphs = std::max(1, (int)((left + stalled) / kResyncEvery));
             for (int k = 0; k < graphs; ++k) CK(cudaGraphLaunch(g, st));
         }
         CK(cudaEventRecord(ctx->ev1, st));
         CK(cudaMemcpyAsync(ctx->h_step, ctx->d_step, sizeof(StepBlock), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
         const int now = ctx->h_lctl->left;
+        due = (double)(ctx->h_lctl->body_runs - ctx->body_runs_seen) - (ctx->list_begun ? 1.0 : 0.0);
         const bool over = precision == BMXG_FP64 && ctx->h_lctl->overflow;  // (the step of that build did not run)
         if (over || ctx->h_lctl->bail) {
             ctx->list64_bail = true;
@@ -1469,7 +1486,13 @@ int list_steps(bmxg_ctx *ctx, double dt, int32_t nsteps, int precision, int32_t 
     const unsigned long long runs = ctx->h_lctl->body_runs - ctx->body_runs_seen;
     ctx->body_runs_seen = ctx->h_lctl->body_runs;
     ctx->launches += (int64_t)runs * (kListBodyKernels + (precision == BMXG_FP64 ? 1 : 0)) + 2 * (int64_t)*done;
-    if (runs > 0) ctx->list_period = 0.5f * (ctx->list_period + (float)*done / (float)runs);
+    ctx->list_begun = ctx->list_begun && runs == 0;
+    ctx->period_steps += *done;
+    ctx->period_builds += std::max(due, 0.0);
+    while (ctx->period_steps > 64.0) {
+        ctx->period_steps *= 0.5;
+        ctx->period_builds *= 0.5;
+    }
     ctx->stats.n_rebins += (int64_t)runs;
     if (*done > 0) {
         ctx->bins_exact = false;
