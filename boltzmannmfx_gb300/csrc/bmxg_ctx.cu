@@ -143,6 +143,10 @@ struct bmxg_ctx {
     bool list_room = true;        // (false: no room for the list, FP64 steps go without)
     bool list64_bail = false;     // the loaded state left what FP64 list steps cover
     int64_t plain64 = 0;          // FP64 steps of this state's size that went without a list
+    bool list64_live = false;     // FP64 steps follow a list; it has lasted list64_lived steps
+    int64_t list64_lived = 0;
+    int list64_short = 0;         // lists in a row that did not last kList64MinSteps steps
+    int64_t list64_since = 0;     // FP64 steps in a row without one
     // list steps and the builds that fell due among them, over the last calls
     // (16 steps a build to begin with)
     double period_steps = 4.0, period_builds = 0.25;
@@ -178,6 +182,7 @@ struct bmxg_ctx {
 namespace {
 
 int sync_fp64(bmxg_ctx *ctx);
+void list64_end(bmxg_ctx *ctx, bool poor = false);
 
 // What a load checks of a state (launch_check_state), when the caller has done so.
 struct StateCheck {
@@ -282,6 +287,8 @@ void free_state(bmxg_ctx *ctx)
     ctx->rod_walk = false;
     ctx->list_room = true;
     ctx->plain64 = 0;
+    list64_end(ctx);
+    ctx->list64_short = 0;
     ctx->d_geoms = nullptr;
     ctx->d_cbase = nullptr;
     ctx->scan_scratch = nullptr;
@@ -543,6 +550,7 @@ int bmxg_set_params(bmxg_ctx *ctx, const bmxg_params *params)
     if (int rc = sync_fp64(ctx)) return rc;  // the list's fixed point restarts from the FP64 positions
     ctx->prm = *params;
     drop_graphs(ctx);
+    list64_end(ctx);
     ctx->list_valid = false;
     if (ctx->have_state) {
         build_geoms(ctx);
@@ -855,6 +863,7 @@ int load_state(bmxg_ctx *ctx, const bmxg_particles *p, const int64_t *colony_off
     ctx->vel64_zero = !p->velx && !p->vely && !p->velz && !p->wx && !p->wy && !p->wz;
     ctx->step_count = 0;
     ctx->list64_bail = false;
+    list64_end(ctx);
     ctx->parity = 0;
     ctx->rmax = rmax;
     ctx->list_valid = false;
@@ -1159,12 +1168,29 @@ float list_skin(const bmxg_ctx *ctx)
     return (float)skin;
 }
 
+// The FP64 steps in a row over one list, or without one, end (poor: its builds fell due
+// too often).
+void list64_end(bmxg_ctx *ctx, bool poor)
+{
+    if (ctx->list64_live) ctx->list64_short = (poor || ctx->list64_lived < kList64MinSteps) ? ctx->list64_short + 1 : 0;
+    ctx->list64_live = false;
+    ctx->list64_lived = 0;
+    ctx->list64_since = 0;
+}
+
 // Whether FP64 steps go over the list (which covers the state: list_skin).
+// A list pays from kList64MinSteps on, and those are not known beforehand: a reader of
+// the bins, another form or a load ends it, or the state moves so fast that it is built
+// again too soon.  From the second list in a row that did not last, twice as many steps
+// without one, or in the call, are asked for each time.  One step and an export of the
+// neighbour list in turn, us: 20 000 slots 100 without, 154 with a list for every step, 400 000
+// 230 and 263.
 bool list64_pays(const bmxg_ctx *ctx, int32_t nsteps)
 {
     if (!ctx->list_room || ctx->list64_bail || ctx->n <= kList64Slots) return false;
     if (ctx->list_valid && ctx->list_prec == BMXG_FP64) return true;
-    if (ctx->step_count + nsteps < kList64MinSteps) return false;
+    if (ctx->list64_since + nsteps < (int64_t)kList64MinSteps << std::min(std::max(ctx->list64_short - 1, 0), 10))
+        return false;
     if (ctx->S.nbr) return true;
     const double steps = (double)(ctx->plain64 + nsteps), n = (double)ctx->n;
     if (steps < 12.0 + 2.4e6 / n && steps < 6.0e6 / n) return false;
@@ -1269,6 +1295,13 @@ int ensure_exact(bmxg_ctx *ctx)
     ctx->bins_exact = true;
     ctx->list_valid = false;
     return BMXG_OK;
+}
+
+// The same for a reader of the bins between steps.
+int read_bins(bmxg_ctx *ctx)
+{
+    list64_end(ctx);
+    return ensure_exact(ctx);
 }
 
 // Steps of a list call from here on: their number and the buffer the first reads.
@@ -1450,6 +1483,7 @@ int list_steps(bmxg_ctx *ctx, double dt, int32_t nsteps, int precision, int32_t 
     ctx->list_valid = false;  // until the steps have run
     int left = nsteps;
     double due = 0.0;  // builds of this call that fell due
+    bool poor = false;
     while (left > 0) {
         cudaGraphExec_t g = nullptr;
         const double period = (ctx->period_steps + (nsteps - left)) / (ctx->period_builds + due);
@@ -1477,6 +1511,12 @@ int list_steps(bmxg_ctx *ctx, double dt, int32_t nsteps, int precision, int32_t 
             left = now + (over ? 1 : 0);
             break;
         }
+        // (FP64: the rest of the call goes without)
+        poor = precision == BMXG_FP64 && due >= 2.0 && (nsteps - now) < kList64MinSteps * due;
+        if (poor) {
+            left = now;
+            break;
+        }
         if (now >= left || now < 0) return fail(ctx, BMXG_ERR_STATE, "internal: list steps made no progress");
         left = now;
     }
@@ -1498,7 +1538,12 @@ int list_steps(bmxg_ctx *ctx, double dt, int32_t nsteps, int precision, int32_t 
         ctx->bins_exact = false;
         if (precision == BMXG_FP32F) ctx->fx_ahead = true;
     }
-    ctx->list_valid = !(precision == BMXG_FP64 && ctx->list64_bail);
+    ctx->list_valid = !(precision == BMXG_FP64 && (ctx->list64_bail || poor));
+    if (precision == BMXG_FP64) {
+        ctx->list64_live = true;
+        ctx->list64_lived += *done;
+        if (!ctx->list_valid) list64_end(ctx, poor);
+    }
     return BMXG_OK;
 }
 
@@ -1507,6 +1552,7 @@ int list_steps(bmxg_ctx *ctx, double dt, int32_t nsteps, int precision, int32_t 
 // before an allocation are dropped: they hold the state's pointers by value).
 int step_setup(bmxg_ctx *ctx, int32_t nsteps, int32_t precision)
 {
+    if (precision == BMXG_FP32F) list64_end(ctx);
     float skin = (ctx->list_mode && (precision == BMXG_FP32F || list64_pays(ctx, nsteps))) ? list_skin(ctx) : 0.0f;
     if (skin > 0.0f && precision == BMXG_FP32F && !ctx->list_valid && nsteps < kListMinSteps && ctx->step_count == 0)
         skin = 0.0f;
@@ -1688,7 +1734,10 @@ int bmxg_step(bmxg_ctx *ctx, double dt, int32_t nsteps, int32_t precision)
         CK(cudaMemcpyAsync(ctx->h_cnt, ctx->d_cnt, sizeof(DevCounters), cudaMemcpyDeviceToHost, ctx->stream));
         CK(cudaStreamSynchronize(ctx->stream));
         ctx->stats.n_rebins += per_step;
-        if (precision == BMXG_FP64) ctx->plain64 += per_step;
+        if (precision == BMXG_FP64) {
+            ctx->plain64 += per_step;
+            ctx->list64_since += per_step;
+        }
         ctx->list_valid = false;
     }
     ctx->stepped = true;
@@ -2017,7 +2066,7 @@ int bmxg_get_pairs(bmxg_ctx *ctx, int64_t *offs, int32_t *idx, int8_t *img, int6
     offs[0] = 0;
     *total = 0;
     if (n == 0) return BMXG_OK;
-    if (int rc0 = ensure_exact(ctx)) return rc0;
+    if (int rc0 = read_bins(ctx)) return rc0;
     cudaStream_t st = ctx->stream;
     const DevParams P = dev_params(ctx->prm);
     int64_t *d_offs = nullptr;
@@ -2071,7 +2120,7 @@ int bmxg_particle_exchange(bmxg_ctx *ctx, const double *vol, double *conc, doubl
     if (where != BMXG_HOST && where != BMXG_DEVICE) return fail(ctx, BMXG_ERR_ARG, "bad `where`");
     const int64_t n = ctx->n;
     if (n == 0 || !ctx->S.has_rods) return BMXG_OK;  // only FUNGI segments exchange
-    if (int rc0 = ensure_exact(ctx)) return rc0;
+    if (int rc0 = read_bins(ctx)) return rc0;
     cudaStream_t st = ctx->stream;
     const cudaMemcpyKind in = (where == BMXG_HOST) ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice;
     const cudaMemcpyKind back = (where == BMXG_HOST) ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice;
@@ -2108,6 +2157,7 @@ int bmxg_set_list_mode(bmxg_ctx *ctx, int32_t mode)
     if (mode != 0 && mode != 1) return fail(ctx, BMXG_ERR_ARG, "list mode must be 0 or 1");
     if (ctx->list_mode != mode) {
         ctx->list_mode = mode;
+        list64_end(ctx);
         ctx->list_valid = false;
         drop_graphs(ctx);
     }
@@ -2124,7 +2174,7 @@ int bmxg_init_bonds(bmxg_ctx *ctx, double rlim, int64_t *added, int64_t *overflo
     if (!ctx->have_state) return fail(ctx, BMXG_ERR_STATE, "no state loaded");
     if (!(rlim > 0.0)) rlim = 1.0e-7;
     if (ctx->n == 0 || !ctx->S.has_rods) return BMXG_OK;
-    if (int rc0 = ensure_exact(ctx)) return rc0;
+    if (int rc0 = read_bins(ctx)) return rc0;
     cudaStream_t st = ctx->stream;
     const DevParams P = dev_params(ctx->prm);
     unsigned long long *d_cnt = nullptr;
@@ -2154,7 +2204,7 @@ int bmxg_autotune(bmxg_ctx *ctx, const char *cache_path)
     (void)cudaGetLastError();  // drop a non-sticky error another library left on this thread
     if (!ctx->have_state) return fail(ctx, BMXG_ERR_STATE, "no state loaded");
     if (ctx->n == 0 || ctx->S.has_rods) return BMXG_OK;
-    if (int rc0 = ensure_exact(ctx)) return rc0;
+    if (int rc0 = read_bins(ctx)) return rc0;
     ctx->list_valid = false;  // the sweep writes the other buffer
     const int64_t n = ctx->n;
     char devname[256] = {0};
@@ -2532,7 +2582,7 @@ int bmxg_forward(bmxg_ctx *ctx, double dt, int32_t nsteps, int32_t ckpt_every)
     if (ctx->S.has_rods) return fail(ctx, BMXG_ERR_UNSUPPORTED, "the differentiation form covers spheres");
     if (nsteps < 0 || ckpt_every < 1 || !std::isfinite(dt)) return fail(ctx, BMXG_ERR_ARG, "bad dt, nsteps or ckpt_every");
     (void)cudaGetLastError();
-    if (int rc0 = ensure_exact(ctx)) return rc0;
+    if (int rc0 = read_bins(ctx)) return rc0;
     ctx->list_valid = false;
     const int64_t n = ctx->n;
     free_adjoint(ctx);
