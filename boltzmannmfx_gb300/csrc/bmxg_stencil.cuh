@@ -162,6 +162,13 @@ __device__ __forceinline__ void col_to_bxy(const DevGeom &G, int col, int &bx, i
 // adjacent columns.
 constexpr int kWalkCols = 9;
 constexpr int kWalkBlock = 32 * kWalkCols;
+// Candidates staged per slot and column (sphere step, adjoint; up to 65 536 slots): one word
+// each, in the room of six of two words.  A slot with more in some column is walked again by
+// one lane while the block waits.  Adjoint of 20 000 / 50 000 spheres over 20 steps, ms: at 10
+// a column 2.3 / 4.0 (6.3 / 6.3 with six), 2.7 / 4.8 at 15 (8.8 / 11.6; one thread per slot with
+// its pairs staged by the block 6.5 / 7.7), 3.4 / 10.4 at 24 (15.4 / 22.4); 1.77 / 3.06 at 3 (1.76 /
+// 3.06).  14: 3.5 / 10.4 at 24, 1.79 / 3.07 at 3.
+constexpr int kWalkStage = 12;
 
 // Blocks an SM a launch of `blocks` is compiled for, `least` to 5: as few (as many
 // registers a thread, as few spills) as hold the grid in the fewest waves.  The
@@ -211,13 +218,20 @@ __device__ __forceinline__ void walk_column(const DevState &S, int a, int lo, in
     }
 }
 
+// A staged candidate: slot j and its code; in one word where the slots are below 2^28
+// and the code is an image's (0..8).
+__device__ __forceinline__ void put_entry(int2 &e, int j, int code) { e = make_int2(j, code); }
+__device__ __forceinline__ void put_entry(unsigned &e, int j, int code) { e = (unsigned)j | ((unsigned)code << 28); }
+__device__ __forceinline__ int2 get_entry(const int2 &e) { return e; }
+__device__ __forceinline__ int2 get_entry(unsigned e) { return make_int2((int)(e & 0xfffffffu), (int)(e >> 28)); }
+
 // Shared memory of a block's walk over NS slots (32 per pass of the warps): per
 // column and slot the staged candidates (slot of the neighbour, image code)
 // and, after walk_scan, the end of the column's run among the slot's pairs;
 // the slots' first pairs.
-template <int NS, int STAGE>
+template <int NS, int STAGE, class Entry = int2>
 struct WalkMem {
-    int2 stage[kWalkCols * NS][STAGE];
+    Entry stage[kWalkCols * NS][STAGE];
     int end[kWalkCols][NS];
     int first[NS + 1];
     int over[NS];  // the slot staged too many in some column: no pairs here
@@ -227,8 +241,8 @@ struct WalkMem {
 // After every warp wrote its counts into end[w][slot] (more than STAGE, or
 // more than `most` in all: overflow): the counts into runs, over the whole
 // block (it synchronises).
-template <int NS, int STAGE>
-__device__ __forceinline__ void walk_scan(WalkMem<NS, STAGE> &M, int most = 0x7fffffff)
+template <int NS, int STAGE, class Entry>
+__device__ __forceinline__ void walk_scan(WalkMem<NS, STAGE, Entry> &M, int most = 0x7fffffff)
 {
     const int tid = threadIdx.x, lane = tid & 31;
     __syncthreads();
@@ -267,8 +281,8 @@ __device__ __forceinline__ void walk_scan(WalkMem<NS, STAGE> &M, int most = 0x7f
 }
 
 // Pair t of the block: its slot o and its staged candidate.
-template <int NS, int STAGE>
-__device__ __forceinline__ int2 walk_pair(const WalkMem<NS, STAGE> &M, int t, int &o)
+template <int NS, int STAGE, class Entry>
+__device__ __forceinline__ int2 walk_pair(const WalkMem<NS, STAGE, Entry> &M, int t, int &o)
 {
     o = 0;
 #pragma unroll
@@ -284,7 +298,7 @@ __device__ __forceinline__ int2 walk_pair(const WalkMem<NS, STAGE> &M, int t, in
             at = e;
         }
     }
-    return M.stage[w * NS + o][k - at];
+    return get_entry(M.stage[w * NS + o][k - at]);
 }
 
 // The column of warp w around slot i's bin (false: outside a closed face).
@@ -323,8 +337,8 @@ __device__ __forceinline__ float screen_slack(const DevGeom &G)
 
 // The block's walk of buffer a: every slot's candidates staged, the runs of
 // pairs set up (walk_scan).  own(s, i, colony): the first warp, for each slot.
-template <int NS, int STAGE, class Own>
-__device__ __forceinline__ void walk_block(const DevState &S, int a, float bwf, WalkMem<NS, STAGE> &M, Own &&own)
+template <int NS, int STAGE, class Entry, class Own>
+__device__ __forceinline__ void walk_block(const DevState &S, int a, float bwf, WalkMem<NS, STAGE, Entry> &M, Own &&own)
 {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     for (int g = 0; g < NS; g += 32) {
@@ -348,7 +362,7 @@ __device__ __forceinline__ void walk_block(const DevState &S, int a, float bwf, 
                     if (!near_pair32(me, q, ox, oy, (float)dzs * dzb, bwf, slack)) return;
                     const int j = __ldg(&S.perm[a][t]);
                     if ((sx | sy) && !image_in_row(S, G, a, j, ii, jj, sx, sy)) return;
-                    if (cnt < STAGE) M.stage[w * NS + s][cnt] = make_int2(j, (sx + 1) * 3 + (sy + 1));
+                    if (cnt < STAGE) put_entry(M.stage[w * NS + s][cnt], j, (sx + 1) * 3 + (sy + 1));
                     ++cnt;
                 });
             }
@@ -362,8 +376,8 @@ __device__ __forceinline__ void walk_block(const DevState &S, int a, float bwf, 
 // slot o into t[NT] (false: no term); add(t, stride) adds one pair's terms to
 // the sums of slot threadIdx.x, in staging order (the slots' threads are the
 // block's first NS).  term: NT x kWalkBlock values.
-template <int NT, int NS, int STAGE, class Eval, class Add>
-__device__ __forceinline__ void walk_pairs(const WalkMem<NS, STAGE> &M, double *term, unsigned char *opass, Eval &&eval,
+template <int NT, int NS, int STAGE, class Entry, class Eval, class Add>
+__device__ __forceinline__ void walk_pairs(const WalkMem<NS, STAGE, Entry> &M, double *term, unsigned char *opass, Eval &&eval,
                                            Add &&add)
 {
     const int tid = threadIdx.x;

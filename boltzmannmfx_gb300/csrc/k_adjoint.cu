@@ -418,7 +418,7 @@ __global__ void __launch_bounds__(kWalkBlock, RESIDENT) k_dfwdw(const DevState S
                                                          int a)
 {
     extern __shared__ __align__(16) unsigned char smw[];
-    auto &M = *reinterpret_cast<WalkMem<NS, STAGE> *>(smw);
+    auto &M = *reinterpret_cast<WalkMem<NS, STAGE, unsigned> *>(smw);
     __shared__ double own[6][NS];
     __shared__ int ocol[NS];
     __shared__ double term[3 * kWalkBlock];
@@ -488,7 +488,7 @@ __global__ void __launch_bounds__(kWalkBlock, RESIDENT) k_dadjw(const DevState S
 {
     constexpr int NO = 10, NT = 7;
     extern __shared__ __align__(16) unsigned char smw[];
-    auto &M = *reinterpret_cast<WalkMem<NS, STAGE> *>(smw);
+    auto &M = *reinterpret_cast<WalkMem<NS, STAGE, unsigned> *>(smw);
     __shared__ double own[NS][NO + 1];  // (odd pitch: no bank conflicts between the slots' rows)
     __shared__ int ocol[NS];
     __shared__ double term[NT * kWalkBlock];
@@ -604,8 +604,9 @@ int launch_dfwd(const DevState &S, const DevParams &P, const DiffParams &D, doub
     // 20 000 spheres take 35 / 82)
     if (S.srel[a] && !pinned && S.n <= kWalkNarrow) {
         const int blocks = (S.n + 31) / 32, fit = wave_fit(blocks, 3);
-        launch_after(fit == 3 ? k_dfwdw<32, 6, 3> : (fit == 4 ? k_dfwdw<32, 6, 4> : k_dfwdw<32, 6, 5>), blocks,
-                     kWalkBlock, sizeof(WalkMem<32, 6>), st, S, P, D, dt, a);
+        launch_after(fit == 3 ? k_dfwdw<32, kWalkStage, 3>
+                              : (fit == 4 ? k_dfwdw<32, kWalkStage, 4> : k_dfwdw<32, kWalkStage, 5>),
+                     blocks, kWalkBlock, sizeof(WalkMem<32, kWalkStage, unsigned>), st, S, P, D, dt, a);
     } else if (S.srel[a]) {
         allow_smem(k_dfwd<true>, smem);
         k_dfwd<true><<<grid, block, smem, st>>>(S, P, D, dt, a);
@@ -622,9 +623,11 @@ int launch_dadj(const DevState &S, const DevParams &P, const DiffParams &D, doub
     const size_t smem = staged_smem(block, 10, 7);
     if (S.srel[a] && !pinned && S.n <= kWalkNarrow) {
         const int blocks = (S.n + 31) / 32, fit = wave_fit(blocks, 2);
-        launch_after(fit == 2 ? k_dadjw<32, 6, 2>
-                              : (fit == 3 ? k_dadjw<32, 6, 3> : (fit == 4 ? k_dadjw<32, 6, 4> : k_dadjw<32, 6, 5>)),
-                     blocks, kWalkBlock, sizeof(WalkMem<32, 6>), st, S, P, D, dt, a, lin, lout, gacc, gadh);
+        launch_after(fit == 2 ? k_dadjw<32, kWalkStage, 2>
+                              : (fit == 3 ? k_dadjw<32, kWalkStage, 3>
+                                          : (fit == 4 ? k_dadjw<32, kWalkStage, 4> : k_dadjw<32, kWalkStage, 5>)),
+                     blocks, kWalkBlock, sizeof(WalkMem<32, kWalkStage, unsigned>), st, S, P, D, dt, a, lin, lout,
+                     gacc, gadh);
     } else if (S.srel[a]) {
         allow_smem(k_dadj<true>, smem);
         k_dadj<true><<<grid, block, smem, st>>>(S, P, D, dt, a, lin, lout, gacc, gadh);

@@ -61,14 +61,19 @@ __device__ __forceinline__ bool sphere_term64(const DevState &S, const DevGeom &
 // the sorted copies takes a column at a time, four entries in flight, and three blocks of
 // 256 threads fit an SM (80 registers): 500 000 slots 223 -> 172 us, 2 million 687 -> 507,
 // 688 000 in 64 colonies 379 -> 245 against entry by entry with the crowded slots'
-// evaluation inside the walk (128 registers).  64 registers: 183; a stage of 16: 174;
-// the next column's bounds a column ahead: 179; three columns unrolled: 216.
-constexpr int kStage64 = 12;
+// evaluation inside the walk (128 registers).  64 registers: 183; the next column's bounds
+// a column ahead: 179; three columns unrolled: 216.
+// A staged candidate is one word: its slot (below 2^30) and whether it is an image along
+// x and y; which one the slot's own bin says (a periodic axis has three bins or more).
+// 24 of them in the room of 12 of two words, whose crowded slots' second walk cost more than
+// staging saved: a load and 24 steps of 50 000 spheres, 15 / 24 a column, 3.51 / 5.06 -> 2.03 /
+// 2.72 ms, 2 million 29.1 / 60.2 -> 28.0 / 40.9; 3 a column 1.18 / 14.3 -> 1.18 / 14.4.
+constexpr int kStage64 = 24;
 
 // dynamic shared memory of k_sphere64 for a block of `block` threads
 __host__ __device__ constexpr size_t sphere64_smem(int block)
 {
-    return (size_t)block * (kStage64 * sizeof(int2) + 4 * sizeof(double) + 3 * sizeof(double) + 4 * sizeof(int)) +
+    return (size_t)block * (kStage64 * sizeof(unsigned) + 4 * sizeof(double) + 3 * sizeof(double) + 4 * sizeof(int)) +
            2 * 32 * sizeof(int);
 }
 
@@ -81,13 +86,13 @@ __global__ void __launch_bounds__(256, 3) k_sphere64(const DevState S, const Dev
     extern __shared__ __align__(16) unsigned char sm64[];
     const int B = blockDim.x, tid = threadIdx.x;
     const int lane = tid & 31, w = tid >> 5, nw = B >> 5;
-    int2 *stage = reinterpret_cast<int2 *>(sm64);
+    unsigned *stage = reinterpret_cast<unsigned *>(sm64);
     double *opos = reinterpret_cast<double *>(stage + (size_t)B * kStage64);  // 4 per thread: x, y, z, r
     double *term = opos + 4 * B;                                               // 3 per thread
     int *ocol = reinterpret_cast<int *>(term + 3 * B);
     int *orun = ocol + B;   // first staged pair of the slot in the block's run
-    int *olen = orun + B;   // its staged pairs
-    int *opass = olen + B;  // the round's gate result per thread
+    int *oimg = orun + B;   // the shifts its images have: (sx + 1) * 3 + (sy + 1)
+    int *opass = oimg + B;  // the round's gate result per thread
     int *wsum = opass + B;  // per warp: staged pairs, then their exclusive scan
     const int b = a ^ 1;
     const float bwf = P.bw32;
@@ -97,11 +102,10 @@ __global__ void __launch_bounds__(256, 3) k_sphere64(const DevState S, const Dev
         const bool act = i < S.n;
         double xi = 0.0, yi = 0.0, zi = 0.0, ri = 0.0;
         double fx = 0.0, fy = 0.0, fz = 0.0;
-        int col = 0, cnt = 0;
+        int col = 0, cnt = 0, bx = 1, by = 1;
         if (act) {
             col = colony_of(S.cbase, S.ncol, i);
             const DevGeom &G = S.geoms[col];
-            int bx, by;
             col_to_bxy(G, S.col[a][i], bx, by);
             const int izi = S.iz[a][i];
             xi = S.x[a][i];
@@ -110,9 +114,9 @@ __global__ void __launch_bounds__(256, 3) k_sphere64(const DevState S, const Dev
             ri = S.rad[i];
             const float4 me = S.rel[a][i];
             const float slack = screen_slack(G), dzb = G.dxf[2];
-            int2 *mine = stage + (size_t)tid * kStage64;
+            unsigned *mine = stage + (size_t)tid * kStage64;
             auto take = [&](int j, int sx, int sy) {
-                if (cnt < kStage64) mine[cnt] = make_int2(j, (sx + 1) * 3 + (sy + 1));
+                if (cnt < kStage64) mine[cnt] = (unsigned)j | (sx ? 1u << 30 : 0u) | (sy ? 1u << 31 : 0u);
                 ++cnt;
             };
             if constexpr (SORTED) {
@@ -161,7 +165,7 @@ __global__ void __launch_bounds__(256, 3) k_sphere64(const DevState S, const Dev
         opos[4 * tid + 2] = zi;
         opos[4 * tid + 3] = ri;
         ocol[tid] = col;
-        olen[tid] = xl;
+        oimg[tid] = (bx == 1 ? 0 : 6) + (by == 1 ? 0 : 2);
         __syncthreads();
         if (tid == 0) {
             int run = 0;
@@ -186,9 +190,11 @@ __global__ void __launch_bounds__(256, 3) k_sphere64(const DevState S, const Dev
                     int o = 0;  // the slot that owns pair t: the last thread whose run starts at or before t
                     for (int s2 = 1 << (31 - __clz(max(B - 1, 1))); s2 >= 1; s2 >>= 1)
                         if (o + s2 < B && orun[o + s2] <= t) o += s2;
-                    const int2 e = stage[(size_t)o * kStage64 + (t - orun[o])];
+                    const unsigned e = stage[(size_t)o * kStage64 + (t - orun[o])];
+                    const int im = oimg[o];
                     pass = sphere_term64(S, S.geoms[ocol[o]], P, a, opos[4 * o], opos[4 * o + 1], opos[4 * o + 2],
-                                         opos[4 * o + 3], e.x, e.y / 3 - 1, e.y % 3 - 1, tt)
+                                         opos[4 * o + 3], (int)(e & 0x3fffffffu), (e >> 30) & 1u ? im / 3 - 1 : 0,
+                                         e >> 31 ? im % 3 - 1 : 0, tt)
                                ? 1
                                : 0;
                 }
@@ -237,7 +243,7 @@ template <int NS, int STAGE, int RESIDENT>
 __global__ void __launch_bounds__(kWalkBlock, RESIDENT) k_sphere64w(const DevState S, const DevParams P, double dt, int a)
 {
     extern __shared__ __align__(16) unsigned char smw[];
-    auto &M = *reinterpret_cast<WalkMem<NS, STAGE> *>(smw);
+    auto &M = *reinterpret_cast<WalkMem<NS, STAGE, unsigned> *>(smw);
     __shared__ double opos[NS][4];
     __shared__ int ocol[NS];
     __shared__ double term[3 * kWalkBlock];
@@ -419,8 +425,9 @@ int launch_sphere_step(const DevState &S, const DevParams &P, double dt, int a, 
     if (precision == BMXG_FP64_FORM) {
         if (sorted && !pinned && S.n <= kColumnSlots64) {
             const int blocks = (S.n + 31) / 32, fit = wave_fit(blocks, 3);
-            launch_after(fit == 3 ? k_sphere64w<32, 6, 3> : (fit == 4 ? k_sphere64w<32, 6, 4> : k_sphere64w<32, 6, 5>),
-                         blocks, kWalkBlock, sizeof(WalkMem<32, 6>), st, S, P, dt, a);
+            launch_after(fit == 3 ? k_sphere64w<32, kWalkStage, 3>
+                                  : (fit == 4 ? k_sphere64w<32, kWalkStage, 4> : k_sphere64w<32, kWalkStage, 5>),
+                         blocks, kWalkBlock, sizeof(WalkMem<32, kWalkStage, unsigned>), st, S, P, dt, a);
             return 1;
         }
         // (block a multiple of 32, at most 256: the block stages and evaluates its pairs together)
