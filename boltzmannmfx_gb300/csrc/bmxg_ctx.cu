@@ -755,6 +755,7 @@ int load_state(bmxg_ctx *ctx, const bmxg_particles *p, const int64_t *colony_off
     S.n = (int)n;
     S.ncol = ctx->ncol;
     S.ncols_total = (int)ncols;
+    S.nsm = ctx->nsm;
     S.has_rods = rods ? 1 : 0;
     int rc = BMXG_OK;
 #define AL(ptr, cnt)                       \
@@ -1116,22 +1117,29 @@ void prof_events(bmxg_ctx *ctx, cudaEvent_t *k0, cudaEvent_t *k1)
 
 // ---- neighbour list with a skin ---------------------------------------
 constexpr int kListMaxAge = 64;      // builds at least this often
-// FP64 spheres step over the list where it is the faster path, per-step path / list:
-// 10 000 slots 19 / 22 us a step, 20 000 29 / 22, 40 000 37 / 24, 160 000 69 / 48,
-// 400 000 128 / 95, 688 000 in 64 colonies 295 / 236 (up to 16 384 slots the
-// per-step path's sort is one cluster and its step little more than two launches).
-// From a load on, with the build: 6 steps of 40 000 slots 446 / 444 us, 400 000
-// 1180 / 1047; fewer steps keep the per-step path.  The list's buffers and graphs
-// cost 0.6-0.7 ms once, which 12 + 2.4e6 / slots steps pay back, above 300 000 slots
-// 6e6 / slots (fresh context, 20 steps: 40 000 slots 2086 / 2335, 160 000 3943 / 4145,
-// 400 000 6159 / 6245; 100 steps: 4726 / 4289, 9066 / 7385, 15 604 / 12 924; the 64
-// colonies, 10 steps: 4702 / 4412).
+// FP64 spheres step over the list where it is the faster path.  A load and 100 steps, per-step
+// path / list, us, 3 and 10 slots a column: 16 000 slots 2008 / 2344, 2466 / 3443, 20 000 2374 /
+// 2399, 3115 / 3733, 24 000 2501 / 2399, 2995 / 3330, 28 000 3101 / 2371, 3663 / 3416, 40 000 3996 /
+// 2581, 6007 / 3755, 160 000 7459 / 5019, 12 292 / 8041, 400 000 13 864 / 9613, 22 939 / 15 815
+// (between kList64Slots and kList64Sure it gains 4 % at best and loses up to 20 %: there
+// it is for states that step for long).
+// From a load on, with the build: 6 steps of 28 000 slots 396 / 377, 441 / 451, 40 000 476 /
+// 410, 578 / 482, 400 000 1279 / 1069, 1791 / 1424; fewer steps keep the per-step path.
 constexpr int kList64Slots = 16384;
+constexpr int kList64Sure = 28672;
 constexpr int kList64MinSteps = 6;
+// Steps of a state's size that pay for the list's buffers and graphs.  In a fresh
+// context, per-step path / list, us, 3 and 10 slots a column: 50 000 slots 13 steps 653 / 692,
+// 933 / 837, 20 941 / 972, 1352 / 1210, 25 1115 / 996, 1638 / 1269; 100 000 20 1218 / 1346,
+// 1760 / 1729, 25 1447 / 1413, 2110 / 1904; 200 000 10 1039 / 1107, 1511 / 1406, 13 1286 / 1194,
+// 1879 / 1600; 400 000 8 1319 / 1274, 2010 / 1725; 900 000 6 1641 / 1726, 2617 / 2479, 8 2336 /
+// 2007, 3656 / 3037.
+inline double list64_pays_back(double n) { return n < kList64Sure ? 150.0 : std::min(26.0, 5.0 + 1.6e6 / n); }
 // So few list steps go as a graph (with its conditional node) for each, more as graphs of
 // kResyncEvery whose surplus steps return at once: the node costs 7 us, a surplus step its
-// blocks' launch.  3 / 4 steps as singles and as one graph, us: 20 000 slots 66, 81 and 53, 63;
-// 200 000 79, 93 and 68, 77; 1 million 128, 167 and 163, 177.
+// blocks' launch.  2 / 3 / 4 FP32F steps as singles and as one graph, us: 20 000 slots 53, 68,
+// 84 and 55, 66, 66; 400 000 66, 92, 122 and 90, 92, 103; 700 000 78, 109, 133 and 115, 127, 139;
+// 1 million 91, 129, 172 and 139, 155, 176.
 inline int list_singles(int64_t n) { return n <= 400000 ? 2 : 4; }
 // Fewer steps a build than this: graphs with a conditional node before every step, where
 // none stalls.  48 FP32F steps with one node per graph / one per step, by steps a build, us:
@@ -1193,7 +1201,7 @@ bool list64_pays(const bmxg_ctx *ctx, int32_t nsteps)
         return false;
     if (ctx->S.nbr) return true;
     const double steps = (double)(ctx->plain64 + nsteps), n = (double)ctx->n;
-    if (steps < 12.0 + 2.4e6 / n && steps < 6.0e6 / n) return false;
+    if (steps < list64_pays_back(n)) return false;
     // (and leaves three quarters of the free memory)
     size_t room = 0, all = 0;
     const size_t need = (size_t)ctx->n * 320 + (size_t)ctx->ncells_total * sizeof(int);

@@ -67,8 +67,7 @@ constexpr int kListBins = 0;         // list mode keeps its frozen bins in buffe
 constexpr int kListStepBlock = 128;  // k_list_step's default block (at most 256; autotuned)
 constexpr int kListBuildBlock = 128; // k_list_build's default block (one slot per thread; at most 256)
 constexpr int kSphereBlock = 64;     // per-step sphere kernels' block (one slot per thread)
-constexpr int kSMs = 152;            // of a GB300: launch rules count in waves of blocks over them
-constexpr int kWalkNarrow = 65536;   // adjoint, tile: 32 slots per block, a warp per neighbour column, up to here
+constexpr int kWalkNarrow = 65536;   // tile: 32 slots per block up to here, then 128
 constexpr int kRodCap = 32;          // gated pairs per segment the rod pipelines hold (more: the
                                      // segment walks its stencil in the segment kernel)
 
@@ -85,6 +84,7 @@ struct DevState {
     int n;             // particles (slots)
     int ncol;          // colonies
     int ncols_total;   // columns over all colonies
+    int nsm;           // SMs of the device (launch rules count in waves of blocks over them)
     const DevGeom *geoms;
     const int *cbase;  // ncol + 1: first slot of each colony, then n (a compact copy for colony lookups)
     DevCounters *cnt;

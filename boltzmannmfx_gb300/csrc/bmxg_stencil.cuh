@@ -3,6 +3,8 @@
 // -fmad=false so that every FP64 expression rounds exactly like the host
 // oracle's (FP32 code uses explicit __fmaf_rn where it wants a fused op).
 #pragma once
+#include <algorithm>
+
 #include "bmxg_kernels.cuh"
 
 namespace bmxg {
@@ -178,11 +180,12 @@ constexpr int kWalkStage = 12;
 // (6) 22.7 / 22.8 / 23.9, 32 768 (7) 29.5 / 23.1 / 25.1; the adjoint's two kernels with 3 and 2 / 3 and
 // 3 / 5 and 5, forward and backward of 40 steps: 9000 slots 2634 / 2686 / 2923, 14 000 3171 / 2767 /
 // 3252, 24 000 4651 / 4307 / 3595, 48 000 7500 / 7120 / 5794.
-inline int wave_fit(int blocks, int least)
+inline int wave_fit(int blocks, int least, int nsm)
 {
+    nsm = std::max(nsm, 1);
     int best = least;
     for (int k = least + 1; k <= 5; ++k)
-        if ((blocks + kSMs * k - 1) / (kSMs * k) < (blocks + kSMs * best - 1) / (kSMs * best)) best = k;
+        if ((blocks + nsm * k - 1) / (nsm * k) < (blocks + nsm * best - 1) / (nsm * best)) best = k;
     return best;
 }
 

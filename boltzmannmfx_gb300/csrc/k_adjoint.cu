@@ -594,16 +594,18 @@ void allow_smem(K kernel, size_t need)
     if (need > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need);
 }
 
+// The kernels with a warp per neighbour column up to here, above with a thread per
+// slot.  Forward and backward of 20 steps, one thread per slot / a warp per column, us, 3 and 10
+// slots a column: 20 000 slots 3347, 5257 / 1758, 2352, 65 000 3888, 6208 / 3590, 4844, 100 000 5924,
+// 9445 / 5314, 7299, 130 000 6133, 9931 / 6242, 8668, 200 000 7928, 13 295 / 8671, 12 101.
+constexpr int kAdjointColumns = 114688;
+
 int launch_dfwd(const DevState &S, const DevParams &P, const DiffParams &D, double dt, int a, int grid, int block,
                 cudaStream_t st, bool pinned)
 {
     const size_t smem = staged_smem(block, 6, 3);
-    // (a warp per column up to kWalkNarrow slots.  Measured, us per step of the forward / the backward sweep
-    // with recomputation, one thread per slot -> a warp per column: 1000 spheres 57 -> 23 / 144 -> 77, 20 000
-    // 79 -> 40 / 195 -> 129, 40 000 82 -> 61 / 207 -> 192; with the resident blocks chosen by wave_fit
-    // 20 000 spheres take 35 / 82)
-    if (S.srel[a] && !pinned && S.n <= kWalkNarrow) {
-        const int blocks = (S.n + 31) / 32, fit = wave_fit(blocks, 3);
+    if (S.srel[a] && !pinned && S.n <= kAdjointColumns) {
+        const int blocks = (S.n + 31) / 32, fit = wave_fit(blocks, 3, S.nsm);
         launch_after(fit == 3 ? k_dfwdw<32, kWalkStage, 3>
                               : (fit == 4 ? k_dfwdw<32, kWalkStage, 4> : k_dfwdw<32, kWalkStage, 5>),
                      blocks, kWalkBlock, sizeof(WalkMem<32, kWalkStage, unsigned>), st, S, P, D, dt, a);
@@ -621,8 +623,8 @@ int launch_dadj(const DevState &S, const DevParams &P, const DiffParams &D, doub
                 double *lout, double *gacc, double *gadh, int grid, int block, cudaStream_t st, bool pinned)
 {
     const size_t smem = staged_smem(block, 10, 7);
-    if (S.srel[a] && !pinned && S.n <= kWalkNarrow) {
-        const int blocks = (S.n + 31) / 32, fit = wave_fit(blocks, 2);
+    if (S.srel[a] && !pinned && S.n <= kAdjointColumns) {
+        const int blocks = (S.n + 31) / 32, fit = wave_fit(blocks, 2, S.nsm);
         launch_after(fit == 2 ? k_dadjw<32, kWalkStage, 2>
                               : (fit == 3 ? k_dadjw<32, kWalkStage, 3>
                                           : (fit == 4 ? k_dadjw<32, kWalkStage, 4> : k_dadjw<32, kWalkStage, 5>)),

@@ -412,11 +412,11 @@ static void allow_smem_once(K kernel, size_t bytes, std::atomic<unsigned long lo
 // Which FP64 kernel a sorted state takes: one warp per neighbour column where
 // the slots are too few for a thread each to hide the walk's dependent loads,
 // one thread per slot above, where the walk's instructions count and not its
-// latency.  Measured, us a step of the kernel alone, one thread per slot / one warp
-// per column, on a sparse and a dense monolayer: 10 000 slots 36, 35 / 28, 21,
-// 20 000 25, 36 / 23, 27, 40 000 27, 42 / 31, 45, 100 000 34, 53 / 62, 87, 400 000
-// 105, 167 / 226, 276.
-constexpr int kColumnSlots64 = 32768;
+// latency.  Measured, us a load and 40 steps, one thread per slot / one warp per
+// column, 3 and 10 slots a column: 16 000 slots 1365, 2068 / 911, 1086, 32 768 1597,
+// 2303 / 1402, 1654, 48 000 1776, 2485 / 1651, 2007, 56 000 1866, 2694 / 1904, 2317, 80 000
+// 1954, 2884 / 2400, 3018.
+constexpr int kColumnSlots64 = 49152;
 
 int launch_sphere_step(const DevState &S, const DevParams &P, double dt, int a, int precision, int grid,
                        int block, cudaStream_t st, int resync, bool pinned)
@@ -424,7 +424,7 @@ int launch_sphere_step(const DevState &S, const DevParams &P, double dt, int a, 
     const bool sorted = S.srel[a] != nullptr;  // the context keeps sorted copies; bare callers do not
     if (precision == BMXG_FP64_FORM) {
         if (sorted && !pinned && S.n <= kColumnSlots64) {
-            const int blocks = (S.n + 31) / 32, fit = wave_fit(blocks, 3);
+            const int blocks = (S.n + 31) / 32, fit = wave_fit(blocks, 3, S.nsm);
             launch_after(fit == 3 ? k_sphere64w<32, kWalkStage, 3>
                                   : (fit == 4 ? k_sphere64w<32, kWalkStage, 4> : k_sphere64w<32, kWalkStage, 5>),
                          blocks, kWalkBlock, sizeof(WalkMem<32, kWalkStage, unsigned>), st, S, P, dt, a);
