@@ -2353,7 +2353,8 @@ int bmxg_autotune(bmxg_ctx *ctx, const char *cache_path)
             // a list built on the loaded positions; then the step launches read
             // buffer a and write buffer b (dt = 0), and the build launches
             // rewrite the same list: the loaded state is untouched, and the
-            // list path starts afresh at the next step (list_valid = false)
+            // list path starts afresh at the next step (list_valid = false), any other
+            // reader of the bins re-bins first
             if (int rc = ensure_list(ctx, skin, BMXG_FP32F)) return rc;
             cudaStream_t st = ctx->stream;
             if (int rc = set_list_run(ctx, 1)) return rc;  // (the timed launches repeat that step)
@@ -2395,6 +2396,7 @@ int bmxg_autotune(bmxg_ctx *ctx, const char *cache_path)
             ctx->ls_persist = best_pe;
             ctx->lb_block = best_bb;
             ctx->list_valid = false;
+            ctx->bins_exact = false;  // (the builds left the list's in buffer kListBins)
             std::snprintf(entry, sizeof(entry),
                           "%s: {\"step_block\": %d, \"step_passes\": %d, \"step_persistent\": %d, \"build_block\": "
                           "%d, \"step_ms_per_5\": %.4f, \"build_ms_per_3\": %.4f}",

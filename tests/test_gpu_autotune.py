@@ -1,0 +1,51 @@
+"""After bmxg_autotune the bins are the reference's for whatever comes next: the FP64
+steps, the neighbour list and the FP32F per-step path of a tuned context are those
+of an untuned one."""
+import numpy as np
+import pytest
+
+from boltzmannmfx_gb300 import Context, configs
+from boltzmannmfx_gb300.abi import BMXG_FP32F, BMXG_FP64
+
+pytestmark = pytest.mark.gpu
+
+OUT = ("x", "y", "z", "velx", "vely", "velz")
+PRM = configs.deck_params()
+
+
+def loaded(n, side, seed):
+    g = configs.box_geometry(side, side)
+    P = configs.sphere_colony(n, side, side, np.random.default_rng(seed))
+    ctx = Context(PRM, [g])
+    ctx.set_state(P)
+    return ctx, g, P
+
+
+def read(ctx, P):
+    Q = P.copy()
+    ctx.get_state(Q)
+    return Q
+
+
+@pytest.mark.parametrize("then", ["step", "pairs", "forward", "fp32f"])
+def test_first_call_after_autotune(gpu_lib, oracle_lib, then):
+    n = 5000
+    A, g, P = loaded(n, 0.064, 41)
+    B, _, _ = loaded(n, 0.064, 41)
+    A.autotune()
+    if then == "pairs":
+        assert all(np.array_equal(x, y) for x, y in zip(A.pairs(), B.pairs()))
+        assert all(np.array_equal(x, y) for x, y in zip(A.pairs(), oracle_lib.pairs(PRM, g, P)))
+    elif then == "forward":
+        for c in (A, B):
+            c.forward(0.25, 3, 2)
+    else:
+        for c in (A, B):
+            if then == "fp32f":
+                c.set_list_mode(0)
+            c.step(0.25, 3, BMXG_FP32F if then == "fp32f" else BMXG_FP64)
+    QA, QB = read(A, P), read(B, P)
+    for k in OUT if then != "pairs" else OUT[:3]:
+        assert np.array_equal(QA[k], QB[k]), k
+    A.close()
+    B.close()
