@@ -106,6 +106,7 @@ struct bmxg_ctx {
     std::map<GraphKey, cudaGraphExec_t> graphs;
     std::map<GraphKey, int> graph_kernels;  // kernels per replay of each graph
     Shape sh_sphere[2], sh_rod, sh_misc;
+    bool adj_pinned = false;  // sh_sphere[0]'s grid is the caller's (bmxg_set_shapes): the adjoint's too
     // list path shapes (bmxg_autotune): k_list_step's block and passes per
     // chunk (0: the launcher's rule), k_list_build's block
     int ls_block = kListStepBlock, ls_passes = 0, lb_block = kListBuildBlock;
@@ -2288,6 +2289,7 @@ int bmxg_autotune(bmxg_ctx *ctx, const char *cache_path)
                 bb > 0) {
                 ctx->sh_sphere[prec].block = bb;
                 ctx->sh_sphere[prec].grid = gg;
+                if (prec == 0) ctx->adj_pinned = false;
                 continue;
             }
         }
@@ -2327,6 +2329,7 @@ int bmxg_autotune(bmxg_ctx *ctx, const char *cache_path)
         CK(cudaMemsetAsync(ctx->d_cnt, 0, sizeof(DevCounters), ctx->stream));
         CK(cudaStreamSynchronize(ctx->stream));
         ctx->sh_sphere[prec] = bs;
+        if (prec == 0) ctx->adj_pinned = false;  // (the sweep does not time the adjoint)
         std::snprintf(entry, sizeof(entry), "%s: {\"block\": %d, \"grid\": %d, \"ms_per_5\": %.4f}", key, bs.block,
                       bs.grid, best);
         cache_add(entry);
@@ -2419,6 +2422,9 @@ int bmxg_set_shapes(bmxg_ctx *ctx, const bmxg_shapes *in)
     if (!block_ok(in->list_step_block) || !block_ok(in->list_build_block) || in->list_step_passes < 0 ||
         in->list_step_passes > 64)
         return fail(ctx, BMXG_ERR_ARG, "list blocks: a multiple of 32 up to 256; passes 0..64");
+    // (a tuned FP64 shape handed back as it is stays one)
+    if (in->sphere_block[0] != ctx->sh_sphere[0].block || in->sphere_grid[0] != ctx->sh_sphere[0].grid)
+        ctx->adj_pinned = in->sphere_grid[0] > 0;
     for (int k = 0; k < 2; ++k) {
         ctx->sh_sphere[k].block = in->sphere_block[k];
         ctx->sh_sphere[k].grid = in->sphere_grid[k];
@@ -2575,7 +2581,7 @@ int dfwd_step(bmxg_ctx *ctx, const DevState &S, int a, double dt)
     const Shape &sh = ctx->sh_sphere[0];
     int sg, sb;
     stencil_shape(ctx, sh, ctx->n, &sg, &sb);
-    LAUNCH(launch_dfwd(S, dev_params(ctx->prm), diff_params(ctx), dt, a, sg, sb, ctx->stream, sh.grid > 0));
+    LAUNCH(launch_dfwd(S, dev_params(ctx->prm), diff_params(ctx), dt, a, sg, sb, ctx->stream, ctx->adj_pinned));
     LAUNCH(launch_rebuild(S, a ^ 1, ctx->scan_scratch, mgrd, mblk, ctx->stream));
     return BMXG_OK;
 }
@@ -2693,7 +2699,8 @@ int bmxg_backward(bmxg_ctx *ctx, const double *dL_dx, double *dL_dx0, double *dL
     int ag, ab;
     stencil_shape(ctx, sh, n, &ag, &ab);
     auto reverse = [&](const DevState &Q, int a) -> int {
-        LAUNCH(launch_dadj(Q, P, D, ctx->traj_dt, a, lam[cur], lam[cur ^ 1], gacc, gadh, ag, ab, st, sh.grid > 0));
+        LAUNCH(launch_dadj(Q, P, D, ctx->traj_dt, a, lam[cur], lam[cur ^ 1], gacc, gadh, ag, ab, st,
+                           ctx->adj_pinned));
         cur ^= 1;
         return BMXG_OK;
     };

@@ -49,3 +49,45 @@ def test_first_call_after_autotune(gpu_lib, oracle_lib, then):
         assert np.array_equal(QA[k], QB[k]), k
     A.close()
     B.close()
+
+
+def cached(path, n, side, **shape):
+    """A tuning file whose FP64 sphere entry is replaced."""
+    import json
+    ctx, _, _ = loaded(n, side, 43)
+    ctx.autotune(str(path))
+    ctx.close()
+    d = json.loads(path.read_text())
+    key, = [k for k in d if "|sphere" in k and "|0|" in k]
+    d[key].update(shape)
+    path.write_text(json.dumps(d, separators=(", ", ": ")))
+    return d, key
+
+
+def test_a_tuned_sphere_shape_leaves_the_adjoint_its_kernels(gpu_lib, tmp_path):
+    """The adjoint's kernels are chosen by its own rule, not by the grid that the
+    tuning found for the FP64 step (one thread per slot takes twice as long here)."""
+    import time
+    n, side = 20_000, 0.128
+    cached(tmp_path / "t.json", n, side, block=64, grid=4864)
+    grad = np.random.default_rng(2).normal(0.0, 1.0, (3, n))
+    best, got = [], []
+    for tuned in (True, False):
+        ctx, _, P = loaded(n, side, 43)
+        if tuned:
+            ctx.autotune(str(tmp_path / "t.json"))
+            assert ctx.shapes()["sphere_grid"][0] == 4864
+            ctx.set_shapes(list_step_passes=1)  # (the others as they are)
+        t = []
+        for _ in range(8):
+            ctx.set_state(P)
+            a = time.perf_counter()
+            ctx.forward(0.25, 20, 10)
+            out = ctx.backward(grad)
+            t.append(time.perf_counter() - a)
+        got.append(out)
+        best.append(min(t[2:]))
+        ctx.close()
+    for x, y in zip(*got):
+        assert np.array_equal(x, y)
+    assert best[0] < 1.4 * best[1]
