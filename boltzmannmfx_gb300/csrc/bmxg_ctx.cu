@@ -2206,6 +2206,10 @@ int bmxg_init_bonds(bmxg_ctx *ctx, double rlim, int64_t *added, int64_t *overflo
     return BMXG_OK;
 }
 
+// The kernels that the cached shapes were timed on: entries of another set (before it
+// was in the key, of kernels with one thread per slot alone) are timed again.
+static constexpr int kTuneSet = 2;
+
 int bmxg_autotune(bmxg_ctx *ctx, const char *cache_path)
 {
     if (!ctx) return BMXG_ERR_ARG;
@@ -2278,8 +2282,8 @@ int bmxg_autotune(bmxg_ctx *ctx, const char *cache_path)
     const DevParams P = dev_params(ctx->prm);
     // the per-step stencil kernels of both forms
     for (int prec = 0; prec < 2; ++prec) {
-        std::snprintf(key, sizeof(key), "\"%s|sphere|%d|n=%lld|ncol=%d|h=%s\"", devname, prec, (long long)n,
-                      ctx->ncol, hist.c_str());
+        std::snprintf(key, sizeof(key), "\"%s|sphere %d|%d|n=%lld|ncol=%d|h=%s\"", devname, kTuneSet, prec,
+                      (long long)n, ctx->ncol, hist.c_str());
         {
             const std::string txt = cache_read();
             const size_t pos = txt.find(key);
@@ -2338,7 +2342,7 @@ int bmxg_autotune(bmxg_ctx *ctx, const char *cache_path)
     // k_list_build's block
     const float skin = ctx->list_mode ? list_skin(ctx) : 0.0f;
     if (skin > 0.0f) {
-        std::snprintf(key, sizeof(key), "\"%s|list|n=%lld|ncol=%d|h=%s\"", devname, (long long)n, ctx->ncol,
+        std::snprintf(key, sizeof(key), "\"%s|list %d|n=%lld|ncol=%d|h=%s\"", devname, kTuneSet, (long long)n, ctx->ncol,
                       hist.c_str());
         const std::string txt = cache_read();
         const size_t pos = txt.find(key);

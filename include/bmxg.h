@@ -454,8 +454,8 @@ int  bmxg_set_list_mode(bmxg_ctx *ctx, int32_t mode);
  * the fastest: the per-step stencil kernels of both forms (block, grid) and,
  * where the FP32F list path applies, the list step (block, passes of the
  * block per chunk of slots) and the list build (block).  Results are cached
- * in a JSON file at cache_path (may be NULL: no cache), keyed by the device,
- * the particle count and the colony-size histogram.  The loaded state is left
+ * in a JSON file at cache_path (may be NULL: no cache), keyed by the device, the
+ * library's set of kernels, the particle count and the colony-size histogram.  The loaded state is left
  * as it was.  The reference has no counterpart (AMReX tiles its loops by a
  * fixed tile size, bmx_pc_interaction.cpp:111-114). */
 int  bmxg_autotune(bmxg_ctx *ctx, const char *cache_path);

@@ -91,3 +91,21 @@ def test_a_tuned_sphere_shape_leaves_the_adjoint_its_kernels(gpu_lib, tmp_path):
     for x, y in zip(*got):
         assert np.array_equal(x, y)
     assert best[0] < 1.4 * best[1]
+
+
+def test_entries_of_other_kernels_are_timed_again(gpu_lib, tmp_path):
+    import json
+    n, side = 2000, 0.064
+    path = tmp_path / "t.json"
+    d, key = cached(path, n, side)
+    old = {k.replace("|sphere 2|", "|sphere|").replace("|list 2|", "|list|"): v for k, v in d.items()}
+    assert not set(old) & set(d)
+    for k in old:
+        if "|sphere|0|" in k:
+            old[k] = {"block": 96, "grid": 4097, "ms_per_5": 0.0}
+    path.write_text(json.dumps(old, separators=(", ", ": ")))
+    ctx, _, _ = loaded(n, side, 43)
+    ctx.autotune(str(path))
+    assert ctx.shapes()["sphere_block"][0] != 96
+    ctx.close()
+    assert set(json.loads(path.read_text())) == set(old) | set(d)  # (the file keeps both)
