@@ -126,6 +126,7 @@ struct bmxg_ctx {
     double traj_dt = 0.0;
 
     bool rod_walk = false;    // no room for the rod pair lists: FP64 rod steps walk the stencil
+    int64_t scratch_limit = -1;   // bmxg_set_scratch_limit
     bool vel32 = false;       // the last step's velocities are in the FP32F buffers
     bool vel64_zero = false;  // the FP64 velocity planes (vx .. wz) hold zeros: a load zeroed them
                               // and no kernel that writes them ran since
@@ -276,6 +277,19 @@ struct JoinIo {
         if (s) cudaStreamSynchronize(s);
     }
 };
+
+// Whether `need` bytes of buffers that a call can do without may be taken: up to the caller's
+// limit, else one `share`-th of the device's free memory.
+bool room_for(const bmxg_ctx *ctx, size_t need, size_t share)
+{
+    if (ctx->scratch_limit >= 0) return need <= (size_t)ctx->scratch_limit;
+    size_t room = 0, all = 0;
+    if (cudaMemGetInfo(&room, &all) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return false;
+    }
+    return need <= room / share;
+}
 
 void free_state(bmxg_ctx *ctx)
 {
@@ -1148,6 +1162,7 @@ inline int list_singles(int64_t n) { return n <= 400000 ? 2 : 4; }
 // 200 000 slots 5: 1529 / 1681, 3: 2151 / 2058, 1.2: 4548 / 3658; 1 million 5: 3977 / 4018,
 // 3: 5676 / 5092, 1.2: 12 479 / 9857.
 constexpr double kStallPeriod = 4.0;
+constexpr size_t kRodBytes = 4 + kRodCap * (sizeof(int4) + sizeof(int) + 6 * sizeof(double));  // rod queues, a segment
 constexpr int kListMinSteps = 2;     // a shorter first call after a load runs the per-step path
 
 // Skin of the list for the loaded state and parameters, or 0 where the list
@@ -1194,7 +1209,7 @@ void list64_end(bmxg_ctx *ctx, bool poor)
 // without one, or in the call, are asked for each time.  One step and an export of the
 // neighbour list in turn, us: 20 000 slots 100 without, 154 with a list for every step, 400 000
 // 230 and 263.
-bool list64_pays(const bmxg_ctx *ctx, int32_t nsteps)
+bool list64_pays(bmxg_ctx *ctx, int32_t nsteps)
 {
     if (!ctx->list_room || ctx->list64_bail || ctx->n <= kList64Slots) return false;
     if (ctx->list_valid && ctx->list_prec == BMXG_FP64) return true;
@@ -1203,14 +1218,10 @@ bool list64_pays(const bmxg_ctx *ctx, int32_t nsteps)
     if (ctx->S.nbr) return true;
     const double steps = (double)(ctx->plain64 + nsteps), n = (double)ctx->n;
     if (steps < list64_pays_back(n)) return false;
-    // (and leaves three quarters of the free memory)
-    size_t room = 0, all = 0;
+    // (refused once, this state size goes without)
     const size_t need = (size_t)ctx->n * 320 + (size_t)ctx->ncells_total * sizeof(int);
-    if (cudaMemGetInfo(&room, &all) != cudaSuccess) {
-        (void)cudaGetLastError();
-        return false;
-    }
-    return need <= room / 4;
+    if (!room_for(ctx, need, 4)) ctx->list_room = false;
+    return ctx->list_room;
 }
 
 // Allocate the list on first use; (re)initialise its control block when the
@@ -1594,9 +1605,11 @@ int step_setup(bmxg_ctx *ctx, int32_t nsteps, int32_t precision)
         if (rc) return rc;
         drop_graphs(ctx);
     }
-    // the rod pipelines' buffers (the queue's length is an int)
-    if (ctx->S.has_rods && !ctx->S.rwork &&
-        !(precision == BMXG_FP64 && (ctx->rod_walk || ctx->n > (1LL << 26)))) {
+    // the rod pipelines' buffers (the queue's length is an int), which the FP64 form can
+    // do without
+    if (ctx->S.has_rods && !ctx->S.rwork && precision == BMXG_FP64 && !ctx->rod_walk)
+        ctx->rod_walk = ctx->n > (1LL << 26) || !room_for(ctx, (size_t)ctx->n * kRodBytes, 4);
+    if (ctx->S.has_rods && !ctx->S.rwork && !(precision == BMXG_FP64 && ctx->rod_walk)) {
         const size_t n = (size_t)ctx->n;
         int4 *work = nullptr;
         int *cnt = nullptr, *q64 = nullptr;
@@ -1609,7 +1622,7 @@ int step_setup(bmxg_ctx *ctx, int32_t nsteps, int32_t precision)
         if (!rc) rc = dalloc(ctx, &work, n * kRodCap);
         if (!rc) rc = dalloc(ctx, &ctl, 1);
         if (rc) {
-            // no room for the queues (2 KB per segment): the FP64 form walks
+            // no room for the queues after all: the FP64 form walks
             while (ctx->allocs.size() > held) {
                 cudaFree(ctx->allocs.back());
                 ctx->allocs.pop_back();
@@ -2173,6 +2186,15 @@ int bmxg_set_list_mode(bmxg_ctx *ctx, int32_t mode)
     return BMXG_OK;
 }
 
+int bmxg_set_scratch_limit(bmxg_ctx *ctx, int64_t bytes)
+{
+    if (!ctx) return BMXG_ERR_ARG;
+    ctx->scratch_limit = bytes < 0 ? -1 : bytes;
+    ctx->list_room = true;  // (refused ones are asked for again)
+    ctx->rod_walk = false;
+    return BMXG_OK;
+}
+
 int bmxg_init_bonds(bmxg_ctx *ctx, double rlim, int64_t *added, int64_t *overflow)
 {
     if (!ctx) return BMXG_ERR_ARG;
@@ -2680,9 +2702,7 @@ int bmxg_backward(bmxg_ctx *ctx, const double *dL_dx, double *dL_dx0, double *dL
     const int kseg = std::min(K, std::max(T, 1));
     {
         const size_t need = trail.stride * (size_t)kseg;
-        size_t free_b = 0, total_b = 0;
-        CK(cudaMemGetInfo(&free_b, &total_b));
-        if (need <= ctx->adj[kAdjTrail].bytes || need <= free_b / 2) {
+        if (need <= ctx->adj[kAdjTrail].bytes || room_for(ctx, need, 2)) {
             if (adj_buf(ctx, kAdjTrail, &trail.base, need)) {
                 (void)cudaGetLastError();
                 trail.base = nullptr;

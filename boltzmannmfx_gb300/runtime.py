@@ -28,7 +28,7 @@ ABI_SYMBOLS = ("bmxg_version", "bmxg_last_error", "bmxg_create", "bmxg_destroy",
                "bmxg_particle_exchange", "bmxg_read_ascii", "bmxg_write_ascii", "bmxg_write_vtk",
                "bmxg_read_checkpoint",
                "bmxg_io_last_error", "bmxg_autotune", "bmxg_get_shapes", "bmxg_step_tile", "bmxg_prepare", "bmxg_set_shapes", "bmxg_split_cells_aos", "bmxg_set_pair_capture",
-               "bmxg_get_step_pairs")
+               "bmxg_get_step_pairs", "bmxg_set_scratch_limit")
 
 
 class Ext(C.Structure):
@@ -79,6 +79,7 @@ def load_library(path=None):
     L.bmxg_set_shapes.argtypes = [vp, C.POINTER(abi.Shapes)]
     L.bmxg_init_bonds.argtypes = [vp, C.c_double, C.POINTER(C.c_int64), C.POINTER(C.c_int64)]
     L.bmxg_set_list_mode.argtypes = [vp, C.c_int32]
+    L.bmxg_set_scratch_limit.argtypes = [vp, C.c_int64]
     L.bmxg_set_pair_capture.argtypes = [vp, C.c_int32]
     L.bmxg_get_step_pairs.argtypes = [vp, C.POINTER(C.c_int64), C.POINTER(C.c_int32), C.c_int64,
                                       C.POINTER(C.c_int64)]
@@ -231,8 +232,13 @@ class Context:
         return c.reshape(3, self.n)
 
     def set_list_mode(self, mode):
-        """1: FP32F sphere steps use the skin neighbour list where it is exact; 0: never."""
+        """1: sphere steps use the skin neighbour list where it is exact (FP64: and pays); 0: never."""
         self._check(self.lib.bmxg_set_list_mode(self.h, int(mode)))
+
+    def set_scratch_limit(self, nbytes):
+        """Bytes up to which each buffer that calls can do without is taken (negative:
+        shares of the free memory)."""
+        self._check(self.lib.bmxg_set_scratch_limit(self.h, int(nbytes)))
 
     def set_pair_capture(self, on):
         """list steps record the pairs that pass the force gate (debug export)."""

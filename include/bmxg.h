@@ -450,6 +450,14 @@ int  bmxg_get_step_pairs(bmxg_ctx *ctx, int64_t *offs, int32_t *idx, int64_t cap
  * this switch has no counterpart there. */
 int  bmxg_set_list_mode(bmxg_ctx *ctx, int32_t mode);
 
+/* Device memory, in bytes, up to which the context takes each of the buffers that
+ * its calls can do without: the neighbour list of FP64 sphere steps, the pair
+ * queues of FP64 rod steps, the states that bmxg_backward keeps of a segment.  A
+ * call whose buffer would need more runs without it, with the same results, in
+ * more time.  Negative (the default): a quarter, a quarter and half of the
+ * device's free memory.  Buffers that are there already stay. */
+int  bmxg_set_scratch_limit(bmxg_ctx *ctx, int64_t bytes);
+
 /* Time the launch shapes of the step kernels on the loaded state and keep
  * the fastest: the per-step stencil kernels of both forms (block, grid) and,
  * where the FP32F list path applies, the list step (block, passes of the
