@@ -242,17 +242,36 @@ void drop_graphs(bmxg_ctx *ctx)
 // (kAdjointKeep) and the state's arrays stay, else they are given back.
 constexpr size_t kAdjointKeep = 256u << 20;
 
+size_t adjoint_bytes(const bmxg_ctx *ctx)
+{
+    size_t held = 0;
+    for (const AdjBuf &b : ctx->adj) held += b.bytes;
+    return held;
+}
+
+void free_adj_buf(AdjBuf &b)
+{
+    if (b.p) cudaFree(b.p);  // (waits for the work that uses it)
+    b = AdjBuf{};
+}
+
 void free_adjoint(bmxg_ctx *ctx, bool all = false)
 {
     ctx->traj_T = -1;
-    size_t held = 0;
-    for (const AdjBuf &b : ctx->adj) held += b.bytes;
-    if (!all && held <= kAdjointKeep) return;
-    for (AdjBuf &b : ctx->adj) {
-        if (b.p) cudaFree(b.p);
-        b = AdjBuf{};
-    }
+    if (!all && adjoint_bytes(ctx) <= kAdjointKeep) return;
+    for (AdjBuf &b : ctx->adj) free_adj_buf(b);
 }
+
+// The buffers of a reverse sweep alone, after it: the states of a segment can be
+// half of the device's memory.  (The trajectory stays: another sweep may follow.)
+struct SweepBufs {
+    bmxg_ctx *ctx;
+    ~SweepBufs()
+    {
+        for (int k : {kAdjTrail, kAdjSeg})
+            if (adjoint_bytes(ctx) > kAdjointKeep) free_adj_buf(ctx->adj[k]);
+    }
+};
 
 // Device staging of at least `bytes` for host loads and stores.
 int ensure_io(bmxg_ctx *ctx, size_t bytes)
@@ -2522,8 +2541,7 @@ int adj_buf(bmxg_ctx *ctx, int k, T **p, size_t count)
     AdjBuf &b = ctx->adj[k];
     const size_t need = std::max<size_t>(count, 1) * sizeof(T);
     if (b.bytes < need) {
-        if (b.p) cudaFree(b.p);  // (waits for the work that uses it)
-        b = AdjBuf{};
+        free_adj_buf(b);
         CK(cudaMalloc(&b.p, need));
         b.bytes = need;
     }
@@ -2697,6 +2715,7 @@ int bmxg_backward(bmxg_ctx *ctx, const double *dL_dx, double *dL_dx0, double *dL
     // memory (100 B per slot and step): the reverse sweep then runs one kernel
     // per step.  Otherwise the positions alone are kept (24 B) and binned and
     // sorted again.
+    SweepBufs give_back{ctx};
     Trail trail((size_t)n, (size_t)S.ncols_total);
     double *segbuf = nullptr;
     const int kseg = std::min(K, std::max(T, 1));

@@ -105,3 +105,23 @@ def test_reverse_sweep(gpu_lib, n, steps, every):
         ctx.close()
     for a, b in zip(*got):
         assert np.array_equal(a, b)
+
+
+def test_a_sweep_gives_its_states_back(gpu_lib):
+    """The kept states (here 460 MB) are not held after the sweep; another may follow."""
+    import torch
+    n, side, steps = 100_000, 0.384, 60
+    g, P = configs.box_geometry(side, side), configs.sphere_colony(n, side, side, np.random.default_rng(61))
+    grad = np.random.default_rng(62).normal(0.0, 1.0, (3, n))
+    ctx = Context(PRM, [g])
+    ctx.set_state(P)
+    ctx.forward(0.25, steps, steps)
+    ctx.step(0.25, 0, BMXG_FP64)
+    torch.cuda.synchronize()
+    free0 = torch.cuda.mem_get_info()[0]
+    a = ctx.backward(grad)
+    free1 = torch.cuda.mem_get_info()[0]
+    assert free0 - free1 < 256 << 20
+    for x, y in zip(a, ctx.backward(grad)):
+        assert np.array_equal(x, y)
+    ctx.close()
