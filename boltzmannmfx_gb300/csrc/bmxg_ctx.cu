@@ -1679,13 +1679,25 @@ int bmxg_prepare(bmxg_ctx *ctx, double dt, int32_t precision)
     if (int rc = step_setup(ctx, 2 * kResyncEvery, precision)) return rc;
     // the replayed graph of kResyncEvery steps and the one-step graphs (with and
     // without the re-sync), from either parity
-    for (int parity = 0; parity < 2; ++parity) {
-        cudaGraphExec_t g = nullptr;
-        if (int rc = get_graph(ctx, subdt, precision, parity, &g)) return rc;
-        for (int resync = 0; resync < (ctx->list_on ? 3 : 2); ++resync)
-            if (int rc = get_graph(ctx, subdt, precision, parity, &g, resync)) return rc;
-    }
-    return BMXG_OK;
+    auto capture = [&]() -> int {
+        for (int parity = 0; parity < 2; ++parity) {
+            cudaGraphExec_t g = nullptr;
+            if (int rc = get_graph(ctx, subdt, precision, parity, &g)) return rc;
+            for (int resync = 0; resync < (ctx->list_on ? 3 : 2); ++resync)
+                if (int rc = get_graph(ctx, subdt, precision, parity, &g, resync)) return rc;
+            if (ctx->list_on && ctx->period_steps < kStallPeriod * ctx->period_builds)
+                if (int rc = get_graph(ctx, subdt, precision, parity, &g, -2)) return rc;
+        }
+        return BMXG_OK;
+    };
+    if (int rc = capture()) return rc;
+    if (!ctx->list_on || precision != BMXG_FP64) return BMXG_OK;
+    // FP64 steps take the list where they are many enough (list64_pays): the others' graphs
+    // too
+    ctx->list_on = false;
+    const int rc = capture();
+    ctx->list_on = true;
+    return rc;
 }
 
 int bmxg_step(bmxg_ctx *ctx, double dt, int32_t nsteps, int32_t precision)

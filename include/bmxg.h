@@ -188,9 +188,11 @@ int  bmxg_step(bmxg_ctx *ctx, double dt, int32_t nsteps, int32_t precision);
 /* Instantiate, without running a step, the CUDA graphs that bmxg_step(ctx, dt,
  * n, precision) replays (the graph of the re-sync period and the one-step
  * graphs, from either parity) and allocate the buffers of that path, so that
- * the first long call captures nothing.  The FP32F list path counts as chosen
- * (a later one-step call then steps over the list too).  No counterpart in the
- * reference (it has no graphs). */
+ * the first long call captures nothing.  Where calls of sixteen steps would
+ * take the neighbour list it counts as chosen (a later one-step call then steps
+ * over the list too, until a load or a call that needs the bins); for FP64 steps
+ * the graphs of steps without it are instantiated as well.  No counterpart in
+ * the reference (it has no graphs). */
 int  bmxg_prepare(bmxg_ctx *ctx, double dt, int32_t precision);
 
 /* Drop-in for the reference member function, on the state loaded with
