@@ -338,7 +338,7 @@ int launch_dadj(const DevState &S, const DevParams &P, const DiffParams &D, doub
                 double *lout, double *gacc, double *gadh, int grid, int block, cudaStream_t st, bool pinned = false);
 // out: kReduceOut values, the planes' sums first
 constexpr int kReduceBlocks = 64;
-constexpr int kReduceOut = 4 + 4 * kReduceBlocks;  // (up to four planes)
+constexpr int kReduceOut = 4 + 4 * 2 * kReduceBlocks;  // (up to four planes; a sum and its remainder)
 int launch_dreduce(const double *gacc, int n, int planes, double *out, cudaStream_t st);
 
 }  // namespace bmxg

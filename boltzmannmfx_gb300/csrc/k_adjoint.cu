@@ -551,37 +551,60 @@ __global__ void __launch_bounds__(kWalkBlock, RESIDENT) k_dadjw(const DevState S
 
 // Deterministic sum of per-slot gradient planes: every block of a plane sums a
 // fixed share of it, the second kernel the blocks' sums, each in a fixed order
-// (one block over all planes took 114 us for 20 000 slots; 6 us for both).
+// (one block over all planes took 114 us for 20 000 slots; 6 us for both).  The
+// rounding of every addition is kept beside the sum (two_add, the exact difference
+// of Knuth's sum), so the order costs no digits: the result is the planes' sum
+// rounded about once, however the shares fall.
 constexpr int kReduceThreads = 256;
 
-__device__ __forceinline__ double block_sum(double s, double *sh)
+__device__ __forceinline__ void two_add(double &s, double &c, double v)
 {
-    sh[threadIdx.x] = s;
+    const double t = s + v, z = t - s;
+    c += (s - (t - z)) + (v - z);
+    s = t;
+}
+
+// The block's sum and what its roundings left, in thread 0.
+__device__ __forceinline__ void block_sum(double &s, double &c, double (*sh)[2])
+{
+    sh[threadIdx.x][0] = s;
+    sh[threadIdx.x][1] = c;
     __syncthreads();
     for (int w = kReduceThreads / 2; w > 0; w >>= 1) {
-        if (threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w];
+        if (threadIdx.x < w) {
+            two_add(s, c, sh[threadIdx.x + w][0]);
+            c += sh[threadIdx.x + w][1];
+            sh[threadIdx.x][0] = s;
+            sh[threadIdx.x][1] = c;
+        }
         __syncthreads();
     }
-    return sh[0];
 }
 
 __global__ void __launch_bounds__(kReduceThreads) k_dreduce(const double *gacc, int n, double *out)
 {
-    __shared__ double sh[kReduceThreads];
+    __shared__ double sh[kReduceThreads][2];
     const int p = blockIdx.y;
-    double s = 0.0;
+    double s = 0.0, c = 0.0;
     for (int i = blockIdx.x * kReduceThreads + threadIdx.x; i < n; i += gridDim.x * kReduceThreads)
-        s += gacc[(size_t)p * n + i];
-    s = block_sum(s, sh);
-    if (threadIdx.x == 0) out[4 + p * kReduceBlocks + blockIdx.x] = s;
+        two_add(s, c, gacc[(size_t)p * n + i]);
+    block_sum(s, c, sh);
+    if (threadIdx.x == 0) {
+        double *o = out + 4 + 2 * (p * kReduceBlocks + blockIdx.x);
+        o[0] = s;
+        o[1] = c;
+    }
 }
 
 __global__ void __launch_bounds__(kReduceThreads) k_dreduce_top(double *out, int blocks)
 {
-    __shared__ double sh[kReduceThreads];
+    __shared__ double sh[kReduceThreads][2];
     const int p = blockIdx.x;
-    const double s = block_sum((int)threadIdx.x < blocks ? out[4 + p * kReduceBlocks + threadIdx.x] : 0.0, sh);
-    if (threadIdx.x == 0) out[p] = s;
+    const double *o = out + 4 + 2 * (p * kReduceBlocks + min((int)threadIdx.x, blocks - 1));
+    const bool mine = (int)threadIdx.x < blocks;
+    double s = mine ? o[0] : 0.0, c = mine ? o[1] : 0.0;
+    block_sum(s, c, sh);
+    if (threadIdx.x == 0) out[p] = finite_bits(s) ? s + c : s;
 }
 
 }  // namespace
