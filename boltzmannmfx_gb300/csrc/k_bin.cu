@@ -315,7 +315,7 @@ struct SortJob {
 constexpr int kSortBlock = 1024;
 constexpr int kSortItems = 4;    // slots per thread
 constexpr int kSortCols = 16;    // columns per thread
-constexpr int kSortCluster = 16; // blocks (non-portable size; 8 where the device refuses it)
+constexpr int kSortCluster = 16; // blocks at most (a non-portable size)
 
 // The rest of k_sort_cluster, after the keys' scatter, for a state with a long
 // column; at: the places the thread's slots drew.  (Out of line, and found out from
@@ -703,46 +703,40 @@ int launch_scan(const int *in, int *out, int n, int *scratch, cudaStream_t st, c
     return 3;
 }
 
-// Blocks of the sort's cluster on the current device (0: none fits), looked up
-// once per device.
-static int sort_cluster_size()
+// Whether the current device takes the sort's cluster, looked up once per device.
+static bool sort_cluster_fits()
 {
-    static std::atomic<int> known[64];  // size + 1; 0: not looked up yet
+    static std::atomic<int> known[64];  // 0: not looked up yet, 1: no, 2: yes
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
     int v = known[dev].load(std::memory_order_relaxed);
-    if (v) return v - 1;
-    int size = 0;
-    const bool wide = cudaFuncSetAttribute(k_sort_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
-                      cudaSuccess;
-    for (int c = wide ? kSortCluster : 8; c >= 8 && !size; c -= 8) {
-        cudaLaunchConfig_t cfg = {};
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = (unsigned)c;
-        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-        cfg.gridDim = dim3((unsigned)c);
-        cfg.blockDim = dim3(kSortBlock);
-        cfg.attrs = at;
-        cfg.numAttrs = 1;
-        int fit = 0;
-        if (cudaOccupancyMaxActiveClusters(&fit, k_sort_cluster, &cfg) == cudaSuccess && fit > 0) size = c;
-    }
-    (void)cudaGetLastError();
-    known[dev].store(size + 1, std::memory_order_relaxed);
-    return size;
+    if (v) return v == 2;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)kSortCluster;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3((unsigned)kSortCluster);
+    cfg.blockDim = dim3(kSortBlock);
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int fit = 0;
+    const bool yes = cudaFuncSetAttribute(k_sort_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
+                         cudaSuccess &&
+                     cudaOccupancyMaxActiveClusters(&fit, k_sort_cluster, &cfg) == cudaSuccess && fit > 0;
+    if (!yes) (void)cudaGetLastError();
+    known[dev].store(yes ? 2 : 1, std::memory_order_relaxed);
+    return yes;
 }
 
 // Runs the job in one cluster where it fits (J.lkey set); false: the caller's
 // separate kernels.
 static bool sort_in_cluster(const SortJob &J, cudaStream_t st)
 {
-    if (!J.lkey) return false;
-    const int c = sort_cluster_size();
-    const long long T = (long long)c * kSortBlock;
-    if (J.n > T * kSortItems || J.ncols > T * kSortCols) return false;
+    constexpr int T = kSortCluster * kSortBlock;
+    if (!J.lkey || J.n > T * kSortItems || J.ncols > T * kSortCols || !sort_cluster_fits()) return false;
     // no more blocks than the slots and columns fill
-    int use = c;
+    int use = kSortCluster;
     while (use > 1 && J.n <= (use / 2) * kSortBlock && J.ncols <= (use / 2) * kSortBlock * 4) use /= 2;
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute at[2];
