@@ -714,22 +714,21 @@ int load_state(bmxg_ctx *ctx, const bmxg_particles *p, const int64_t *colony_off
         unsigned long long *diff = ctx->d_chk + 4;
         CK(cudaMemsetAsync(ctx->d_chk, 0, 5 * sizeof(unsigned long long), st));
         // (the checks of a full load go along: one read-back decides both)
-        Shape sh;
-        LAUNCH(launch_check_state(src_ct, src_r, (int)n, ctx->d_chk, grid_for(ctx, sh, n), sh.block, st));
         if (join.s) {  // each field as its copy lands: only the last comparison follows the copies
-            LAUNCH(launch_same_state(S, ctx->parity, nullptr, nullptr, nullptr, src_r, src_ct, diff, grd, blk,
-                                     st));
+            LAUNCH(launch_same_state(S, ctx->parity, nullptr, nullptr, nullptr, src_r, src_ct, diff, ctx->d_chk, grd,
+                                     blk, st));
             CK(cudaStreamWaitEvent(st, ctx->io_ev[6], 0));
-            LAUNCH(launch_same_state(S, ctx->parity, src_x, nullptr, nullptr, nullptr, nullptr, diff, grd, blk,
-                                     st));
+            LAUNCH(launch_same_state(S, ctx->parity, src_x, nullptr, nullptr, nullptr, nullptr, diff, nullptr, grd,
+                                     blk, st));
             CK(cudaStreamWaitEvent(st, ctx->io_ev[7], 0));
-            LAUNCH(launch_same_state(S, ctx->parity, nullptr, src_y, nullptr, nullptr, nullptr, diff, grd, blk,
-                                     st));
+            LAUNCH(launch_same_state(S, ctx->parity, nullptr, src_y, nullptr, nullptr, nullptr, diff, nullptr, grd,
+                                     blk, st));
             CK(cudaStreamWaitEvent(st, ctx->io_ev[1], 0));
-            LAUNCH(launch_same_state(S, ctx->parity, nullptr, nullptr, src_z, nullptr, nullptr, diff, grd, blk,
-                                     st));
+            LAUNCH(launch_same_state(S, ctx->parity, nullptr, nullptr, src_z, nullptr, nullptr, diff, nullptr, grd,
+                                     blk, st));
         } else {
-            LAUNCH(launch_same_state(S, ctx->parity, src_x, src_y, src_z, src_r, src_ct, diff, grd, blk, st));
+            LAUNCH(launch_same_state(S, ctx->parity, src_x, src_y, src_z, src_r, src_ct, diff, ctx->d_chk, grd, blk,
+                                     st));
         }
         CK(cudaMemcpyAsync(ctx->h_chk, ctx->d_chk, 5 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));

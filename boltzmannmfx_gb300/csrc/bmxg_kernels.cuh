@@ -216,9 +216,11 @@ int launch_aos_load(const unsigned char *rec, const AosLayout &L, int n, bool ro
 // What a step writes, from buffer a into the records.
 int launch_aos_store(unsigned char *rec, const AosLayout &L, const DevState &S, int a, cudaStream_t st);
 // *diff |= 1 when a given field (null: not compared) differs bit for bit from
-// the device state of buffer a (slot s against caller index orig[s])
+// the device state of buffer a (slot s against caller index orig[s]); chk (null: not):
+// launch_check_state's out, from the same pass over r and ct
 int launch_same_state(const DevState &S, int a, const double *x, const double *y, const double *z, const double *r,
-                      const int *ct, unsigned long long *diff, int grid, int block, cudaStream_t st);
+                      const int *ct, unsigned long long *diff, unsigned long long *chk, int grid, int block,
+                      cudaStream_t st);
 // state checks before a load: out[4] = {bad cell type, any FUNGI, largest radius bits, NaN radius}
 int launch_check_state(const int *ct, const double *r, int n, unsigned long long *out, int grid, int block,
                        cudaStream_t st);
