@@ -874,10 +874,22 @@ int load_state(bmxg_ctx *ctx, const bmxg_particles *p, const int64_t *colony_off
     auto fi = [&](const int32_t *src, int planes) {
         return static_cast<const int *>(field(src, sizeof(int) * n * planes, 4));
     };
-    const double *const vel[6] = {fd(p->velx), fd(p->vely), fd(p->velz), fd(p->wx), fd(p->wy), fd(p->wz)};
+    const double *vel[6] = {fd(p->velx), fd(p->vely), fd(p->velz), fd(p->wx), fd(p->wy), fd(p->wz)};
     if (rc) return rc;
+    // velocities that the gather of the positions has no room for in its pass: one by one
+    // after it (3 million spheres with six: 652 us, 829 in one pass)
+    const double *later[6] = {};
+    size_t pass = (size_t)n * 36;
+    for (int k = 0; k < 6; ++k) {
+        if (!vel[k]) continue;
+        pass += (size_t)n * sizeof(double);
+        if (pass > kScatterPass) std::swap(vel[k], later[k]);
+    }
     LAUNCH(launch_load_slots(S, src_x, src_y, src_z, src_r, src_ct, vel, S.col[1], S.iz[1], ctx->uperm, grd, blk,
                              st));
+    double *const vdst[6] = {S.vx, S.vy, S.vz, S.wx, S.wy, S.wz};
+    for (int k = 0; k < 6; ++k)
+        if (later[k]) LAUNCH(launch_gather_d(vdst[k], later[k], ctx->uperm, (int)n, grd, blk, st));
     if (rods) {
         const RodFields F{fd(p->c_length), fd(p->area), fd(p->bond_scale), fd(p->theta), fd(p->phi),
                           fi(p->id, 1), fi(p->cpu, 1), fi(p->fuse_tip, 1), fi(p->position, 1), fi(p->fix_site, 1),
@@ -1000,6 +1012,10 @@ int store_fused(bmxg_ctx *ctx, bmxg_particles *p, bool host, bool fx)
     F.sflag = (int *)at[18];
     F.nflag = (int *)at[19];
     F.dltd = (int *)at[20];
+    if (fx && store_bytes(F, (int)n) + 3 * d8 > kScatterPass) {  // (a pass for each field: converted before them)
+        if (int rc = sync_fp64(ctx)) return rc;
+        fx = false;
+    }
     LAUNCH(launch_store(S, ctx->parity, F, fx, ctx->vel32, st));
     if (fx) ctx->fx_ahead = false;
     for (const Out &o : outs) CK(cudaMemcpyAsync(o.dst, o.from, o.bytes, cudaMemcpyDeviceToHost, st));

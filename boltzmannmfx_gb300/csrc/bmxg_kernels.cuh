@@ -195,13 +195,16 @@ struct RodFields {
 };
 int launch_load_rods(const DevState &S, const DevParams &P, const RodFields &F, const int *uperm, int grid, int block,
                      cudaStream_t st);
-// The state of buffer a scattered to caller order in one pass, the fields asked
-// for (null: not).  fx: the positions come from the list's fixed point (the FP64
+// The state of buffer a scattered to caller order, the fields asked for (null: not).  fx: the positions come from the list's fixed point (the FP64
 // ones are written too); vel32: the velocities from the FP32F planes.
 struct StoreFields {
     double *x, *y, *z, *v[6], *theta, *phi;
     int *n_bnds, *seg_id1, *seg_id2, *site, *position, *fix_site, *fflag, *sflag, *nflag, *dltd;
 };
+// Bytes up to which one pass scatters several fields: past it their lines leave L2 (129 MB,
+// the sources' lines with them) before they are whole.
+constexpr size_t kScatterPass = 76u << 20;
+size_t store_bytes(const StoreFields &F, int n);
 int launch_store(const DevState &S, int a, const StoreFields &F, bool fx, bool vel32, cudaStream_t st);
 // AoS records (k_io.cu): bytes per record, of rdata and idata in a record
 struct AosLayout {
