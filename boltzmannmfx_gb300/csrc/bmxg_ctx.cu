@@ -273,6 +273,14 @@ struct SweepBufs {
     }
 };
 
+// What the last sort found (the captured steps hold the choice of its kernel).
+void set_long_cols(bmxg_ctx *ctx, bool some)
+{
+    if ((ctx->S.long_cols != 0) == some) return;
+    ctx->S.long_cols = some ? 1 : 0;
+    drop_graphs(ctx);
+}
+
 // Device staging of at least `bytes` for host loads and stores.
 int ensure_io(bmxg_ctx *ctx, size_t bytes)
 {
@@ -903,6 +911,7 @@ int load_state(bmxg_ctx *ctx, const bmxg_particles *p, const int64_t *colony_off
     CK(cudaMemcpyAsync(ctx->h_cnt, ctx->d_cnt, sizeof(DevCounters), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     if (ctx->h_cnt->bad_index) return fail(ctx, BMXG_ERR_STATE, "internal: inconsistent bin counts in the load sort");
+    set_long_cols(ctx, ctx->h_cnt->long_column != 0);
     ctx->have_state = true;
     ctx->stepped = false;
     ctx->vel32 = false;
@@ -1551,7 +1560,7 @@ int list_steps(bmxg_ctx *ctx, double dt, int32_t nsteps, int precision, int32_t 
             const bool each = period < kStallPeriod;
             if (int rc = get_graph(ctx, dt, precision, 0, &g, each ? -2 : -1)) return rc;
             const double stalled = each ? 0.0 : 0.5 * (kResyncEvery - 1) * left / std::max(period, 1.0);
-            const int graphs = std::max(1, (int)((left + stalled) / kResyncEvery));
+            const int graphs = std::max(1, (int)((left + stalled) / kResyncEvery + 0.5));
             for (int k = 0; k < graphs; ++k) CK(cudaGraphLaunch(g, st));
         }
         CK(cudaEventRecord(ctx->ev1, st));
@@ -1802,6 +1811,7 @@ int bmxg_step(bmxg_ctx *ctx, double dt, int32_t nsteps, int32_t precision)
         CK(cudaMemcpyAsync(ctx->h_cnt, ctx->d_cnt, sizeof(DevCounters), cudaMemcpyDeviceToHost, ctx->stream));
         CK(cudaStreamSynchronize(ctx->stream));
         ctx->stats.n_rebins += per_step;
+        if (ctx->h_cnt->long_column) set_long_cols(ctx, true);
         if (precision == BMXG_FP64) {
             ctx->plain64 += per_step;
             ctx->list64_since += per_step;
@@ -2019,6 +2029,7 @@ int bmxg_step_tile(bmxg_ctx *ctx, const bmxg_tile *tile, const bmxg_particles *r
     S.n = (int)nt;
     S.ncol = 1;
     S.ncols_total = ncols;
+    S.long_cols = nt / ncols > kLongColumn;  // (by the average: nothing was sorted before)
     S.cnt = reinterpret_cast<DevCounters *>(base + o_bad + 3 * sizeof(unsigned long long));
     S.x[0] = reinterpret_cast<double *>(base + o_pos);
     S.y[0] = S.x[0] + N;

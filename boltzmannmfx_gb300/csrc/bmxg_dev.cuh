@@ -99,6 +99,7 @@ struct DevCounters {
     unsigned long long nonfinite;  // sticky
     unsigned long long bad_index;  // counting-sort slots outside 0..n-1 (skipped; an internal error, sticky)
     unsigned long long range;      // list path: a z left the fixed-point range (sticky)
+    unsigned long long long_column;  // a column sort met one longer than kLongColumn (sticky)
     unsigned long long last_out_of_domain, last_edge_ghost, last_bond_repairs;
 };
 constexpr int kStepCounters = 5;

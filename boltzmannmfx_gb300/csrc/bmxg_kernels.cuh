@@ -68,6 +68,7 @@ constexpr int kListStepBlock = 128;  // k_list_step's default block (at most 256
 constexpr int kListBuildBlock = 128; // k_list_build's default block (one slot per thread; at most 256)
 constexpr int kSphereBlock = 64;     // per-step sphere kernels' block (one slot per thread)
 constexpr int kWalkNarrow = 65536;   // tile: 32 slots per block up to here, then 128
+constexpr int kLongColumn = 160;     // slots of a column above which its runs are sorted (k_bin.cu)
 constexpr int kRodCap = 32;          // gated pairs per segment the rod pipelines hold (more: the
                                      // segment walks its stencil in the segment kernel)
 
@@ -85,6 +86,7 @@ struct DevState {
     int ncol;          // colonies
     int ncols_total;   // columns over all colonies
     int nsm;           // SMs of the device (launch rules count in waves of blocks over them)
+    int long_cols;     // some column is longer than kLongColumn: what its sort found last
     const DevGeom *geoms;
     const int *cbase;  // ncol + 1: first slot of each colony, then n (a compact copy for colony lookups)
     DevCounters *cnt;

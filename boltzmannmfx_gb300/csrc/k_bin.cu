@@ -171,12 +171,13 @@ __device__ __forceinline__ void publish_counters(DevCounters *c, RodCtl *rctl)
 // ascending order kRun at a time (one warp per run of them from the column's start),
 // then a rank is a binary search per run, eight reads for 128 keys.  In the cluster sort,
 // whose 16 SMs counted slower than the separate kernels' blocks do, 60 000 FP64 spheres in
-// 1 / 4 / 16 / 64 columns, 5 steps: 54.4 / 16.2 / 5.35 / 2.12 -> 12.7 / 4.5 / 1.90 / 1.29 ms
+// 1 / 4 / 16 / 64 columns, 5 steps: 54.4 / 16.2 / 5.35 / 2.12 -> 12.8 / 4.46 / 1.93 / 1.23 ms
 // (separate kernels, every key counted: 16.6 / 5.21 / 2.25 / 1.37); runs of 32: 33.9 / 10.4 /
 // 3.32 / 1.46.  In a tile of 50 451 + 62 038 in 36 columns 2006 -> 1653 us (cell by cell 1791).
-// Where it starts: 65 000 spheres at 253 / 112 a column, 5 steps, from 128 slots on 980 / 836, from
-// 512 on 1075 / 786 us.
-constexpr int kLongColumn = 160;  // slots of a column above which its runs are sorted
+// Whether a state has such columns its sorts say in DevCounters::long_column, which the host
+// reads with the other counters.
+// kLongColumn: 65 000 spheres at 253 / 112 a column, 5 steps, from 128 slots on
+// 980 / 836, from 512 on 1075 / 786 us.
 constexpr int kRun = 128;
 
 // The warp sorts the run at t (keys t .. end - 1, at most kRun of them): a bitonic
@@ -240,6 +241,7 @@ __global__ void k_scatter(const DevState S, int b)
         const int c = S.col[b][i];
         const int r = atomicSub(&S.colcnt[c], 1) - 1;  // leaves colcnt at zero
         const int t = S.colstart[b][c] + r;
+        if (r == kLongColumn) S.cnt->long_column = 1ull;
         if (t >= 0 && t < S.n) {
             if (S.lkey) S.lkey[t] = col_key(S.iz[b][i], S.orig ? S.orig[i] : i);
             else S.tmp[t] = i;
@@ -317,11 +319,10 @@ constexpr int kSortItems = 4;    // slots per thread
 constexpr int kSortCols = 16;    // columns per thread
 constexpr int kSortCluster = 16; // blocks at most (a non-portable size)
 
-// The rest of k_sort_cluster, after the keys' scatter, for a state with a long
-// column; at: the places the thread's slots drew.  (Out of line, and found out from
-// the scatter: with the columns' lengths looked at in the scan and this in line the sort of
-// 50 000 segments in 65 536 columns took 2 us more; so, 1 us.)
-__device__ __noinline__ void rank_long(const SortJob &J, int g, int T, int4 at)
+// The rest of k_sort_cluster, after the keys' scatter, for a state with long
+// columns; at: the places the thread's slots drew.  (Of an instantiation of its own: in
+// the common kernel it cost every sort 0.3 us in line, as a function 1.6.)
+__device__ __forceinline__ void rank_long(const SortJob &J, int g, int T, int4 at)
 {
     for (int k = 0; k < kSortItems; ++k) {  // a run is sorted by the warp whose slot drew its first place
         const int i = g + k * T;
@@ -360,12 +361,13 @@ __device__ __noinline__ void rank_long(const SortJob &J, int g, int T, int4 at)
     }
 }
 
+template <bool LONG>
 __global__ void __launch_bounds__(kSortBlock) k_sort_cluster(const SortJob J)
 {
     namespace cg = cooperative_groups;
     cg::cluster_group cl = cg::this_cluster();
     __shared__ int warp_sums[kSortBlock / 32];
-    __shared__ int block_sum, some_long;
+    __shared__ int block_sum;
     const int nb = (int)cl.num_blocks(), rank = (int)cl.block_rank();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int T = nb * kSortBlock, g = rank * kSortBlock + tid;
@@ -395,7 +397,6 @@ __global__ void __launch_bounds__(kSortBlock) k_sort_cluster(const SortJob J)
         if (lane >= d) x += y;
     }
     if (lane == 31) warp_sums[warp] = x;
-    if (tid == 0) some_long = 0;
     __syncthreads();
     if (warp == 0) {
         int w = warp_sums[lane];
@@ -420,6 +421,7 @@ __global__ void __launch_bounds__(kSortBlock) k_sort_cluster(const SortJob J)
     }
     if (q0 < J.ncols && q1 == J.ncols) J.colstart[J.ncols] = run;
     cl.sync();
+    bool is_long = false;
 #pragma unroll
     for (int k = 0; k < kSortItems; ++k) {
         if (c[k] < 0) continue;
@@ -427,12 +429,12 @@ __global__ void __launch_bounds__(kSortBlock) k_sort_cluster(const SortJob J)
         const int t = J.colstart[c[k]] + r;
         if (t >= 0 && t < J.n) J.lkey[t] = col_key(z[k], o[k]);
         else atomicAdd(&J.cnt->bad_index, 1ULL);
-        at[k] = t;
-        if (r == kLongColumn)  // (one slot of each long column: every block learns of it)
-            for (int v = 0; v < nb; ++v) *cl.map_shared_rank(&some_long, v) = 1;
+        if (LONG) at[k] = t;
+        is_long |= r == kLongColumn;
     }
+    if (is_long) J.cnt->long_column = 1ull;  // (one slot of each long column)
     cl.sync();
-    if (some_long) {  // (the same in every block)
+    if constexpr (LONG) {
         rank_long(J, g, T, make_int4(at[0], at[1], at[2], at[3]));
         return;
     }
@@ -482,6 +484,7 @@ __global__ void k_user_scatter(const DevState S, const int *ucol, const int *uiz
     for (int u = blockIdx.x * blockDim.x + threadIdx.x; u < S.n; u += gridDim.x * blockDim.x) {
         const int c = ucol[u];
         const int r = atomicSub(&S.colcnt[c], 1) - 1;
+        if (r == kLongColumn) S.cnt->long_column = 1ull;
         const int t = colstart[c] + r;
         if (t >= 0 && t < S.n) S.lkey[t] = col_key(uiz[u], u);
         else atomicAdd(&S.cnt->bad_index, 1ULL);
@@ -559,19 +562,25 @@ struct StateFlags {
     __device__ __forceinline__ void publish(unsigned long long *out)
     {
         __shared__ unsigned long long most[32];
-        bad = __syncthreads_or(bad);
-        fungi = __syncthreads_or(fungi);
-        nan = __syncthreads_or(nan);
+        __shared__ unsigned flags[32];
+        const unsigned all = __reduce_or_sync(0xffffffffu, bad | (fungi << 1) | (nan << 2));
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) rmax = max(rmax, __shfl_xor_sync(0xffffffffu, rmax, o));
-        if ((threadIdx.x & 31) == 0) most[threadIdx.x >> 5] = rmax;
+        if ((threadIdx.x & 31) == 0) {
+            most[threadIdx.x >> 5] = rmax;
+            flags[threadIdx.x >> 5] = all;
+        }
         __syncthreads();
         if (threadIdx.x) return;
-        for (int v = 1; v < (int)(blockDim.x >> 5); ++v) rmax = max(rmax, most[v]);
-        if (bad) atomicOr(&out[0], 1ull);
-        if (fungi) atomicOr(&out[1], 1ull);
+        unsigned f = all;
+        for (int v = 1; v < (int)(blockDim.x >> 5); ++v) {
+            rmax = max(rmax, most[v]);
+            f |= flags[v];
+        }
+        if (f & 1u) atomicOr(&out[0], 1ull);
+        if (f & 2u) atomicOr(&out[1], 1ull);
         if (rmax > *static_cast<volatile unsigned long long *>(&out[2])) atomicMax(&out[2], rmax);
-        if (nan) atomicOr(&out[3], 1ull);
+        if (f & 4u) atomicOr(&out[3], 1ull);
     }
 };
 
@@ -739,9 +748,12 @@ static bool sort_cluster_fits()
     cfg.attrs = at;
     cfg.numAttrs = 1;
     int fit = 0;
-    const bool yes = cudaFuncSetAttribute(k_sort_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
+    const bool yes = cudaFuncSetAttribute(k_sort_cluster<false>, cudaFuncAttributeNonPortableClusterSizeAllowed,
+                                          1) == cudaSuccess &&
+                     cudaOccupancyMaxActiveClusters(&fit, k_sort_cluster<false>, &cfg) == cudaSuccess && fit > 0 &&
+                     cudaFuncSetAttribute(k_sort_cluster<true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
                          cudaSuccess &&
-                     cudaOccupancyMaxActiveClusters(&fit, k_sort_cluster, &cfg) == cudaSuccess && fit > 0;
+                     cudaOccupancyMaxActiveClusters(&fit, k_sort_cluster<true>, &cfg) == cudaSuccess && fit > 0;
     if (!yes) (void)cudaGetLastError();
     known[dev].store(yes ? 2 : 1, std::memory_order_relaxed);
     return yes;
@@ -749,7 +761,7 @@ static bool sort_cluster_fits()
 
 // Runs the job in one cluster where it fits (J.lkey set); false: the caller's
 // separate kernels.
-static bool sort_in_cluster(const SortJob &J, cudaStream_t st)
+static bool sort_in_cluster(const SortJob &J, bool long_cols, cudaStream_t st)
 {
     constexpr int T = kSortCluster * kSortBlock;
     if (!J.lkey || J.n > T * kSortItems || J.ncols > T * kSortCols || !sort_cluster_fits()) return false;
@@ -768,7 +780,7 @@ static bool sort_in_cluster(const SortJob &J, cudaStream_t st)
     cfg.stream = st;
     cfg.attrs = at;
     cfg.numAttrs = 2;
-    cudaLaunchKernelEx(&cfg, k_sort_cluster, J);  // (an error is the launch status the caller reads)
+    cudaLaunchKernelEx(&cfg, long_cols ? k_sort_cluster<true> : k_sort_cluster<false>, J);  // (an error is the launch status the caller reads)
     return true;
 }
 
@@ -776,13 +788,12 @@ int launch_rebuild(const DevState &S, int b, int *scan_scratch, int grid, int bl
 {
     const SortJob J{S.n,       S.ncols_total, S.col[b], S.iz[b],  S.orig, S.colcnt, S.colstart[b],  S.lkey, S.perm[b],
                     S.rel[b],  S.srel[b],     S.siz[b], S.rank[b], S.cnt, S.rctl,   publish ? 1 : 0};
-    if (sort_in_cluster(J, st)) return 1;
+    if (sort_in_cluster(J, S.long_cols, st)) return 1;
     const int k = launch_scan(S.colcnt, S.colstart[b], S.ncols_total, scan_scratch, st);
     k_scatter<<<grid, block, 0, st>>>(S, b);
-    // (the host knows the columns' average alone)
-    const bool runs = S.lkey && S.n / std::max(S.ncols_total, 1) > kLongColumn;
+    const bool runs = S.lkey && S.long_cols;
     if (runs)
-        k_sort_runs<<<dim3(S.ncols_total, std::max(1, std::min(64, S.n / S.ncols_total / 256))), 256, 0, st>>>(S, b);
+        k_sort_runs<<<dim3(S.ncols_total, std::max(1, std::min(64, S.n / S.ncols_total / (2 * kRun)))), 256, 0, st>>>(S, b);
     k_canon<<<grid, block, 0, st>>>(S, b, publish ? 1 : 0, runs ? 1 : 0);
     return k + 2 + (runs ? 1 : 0);
 }
@@ -799,7 +810,10 @@ int launch_user_sort(const DevState &S, const int *ucol, const int *uiz, int *co
 {
     const SortJob J{S.n,     S.ncols_total, ucol,    uiz,     nullptr, S.colcnt, colstart, S.lkey, uperm,
                     nullptr, nullptr,       nullptr, nullptr, S.cnt,   nullptr,  0};
-    if (sort_in_cluster(J, st)) return 1;
+    // (what this sort will find out the last load of the size or the average says for now;
+    // above 32 768 slots a long column that neither shows costs more than looking out for it)
+    const bool runs = S.long_cols || S.n > 32768 || S.n / std::max(S.ncols_total, 1) > kLongColumn;
+    if (sort_in_cluster(J, runs, st)) return 1;
     const int k = launch_scan(S.colcnt, colstart, S.ncols_total, scan_scratch, st);
     k_user_scatter<<<grid, block, 0, st>>>(S, ucol, uiz, colstart);
     k_user_canon<<<grid, block, 0, st>>>(S, ucol, uiz, colstart, uperm);

@@ -59,3 +59,28 @@ def test_tile_of_long_columns(gpu_lib, n, m, nz):
     ctx.close()
     for k in OUT:
         assert np.array_equal(R[k], ref[k][idx]), k
+
+
+@pytest.mark.parametrize("n, crowd", [(3000, 161), (3000, 1500), (70_000, 900)])
+def test_one_long_column_among_many(gpu_lib, n, crowd):
+    """A column that the average does not show: found by the load's sort, and gone with
+    the next load; a column that grows long during the steps likewise."""
+    m, nz = 64, 400
+    g, P = tall(n, m, m, nz, n, 1)
+    L = P.copy()
+    rng = np.random.default_rng(n + 1)
+    L["x"][:crowd] = 0.0210 + rng.uniform(-9.0e-4, 9.0e-4, crowd)
+    L["y"][:crowd] = 0.0210 + rng.uniform(-9.0e-4, 9.0e-4, crowd)
+    ctx = Context(PRM, [g])
+    for S in (L, P, L):
+        ctx.set_state(S)
+        for steps in (1, 9):
+            ctx.step(0.25, steps, BMXG_FP64)
+        Q, R = S.copy(), S.copy()
+        ctx.get_state(Q)
+        O.evolve(PRM, [g], [0, n], R, 0.25, 10)
+        for k in ("x", "y", "z", "velx", "vely", "velz"):
+            assert np.array_equal(Q[k], R[k]), k
+        if n <= 20_000:
+            assert same_pairs(ctx.pairs(), O.pairs(PRM, g, Q))
+    ctx.close()
