@@ -84,3 +84,20 @@ def test_one_long_column_among_many(gpu_lib, n, crowd):
         if n <= 20_000:
             assert same_pairs(ctx.pairs(), O.pairs(PRM, g, Q))
     ctx.close()
+
+
+@pytest.mark.parametrize("n, mx, my", [(700, 256, 256), (700, 257, 256), (40_000, 256, 256), (40_000, 255, 258)])
+def test_column_counts_around_the_cluster_sorts(gpu_lib, n, mx, my):
+    """65 536 columns and a few more."""
+    g, P = tall(n, mx, my, 32, n + mx, 1)
+    ctx = Context(PRM, [g])
+    ctx.set_state(P)
+    if n <= 20_000:
+        assert same_pairs(ctx.pairs(), O.pairs(PRM, g, P))
+    ctx.step(0.25, 3, BMXG_FP64)
+    Q, R = P.copy(), P.copy()
+    ctx.get_state(Q)
+    ctx.close()
+    O.evolve(PRM, [g], [0, n], R, 0.25, 3)
+    for k in ("x", "y", "z", "velx", "vely", "velz"):
+        assert np.array_equal(Q[k], R[k]), k
