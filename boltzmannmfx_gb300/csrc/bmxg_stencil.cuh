@@ -164,7 +164,7 @@ __device__ __forceinline__ void col_to_bxy(const DevGeom &G, int col, int &bx, i
 // adjacent columns.
 constexpr int kWalkCols = 9;
 constexpr int kWalkBlock = 32 * kWalkCols;
-// Candidates staged per slot and column (sphere step, adjoint; up to 65 536 slots): one word
+// Candidates staged per slot and column (sphere step, adjoint): one word
 // each, in the room of six of two words.  A slot with more in some column is walked again by
 // one lane while the block waits.  Adjoint of 20 000 / 50 000 spheres over 20 steps, ms: at 10
 // a column 2.3 / 4.0 (6.3 / 6.3 with six), 2.7 / 4.8 at 15 (8.8 / 11.6; one thread per slot with

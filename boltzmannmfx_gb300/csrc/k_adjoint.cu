@@ -622,6 +622,7 @@ void allow_smem(K kernel, size_t need)
 // slots a column: 20 000 slots 3347, 5257 / 1758, 2352, 65 000 3888, 6208 / 3590, 4844, 100 000 5924,
 // 9445 / 5314, 7299, 130 000 6133, 9931 / 6242, 8668, 200 000 7928, 13 295 / 8671, 12 101.
 constexpr int kAdjointColumns = 114688;
+static_assert(kAdjointColumns < (1 << 28), "a staged slot in 28 bits");
 
 int launch_dfwd(const DevState &S, const DevParams &P, const DiffParams &D, double dt, int a, int grid, int block,
                 cudaStream_t st, bool pinned)

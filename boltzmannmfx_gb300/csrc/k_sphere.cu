@@ -417,6 +417,7 @@ static void allow_smem_once(K kernel, size_t bytes, std::atomic<unsigned long lo
 // 2303 / 1402, 1654, 48 000 1776, 2485 / 1651, 2007, 56 000 1866, 2694 / 1904, 2317, 80 000
 // 1954, 2884 / 2400, 3018.
 constexpr int kColumnSlots64 = 49152;
+static_assert(kColumnSlots64 < (1 << 28), "a staged slot in 28 bits");
 
 int launch_sphere_step(const DevState &S, const DevParams &P, double dt, int a, int precision, int grid,
                        int block, cudaStream_t st, int resync, bool pinned)
